@@ -105,12 +105,13 @@ __global__ void __launch_bounds__(256) cleansc_steer_kernel(CscArgs a, double2 *
         r0 = a.ref_mode == 1 ? a.ref_dist : dist3(gx, gy, gz, a.ref0, a.ref1, a.ref2);
     }
     double2 *o = out + ((int64_t)b * a.G + g) * M;
+    const SincosTable sct = sincos_table(a.table, a.mask, a.faithful != 0);
     double S = 0.0;
     for (int m = lane; m < M; m += 32) {
         const double r = a.rm ? a.rm[g * M + m] : dist3(gx, gy, gz, a.mpos[m], a.mpos[M + m], a.mpos[2 * M + m]);
         const float arg = __double2float_rn(__dmul_rn(k, r));
         float c, sn;
-        sincos_f32_arg(arg, a.table, a.mask, a.faithful != 0, c, sn);
+        sincos_f32_arg(arg, sct, c, sn);
         double2 v = make_double2((double)c, -(double)sn);
         if (a.steer_type == 2) {
             v.x = __dmul_rn(v.x, r);
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(kCscThreads) cleansc_step_kernel(CscArgs a, in
     } else {
     // 2. steering vector of the peak: transfer x_m = (cos p - i sin p) r0 / rm, p = fl32(k (rm - r0))
     const double k = a.k[b];
+    const SincosTable sct = sincos_table(a.table, a.mask, a.faithful != 0);
     double gx = 0, gy = 0, gz = 0, r0x;
     if (a.rm) {
         r0x = a.r0[xi];
@@ -238,7 +240,7 @@ __global__ void __launch_bounds__(kCscThreads) cleansc_step_kernel(CscArgs a, in
         const double rmm = a.rm ? a.rm[xi * M + m] : dist3(gx, gy, gz, a.mpos[m], a.mpos[M + m], a.mpos[2 * M + m]);
         const float arg = __double2float_rn(__dmul_rn(k, __dsub_rn(rmm, r0x)));
         float c, s;
-        sincos_f32_arg(arg, a.table, a.mask, a.faithful != 0, c, s);
+        sincos_f32_arg(arg, sct, c, s);
         const double xr = __ddiv_rn(__dmul_rn((double)c, r0x), rmm);
         const double xim = __ddiv_rn(__dmul_rn(-(double)s, r0x), rmm);
         w[m] = make_double2(xr, xim);

@@ -38,18 +38,53 @@ __device__ __forceinline__ double dist3(double g0, double g1, double g2, double 
     return __dsqrt_rn(__fma_rn(d2, d2, __fma_rn(d1, d1, __dmul_rn(d0, d0))));
 }
 
-// Look up float32 argument `x` in the sincos exception table (open addressing, linear probing).
-// Entry layout: bits 63..32 = float bits of x, bits 15..8 = int8 ulp delta of cos, bits 7..0 =
-// int8 ulp delta of sin; an all-ones word marks an empty slot.
-__device__ __forceinline__ void sincos_exception(const uint64_t *__restrict__ table, uint64_t mask, float x,
-                                                 int &dcos, int &dsin)
+// Exception table of the host C library's float32 cosf/sinf (built by acb_sincos_table_build_host): open
+// addressing, linear probing.  Entry layout: bits 63..32 = float bits of x, bits 31..16 = tags of the slot (below),
+// bits 15..8 = int8 ulp delta of cos, bits 7..0 = int8 ulp delta of sin; an all-ones word marks an empty slot.
+// Two things keep the lookups (random 32-byte sectors of a 64 MB table) few and short:
+//   tol   An exception can only occur where the FP64 value lies within tol units (of 2^-29 float32 ulp) of the
+//         midpoint of two float32 values: the table holds, under kSincosMetaKey, the largest distance of any of its
+//         entries (0.0607 ulp for glibc 2.39), so three arguments in four are never looked up.  tol < 0: no table.
+//   tags  Bit 16 + tag of a slot's word is set for every key with this home slot (whoever occupies it), tag = 4
+//         other bits of the key's hash: unless the bit is set, one load answers the lookup, with no walk.
+// A table without the meta entry has no tags: tol is then half an ulp and every occupied home slot is walked.
+// Bound: issue slots (about 100 instructions per value); with a lookup and its walk for every value and the library's
+// sincos it was 194 instructions.  Measured (B200): map of one eigen-component, 16 bins x 160,801 points x 256 mics,
+// 7.9 -> 5.1 ms; point-spread function 1681 x 1681 x 64 mics 1.72 -> 1.03 ms.
+struct SincosTable {
+    const uint64_t *table;
+    uint64_t mask;
+    int tol;
+    uint32_t untagged;   // all tag bits if the table has none
+};
+
+constexpr uint32_t kSincosMetaKey = 0xfffffffeu;   // sign bit set: never the magnitude of an argument
+__host__ __device__ constexpr uint64_t sincos_hash(uint32_t key)
+{
+    return static_cast<uint64_t>(key) * 0x9E3779B97F4A7C15ull;   // home slot: bits 20 and up; tag: bits 60..63
+}
+
+__device__ __forceinline__ SincosTable sincos_table(const uint64_t *table, uint64_t mask, bool faithful)
+{
+    SincosTable t{table, mask, -1, 0u};
+    if (faithful) {
+        const uint64_t e = __ldg(table + ((sincos_hash(kSincosMetaKey) >> 20) & mask));
+        const bool meta = static_cast<uint32_t>(e >> 32) == kSincosMetaKey;
+        t.tol = meta ? static_cast<int>((static_cast<uint32_t>(e) & 0xffffu) << 13) : 0x10000000;
+        t.untagged = meta ? 0u : 0xffff0000u;
+    }
+    return t;
+}
+
+// Walk the table for float32 argument magnitude `x`.
+__device__ __forceinline__ void sincos_exception(const SincosTable &t, float x, int &dcos, int &dsin)
 {
     const uint32_t key = __float_as_uint(x);
-    uint64_t slot = (static_cast<uint64_t>(key) * 0x9E3779B97F4A7C15ull) >> 20;
+    uint64_t slot = sincos_hash(key) >> 20;
     dcos = 0;
     dsin = 0;
     for (int probe = 0; probe < 64; ++probe) {  // bounded: the table is built at < 50 % load
-        const uint64_t e = __ldg(table + (slot & mask));
+        const uint64_t e = __ldg(t.table + (slot & t.mask));
         if (e == ~0ull) return;
         if (static_cast<uint32_t>(e >> 32) == key) {
             dcos = static_cast<int8_t>((e >> 8) & 0xff);
@@ -60,23 +95,83 @@ __device__ __forceinline__ void sincos_exception(const uint64_t *__restrict__ ta
     }
 }
 
+static __device__ const double2 kSincosPoints[64] = {
+#include "sincos_points.inc"
+};
+
+// The general FP64 sincos, out of line: only arguments beyond the table-driven range come here.
+static __device__ __noinline__ void sincos_any(double x, double *s, double *c) { sincos(x, s, c); }
+
+// FP64 cos/sin of a float32 argument, table driven (the scheme of P. T. P. Tang, Table-lookup algorithms for
+// elementary functions, 1991): x = n pi/32 + r with |r| <= pi/64, pi/32 split in a part of 38 bits (n times it is
+// exact for n < 2^15) and its remainder; cos/sin of n pi/32 from the table, those of r from their Taylor series
+// (next terms 2e-20 and 4e-18), combined as C + (C (cos r - 1) - S sin r).  About one FP64 ulp; results near zero
+// (C = 0 exactly) keep the relative accuracy of r.  17 FP64 operations, no branch but the range check.
+__device__ __forceinline__ void sincos_reduced(float x, double &c, double &s)
+{
+    const double xd = static_cast<double>(x);
+    if (!(fabsf(x) < 3000.0f)) {   // NaN and infinities too
+        sincos_any(xd, &s, &c);
+        return;
+    }
+    const double magic = 6755399441055744.0;   // 1.5 2^52: the addition rounds to an integer
+    const double t = fma(xd, 0x1.45f306dc9c883p+3, magic);
+    const double nd = t - magic;
+    const double2 p = __ldg(kSincosPoints + (__double2loint(t) & 63));
+    double r = fma(-nd, 0x1.921fb54440000p-4, xd);
+    r = fma(-nd, 0x1.68c234c4c6629p-43, r);
+    const double r2 = r * r;
+    const double cm = r2 * fma(r2, fma(r2, fma(r2, 1.0 / 40320.0, -1.0 / 720.0), 1.0 / 24.0), -0.5);
+    const double sr = fma(r * r2, fma(r2, fma(r2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), r);
+    c = fma(p.x, cm, fma(-p.y, sr, p.x));
+    s = fma(p.y, cm, fma(p.x, sr, p.y));
+}
+
 // Float32 cos/sin of a float32 argument: correctly rounded value through FP64 evaluation,
 // optionally corrected to the host C library's cosf/sinf by the exception table.  The table holds
 // non-negative arguments; a negative one is looked up by its magnitude (the C library's cosf is even
 // and its sinf odd, bit for bit, and a delta on the bits of a float changes its magnitude).
-__device__ __forceinline__ void sincos_f32_arg(float x, const uint64_t *table, uint64_t mask, bool faithful,
-                                               float &c, float &s)
+// In two halves, so that the loads of several arguments are in flight together: begin evaluates and loads the home
+// slot's word, finish corrects (about one lane in 150 walks the table).
+struct SincosPending {
+    float x, c, s;
+    uint64_t word;   // the home slot's word, all ones where no lookup is needed
+};
+
+__device__ __forceinline__ SincosPending sincos_begin(float x, const SincosTable &t)
 {
+    SincosPending v;
     double sd, cd;
-    sincos(static_cast<double>(x), &sd, &cd);
-    c = __double2float_rn(cd);
-    s = __double2float_rn(sd);
-    if (faithful) {
+    sincos_reduced(x, cd, sd);
+    v.x = x;
+    v.c = __double2float_rn(cd);
+    v.s = __double2float_rn(sd);
+    // distance of the FP64 values from a float32 rounding midpoint, from their 29 low mantissa bits
+    const int mc = abs((__double2loint(cd) & 0x1fffffff) - 0x10000000);
+    const int ms = abs((__double2loint(sd) & 0x1fffffff) - 0x10000000);
+    v.word = ~0ull;
+    if (min(mc, ms) <= t.tol) v.word = __ldg(t.table + ((sincos_hash(__float_as_uint(fabsf(x))) >> 20) & t.mask));
+    return v;
+}
+
+__device__ __forceinline__ void sincos_finish(SincosPending &v, const SincosTable &t)
+{
+    const uint32_t key = __float_as_uint(fabsf(v.x));
+    const uint32_t tag = 16u + static_cast<uint32_t>(sincos_hash(key) >> 60);
+    if (v.word != ~0ull && (((static_cast<uint32_t>(v.word) | t.untagged) >> tag) & 1u)) {
         int dc, ds;
-        sincos_exception(table, mask, fabsf(x), dc, ds);
-        if (dc) c = __int_as_float(__float_as_int(c) + dc);
-        if (ds) s = __int_as_float(__float_as_int(s) + ds);
+        sincos_exception(t, fabsf(v.x), dc, ds);
+        if (dc) v.c = __int_as_float(__float_as_int(v.c) + dc);
+        if (ds) v.s = __int_as_float(__float_as_int(v.s) + ds);
     }
+}
+
+__device__ __forceinline__ void sincos_f32_arg(float x, const SincosTable &t, float &c, float &s)
+{
+    SincosPending v = sincos_begin(x, t);
+    sincos_finish(v, t);
+    c = v.c;
+    s = v.s;
 }
 
 }  // namespace acb

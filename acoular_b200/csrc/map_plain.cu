@@ -50,11 +50,11 @@ __device__ __forceinline__ double grid_mic_dist(const MapArgs &a, const double *
 // Steering value of a grid point and a mic at distance r (acoular/fastFuncs.py:258-273): the phase
 // rounded to float32, cos - i sin of it as the C library's float32 functions give them, then the
 // weight r (inverse) or 1/r (true level, true location).
-__device__ __forceinline__ double2 steer_value(const MapArgs &a, double k, double r)
+__device__ __forceinline__ double2 steer_value(const MapArgs &a, const SincosTable &sct, double k, double r)
 {
     const float arg = __double2float_rn(__dmul_rn(k, r));
     float c, s;
-    sincos_f32_arg(arg, a.table, a.table_mask, a.faithful != 0, c, s);
+    sincos_f32_arg(arg, sct, c, s);
     double2 h = make_double2((double)c, -(double)s);
     if (a.steer_type == 2) {
         h.x = __dmul_rn(h.x, r);
@@ -74,12 +74,13 @@ __device__ __forceinline__ void synth_chunk(const MapArgs &a, const double *__re
                                            int n, double2 *hs, const double2 *__restrict__ hv = nullptr)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const SincosTable sct = sincos_table(a.table, a.table_mask, !CUSTOM && a.faithful != 0);
     for (int i = warp; i < n; i += NW) {
         double2 h = make_double2(0.0, 0.0);
         if (CUSTOM) {
             if (gvalid) h = __ldg(hv + g * a.M + m0 + i);
         } else if (gvalid) {
-            h = steer_value(a, k, grid_mic_dist<USE_RM>(a, rm, g, m0 + i, g0, g1, g2, mp));
+            h = steer_value(a, sct, k, grid_mic_dist<USE_RM>(a, rm, g, m0 + i, g0, g1, g2, mp));
         }
         hs[i * kLanes + lane] = h;
     }
@@ -657,6 +658,7 @@ __global__ void __launch_bounds__(kEigSmallThreads)
 #pragma unroll
     for (int j = 0; j < EMAX; ++j) fr[j] = fi[j] = dg[j] = 0.0;
     double S = 0.0;
+    const SincosTable sct = sincos_table(a.table, a.table_mask, !CUSTOM && a.faithful != 0);
     for (int m = 0; m < M; ++m) {
         double2 h;
         if (CUSTOM) {
@@ -665,7 +667,7 @@ __global__ void __launch_bounds__(kEigSmallThreads)
         } else {
             const double r = USE_RM ? __ldg(rm + g * M + m)
                                     : dist3(g0, g1, g2, __ldg(mpos + m), __ldg(mpos + M + m), __ldg(mpos + 2 * M + m));
-            h = steer_value(a, k, r);
+            h = steer_value(a, sct, k, r);
             if (a.steer_type >= 2) S += (a.steer_type == 2) ? r * r : 1.0 / (r * r);
         }
         const double2 *vrow = V + (int64_t)m * E;

@@ -28,6 +28,7 @@ namespace acb {
 
 constexpr int kPsfLanes = 32;
 constexpr int kPsfWarps = 8;
+constexpr int kPsfMics = 4;     // mics whose phases a lane evaluates together
 
 template <int ST>
 __global__ void __launch_bounds__(256) psf_kernel(int M, int64_t G, int S, const int64_t *__restrict__ src,
@@ -44,6 +45,7 @@ __global__ void __launch_bounds__(256) psf_kernel(int M, int64_t G, int S, const
     s = src_ok ? s : 0;
     const bool valid = g < G && sidx < S;
     const double *rs = rm + s * M;
+    const SincosTable sct = sincos_table(table, mask, faithful != 0);
     double re = 0.0, im = 0.0, help = 0.0;
     double rs_l = 1.0, irs_l = 1.0;
     for (int m0 = 0; m0 < M; m0 += mc) {
@@ -55,32 +57,41 @@ __global__ void __launch_bounds__(256) psf_kernel(int M, int64_t G, int S, const
             rg_s[i] = gg < G ? rm[gg * M + m0 + mm] : 1.0;
         }
         __syncthreads();
-        // every lane runs the loop (the shuffles need the whole warp); invalid lanes write nothing
-        for (int mm = 0; mm < n; ++mm) {
+        // every lane runs the loop (the shuffles need the whole warp); invalid lanes write nothing.  Four mics at
+        // a time, so that their table lookups are in flight together (four divide the 32 of a shuffle block)
+        for (int mm = 0; mm < n; mm += kPsfMics) {
             if ((mm & 31) == 0) {   // lane l holds the source distance of mic mm + l and its reciprocal
                 rs_l = mm + lane < n ? __ldg(rs + m0 + mm + lane) : 1.0;
                 irs_l = 1.0 / rs_l;
             }
-            const double rsm = __shfl_sync(0xffffffffu, rs_l, mm & 31);
-            const double irs = __shfl_sync(0xffffffffu, irs_l, mm & 31);
-            const double rg = rg_s[mm * kPsfLanes + lane];
-            const float arg = __double2float_rn(__dmul_rn(k, __dsub_rn(rg, rsm)));
-            float c, sn;
-            sincos_f32_arg(arg, table, mask, faithful != 0, c, sn);
-            // (cos - i sin) / rs  [* rg (inverse) | / rg (true level, true location)]; the divisions as
-            // products with reciprocals (within an ulp of the quotients)
-            double tr = __dmul_rn((double)c, irs), ti = __dmul_rn(-(double)sn, irs);
-            if (ST == 2) {
-                tr = __dmul_rn(tr, rg);
-                ti = __dmul_rn(ti, rg);
-            } else if (ST >= 3) {
-                const double ig = 1.0 / rg;
-                tr = __dmul_rn(tr, ig);
-                ti = __dmul_rn(ti, ig);
-                help += ig * ig;
+            SincosPending pend[kPsfMics];
+#pragma unroll
+            for (int u = 0; u < kPsfMics; ++u) {
+                const double rsm = __shfl_sync(0xffffffffu, rs_l, (mm + u) & 31);
+                const double rg = rg_s[min(mm + u, n - 1) * kPsfLanes + lane];
+                pend[u] = sincos_begin(__double2float_rn(__dmul_rn(k, __dsub_rn(rg, rsm))), sct);
             }
-            re += tr;
-            im += ti;
+#pragma unroll
+            for (int u = 0; u < kPsfMics; ++u) {
+                const double irs = __shfl_sync(0xffffffffu, irs_l, (mm + u) & 31);
+                if (mm + u >= n) break;   // uniform
+                const double rg = rg_s[(mm + u) * kPsfLanes + lane];
+                sincos_finish(pend[u], sct);
+                // (cos - i sin) / rs  [* rg (inverse) | / rg (true level, true location)]; the divisions as
+                // products with reciprocals (within an ulp of the quotients)
+                double tr = __dmul_rn((double)pend[u].c, irs), ti = __dmul_rn(-(double)pend[u].s, irs);
+                if (ST == 2) {
+                    tr = __dmul_rn(tr, rg);
+                    ti = __dmul_rn(ti, rg);
+                } else if (ST >= 3) {
+                    const double ig = 1.0 / rg;
+                    tr = __dmul_rn(tr, ig);
+                    ti = __dmul_rn(ti, ig);
+                    help += ig * ig;
+                }
+                re += tr;
+                im += ti;
+            }
         }
     }
     if (!valid) return;

@@ -196,7 +196,7 @@ def sincos_table_host() -> np.ndarray:
         if _table_host is not None:
             return _table_host
         libc_ver = os.confstr('CS_GNU_LIBC_VERSION') if hasattr(os, 'confstr') else 'unknown'
-        tag = hashlib.blake2b(f'{libc_ver}|{SINCOS_MAX_ARG}|{SINCOS_SLOTS}|v1'.encode(), digest_size=8).hexdigest()
+        tag = hashlib.blake2b(f'{libc_ver}|{SINCOS_MAX_ARG}|{SINCOS_SLOTS}|v2'.encode(), digest_size=8).hexdigest()
         path = _cache_dir() / f'sincos_exc_{tag}.npy'
         if path.exists():
             try:
