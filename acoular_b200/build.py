@@ -39,7 +39,7 @@ def needs_build() -> bool:
     if not LIB.exists():
         return True
     t = LIB.stat().st_mtime
-    deps = sources() + list(CSRC.glob('*.cuh')) + list(CSRC.glob('*.h')) + list((ROOT / 'include').glob('*.h'))
+    deps = sources() + list(CSRC.glob('*.cuh')) + list(CSRC.glob('*.inc')) + list(CSRC.glob('*.h')) + list((ROOT / 'include').glob('*.h'))
     return any(p.stat().st_mtime > t for p in deps)
 
 

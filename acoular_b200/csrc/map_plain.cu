@@ -1,29 +1,33 @@
 // Stage B, plain FP64 form: h^H C h per (grid point, bin) as in _freqBeamformer_FullCSM
-// (acoular/fastFuncs.py:217-311), batched over bins.
+// (acoular/fastFuncs.py:217-311), batched over bins, and its eigenvalue and custom-steering forms.
 //
-// CTA = 32 grid points (one per lane) x one bin, 8 warps.
+// CTA = 16 grid points x one bin.
 //   1. distances |g - m| in FP64 (same contraction as the reference's dist_mat), phase
 //      fl32(k*r), float32 cos/sin (correctly rounded, optionally corrected to the C library's
-//      cosf/sinf by the exception table), steering h = cos - i sin, scaled by r (inverse) or 1/r
-//      (true level / true location); h lives only in shared memory, chunk by chunk.
-//   2. B = 2 Re sum_{a<b} conj(h_a) C_ab h_b (+ sum_a C_aa |h_a|^2 without diagonal removal):
-//      warps take 8-row blocks of C (snake order for balance), each lane accumulates
-//      y_r = sum_b C_{a_r b} h_b for its grid point with C_ab broadcast from L1/L2 and h_b from
-//      shared memory, then conj(h_a) y.
+//      cosf/sinf by the exception table), steering h = cos - i sin, times r (inverse) or 1/r
+//      (true level / true location); h lives only in shared memory.
+//   2. B = 2 Re sum_{a<b} conj(h_a) C_ab h_b (+ sum_a C_aa |h_a|^2 without diagonal removal) on the FP64
+//      matrix instruction (mma.sync m16n8k8: tcgen05 has no FP64 kind): Y = H C^T for the 16 points, a warp
+//      per group of 16 rows a, then Re(conj(h_a) y_a).
 //   3. cross-warp sum, normalisation of the steering type, optional clipping of negatives.
-// Mic chunks: M <= 256 is one chunk; larger arrays use 128-mic chunks and loop over chunk pairs.
+// Bound: the FP64 pipe (4 M^2 flop per point and bin at 37 TFLOP/s, DFMA and the matrix instruction alike).  The
+// matrix instruction needs no masks, no broadcasts and 1/30 of the instructions of an FMA form, and 16-point tiles
+// leave room for three CTAs per SM at 256 mics.  Measured (B200): 12 bins x 160,801 points x 256 mics 41.0 -> 20.9 ms
+// (14.5 ms of it the matrix instruction alone, 24.4 TFLOP/s of its 4 M^2); 6 bins x 15,903 points x 300 mics
+// 8.1 -> 1.41 ms; 5 bins x 1681 points x 64 mics 45 -> 22 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "common.cuh"
 #include "map_internal.h"
-#include "tc_common.cuh"
 
 namespace acb {
 
-constexpr int kLanes = 32;
-constexpr int kWarps = 8;
-constexpr int kRowBlock = 8;
+constexpr int kPts = 16;       // grid points per CTA (the M of the matrix instruction)
+// double2 slots per mic in the steering tile: 18 instead of 16, so that the 8 lanes of one 128-bit shared-memory
+// phase (2 points x 4 mics) fall on different banks
+constexpr int kPtsPad = 18;
+constexpr int kGroup = 16;     // rows of C (or eigenvectors) per warp and pass: two 8-column accumulators
 
 struct MapArgs {
     int M;
@@ -39,100 +43,208 @@ struct MapArgs {
     uint64_t table_mask;
 };
 
-template <bool USE_RM>
-__device__ __forceinline__ double grid_mic_dist(const MapArgs &a, const double *__restrict__ rm, int64_t g, int m,
-                                                double g0, double g1, double g2, const double *mp)
-{
-    if (USE_RM) return rm[g * a.M + m];
-    return dist3(g0, g1, g2, mp[m], mp[a.M + m], mp[2 * a.M + m]);
-}
 
 // Steering value of a grid point and a mic at distance r (acoular/fastFuncs.py:258-273): the phase
 // rounded to float32, cos - i sin of it as the C library's float32 functions give them, then the
-// weight r (inverse) or 1/r (true level, true location).
-__device__ __forceinline__ double2 steer_value(const MapArgs &a, const SincosTable &sct, double k, double r)
+// weight w: r (inverse) or 1/r (true level, true location; the product is within an ulp of the quotient).
+// In two halves, so that a caller with several values has their table lookups in flight together.
+__device__ __forceinline__ SincosPending steer_begin(const SincosTable &sct, double k, double r)
 {
-    const float arg = __double2float_rn(__dmul_rn(k, r));
-    float c, s;
-    sincos_f32_arg(arg, sct, c, s);
-    double2 h = make_double2((double)c, -(double)s);
-    if (a.steer_type == 2) {
-        h.x = __dmul_rn(h.x, r);
-        h.y = __dmul_rn(h.y, r);
-    } else if (a.steer_type >= 3) {
-        h.x = __ddiv_rn(h.x, r);
-        h.y = __ddiv_rn(h.y, r);
+    return sincos_begin(__double2float_rn(__dmul_rn(k, r)), sct);
+}
+
+__device__ __forceinline__ double2 steer_finish(int steer_type, const SincosTable &sct, SincosPending &v, double w)
+{
+    sincos_finish(v, sct);
+    double2 h = make_double2((double)v.c, -(double)v.s);
+    if (steer_type >= 2) {
+        h.x *= w;
+        h.y *= w;
     }
     return h;
 }
 
-// Synthesise h for mics [m0, m0+n) of this CTA's 32 grid points into hs[m - m0][lane]; with CUSTOM,
-// copy the caller's steering vectors hv[g][m] instead (custom steering, acoular/fastFuncs.py:414-559).
-template <bool USE_RM, bool CUSTOM = false, int NW = kWarps>
-__device__ __forceinline__ void synth_chunk(const MapArgs &a, const double *__restrict__ rm, double k, int64_t g,
-                                           bool gvalid, double g0, double g1, double g2, const double *mp, int m0,
-                                           int n, double2 *hs, const double2 *__restrict__ hv = nullptr)
+__device__ __forceinline__ double steer_weight(int steer_type, double r)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const SincosTable sct = sincos_table(a.table, a.table_mask, !CUSTOM && a.faithful != 0);
-    for (int i = warp; i < n; i += NW) {
-        double2 h = make_double2(0.0, 0.0);
-        if (CUSTOM) {
-            if (gvalid) h = __ldg(hv + g * a.M + m0 + i);
-        } else if (gvalid) {
-            h = steer_value(a, sct, k, grid_mic_dist<USE_RM>(a, rm, g, m0 + i, g0, g1, g2, mp));
+    return steer_type == 2 ? r : steer_type >= 3 ? 1.0 / r : 1.0;
+}
+
+// D (16 x 8) += A (16 x 8) B (8 x 8), FP64.  Lane (g = lane / 4, t = lane % 4) holds A rows g, g + 8 at columns
+// t, t + 4 (a0: g,t  a1: g+8,t  a2: g,t+4  a3: g+8,t+4), B rows t, t + 4 of column g, and D rows g, g + 8 at
+// columns 2t, 2t + 1.  The products of one element are added as a chain of FMAs.
+__device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, double a2, double a3, double b0,
+                                        double b1)
+{
+    asm(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64.rn {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+        : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
+}
+
+// Distance of a grid point and a mic, and the steering weight: r (inverse) or 1/r (true level, true location; within
+// an ulp).  r is the correctly rounded square root that dist3 gives, formed from one reciprocal square root y, which
+// the weight needs anyway (P. Markstein's correction: s = d y, r = s + (d - s^2) y / 2).
+__device__ __forceinline__ double dist3_weight(int steer_type, double g0, double g1, double g2, double m0, double m1,
+                                               double m2, double &w)
+{
+    const double d0 = __dsub_rn(g0, m0), d1 = __dsub_rn(g1, m1), d2 = __dsub_rn(g2, m2);
+    const double d = __fma_rn(d2, d2, __fma_rn(d1, d1, __dmul_rn(d0, d0)));
+    const double y = rsqrt(d);
+    const double s = d * y;
+    double r = fma(fma(-s, s, d), 0.5 * y, s);
+    if (!(d > 0.0)) r = d;   // a grid point on a microphone: r = 0, w = infinity; NaN stays NaN
+    w = steer_type == 2 ? r : y;
+    return r;
+}
+
+// Steering values of mics [m0, m0 + n) for this CTA's 16 grid points into hs[(m - m0) * kPtsPad + point], zeros
+// for points past the grid and rows n .. up to a multiple of 16.  With `sum` the steering type's normalisation
+// terms (inverse: r^2; true level / true location: 1/r^2; custom: |h|^2) are added to S: without given distances
+// a thread owns point tid % 16 (S[0]), else a warp owns points warp + NW i (S[i], partial per lane; the given
+// values are contiguous along the mics).
+template <bool USE_RM, bool CUSTOM, int NW>
+__device__ __forceinline__ void synth_tile(const MapArgs &a, const SincosTable &sct, const double *__restrict__ rm,
+                                           double k, int64_t gb, double g0, double g1, double g2,
+                                           const double *__restrict__ mpos, const double2 *__restrict__ hv, int m0,
+                                           int n, double2 *hs, bool sum, double (&S)[kPts / NW])
+{
+    const int np = (n + 15) & ~15;
+    if (USE_RM || CUSTOM) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+        for (int i = 0; i < kPts / NW; ++i) {
+            const int p = warp + NW * i;
+            const int64_t g = gb + p;
+            for (int m = lane; m < np; m += 32) {
+                double2 h = make_double2(0.0, 0.0);
+                if (m < n && g < a.G) {
+                    if (CUSTOM) {
+                        h = __ldg(hv + g * a.M + m0 + m);
+                        if (sum) S[i] += h.x * h.x + h.y * h.y;
+                    } else {
+                        const double r = __ldg(rm + g * a.M + m0 + m);
+                        const double w = steer_weight(a.steer_type, r);
+                        SincosPending v = steer_begin(sct, k, r);
+                        h = steer_finish(a.steer_type, sct, v, w);
+                        if (sum) S[i] += w * w;
+                    }
+                }
+                hs[m * kPtsPad + p] = h;
+            }
         }
-        hs[i * kLanes + lane] = h;
+    } else {
+        // kSynth mics at a time per thread; mics past the chunk repeat its last one and are stored as zeros
+        constexpr int kStep = 32 * NW / kPts, kSynth = 4;
+        const int p = threadIdx.x & (kPts - 1);
+        const bool ok = gb + p < a.G;
+        for (int mb = threadIdx.x / kPts; mb < np; mb += kSynth * kStep) {
+            double w[kSynth];
+            SincosPending v[kSynth];
+#pragma unroll
+            for (int u = 0; u < kSynth; ++u) {
+                const int m = m0 + min(mb + u * kStep, n - 1);
+                const double r = dist3_weight(a.steer_type, g0, g1, g2, __ldg(mpos + m), __ldg(mpos + a.M + m),
+                                              __ldg(mpos + 2 * a.M + m), w[u]);
+                v[u] = steer_begin(sct, k, r);
+            }
+#pragma unroll
+            for (int u = 0; u < kSynth; ++u) {
+                const int m = mb + u * kStep;
+                double2 h = steer_finish(a.steer_type, sct, v[u], w[u]);
+                if (!ok || m >= n) h = make_double2(0.0, 0.0);
+                else if (sum) S[0] += w[u] * w[u];
+                if (m < np) hs[m * kPtsPad + p] = h;
+            }
+        }
     }
 }
 
-// Quadratic-form contribution of rows [ra0, ra0+na) x cols [cb0, cb0+nb) of C for this lane.
-// If `diag_block` the block pair is the same chunk: only b > a counts (plus the diagonal when
-// requested).  Returns (off-diagonal sum, diagonal sum).
-__device__ __forceinline__ void quad_block(const double2 *__restrict__ C, int M, const double2 *ha, int ra0, int na,
-                                           const double2 *hb, int cb0, int nb, bool diag_block, bool with_diag,
-                                           double &off, double &dsum)
+// Quadratic-form contribution of rows [ra0, ra0 + na) x columns [cb0, cb0 + nb) of C: returns this lane's parts of
+// sum Re(conj(h_a) C_ab h_b) for points g = lane / 4 and g + 8.  `diag`: the two ranges are the same mics, only
+// b > a counts, and half the (real) diagonal with `with_diag`.  Rows of C are read from global memory (L2) straight
+// into the B operand, two steps of 4 columns ahead: a lane's element C[a][b] serves the real and the imaginary
+// product, and every element is read once per CTA.  Rows and columns past the range repeat the last one: their
+// steering values are zeros.
+template <int NW, int Q>
+__device__ __forceinline__ void quad_tile(const double2 *__restrict__ C, int M, const double2 *ha, int ra0, int na,
+                                          const double2 *hb, int cb0, int nb, bool diag, bool with_diag, double &off0,
+                                          double &off1)
 {
+    constexpr int kRows = 8 * Q;   // rows per group
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nrb = (na + kRowBlock - 1) / kRowBlock;
-    for (int j = 0; j < nrb; ++j) {
-        // snake assignment of row blocks to warps: 0..7, 7..0, 0..7, ...
-        const int owner = ((j / kWarps) & 1) ? (kWarps - 1 - (j % kWarps)) : (j % kWarps);
-        if (owner != warp) continue;
-        const int a0 = j * kRowBlock;  // local row index in chunk A
-        double yr[kRowBlock], yi[kRowBlock];
-        const double2 *crow[kRowBlock];
+    const int g = lane >> 2, t = lane & 3;
+    const int ngrp = (na + kRows - 1) / kRows;
+    const double dscale = with_diag ? 0.5 : 0.0;
+    for (int j = 0; j < ngrp; ++j) {
+        // snake order over the warps (the groups' lengths fall with j), started at another warp in each CTA
+        const int pos = j % NW;
+        if ((((j / NW) & 1 ? NW - 1 - pos : pos) + (int)blockIdx.x) % NW != warp) continue;
+        const int a0 = j * kRows;
+        const double2 *cp[Q];   // this lane's rows
 #pragma unroll
-        for (int r = 0; r < kRowBlock; ++r) {
-            yr[r] = 0.0;
-            yi[r] = 0.0;
-            const int ar = min(a0 + r, na - 1);
-            crow[r] = C + (int64_t)(ra0 + ar) * M + cb0;
+        for (int q = 0; q < Q; ++q) cp[q] = C + (int64_t)(ra0 + min(a0 + 8 * q + g, na - 1)) * M + cb0;
+        double re[Q][4], im[Q][4];
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) re[q][e] = im[q][e] = 0.0;
+        int b = diag ? a0 : 0;
+        const double2 *hp = hb + (b + t) * kPtsPad + g;
+        const double2 *hend = hb + (((nb + 15) & ~15) - 4 + t) * kPtsPad + g;
+        double2 c0[Q], c1[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            c0[q] = __ldg(cp[q] + min(b + t, nb - 1));
+            c1[q] = __ldg(cp[q] + min(b + 4 + t, nb - 1));
         }
-        const int bstart = diag_block ? a0 + 1 : 0;
-        for (int b = bstart; b < nb; ++b) {
-            const double2 h = hb[b * kLanes + lane];
+        double2 n0 = hp[0], n1 = hp[8];
+        if (diag) {   // the group's own columns: left of the diagonal nothing counts
+            const int bend = min(a0 + kRows, nb);
+            for (; b < bend; b += 4) {
+                const double2 h0 = n0, h1 = n1;
+                hp = hp < hend ? hp + 4 * kPtsPad : hp;
+                n0 = hp[0];
+                n1 = hp[8];
 #pragma unroll
-            for (int r = 0; r < kRowBlock; ++r) {
-                const bool use = (a0 + r < na) && (!diag_block || b > a0 + r);
-                double2 c = __ldg(crow[r] + b);
-                if (!use) c = make_double2(0.0, 0.0);
-                yr[r] = fma(c.x, h.x, fma(-c.y, h.y, yr[r]));
-                yi[r] = fma(c.x, h.y, fma(c.y, h.x, yi[r]));
+                for (int q = 0; q < Q; ++q) {
+                    double2 x = c0[q];
+                    c0[q] = c1[q];
+                    c1[q] = __ldg(cp[q] + min(b + 8 + t, nb - 1));
+                    const int d = b + t - a0 - 8 * q - g;   // column less row
+                    if (d <= 0) x = make_double2(d == 0 ? dscale * x.x : 0.0, 0.0);
+                    if (b >= a0 + 8 * q) {
+                        mma_f64(re[q], h0.x, h1.x, h0.y, h1.y, x.x, -x.y);
+                        mma_f64(im[q], h0.x, h1.x, h0.y, h1.y, x.y, x.x);
+                    }
+                }
+            }
+        }
+#pragma unroll 2
+        for (; b < nb; b += 4) {
+            const double2 h0 = n0, h1 = n1;
+            hp = hp < hend ? hp + 4 * kPtsPad : hp;
+            n0 = hp[0];
+            n1 = hp[8];
+            const int o = min(b + 8 + t, nb - 1);
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const double2 x = c0[q];
+                c0[q] = c1[q];
+                c1[q] = __ldg(cp[q] + o);
+                mma_f64(re[q], h0.x, h1.x, h0.y, h1.y, x.x, -x.y);
+                mma_f64(im[q], h0.x, h1.x, h0.y, h1.y, x.y, x.x);
             }
         }
 #pragma unroll
-        for (int r = 0; r < kRowBlock; ++r) {
-            if (a0 + r < na) {
-                const double2 h = ha[(a0 + r) * kLanes + lane];
-                off = fma(h.x, yr[r], fma(h.y, yi[r], off));  // Re(conj(h) y)
-                if (with_diag) {
-                    const double2 c = __ldg(C + (int64_t)(ra0 + a0 + r) * M + (ra0 + a0 + r));
-                    // (C_aa * conj(h)) * h, real part
-                    const double pr = c.x * h.x + c.y * h.y;
-                    const double pi = -c.x * h.y + c.y * h.x;
-                    dsum += pr * h.x - pi * h.y;
-                }
+        for (int q = 0; q < Q; ++q) {
+            if (Q > 2 && a0 + 8 * q >= na) break;   // no such rows (their steering tile ends at a multiple of 16)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const double2 *r = ha + (a0 + 8 * q + 2 * t + e) * kPtsPad + g;
+                double2 h = r[0];
+                off0 = fma(h.x, re[q][e], fma(h.y, im[q][e], off0));
+                h = r[8];
+                off1 = fma(h.x, re[q][2 + e], fma(h.y, im[q][2 + e], off1));
             }
         }
     }
@@ -169,532 +281,345 @@ __device__ __forceinline__ void finish_plain(const MapArgs &a, double scalar, do
     if (out_norm) out_norm[(int64_t)bin * a.G + g] = ns;
 }
 
-template <bool USE_RM, bool CUSTOM = false>
-__global__ void __launch_bounds__(256) map_plain_kernel(MapArgs a, const double2 *__restrict__ csm,
-                                                        const double *__restrict__ wavenumber, double k_scalar,
-                                                        const double *__restrict__ mpos,
-                                                        const double *__restrict__ gpos,
-                                                        const double *__restrict__ r0_in,
-                                                        const double *__restrict__ rm, int mc,
-                                                        double *__restrict__ out_map,
-                                                        double *__restrict__ out_norm,
-                                                        const double2 *__restrict__ steer = nullptr)
+// Cross-warp sums of a point's quadratic form and steering normalisation, in a fixed order.
+template <int NW>
+struct TileSums {
+    double off[NW][kPts];
+    double s[2 * NW][kPts];
+};
+
+template <bool USE_RM, bool CUSTOM, int NW>
+__device__ __forceinline__ void put_sums(TileSums<NW> &red, double off0, double off1, double (&S)[kPts / NW])
 {
-    extern __shared__ double smem[];
-    const int M = a.M;
-    double *mp = smem;                                          // [3][M]
-    double2 *ha = reinterpret_cast<double2 *>(smem + ((3 * M + 1) & ~1));  // [mc][32]
-    double2 *hb = ha + (size_t)mc * kLanes;                      // [mc][32] (only if M > mc)
-    __shared__ double red_off[kWarps][kLanes], red_diag[kWarps][kLanes], red_s[kWarps][kLanes];
-
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int bin = blockIdx.y;
-    const int64_t g = (int64_t)blockIdx.x * kLanes + lane;
-    const bool gvalid = g < a.G;
-    const double k = wavenumber ? wavenumber[bin] : k_scalar;
-    const double2 *C = csm + (int64_t)bin * M * M;
-    const double2 *hv = CUSTOM ? steer + (int64_t)bin * a.G * M : nullptr;
-
-    if (!USE_RM && !CUSTOM)
-        for (int i = threadIdx.x; i < 3 * M; i += blockDim.x) mp[i] = mpos[i];
-    double g0 = 0, g1 = 0, g2 = 0;
-    if (gvalid && !USE_RM && !CUSTOM) {
-        g0 = gpos[g];
-        g1 = gpos[a.G + g];
-        g2 = gpos[2 * a.G + g];
-    }
-    __syncthreads();
-
-    // steering normalisation sum S (inverse: sum r^2; true level / location: sum 1/r^2; custom: sum |h|^2)
-    double s_part = 0.0;
-    if (CUSTOM) {
-        if (gvalid)
-            for (int m = warp; m < M; m += kWarps) {
-                const double2 h = __ldg(hv + g * M + m);
-                s_part += h.x * h.x + h.y * h.y;
-            }
-    } else if (gvalid && a.steer_type >= 2) {
-        for (int m = warp; m < M; m += kWarps) {
-            const double r = grid_mic_dist<USE_RM>(a, rm, g, m, g0, g1, g2, mp);
-            s_part += (a.steer_type == 2) ? r * r : 1.0 / (r * r);
-        }
-    }
-
-    double off = 0.0, dsum = 0.0;
-    const int nchunks = (M + mc - 1) / mc;
-    for (int ca = 0; ca < nchunks; ++ca) {
-        const int ma0 = ca * mc, na = min(mc, M - ma0);
-        synth_chunk<USE_RM, CUSTOM>(a, rm, k, g, gvalid, g0, g1, g2, mp, ma0, na, ha, hv);
-        __syncthreads();
-        quad_block(C, M, ha, ma0, na, ha, ma0, na, true, a.r_diag == 0, off, dsum);
-        for (int cb = ca + 1; cb < nchunks; ++cb) {
-            const int mb0 = cb * mc, nb = min(mc, M - mb0);
-            __syncthreads();
-            synth_chunk<USE_RM, CUSTOM>(a, rm, k, g, gvalid, g0, g1, g2, mp, mb0, nb, hb, hv);
-            __syncthreads();
-            quad_block(C, M, ha, ma0, na, hb, mb0, nb, false, false, off, dsum);
-        }
-        __syncthreads();
-    }
-
-    red_off[warp][lane] = off;
-    red_diag[warp][lane] = dsum;
-    red_s[warp][lane] = s_part;
-    __syncthreads();
-    if (warp == 0 && gvalid) {
-        double o = 0.0, d = 0.0, S = 0.0;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            o += red_off[w][lane];
-            d += red_diag[w][lane];
-            S += red_s[w][lane];
+    for (int o = 1; o <= 2; o <<= 1) {
+        off0 += __shfl_xor_sync(0xffffffffu, off0, o);
+        off1 += __shfl_xor_sync(0xffffffffu, off1, o);
+    }
+    if ((lane & 3) == 0) {
+        red.off[warp][lane >> 2] = off0;
+        red.off[warp][(lane >> 2) + 8] = off1;
+    }
+    if (USE_RM || CUSTOM) {
+#pragma unroll
+        for (int i = 0; i < kPts / NW; ++i) {
+            double v = S[i];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) red.s[0][warp + NW * i] = v;
         }
-        const double scalar = 2.0 * o + d;
-        double r0 = 0.0;
-        if (CUSTOM) r0 = 0.0;
-        else if (a.ref_mode == 1) r0 = a.ref_dist;
-        else if (USE_RM) r0 = r0_in[g];
-        else r0 = dist3(g0, g1, g2, a.ref0, a.ref1, a.ref2);
-        finish_plain(a, scalar, S, r0, bin, g, out_map, out_norm);
+    } else {
+        red.s[threadIdx.x / kPts][threadIdx.x & (kPts - 1)] = S[0];
     }
 }
 
-// ------------------------------------------------------------------------------------------------
-// Staged variant for M <= 256 (one mic chunk): the same steering synthesis and quadratic form, but the
-// CSM rows come through shared memory.  Each warp streams the rows of its 8-row blocks in column
-// chunks of kCB through a two-stage ring that lane 0 fills with bulk copies (cp.async.bulk into this
-// CTA alone; one copy per row, completion on the stage's mbarrier); the next chunk is in flight while
-// the warp works on the current one.  Every loaded C value then feeds the 32 grid points of the warp
-// from shared memory instead of a broadcast load through L1/L2 per complex FMA, and the masking of the
-// triangle is confined to the diagonal 8 x 8 block.  Sixteen warps (four per scheduler, 128 registers
-// each) share the CTA's steering block: the FP64 FMA chains of the 8-row blocks need that many warps
-// to cover their latency at one CTA per SM (8 warps: 19.7 TFLOP/s on the 256-mic workload, 16: 24.7).
-// Waits are bounded; a CTA that gives up raises the error word, writes NaN and returns after its own
-// copies have landed.
-// ------------------------------------------------------------------------------------------------
-constexpr int kSWarps = 16;                              // warps of the staged kernel (4 per scheduler)
-constexpr int kCB = 16;                                  // C columns per staged chunk
-constexpr int kCStageElems = kRowBlock * kCB;            // double2 per (warp, stage)
-constexpr uint64_t kPlainWaitNs = 500ull * 1000 * 1000;  // limit of one wait
-
-struct StagedSmem {
-    // byte offsets; M mics
-    __host__ __device__ static constexpr size_t mp(int) { return 0; }
-    __host__ __device__ static constexpr size_t ha(int M) { return (size_t)((3 * M + 1) & ~1) * 8; }
-    __host__ __device__ static constexpr size_t cst(int M) { return ha(M) + (size_t)M * kLanes * 16; }
-    __host__ __device__ static constexpr size_t bars(int M) { return cst(M) + (size_t)kSWarps * 2 * kCStageElems * 16; }
-    __host__ __device__ static constexpr size_t total(int M) { return bars(M) + kSWarps * 2 * 8 + 16; }
-};
-
-// the chunk sequence of one warp: its row blocks in snake order, each block's columns [a0, M) in kCB chunks
-struct ChunkCursor {
-    int j;    // row block (local index into the warp's list: j-th block of this warp)
-    int c0;   // first column of the chunk
-};
-
-__device__ __forceinline__ int warp_block(int warp, int t)
+template <bool USE_RM, bool CUSTOM, int NW>
+__device__ __forceinline__ void get_sums(const TileSums<NW> &red, int p, double &o, double &S)
 {
-    // t-th row block of `warp` in the snake assignment 0..7, 7..0, 0..7, ...
-    return t * kSWarps + ((t & 1) ? (kSWarps - 1 - warp) : warp);
+    o = S = 0.0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) o += red.off[w][p];
+#pragma unroll
+    for (int w = 0; w < (USE_RM || CUSTOM ? 1 : 2 * NW); ++w) S += red.s[w][p];
 }
 
 template <bool USE_RM, bool CUSTOM>
-__global__ void __launch_bounds__(kLanes * kSWarps, 1)
-    map_plain_staged_kernel(MapArgs a, const double2 *__restrict__ csm, const double *__restrict__ wavenumber,
-                            double k_scalar, const double *__restrict__ mpos, const double *__restrict__ gpos,
-                            const double *__restrict__ r0_in, const double *__restrict__ rm,
-                            double *__restrict__ out_map, double *__restrict__ out_norm,
-                            const double2 *__restrict__ steer, int *err)
+__device__ __forceinline__ double ref_distance(const MapArgs &a, const double *r0_in, int64_t g, double g0, double g1,
+                                               double g2)
 {
-    extern __shared__ __align__(16) uint8_t smem_b[];
-    const int M = a.M;
-    double *mp = reinterpret_cast<double *>(smem_b);
-    double2 *ha = reinterpret_cast<double2 *>(smem_b + StagedSmem::ha(M));     // [M][32]
-    double2 *cst = reinterpret_cast<double2 *>(smem_b + StagedSmem::cst(M));   // [warp][stage][8][kCB]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_b + StagedSmem::bars(M));   // [warp][stage]
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + kSWarps * 2);
-    __shared__ double red_off[kSWarps][kLanes], red_diag[kSWarps][kLanes], red_s[kSWarps][kLanes];
+    if (CUSTOM) return 0.0;
+    if (a.ref_mode == 1) return a.ref_dist;
+    if (USE_RM) return r0_in[g];
+    return dist3(g0, g1, g2, a.ref0, a.ref1, a.ref2);
+}
 
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int bin = blockIdx.y;
-    const int64_t g = (int64_t)blockIdx.x * kLanes + lane;
-    const bool gvalid = g < a.G;
+// Full-CSM map.  Mics in chunks of `mc` (one chunk for all of them where their steering fits shared memory: then
+// every steering value is synthesised once; else the chunk pairs a <= b are walked and the steering of chunk b is
+// synthesised again for each).
+template <bool USE_RM, bool CUSTOM, int NW>
+__global__ void __launch_bounds__(32 * NW, NW == 4 ? 4 : 2) map_f64_kernel(MapArgs a, const double2 *__restrict__ csm,
+                                                          const double *__restrict__ wavenumber, double k_scalar,
+                                                          const double *__restrict__ mpos,
+                                                          const double *__restrict__ gpos,
+                                                          const double *__restrict__ r0_in,
+                                                          const double *__restrict__ rm, int mc,
+                                                          double *__restrict__ out_map, double *__restrict__ out_norm,
+                                                          const double2 *__restrict__ steer)
+{
+    extern __shared__ double2 map_sm[];
+    __shared__ TileSums<NW> red;
+    double2 *ha = map_sm;                                          // [mc to 16][kPtsPad]
+    double2 *hb = ha + (size_t)((mc + 15) & ~15) * kPtsPad;         // the same, only if M > mc
+    const int M = a.M, bin = blockIdx.y;
+    const int64_t gb = (int64_t)blockIdx.x * kPts;
+    const int64_t g = gb + (threadIdx.x & (kPts - 1));
     const double k = wavenumber ? wavenumber[bin] : k_scalar;
     const double2 *C = csm + (int64_t)bin * M * M;
     const double2 *hv = CUSTOM ? steer + (int64_t)bin * a.G * M : nullptr;
-
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < kSWarps * 2; ++i) tc::mbar_init(&bars[i], 1);
-        *abort_flag = 0;
-        tc::fence_mbar_init();
-    }
-    if (!USE_RM && !CUSTOM)
-        for (int i = threadIdx.x; i < 3 * M; i += blockDim.x) mp[i] = mpos[i];
+    const SincosTable sct = sincos_table(a.table, a.table_mask, !CUSTOM && a.faithful != 0);
     double g0 = 0, g1 = 0, g2 = 0;
-    if (gvalid && !USE_RM && !CUSTOM) {
+    if (g < a.G && !USE_RM && !CUSTOM) {
         g0 = gpos[g];
         g1 = gpos[a.G + g];
         g2 = gpos[2 * a.G + g];
     }
+    double S[kPts / NW];
+#pragma unroll
+    for (int i = 0; i < kPts / NW; ++i) S[i] = 0.0;
+    double off0 = 0.0, off1 = 0.0;
+    for (int ma0 = 0; ma0 < M; ma0 += mc) {
+        const int na = min(mc, M - ma0);
+        if (ma0) __syncthreads();   // the previous chunk's readers
+        synth_tile<USE_RM, CUSTOM, NW>(a, sct, rm, k, gb, g0, g1, g2, mpos, hv, ma0, na, ha, true, S);
+        __syncthreads();
+        quad_tile<NW, 2>(C, M, ha, ma0, na, ha, ma0, na, true, a.r_diag == 0, off0, off1);
+        for (int mb0 = ma0 + mc; mb0 < M; mb0 += mc) {
+            const int nb = min(mc, M - mb0);
+            __syncthreads();
+            synth_tile<USE_RM, CUSTOM, NW>(a, sct, rm, k, gb, g0, g1, g2, mpos, hv, mb0, nb, hb, false, S);
+            __syncthreads();
+            quad_tile<NW, 2>(C, M, ha, ma0, na, hb, mb0, nb, false, false, off0, off1);
+        }
+    }
+    put_sums<USE_RM, CUSTOM, NW>(red, off0, off1, S);
     __syncthreads();
-
-    // this warp's chunk sequence
-    const int nblk = (M + kRowBlock - 1) / kRowBlock;
-    int nmine = 0;
-    while (warp_block(warp, nmine) < nblk) ++nmine;
-    double2 *wst = cst + (size_t)warp * 2 * kCStageElems;
-    uint64_t *wbar = bars + warp * 2;
-    // lane 0: issue the copies of chunk (t, c0) into stage st
-    auto issue = [&](int t, int c0, int st) {
-        const int a0 = warp_block(warp, t) * kRowBlock;
-        const int na = min(kRowBlock, M - a0), nc = min(kCB, M - c0);
-        tc::mbar_arrive_expect_tx(&wbar[st], (uint32_t)(na * nc * 16));
-        for (int r = 0; r < na; ++r)
-            tc::bulk_g2s(wst + (size_t)st * kCStageElems + r * kCB, C + (int64_t)(a0 + r) * M + c0, (uint32_t)(nc * 16),
-                         &wbar[st]);
-    };
-    auto next = [&](int &t, int &c0) {
-        c0 += kCB;
-        if (c0 >= M) {
-            ++t;
-            if (t < nmine) c0 = warp_block(warp, t) * kRowBlock;
-        }
-    };
-    // the first two chunks go out before the steering synthesis, so their latency hides under it
-    int it_t = 0, it_c = nmine > 0 ? warp_block(warp, 0) * kRowBlock : 0;   // issue cursor
-    int issued = 0;
-    if (lane == 0)
-        for (int q = 0; q < 2 && it_t < nmine; ++q, ++issued) {
-            issue(it_t, it_c, q);
-            next(it_t, it_c);
-        }
-    issued = __shfl_sync(0xffffffffu, issued, 0);
-    it_t = __shfl_sync(0xffffffffu, it_t, 0);
-    it_c = __shfl_sync(0xffffffffu, it_c, 0);
-
-    // steering normalisation sum S (inverse: sum r^2; true level / location: sum 1/r^2; custom: sum |h|^2)
-    double s_part = 0.0;
-    if (CUSTOM) {
-        if (gvalid)
-            for (int m = warp; m < M; m += kSWarps) {
-                const double2 h = __ldg(hv + g * M + m);
-                s_part += h.x * h.x + h.y * h.y;
-            }
-    } else if (gvalid && a.steer_type >= 2) {
-        for (int m = warp; m < M; m += kSWarps) {
-            const double r = grid_mic_dist<USE_RM>(a, rm, g, m, g0, g1, g2, mp);
-            s_part += (a.steer_type == 2) ? r * r : 1.0 / (r * r);
-        }
+    if (threadIdx.x < kPts && g < a.G) {
+        double o, sn;
+        get_sums<USE_RM, CUSTOM, NW>(red, threadIdx.x, o, sn);
+        finish_plain(a, 2.0 * o, sn, ref_distance<USE_RM, CUSTOM>(a, r0_in, g, g0, g1, g2), bin, g, out_map, out_norm);
     }
-    synth_chunk<USE_RM, CUSTOM, kSWarps>(a, rm, k, g, gvalid, g0, g1, g2, mp, 0, M, ha, hv);
-    __syncthreads();
-
-    double off = 0.0, dsum = 0.0;
-    const bool with_diag = a.r_diag == 0;
-    int q = 0;   // chunk counter: stage q & 1, phase (q >> 1) & 1
-    bool ok = true;
-    for (int t = 0; t < nmine && ok; ++t) {
-        const int a0 = warp_block(warp, t) * kRowBlock;
-        const int na = min(kRowBlock, M - a0);
-        double yr[kRowBlock], yi[kRowBlock];
-#pragma unroll
-        for (int r = 0; r < kRowBlock; ++r) yr[r] = yi[r] = 0.0;
-        for (int c0 = a0; c0 < M; c0 += kCB, ++q) {
-            const int st = q & 1;
-            ok = __all_sync(0xffffffffu, tc::mbar_wait(&wbar[st], (uint32_t)((q >> 1) & 1), abort_flag, kPlainWaitNs));
-            if (!ok) break;
-            const double2 *cs = wst + (size_t)st * kCStageElems;
-            const int nc = min(kCB, M - c0);
-            int bb = 0;
-            if (c0 == a0) {
-                // the diagonal 8 x 8 block: row r takes columns b > a0 + r (and its diagonal term)
-#pragma unroll
-                for (int d = 0; d < kRowBlock; ++d) {
-                    if (d >= nc) break;
-                    const double2 h = ha[(c0 + d) * kLanes + lane];
-#pragma unroll
-                    for (int r = 0; r < kRowBlock; ++r) {
-                        if (r >= na) continue;
-                        const double2 c = cs[r * kCB + d];
-                        if (d > r) {
-                            yr[r] = fma(c.x, h.x, fma(-c.y, h.y, yr[r]));
-                            yi[r] = fma(c.x, h.y, fma(c.y, h.x, yi[r]));
-                        } else if (d == r && with_diag) {
-                            // (C_aa * conj(h)) * h, real part
-                            const double pr = c.x * h.x + c.y * h.y;
-                            const double pi = -c.x * h.y + c.y * h.x;
-                            dsum += pr * h.x - pi * h.y;
-                        }
-                    }
-                }
-                bb = kRowBlock;
-            }
-            if (na == kRowBlock) {
-#pragma unroll 4
-                for (; bb < nc; ++bb) {
-                    const double2 h = ha[(c0 + bb) * kLanes + lane];
-#pragma unroll
-                    for (int r = 0; r < kRowBlock; ++r) {
-                        const double2 c = cs[r * kCB + bb];
-                        yr[r] = fma(c.x, h.x, fma(-c.y, h.y, yr[r]));
-                        yi[r] = fma(c.x, h.y, fma(c.y, h.x, yi[r]));
-                    }
-                }
-            } else {
-                for (; bb < nc; ++bb) {
-                    const double2 h = ha[(c0 + bb) * kLanes + lane];
-#pragma unroll
-                    for (int r = 0; r < kRowBlock; ++r) {
-                        if (r >= na) continue;
-                        const double2 c = cs[r * kCB + bb];
-                        yr[r] = fma(c.x, h.x, fma(-c.y, h.y, yr[r]));
-                        yi[r] = fma(c.x, h.y, fma(c.y, h.x, yi[r]));
-                    }
-                }
-            }
-            // the stage is consumed: lane 0 refills it with the chunk two ahead
-            __syncwarp();
-            if (it_t < nmine) {
-                if (lane == 0) {
-                    tc::fence_proxy_async_smem();
-                    issue(it_t, it_c, st);
-                }
-                next(it_t, it_c);
-                ++issued;
-            }
-        }
-        if (!ok) break;
-#pragma unroll
-        for (int r = 0; r < kRowBlock; ++r) {
-            if (r < na) {
-                const double2 h = ha[(a0 + r) * kLanes + lane];
-                off = fma(h.x, yr[r], fma(h.y, yi[r], off));   // Re(conj(h) y)
-            }
-        }
-    }
-    if (!ok && lane == 0) {
-        // let this warp's copies still in flight (chunks q .. issued - 1) land before the CTA exits
-        for (int qq = q; qq < issued; ++qq)
-            tc::mbar_drain(&wbar[qq & 1], (uint32_t)((qq >> 1) & 1), tc::drain_limit_ns(kPlainWaitNs));
-    }
-
-    red_off[warp][lane] = off;
-    red_diag[warp][lane] = dsum;
-    red_s[warp][lane] = s_part;
-    __syncthreads();
-    if (warp == 0 && gvalid) {
-        double o = 0.0, d = 0.0, S = 0.0;
-#pragma unroll
-        for (int w = 0; w < kSWarps; ++w) {
-            o += red_off[w][lane];
-            d += red_diag[w][lane];
-            S += red_s[w][lane];
-        }
-        double r0 = 0.0;
-        if (CUSTOM) r0 = 0.0;
-        else if (a.ref_mode == 1) r0 = a.ref_dist;
-        else if (USE_RM) r0 = r0_in[g];
-        else r0 = dist3(g0, g1, g2, a.ref0, a.ref1, a.ref2);
-        if (*abort_flag) {
-            out_map[(int64_t)bin * a.G + g] = __longlong_as_double(0x7ff8000000000000ll);
-            if (out_norm) out_norm[(int64_t)bin * a.G + g] = __longlong_as_double(0x7ff8000000000000ll);
-        } else {
-            finish_plain(a, 2.0 * o + d, S, r0, bin, g, out_map, out_norm);
-        }
-    }
-    if (threadIdx.x == 0 && *abort_flag && err) atomicOr(err, 1);
 }
 
 // ------------------------------------------------------------------------------------------------
 // Eigenvalue form of _freqBeamformer_EigValues (acoular/fastFuncs.py:313-411): with eigenvalues
 // lambda_e and eigenvectors V[:, e] of the CSM (E of them),
 //     scalar = sum_e lambda_e (|sum_m conj(V[m][e]) h[m]|^2 - [r_diag] sum_m |conj(V[m][e]) h[m]|^2),
-// then the steering-type normalisation of the full-CSM form.  Same steering synthesis (float32
-// phase, libm-faithful cos/sin) as map_plain_kernel; the warps take the eigenvectors in groups of
-// 32 (four per warp, partial sums in registers across mic chunks), each eigenvector's mic sum in
-// the reference's order.  Cost O(G M E) per bin.
+// then the steering-type normalisation of the full-CSM form.  Same steering synthesis as the full-CSM form;
+// the projections T = H conj(V) are a matrix product on the FP64 matrix instruction, a warp per group of 16
+// eigenvectors, squared and weighted in the epilogue (no cancellation: each term is a square times lambda_e).
+// The diagonal's part is sum_m |h_m|^2 w_m with w_m = sum_e lambda_e |V[m][e]|^2.  Cost O(G M E) per bin.
+// Bound: the FP64 pipe (8 M E flop per point and bin).  Measured (B200): 64 bins x 3721 points x 112 mics and
+// components 7.2 -> 1.09 ms (the earlier form read every eigenvector entry as a broadcast for 32 points).
 // ------------------------------------------------------------------------------------------------
-constexpr int kEigPerWarp = 4;
-
-template <bool USE_RM, bool CUSTOM = false>
-__global__ void __launch_bounds__(256) map_eig_kernel(MapArgs a, int E, const double *__restrict__ eigval,
-                                                      const double2 *__restrict__ eigvec,
-                                                      const double *__restrict__ wavenumber, double k_scalar,
-                                                      const double *__restrict__ mpos, const double *__restrict__ gpos,
-                                                      const double *__restrict__ r0_in, const double *__restrict__ rm,
-                                                      int mc, double *__restrict__ out_map,
-                                                      double *__restrict__ out_norm,
-                                                      const double2 *__restrict__ steer = nullptr,
-                                                      const int *__restrict__ active = nullptr)
+template <bool USE_RM, bool CUSTOM, int NW>
+__global__ void __launch_bounds__(32 * NW) map_eig_kernel(MapArgs a, int E, const double *__restrict__ eigval,
+                                                          const double2 *__restrict__ eigvec,
+                                                          const double *__restrict__ wavenumber, double k_scalar,
+                                                          const double *__restrict__ mpos,
+                                                          const double *__restrict__ gpos,
+                                                          const double *__restrict__ r0_in,
+                                                          const double *__restrict__ rm, int mc,
+                                                          double *__restrict__ out_map, double *__restrict__ out_norm,
+                                                          const double2 *__restrict__ steer,
+                                                          const int *__restrict__ active)
 {
-    extern __shared__ double smem[];
-    if (active && !active[blockIdx.y]) return;   // a bin whose iteration has stopped (CLEAN-SC)
-    const int M = a.M;
-    double *mp = smem;                                                     // [3][M]
-    double2 *hs = reinterpret_cast<double2 *>(smem + ((3 * M + 1) & ~1));  // [mc][32]
-    __shared__ double red_sc[kWarps][kLanes], red_s[kWarps][kLanes];
-
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    extern __shared__ double2 map_sm[];
+    __shared__ TileSums<NW> red;
     const int bin = blockIdx.y;
-    const int64_t g = (int64_t)blockIdx.x * kLanes + lane;
-    const bool gvalid = g < a.G;
+    if (active && !active[bin]) return;   // a bin whose iteration has stopped (CLEAN-SC)
+    const int M = a.M;
+    double2 *hs = map_sm;                                                       // [mc to 16][kPtsPad]
+    double *wd = reinterpret_cast<double *>(hs + (size_t)((mc + 15) & ~15) * kPtsPad);   // [mc], with r_diag only
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int gl = lane >> 2, t = lane & 3;
+    const int64_t gb = (int64_t)blockIdx.x * kPts;
+    const int64_t g = gb + (threadIdx.x & (kPts - 1));
     const double k = wavenumber ? wavenumber[bin] : k_scalar;
     const double *lam = eigval + (int64_t)bin * E;
     const double2 *V = eigvec + (int64_t)bin * M * E;
     const double2 *hv = CUSTOM ? steer + (int64_t)bin * a.G * M : nullptr;
-
-    if (!USE_RM && !CUSTOM)
-        for (int i = threadIdx.x; i < 3 * M; i += blockDim.x) mp[i] = mpos[i];
+    const SincosTable sct = sincos_table(a.table, a.table_mask, !CUSTOM && a.faithful != 0);
     double g0 = 0, g1 = 0, g2 = 0;
-    if (gvalid && !USE_RM && !CUSTOM) {
+    if (g < a.G && !USE_RM && !CUSTOM) {
         g0 = gpos[g];
         g1 = gpos[a.G + g];
         g2 = gpos[2 * a.G + g];
     }
-    __syncthreads();
-
-    double s_part = 0.0;
-    if (CUSTOM) {
-        if (gvalid)
-            for (int m = warp; m < M; m += kWarps) {
-                const double2 h = __ldg(hv + g * M + m);
-                s_part += h.x * h.x + h.y * h.y;
+    double S[kPts / NW];
+#pragma unroll
+    for (int i = 0; i < kPts / NW; ++i) S[i] = 0.0;
+    double off0 = 0.0, off1 = 0.0;
+    // passes of NW groups of 16 eigenvectors; the steering stays in shared memory over the passes when it is one chunk
+    for (int e0 = 0; e0 < E; e0 += NW * kGroup) {
+        const int eb = e0 + ((warp + (int)blockIdx.x) % NW) * kGroup;   // this warp's eigenvectors
+        double re0[4] = {0, 0, 0, 0}, im0[4] = {0, 0, 0, 0}, re1[4] = {0, 0, 0, 0}, im1[4] = {0, 0, 0, 0};
+        for (int m0 = 0; m0 < M; m0 += mc) {
+            const int n = min(mc, M - m0);
+            if (e0 == 0 || mc < M) {
+                if (e0 || m0) __syncthreads();   // the previous chunk's readers
+                synth_tile<USE_RM, CUSTOM, NW>(a, sct, rm, k, gb, g0, g1, g2, mpos, hv, m0, n, hs, e0 == 0, S);
+                if (a.r_diag && e0 == 0)
+                    for (int m = warp; m < n; m += NW) {
+                        double w = 0.0;
+                        for (int e = lane; e < E; e += 32) {
+                            const double2 v = __ldg(V + (int64_t)(m0 + m) * E + e);
+                            w += lam[e] * (v.x * v.x + v.y * v.y);
+                        }
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+                        if (lane == 0) wd[m] = w;
+                    }
+                __syncthreads();
+                if (a.r_diag && e0 == 0)
+                    for (int m = warp * 4 + t; m < n; m += NW * 4) {
+                        const double2 h0 = hs[m * kPtsPad + gl], h1 = hs[m * kPtsPad + gl + 8];
+                        off0 -= (h0.x * h0.x + h0.y * h0.y) * wd[m];
+                        off1 -= (h1.x * h1.x + h1.y * h1.y) * wd[m];
+                    }
             }
-    } else if (gvalid && a.steer_type >= 2) {
-        for (int m = warp; m < M; m += kWarps) {
-            const double r = grid_mic_dist<USE_RM>(a, rm, g, m, g0, g1, g2, mp);
-            s_part += (a.steer_type == 2) ? r * r : 1.0 / (r * r);
-        }
-    }
-
-    double scal = 0.0;
-    const int nchunks = (M + mc - 1) / mc;
-    for (int eg = 0; eg < E; eg += kWarps * kEigPerWarp) {
-        double fr[kEigPerWarp], fi[kEigPerWarp], dg[kEigPerWarp];
-#pragma unroll
-        for (int j = 0; j < kEigPerWarp; ++j) fr[j] = fi[j] = dg[j] = 0.0;
-        const int e0 = eg + warp * kEigPerWarp;
-        for (int ca = 0; ca < nchunks; ++ca) {
-            const int m0 = ca * mc, n = min(mc, M - m0);
-            synth_chunk<USE_RM, CUSTOM>(a, rm, k, g, gvalid, g0, g1, g2, mp, m0, n, hs, hv);
-            __syncthreads();
-            for (int mm = 0; mm < n; ++mm) {
-                const double2 h = hs[mm * kLanes + lane];
-                const double2 *vrow = V + (int64_t)(m0 + mm) * E;
-#pragma unroll
-                for (int j = 0; j < kEigPerWarp; ++j) {
-                    if (e0 + j >= E) break;
-                    const double2 v = __ldg(vrow + e0 + j);
-                    // temp1 = conj(V[m][e]) * h[m]
-                    const double tr = v.x * h.x + v.y * h.y, ti = v.x * h.y - v.y * h.x;
-                    fr[j] += tr;
-                    fi[j] += ti;
-                    if (a.r_diag) dg[j] += tr * tr + ti * ti;
+            if (eb < E) {
+                // eigenvectors and mics past the end repeat the last one (their lambda is not read, their
+                // steering is zero)
+                const double2 *vx = V + (int64_t)m0 * E + min(eb + gl, E - 1);
+                const double2 *vy = V + (int64_t)m0 * E + min(eb + 8 + gl, E - 1);
+                auto load = [&](int m, double2 &x, double2 &y) {
+                    const int64_t o = (int64_t)min(m, n - 1) * E;
+                    x = __ldg(vx + o);
+                    y = __ldg(vy + o);
+                };
+                double2 x0, y0, x1, y1;
+                load(t, x0, y0);
+                load(4 + t, x1, y1);
+                for (int m = 0; m < n; m += 4) {
+                    const double2 h0 = hs[(m + t) * kPtsPad + gl], h1 = hs[(m + t) * kPtsPad + gl + 8];
+                    const double2 x = x0, y = y0;
+                    x0 = x1;
+                    y0 = y1;
+                    load(m + 8 + t, x1, y1);
+                    // conj(V) h: re = v.x h.x + v.y h.y, im = v.x h.y - v.y h.x
+                    mma_f64(re0, h0.x, h1.x, h0.y, h1.y, x.x, x.y);
+                    mma_f64(im0, h0.x, h1.x, h0.y, h1.y, -x.y, x.x);
+                    if (eb + 8 < E) {
+                        mma_f64(re1, h0.x, h1.x, h0.y, h1.y, y.x, y.y);
+                        mma_f64(im1, h0.x, h1.x, h0.y, h1.y, -y.y, y.x);
+                    }
                 }
             }
-            __syncthreads();   // hs is rewritten by the next chunk
         }
 #pragma unroll
-        for (int j = 0; j < kEigPerWarp; ++j) {
-            if (e0 + j >= E) break;
-            const double full = fr[j] * fr[j] + fi[j] * fi[j];
-            scal += (a.r_diag ? full - dg[j] : full) * lam[e0 + j];
+        for (int e = 0; e < 2; ++e) {
+            const int q0 = eb + 2 * t + e, q1 = q0 + 8;
+            if (q0 < E) {
+                const double l = lam[q0];
+                off0 = fma(l, re0[e] * re0[e] + im0[e] * im0[e], off0);
+                off1 = fma(l, re0[2 + e] * re0[2 + e] + im0[2 + e] * im0[2 + e], off1);
+            }
+            if (q1 < E) {
+                const double l = lam[q1];
+                off0 = fma(l, re1[e] * re1[e] + im1[e] * im1[e], off0);
+                off1 = fma(l, re1[2 + e] * re1[2 + e] + im1[2 + e] * im1[2 + e], off1);
+            }
         }
     }
-
-    red_sc[warp][lane] = scal;
-    red_s[warp][lane] = s_part;
+    put_sums<USE_RM, CUSTOM, NW>(red, off0, off1, S);
     __syncthreads();
-    if (warp == 0 && gvalid) {
-        double sc = 0.0, S = 0.0;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            sc += red_sc[w][lane];
-            S += red_s[w][lane];
-        }
-        double r0 = 0.0;
-        if (CUSTOM) r0 = 0.0;
-        else if (a.ref_mode == 1) r0 = a.ref_dist;
-        else if (USE_RM) r0 = r0_in[g];
-        else r0 = dist3(g0, g1, g2, a.ref0, a.ref1, a.ref2);
-        finish_plain(a, sc, S, r0, bin, g, out_map, out_norm);
+    if (threadIdx.x < kPts && g < a.G) {
+        double sc, sn;
+        get_sums<USE_RM, CUSTOM, NW>(red, threadIdx.x, sc, sn);
+        finish_plain(a, sc, sn, ref_distance<USE_RM, CUSTOM>(a, r0_in, g, g0, g1, g2), bin, g, out_map, out_norm);
     }
 }
 
 // Eigenvalue form for a few components (E <= kEigSmall, e.g. BeamformerEig's default n = -1 and each
-// CLEAN-SC iteration's single component): one thread per grid point walks the mics in order,
-// synthesises each steering value once and accumulates the E projections and the normalisation sum in
-// registers.  Without shared memory a CTA of 4 warps holds no resources but registers, so many warps
-// per SM hide the latency of the FP64 synthesis and of the exception-table probes; the shared-memory
-// form above (one CTA of 8 warps per SM) serves larger E, where the projections outnumber the
-// registers.  Each component's mic sum runs in the reference's order.
+// CLEAN-SC iteration's single component): one thread per grid point and NB bins walks the mics in order,
+// computes a mic's distance and weight once, synthesises the steering value of each bin and accumulates the
+// projections and the normalisation sum in registers.  Each component's mic sum runs in the reference's order.
+// Bound: issue slots of the steering synthesis.  Measured (B200): 16 bins x 160,801 points x 256 mics 5.1 -> 3.8 ms
+// with four bins per thread and their table lookups in flight together (two bins: 3.8 too; one: 4.5).
 constexpr int kEigSmall = 4;
 constexpr int kEigSmallThreads = 128;
 
-template <bool USE_RM, bool CUSTOM, int EMAX>
+template <bool USE_RM, bool CUSTOM, int EMAX, int NB>
 __global__ void __launch_bounds__(kEigSmallThreads)
-    map_eig_small_kernel(MapArgs a, int E, const double *__restrict__ eigval, const double2 *__restrict__ eigvec,
-                         const double *__restrict__ wavenumber, double k_scalar, const double *__restrict__ mpos,
-                         const double *__restrict__ gpos, const double *__restrict__ r0_in,
-                         const double *__restrict__ rm, double *__restrict__ out_map, double *__restrict__ out_norm,
+    map_eig_small_kernel(MapArgs a, int nbins, int E, const double *__restrict__ eigval,
+                         const double2 *__restrict__ eigvec, const double *__restrict__ wavenumber, double k_scalar,
+                         const double *__restrict__ mpos, const double *__restrict__ gpos,
+                         const double *__restrict__ r0_in, const double *__restrict__ rm,
+                         double *__restrict__ out_map, double *__restrict__ out_norm,
                          const double2 *__restrict__ steer, const int *__restrict__ active)
 {
-    const int bin = blockIdx.y;
-    if (active && !active[bin]) return;   // a bin whose iteration has stopped (CLEAN-SC)
+    const int bin0 = blockIdx.y * NB;
+    if (active && !active[bin0]) return;   // a bin whose iteration has stopped (CLEAN-SC; NB = 1 there)
     const int64_t g = (int64_t)blockIdx.x * kEigSmallThreads + threadIdx.x;
     if (g >= a.G) return;
     const int M = a.M;
-    const double k = wavenumber ? wavenumber[bin] : k_scalar;
-    const double *lam = eigval + (int64_t)bin * E;
-    const double2 *V = eigvec + (int64_t)bin * M * E;
-    const double2 *hv = CUSTOM ? steer + ((int64_t)bin * a.G + g) * M : nullptr;
+    const SincosTable sct = sincos_table(a.table, a.table_mask, !CUSTOM && a.faithful != 0);
+    double k[NB];
+    const double2 *V[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const int bin = min(bin0 + q, nbins - 1);   // the last group repeats its last bin; not written twice
+        k[q] = wavenumber ? wavenumber[bin] : k_scalar;
+        V[q] = eigvec + (int64_t)bin * M * E;
+    }
+    const double2 *hv = CUSTOM ? steer + ((int64_t)bin0 * a.G + g) * M : nullptr;
     double g0 = 0, g1 = 0, g2 = 0;
     if (!USE_RM && !CUSTOM) {
         g0 = gpos[g];
         g1 = gpos[a.G + g];
         g2 = gpos[2 * a.G + g];
     }
-    double fr[EMAX], fi[EMAX], dg[EMAX];
+    double fr[NB][EMAX], fi[NB][EMAX], dg[NB][EMAX];
 #pragma unroll
-    for (int j = 0; j < EMAX; ++j) fr[j] = fi[j] = dg[j] = 0.0;
+    for (int q = 0; q < NB; ++q)
+#pragma unroll
+        for (int j = 0; j < EMAX; ++j) fr[q][j] = fi[q][j] = dg[q][j] = 0.0;
     double S = 0.0;
-    const SincosTable sct = sincos_table(a.table, a.table_mask, !CUSTOM && a.faithful != 0);
     for (int m = 0; m < M; ++m) {
-        double2 h;
-        if (CUSTOM) {
-            h = __ldg(hv + m);
-            S += h.x * h.x + h.y * h.y;
-        } else {
-            const double r = USE_RM ? __ldg(rm + g * M + m)
-                                    : dist3(g0, g1, g2, __ldg(mpos + m), __ldg(mpos + M + m), __ldg(mpos + 2 * M + m));
-            h = steer_value(a, sct, k, r);
-            if (a.steer_type >= 2) S += (a.steer_type == 2) ? r * r : 1.0 / (r * r);
+        double r = 0.0, w = 0.0;
+        if (!CUSTOM) {
+            if (USE_RM) {
+                r = __ldg(rm + g * M + m);
+                w = steer_weight(a.steer_type, r);
+            } else {
+                r = dist3_weight(a.steer_type, g0, g1, g2, __ldg(mpos + m), __ldg(mpos + M + m),
+                                 __ldg(mpos + 2 * M + m), w);
+            }
+            S = fma(w, w, S);
         }
-        const double2 *vrow = V + (int64_t)m * E;
+        SincosPending pend[NB];
+        if (!CUSTOM) {
+#pragma unroll
+            for (int q = 0; q < NB; ++q) pend[q] = steer_begin(sct, k[q], r);
+        }
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            double2 h;
+            if (CUSTOM) {
+                h = __ldg(hv + m);
+                S += fma(h.x, h.x, __dmul_rn(h.y, h.y));
+            } else {
+                h = steer_finish(a.steer_type, sct, pend[q], w);
+            }
+            const double2 *vrow = V[q] + (int64_t)m * E;
+#pragma unroll
+            for (int j = 0; j < EMAX; ++j) {
+                if (j >= E) break;
+                const double2 v = __ldg(vrow + j);
+                // temp1 = conj(V[m][e]) * h[m]; the FMAs are spelled out, so that every instance of this kernel
+                // gives the same bits
+                const double tr = fma(v.x, h.x, __dmul_rn(v.y, h.y)), ti = fma(v.x, h.y, -__dmul_rn(v.y, h.x));
+                fr[q][j] += tr;
+                fi[q][j] += ti;
+                if (a.r_diag) dg[q][j] = fma(tr, tr, fma(ti, ti, dg[q][j]));
+            }
+        }
+    }
+    const double r0 = ref_distance<USE_RM, CUSTOM>(a, r0_in, g, g0, g1, g2);
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        if (bin0 + q >= nbins) break;
+        const double *lam = eigval + (int64_t)(bin0 + q) * E;
+        double scal = 0.0;
 #pragma unroll
         for (int j = 0; j < EMAX; ++j) {
             if (j >= E) break;
-            const double2 v = __ldg(vrow + j);
-            // temp1 = conj(V[m][e]) * h[m]
-            const double tr = v.x * h.x + v.y * h.y, ti = v.x * h.y - v.y * h.x;
-            fr[j] += tr;
-            fi[j] += ti;
-            if (a.r_diag) dg[j] += tr * tr + ti * ti;
+            const double full = fma(fr[q][j], fr[q][j], __dmul_rn(fi[q][j], fi[q][j]));
+            scal = fma(a.r_diag ? full - dg[q][j] : full, lam[j], scal);
         }
+        finish_plain(a, scal, S, r0, bin0 + q, g, out_map, out_norm);
     }
-    double scal = 0.0;
-#pragma unroll
-    for (int j = 0; j < EMAX; ++j) {
-        if (j >= E) break;
-        const double full = fr[j] * fr[j] + fi[j] * fi[j];
-        scal += (a.r_diag ? full - dg[j] : full) * lam[j];
-    }
-    double r0 = 0.0;
-    if (CUSTOM) r0 = 0.0;
-    else if (a.ref_mode == 1) r0 = a.ref_dist;
-    else if (USE_RM) r0 = r0_in[g];
-    else r0 = dist3(g0, g1, g2, a.ref0, a.ref1, a.ref2);
-    finish_plain(a, scal, S, r0, bin, g, out_map, out_norm);
 }
 
 static int make_args(const acb_map_params *p, MapArgs &a)
@@ -723,30 +648,63 @@ static int make_args(const acb_map_params *p, MapArgs &a)
     return ACB_OK;
 }
 
+// Chunk of mics whose steering tile a CTA holds, and the warps per CTA.  All mics in one tile up to 768 (221 KB);
+// above, pairs of 384-mic tiles.  Four warps per CTA up to 256 mics (three CTAs or more per SM, so that one's
+// synthesis runs under another's matrix products), eight where only one or two CTAs fit.
+constexpr int kMapOneTile = 768, kMapPairTile = 384, kMapFourWarps = 256;
+
+template <bool USE_RM, bool CUSTOM, int NW>
+static int launch_map_nw(const MapArgs &a, int nbins, const void *csm, const double *k, double k_scalar,
+                         const double *mpos, const double *gpos, const double *r0, const double *rm, double *out_map,
+                         double *out_norm, cudaStream_t s, const void *steer)
+{
+    const int mc = a.M <= kMapOneTile ? a.M : kMapPairTile;
+    const size_t smem = (size_t)(a.M <= mc ? 1 : 2) * ((mc + 15) & ~15) * kPtsPad * sizeof(double2);
+    auto kern = map_f64_kernel<USE_RM, CUSTOM, NW>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const dim3 grid((unsigned)((a.G + kPts - 1) / kPts), nbins);
+    kern<<<grid, 32 * NW, smem, s>>>(a, reinterpret_cast<const double2 *>(csm), k, k_scalar, mpos, gpos, r0, rm, mc,
+                                     out_map, out_norm, reinterpret_cast<const double2 *>(steer));
+    return check_launch();
+}
+
 template <bool USE_RM, bool CUSTOM = false>
 static int launch_plain(const MapArgs &a, int nbins, const void *csm, const double *k, double k_scalar,
-                        const double *mpos,
-                        const double *gpos, const double *r0, const double *rm, double *out_map, double *out_norm,
-                        cudaStream_t s, const void *steer = nullptr, int *err = nullptr)
+                        const double *mpos, const double *gpos, const double *r0, const double *rm, double *out_map,
+                        double *out_norm, cudaStream_t s, const void *steer = nullptr)
 {
-    if (a.M <= 256) {   // one mic chunk: the staged kernel
-        const size_t smem = StagedSmem::total(a.M);
-        auto kern = map_plain_staged_kernel<USE_RM, CUSTOM>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        const dim3 grid((unsigned)((a.G + kLanes - 1) / kLanes), nbins);
-        kern<<<grid, kLanes * kSWarps, smem, s>>>(a, reinterpret_cast<const double2 *>(csm), k, k_scalar, mpos, gpos,
-                                                 r0, rm, out_map, out_norm, reinterpret_cast<const double2 *>(steer),
-                                                 err);
-        return check_launch();
-    }
-    const int mc = a.M <= 256 ? a.M : 128;
-    const int nbuf = a.M <= mc ? 1 : 2;
-    const size_t smem = (size_t)(((3 * a.M + 1) & ~1) * sizeof(double)) + (size_t)nbuf * mc * kLanes * sizeof(double2);
-    auto kern = map_plain_kernel<USE_RM, CUSTOM>;
+    if (a.M <= kMapFourWarps)
+        return launch_map_nw<USE_RM, CUSTOM, 4>(a, nbins, csm, k, k_scalar, mpos, gpos, r0, rm, out_map, out_norm, s,
+                                                steer);
+    return launch_map_nw<USE_RM, CUSTOM, 8>(a, nbins, csm, k, k_scalar, mpos, gpos, r0, rm, out_map, out_norm, s,
+                                            steer);
+}
+
+template <bool USE_RM, bool CUSTOM, int NW>
+static int launch_eig_nw(const MapArgs &a, int nbins, int E, const double *eigval, const void *eigvec, const double *k,
+                         double k_scalar, const double *mpos, const double *gpos, const double *r0, const double *rm,
+                         double *out_map, double *out_norm, cudaStream_t s, const void *steer, const int *active)
+{
+    const int mc = a.M <= kMapOneTile ? a.M : kMapPairTile;
+    const size_t smem = (size_t)((mc + 15) & ~15) * kPtsPad * sizeof(double2) + (a.r_diag ? mc * sizeof(double) : 0);
+    auto kern = map_eig_kernel<USE_RM, CUSTOM, NW>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const dim3 grid((unsigned)((a.G + kLanes - 1) / kLanes), nbins);
-    kern<<<grid, kLanes * kWarps, smem, s>>>(a, reinterpret_cast<const double2 *>(csm), k, k_scalar, mpos, gpos, r0,
-                                            rm, mc, out_map, out_norm, reinterpret_cast<const double2 *>(steer));
+    const dim3 grid((unsigned)((a.G + kPts - 1) / kPts), nbins);
+    kern<<<grid, 32 * NW, smem, s>>>(a, E, eigval, reinterpret_cast<const double2 *>(eigvec), k, k_scalar, mpos, gpos,
+                                     r0, rm, mc, out_map, out_norm, reinterpret_cast<const double2 *>(steer), active);
+    return check_launch();
+}
+
+template <bool USE_RM, bool CUSTOM, int EMAX, int NB>
+static int launch_eig_small(const MapArgs &a, int nbins, int E, const double *eigval, const void *eigvec,
+                            const double *k, double k_scalar, const double *mpos, const double *gpos, const double *r0,
+                            const double *rm, double *out_map, double *out_norm, cudaStream_t s, const void *steer,
+                            const int *active)
+{
+    const dim3 grid((unsigned)((a.G + kEigSmallThreads - 1) / kEigSmallThreads), (nbins + NB - 1) / NB);
+    map_eig_small_kernel<USE_RM, CUSTOM, EMAX, NB><<<grid, kEigSmallThreads, 0, s>>>(
+        a, nbins, E, eigval, reinterpret_cast<const double2 *>(eigvec), k, k_scalar, mpos, gpos, r0, rm, out_map,
+        out_norm, reinterpret_cast<const double2 *>(steer), active);
     return check_launch();
 }
 
@@ -756,23 +714,17 @@ static int launch_eig(const MapArgs &a, int nbins, int E, const double *eigval, 
                       double *out_map, double *out_norm, cudaStream_t s, const void *steer = nullptr,
                       const int *active = nullptr)
 {
-    if (E <= kEigSmall) {
-        const dim3 grid((unsigned)((a.G + kEigSmallThreads - 1) / kEigSmallThreads), nbins);
-        auto kern = E == 1 ? map_eig_small_kernel<USE_RM, CUSTOM, 1> : map_eig_small_kernel<USE_RM, CUSTOM, kEigSmall>;
-        kern<<<grid, kEigSmallThreads, 0, s>>>(a, E, eigval, reinterpret_cast<const double2 *>(eigvec), k, k_scalar,
-                                               mpos, gpos, r0, rm, out_map, out_norm,
-                                               reinterpret_cast<const double2 *>(steer), active);
-        return check_launch();
+#define ACB_EIG_ARGS a, nbins, E, eigval, eigvec, k, k_scalar, mpos, gpos, r0, rm, out_map, out_norm, s, steer, active
+    if (E == 1) {
+        // four bins per thread share the distances, as long as that leaves every SM eight CTAs (32 warps)
+        if (!CUSTOM && !active && (a.G + kEigSmallThreads - 1) / kEigSmallThreads * ((nbins + 3) / 4) >= 8 * kNumSMs)
+            return launch_eig_small<USE_RM, CUSTOM, 1, CUSTOM ? 1 : 4>(ACB_EIG_ARGS);
+        return launch_eig_small<USE_RM, CUSTOM, 1, 1>(ACB_EIG_ARGS);
     }
-    const int mc = a.M <= 256 ? a.M : 128;
-    const size_t smem = (size_t)(((3 * a.M + 1) & ~1) * sizeof(double)) + (size_t)mc * kLanes * sizeof(double2);
-    auto kern = map_eig_kernel<USE_RM, CUSTOM>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const dim3 grid((unsigned)((a.G + kLanes - 1) / kLanes), nbins);
-    kern<<<grid, kLanes * kWarps, smem, s>>>(a, E, eigval, reinterpret_cast<const double2 *>(eigvec), k, k_scalar, mpos,
-                                            gpos, r0, rm, mc, out_map, out_norm,
-                                            reinterpret_cast<const double2 *>(steer), active);
-    return check_launch();
+    if (E <= kEigSmall) return launch_eig_small<USE_RM, CUSTOM, kEigSmall, 1>(ACB_EIG_ARGS);
+    if (a.M <= kMapFourWarps) return launch_eig_nw<USE_RM, CUSTOM, 4>(ACB_EIG_ARGS);
+    return launch_eig_nw<USE_RM, CUSTOM, 8>(ACB_EIG_ARGS);
+#undef ACB_EIG_ARGS
 }
 
 // Launchers for other translation units (map_internal.h).
@@ -815,15 +767,16 @@ using namespace acb;
 extern "C" {
 
 int acb_map_f64(const acb_map_params *p, const void *csm, const double *wavenumber, const double *mpos,
-                const double *gpos, double *out_map, double *out_steer_norm, int *error_word, void *stream)
+                const double *gpos, double *out_map, double *out_steer_norm, int * /*error_word: no device-side wait*/,
+                void *stream)
 {
     MapArgs a;
     int st = make_args(p, a);
     if (st) return st;
     if (!csm || !wavenumber || !mpos || !gpos || !out_map) return ACB_ERR_ARG;
-    if ((a.G + kLanes - 1) / kLanes > 0x7fffffffLL) return ACB_ERR_SHAPE;
+    if ((a.G + kPts - 1) / kPts > 0x7fffffffLL) return ACB_ERR_SHAPE;
     return launch_plain<false>(a, p->num_bins, csm, wavenumber, 0.0, mpos, gpos, nullptr, nullptr, out_map,
-                               out_steer_norm, as_stream(stream), nullptr, error_word);
+                               out_steer_norm, as_stream(stream));
 }
 
 int acb_map_eig_f64(const acb_map_params *p, int num_eigs, const double *eigval, const void *eigvec,
@@ -835,7 +788,7 @@ int acb_map_eig_f64(const acb_map_params *p, int num_eigs, const double *eigval,
     if (st) return st;
     if (!eigval || !eigvec || !wavenumber || !mpos || !gpos || !out_map) return ACB_ERR_ARG;
     if (num_eigs < 1 || num_eigs > p->num_mics) return ACB_ERR_SHAPE;
-    if ((a.G + kLanes - 1) / kLanes > 0x7fffffffLL) return ACB_ERR_SHAPE;
+    if ((a.G + kPts - 1) / kPts > 0x7fffffffLL) return ACB_ERR_SHAPE;
     return launch_eig<false>(a, p->num_bins, num_eigs, eigval, eigvec, wavenumber, 0.0, mpos, gpos, nullptr, nullptr,
                              out_map, out_steer_norm, as_stream(stream));
 }
@@ -862,7 +815,7 @@ int acb_map_rm_f64(const acb_map_params *p, const void *csm, const double *waven
     int st = make_args(p, a);
     if (st) return st;
     if (!csm || !wavenumber || !r0 || !rm || !out_map) return ACB_ERR_ARG;
-    if ((a.G + kLanes - 1) / kLanes > 0x7fffffffLL) return ACB_ERR_SHAPE;
+    if ((a.G + kPts - 1) / kPts > 0x7fffffffLL) return ACB_ERR_SHAPE;
     a.ref_mode = 0;
     return launch_plain<true>(a, p->num_bins, csm, wavenumber, 0.0, nullptr, nullptr, r0, rm, out_map, out_steer_norm,
                               as_stream(stream));
@@ -888,7 +841,7 @@ int acb_map_custom_f64(const acb_map_params *p, const void *csm, const void *ste
     int st = custom_args(p, a);
     if (st) return st;
     if (!csm || !steer || !out_map) return ACB_ERR_ARG;
-    if ((a.G + kLanes - 1) / kLanes > 0x7fffffffLL) return ACB_ERR_SHAPE;
+    if ((a.G + kPts - 1) / kPts > 0x7fffffffLL) return ACB_ERR_SHAPE;
     return launch_plain<false, true>(a, p->num_bins, csm, nullptr, 0.0, nullptr, nullptr, nullptr, nullptr, out_map,
                                      out_steer_norm, as_stream(stream), steer);
 }
@@ -901,7 +854,7 @@ int acb_map_eig_custom_f64(const acb_map_params *p, int num_eigs, const double *
     if (st) return st;
     if (!eigval || !eigvec || !steer || !out_map) return ACB_ERR_ARG;
     if (num_eigs < 1 || num_eigs > p->num_mics) return ACB_ERR_SHAPE;
-    if ((a.G + kLanes - 1) / kLanes > 0x7fffffffLL) return ACB_ERR_SHAPE;
+    if ((a.G + kPts - 1) / kPts > 0x7fffffffLL) return ACB_ERR_SHAPE;
     return launch_eig<false, true>(a, p->num_bins, num_eigs, eigval, eigvec, nullptr, 0.0, nullptr, nullptr, nullptr,
                                    nullptr, out_map, out_steer_norm, as_stream(stream), steer);
 }
