@@ -627,6 +627,145 @@ __global__ void __launch_bounds__(256) gram_kernel(const void *__restrict__ spec
 }
 
 // ------------------------------------------------------------------------------------------------
+// The complex128 Gram on the FP64 matrix instruction (mma.sync m16n8k8; tcgen05 has no FP64 kind).  With the windows'
+// (re, im) pairs as the K dimension,
+//     Re C[r][c] = sum_k A[r][k] B[k][c],  A[r] = (x_r, y_r, ..),  B[.][c] = (x_c, y_c, ..),
+//     Im C[r][c] = sum_k A[r][k] B'[k][c],                         B'[.][c] = (-y_c, x_c, ..),
+// and the instruction adds its products to an element as a chain of FMAs in ascending k (checked on 10^5 random
+// elements), so this is the reference's order of two chained FMAs per window and component, bit for bit.
+// CTA = 32 x 32 tile of one bin's upper triangle, 4 warps of 16 x 16; 16 windows per stage, three stages of cp.async,
+// four CTAs per SM.  Rows are padded to 36 mics, so that the operand reads of 4 mics x 2 windows (A) and 8 mics x 2
+// windows (B) fall on different banks.  16 x 8 blocks entirely below the diagonal or past M are skipped.
+// Bound: the FP64 pipe (4 M^2 K flop per bin).  Measured (B200): 513 bins x 256 mics x 999 windows 7.84 -> 5.0 ms
+// (27 TFLOP/s; 64 x 64 tiles of 32 x 16 per warp 5.2 ms, half of the diagonal tiles idle); 65 bins x 64 mics x 799
+// windows 281 -> 115 us (195 CTAs where the 64 x 64 tiles of the FMA form were 65).
+// ------------------------------------------------------------------------------------------------
+constexpr int GF_T = 32;       // tile edge
+constexpr int GF_LD = GF_T + 4;
+constexpr int GF_KW = 16;      // windows per stage
+constexpr int GF_STAGES = 3;
+constexpr int GF_SMEM = GF_STAGES * 2 * GF_KW * GF_LD * (int)sizeof(double2);
+
+__device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], double b0, double b1)
+{
+    asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64.rn {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+
+__global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restrict__ spec, int M, int64_t nw,
+                                                          double2 *__restrict__ csm)
+{
+    constexpr int T = GF_T, LD = GF_LD, NB = 2;
+    extern __shared__ double2 gf_sm[];   // [stage][row mics | column mics][window][LD]
+    // upper-triangular tile index -> (ti, tj), ti <= tj
+    const int NT = (M + T - 1) / T;
+    int tile = blockIdx.x, ti = 0;
+    while (tile >= NT - ti) {
+        tile -= NT - ti;
+        ++ti;
+    }
+    const int tj = ti + tile;
+    const int f = blockIdx.y;
+    const int lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    // warp -> 16 x 16 quarter, rotated over the CTAs: in a diagonal tile the lower-left quarter has nothing to do
+    const int quarter = ((threadIdx.x >> 5) + blockIdx.x + blockIdx.y) & 3;
+    const int wr = quarter >> 1, wc = quarter & 1;
+    const int r0 = ti * T, c0 = tj * T;
+    const int rw = r0 + wr * 16, cw = c0 + wc * 16;   // this warp's first row and column
+    const bool same = ti == tj;
+    const double2 *sp = spec + (int64_t)f * nw * M;
+    double2 *base = csm + (int64_t)f * M * M;
+
+    auto load = [&](int64_t st) {
+        double2 *d = gf_sm + (st % GF_STAGES) * (2 * GF_KW * LD);
+        const int64_t k0 = st * GF_KW;
+#pragma unroll
+        for (int i = 0; i < GF_KW / 4; ++i) {
+            const int kk = i * 4 + (int)threadIdx.x / T, m = threadIdx.x % T;
+            const bool in = k0 + kk < nw;
+            const double2 *src = sp + (in ? k0 + kk : 0) * M;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(d + kk * LD + m);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src + min(r0 + m, M - 1)),
+                         "r"(in && r0 + m < M ? 16 : 0)
+                         : "memory");
+            if (!same)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + GF_KW * LD * 16),
+                             "l"(src + min(c0 + m, M - 1)), "r"(in && c0 + m < M ? 16 : 0)
+                             : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    double re[NB][4], im[NB][4];
+    bool use[NB];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+        const int cb = cw + 8 * j;
+        use[j] = rw <= cb + 7 && rw < M && cb < M;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = rw + g + 8 * (e >> 1), c = cb + 2 * t + (e & 1);
+            double2 v = make_double2(0.0, 0.0);
+            if (c < M && r <= c) v = base[(int64_t)r * M + c];
+            re[j][e] = v.x;
+            im[j][e] = v.y;
+        }
+    }
+
+    const int64_t nst = (nw + GF_KW - 1) / GF_KW;
+    load(0);
+    if (nst > 1) load(1);
+    for (int64_t st = 0; st < nst; ++st) {
+        if (st + 1 < nst) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();   // stage st has landed for every thread; stage st - 1 is read by none any more
+        if (st + 2 < nst) load(st + 2);
+        const double2 *xr = gf_sm + (st % GF_STAGES) * (2 * GF_KW * LD);
+        const double2 *xc = same ? xr : xr + GF_KW * LD;
+        const double *ar = reinterpret_cast<const double *>(xr + (t >> 1) * LD + wr * 16 + g) + (t & 1);
+        const double2 *bc = xc + (t >> 1) * LD + wc * 16 + g;
+#pragma unroll
+        for (int w = 0; w < GF_KW; w += 4) {
+            double b0[NB], b1[NB], q0[NB], q1[NB];
+#pragma unroll
+            for (int j = 0; j < NB; ++j) {
+                const double2 u = bc[w * LD + 8 * j], v = bc[(w + 2) * LD + 8 * j];
+                b0[j] = t & 1 ? u.y : u.x;
+                b1[j] = t & 1 ? v.y : v.x;
+                q0[j] = t & 1 ? u.x : -u.y;
+                q1[j] = t & 1 ? v.x : -v.y;
+            }
+            const double *p = ar + w * LD * 2;
+            const double a[4] = {p[0], p[16], p[4 * LD], p[4 * LD + 16]};
+#pragma unroll
+            for (int j = 0; j < NB; ++j)
+                if (use[j]) {
+                    mma_f64(re[j], a, b0[j], b1[j]);
+                    mma_f64(im[j], a, q0[j], q1[j]);
+                }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = rw + g + 8 * (e >> 1), c = cw + 8 * j + 2 * t + (e & 1);
+            if (c < M && r <= c) base[(int64_t)r * M + c] = make_double2(re[j][e], im[j][e]);
+        }
+}
+
+static int gram_f64_launch(const void *spec, int M, int64_t nw, int nbins, void *csm, cudaStream_t s)
+{
+    const int T = (M + GF_T - 1) / GF_T;
+    cudaFuncSetAttribute(gram_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GF_SMEM);
+    gram_f64_kernel<<<dim3(T * (T + 1) / 2, nbins), 128, GF_SMEM, s>>>(reinterpret_cast<const double2 *>(spec), M, nw,
+                                                                      reinterpret_cast<double2 *>(csm));
+    return check_launch();
+}
+
+// ------------------------------------------------------------------------------------------------
 // Hermitian completion + scale, 32x32 tiles through shared memory for the transposed half.
 // ------------------------------------------------------------------------------------------------
 template <bool C64>
@@ -798,9 +937,7 @@ int acb_calc_csm_c128(void *csm, const void *spec, int num_freqs, int num_mics, 
 {
     if (!csm || !spec) return ACB_ERR_ARG;
     if (num_freqs <= 0 || num_mics <= 0) return ACB_ERR_SHAPE;
-    const int T = (num_mics + GT - 1) / GT;
-    gram_kernel<false><<<dim3(T * (T + 1) / 2, num_freqs), 256, 0, as_stream(stream)>>>(spec, num_mics, 1, csm);
-    return check_launch();
+    return gram_f64_launch(spec, num_mics, 1, num_freqs, csm, as_stream(stream));
 }
 
 int acb_calc_csm_c64(void *csm, const void *spec, int num_freqs, int num_mics, void *stream)
@@ -861,10 +998,9 @@ int acb_csm_accumulate(const void *samples, int sample_dtype, int64_t num_sample
     int st = fft_launch(samples, sample_dtype, precision == ACB_C64 ? OUT_C64 : OUT_C128, num_mics, block_size, hop,
                         first_window, num_windows, window, tw, bin_lo, num_bins, workspace, 0, 0, 0, scratch, s);
     if (st) return st;
+    if (precision == ACB_C128) return gram_f64_launch(workspace, num_mics, num_windows, num_bins, csm_upper, s);
     const int T = (num_mics + GT - 1) / GT;
-    const dim3 g2(T * (T + 1) / 2, num_bins);
-    if (precision == ACB_C64) gram_kernel<true><<<g2, 256, 0, s>>>(workspace, num_mics, num_windows, csm_upper);
-    else gram_kernel<false><<<g2, 256, 0, s>>>(workspace, num_mics, num_windows, csm_upper);
+    gram_kernel<true><<<dim3(T * (T + 1) / 2, num_bins), 256, 0, s>>>(workspace, num_mics, num_windows, csm_upper);
     return check_launch();
 }
 
