@@ -29,14 +29,17 @@ static thread_local std::string g_last_cuda_error;
 void set_cuda_error(cudaError_t e) { g_last_cuda_error = cudaGetErrorString(e); }
 
 // ------------------------------------------------------------------------------------------------
-// Windowed real FFT.  One CTA = one window x `mpb` mics; FFT of the N/2-point complex sequence
+// Windowed real FFT.  One CTA = one window x `mpb` mics (a power of two); FFT of the N/2-point complex sequence
 // z[j] = x[2j] + i x[2j+1], then the split into the N/2+1 real-input bins.
 //
-// The radix-2 DIT stages run in passes of up to three: a thread loads the 2^s points that s
-// consecutive stages combine among themselves, applies the s stages' butterflies in registers
-// (same operands, twiddles and operation order as one stage at a time, so the spectra are the
-// same bits) and stores them back: one shared-memory round trip and one barrier per pass instead
-// of per stage.
+// The radix-2 DIT stages run in passes of up to three: a thread loads the 2^s points that s consecutive stages
+// combine among themselves, applies the s stages' butterflies in registers and stores them back: one
+// shared-memory round trip and one barrier per pass instead of per stage.  The first three stages take their points
+// straight from the samples (bit-reversed order: 8 rows H/8 apart), lanes along the mics.  In the later passes a
+// thread keeps its task's twiddles for all of its mics, and it reads four of the seven: the others are those times -i.
+// Bound: shared memory (seven 16-byte accesses per point) and the FP64 pipe, about 0.5 ms each for 999 windows x 256
+// mics x 1024 samples.  Measured (B200): that transform 2.65 -> 1.24 ms (before: two more trips through shared
+// memory, a twiddle load per butterfly and runtime divisions by the mic count in the index arithmetic).
 // ------------------------------------------------------------------------------------------------
 // Shared-memory slot of point j of a mic's sequence: one padding slot after every 8 points, so that
 // 8 threads reading 16-byte points 8 apart (the first pass) or 64 apart hit different banks.
@@ -44,13 +47,32 @@ __device__ __forceinline__ int zp(int j) { return j + (j >> 3); }
 // padded length of one mic's sequence of H points (an odd number of 16-byte slots past the padding)
 __host__ __device__ constexpr int fft_stride(int H) { return H + (H >> 3) + 1; }
 
-// s (1..3) consecutive radix-2 DIT stages of lengths L1 = 2^(sg + 1), 2 L1, .., on a bit-reversed
-// sequence z of H points (one mic).  Task `task` in [0, H / 2^s) owns points base + t * L1/2,
-// t = 0 .. 2^s - 1.  All lengths are powers of two (logN = log2 N): shifts and masks index the
-// points and the twiddles W_N^e.
+// (a, b) -> (a + w b, a - w b), the difference as 2 a - (a + w b): six FMAs
+__device__ __forceinline__ void butterfly(double2 &a, double2 &b, double2 w)
+{
+    const double re = fma(b.x, w.x, fma(-b.y, w.y, a.x)), im = fma(b.x, w.y, fma(b.y, w.x, a.y));
+    b = make_double2(fma(2.0, a.x, -re), fma(2.0, a.y, -im));
+    a = make_double2(re, im);
+}
+
+// Twiddles of one task of a pass of S stages, the first of length 2 half1: with tb = task mod half1, stage q uses
+// W_{2 half1 2^q}^{tb + u half1}, u < 2^q; w[q] holds u = 0 and w3 u = 1 of the third stage; u + 2^{q-1} is -i times u.
 template <int S>
-__device__ __forceinline__ void fft_pass(double2 *__restrict__ z, int sg, int task, int logN,
-                                         const double2 *__restrict__ tw)
+struct PassTwiddles {
+    double2 w[S], w3;
+    __device__ __forceinline__ void load(int sg, int task, int logN, const double2 *__restrict__ tw)
+    {
+        const int half1 = 1 << sg, tb = task & (half1 - 1);
+#pragma unroll
+        for (int q = 0; q < S; ++q) w[q] = __ldg(tw + (tb << (logN - (sg + 1 + q))));
+        if (S == 3) w3 = __ldg(tw + ((tb + half1) << (logN - (sg + 3))));
+    }
+};
+
+// s (1..3) consecutive radix-2 DIT stages of lengths L1 = 2^(sg + 1), 2 L1, .., on a bit-reversed
+// sequence z (one mic).  Task `task` in [0, H / 2^s) owns points base + t * L1/2, t = 0 .. 2^s - 1.
+template <int S>
+__device__ __forceinline__ void fft_pass(double2 *__restrict__ z, int sg, int task, const PassTwiddles<S> &tws)
 {
     const int half1 = 1 << sg;
     const int base = ((task >> sg) << (sg + S)) + (task & (half1 - 1));   // the pass spans 2^(sg + S) points
@@ -58,24 +80,73 @@ __device__ __forceinline__ void fft_pass(double2 *__restrict__ z, int sg, int ta
 #pragma unroll
     for (int t = 0; t < (1 << S); ++t) v[t] = z[zp(base + t * half1)];
 #pragma unroll
-    for (int q = 0; q < S; ++q) {
-        const int hf = half1 << q;                       // half the stage length L = 2^(sg + 1 + q)
-        const int shift = logN - (sg + 1 + q);           // W_L^i = W_N^(i N / L)
+    for (int q = 0; q < S; ++q)
 #pragma unroll
         for (int t = 0; t < (1 << S); ++t) {
             if (t & (1 << q)) continue;
-            const int i0 = base + t * half1;
-            const double2 w = __ldg(tw + ((i0 & (hf - 1)) << shift));
-            const double2 b = v[t + (1 << q)];
-            const double br = b.x * w.x - b.y * w.y;
-            const double bi = b.x * w.y + b.y * w.x;
-            const double2 a = v[t];
-            v[t] = make_double2(a.x + br, a.y + bi);
-            v[t + (1 << q)] = make_double2(a.x - br, a.y - bi);
+            const int u = t & ((1 << q) - 1);
+            const double2 w1 = S == 3 && q == 2 && (u & 1) ? tws.w3 : tws.w[q];
+            const bool rot = q > 0 && (u >> (q - 1));   // the upper half of the u: times -i
+            butterfly(v[t], v[t + (1 << q)], rot ? make_double2(w1.y, -w1.x) : w1);
         }
-    }
 #pragma unroll
     for (int t = 0; t < (1 << S); ++t) z[zp(base + t * half1)] = v[t];
+}
+
+// The remaining stages st .. logH - 1 of `nm` sequences in shared memory.  A thread keeps one task per pass and
+// its twiddles, and walks the mics (all of them, or every ngrp-th where the CTA holds ngrp threads per task).
+template <int S>
+__device__ __forceinline__ void fft_pass_mics(double2 *zs, int nm, int stride, int st, int logH, int logN,
+                                              const double2 *__restrict__ tw)
+{
+    const int logT = logH - S, T = 1 << logT;   // H / 2^S tasks per mic
+    const int nt = blockDim.x;
+    const int grp = T < nt ? threadIdx.x >> logT : 0, ngrp = T < nt ? nt >> logT : 1;
+    for (int task = T < nt ? threadIdx.x & (T - 1) : threadIdx.x; task < T; task += nt) {
+        PassTwiddles<S> w;
+        w.load(st, task, logN, tw);
+        for (int ml = grp; ml < nm; ml += ngrp) fft_pass<S>(zs + ml * stride, st, task, w);
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ void fft_passes(double2 *zs, int nm, int stride, int st, int logH, int logN,
+                                           const double2 *__restrict__ tw)
+{
+    while (st < logH) {
+        const int left = logH - st;
+        // four left: 2 + 2 rather than 3 + 1
+        const int S = left == 4 ? 2 : (left >= 3 ? 3 : left);
+        if (S == 3) fft_pass_mics<3>(zs, nm, stride, st, logH, logN, tw);
+        else if (S == 2) fft_pass_mics<2>(zs, nm, stride, st, logH, logN, tw);
+        else fft_pass_mics<1>(zs, nm, stride, st, logH, logN, tw);
+        st += S;
+    }
+}
+
+// The first three stages (twiddles 1, -i and the odd eighth roots) of 8 points in bit-reversed order.
+__device__ __forceinline__ void first_stages(double2 (&v)[8])
+{
+    auto pair = [](double2 &a, double2 &b) {
+        const double2 s = make_double2(a.x + b.x, a.y + b.y);
+        b = make_double2(a.x - b.x, a.y - b.y);
+        a = s;
+    };
+    auto turn = [](double2 &a) { a = make_double2(a.y, -a.x); };   // times -i
+#pragma unroll
+    for (int t = 0; t < 8; t += 2) pair(v[t], v[t + 1]);
+#pragma unroll
+    for (int t = 0; t < 8; t += 4) {
+        pair(v[t], v[t + 2]);
+        turn(v[t + 3]);
+        pair(v[t + 1], v[t + 3]);
+    }
+    const double h = 0.70710678118654752440;
+    pair(v[0], v[4]);
+    butterfly(v[1], v[5], make_double2(h, -h));
+    turn(v[6]);
+    pair(v[2], v[6]);
+    butterfly(v[3], v[7], make_double2(-h, -h));
 }
 
 // Output forms of the spectra (OUT): complex128 or complex64 [bin][window][mic] for the FP64 /
@@ -116,61 +187,61 @@ __device__ __forceinline__ void put_bin(void *__restrict__ out, int64_t nw, int 
 }
 
 template <typename TS, int OUT>
-__global__ void __launch_bounds__(256) fft_window_kernel(const TS *__restrict__ samples, int M, int N, int hop,
+__global__ void __launch_bounds__(512) fft_window_kernel(const TS *__restrict__ samples, int M, int N, int hop,
                                                          int64_t w0, int64_t nw, int mpb,
                                                          const double *__restrict__ window,
                                                          const double2 *__restrict__ tw, int bin_lo, int nbins,
                                                          void *__restrict__ out, int R, int KC, int64_t lo_elems)
 {
     extern __shared__ double2 zs[];  // [mpb][fft_stride(H)], point j of mic ml at zs[ml * stride + zp(j)]
-    const int H = N >> 1;
-    int logH = 0;
-    while ((1 << logH) < H) ++logH;
+    const int H = N >> 1, stride = fft_stride(H);
+    const int logH = 31 - __clz(H), logP = 31 - __clz(mpb);
     const int64_t w = w0 + blockIdx.y;
     const int m0 = blockIdx.x * mpb;
     const int nm = min(mpb, M - m0);
-    const TS *src = samples + (w * (int64_t)hop) * M;
+    const TS *src = samples + (w * (int64_t)hop) * M + m0;
 
-    // load + window + bit-reversed placement
-    for (int idx = threadIdx.x; idx < H * nm; idx += blockDim.x) {
-        const int ml = idx % nm;
-        const int j = idx / nm;
-        const double x0 = (double)src[(int64_t)(2 * j) * M + m0 + ml] * window[2 * j];
-        const double x1 = (double)src[(int64_t)(2 * j + 1) * M + m0 + ml] * window[2 * j + 1];
-        const int jr = (int)(__brev((unsigned)j) >> (32 - logH));
-        zs[ml * fft_stride(H) + zp(logH ? jr : 0)] = make_double2(x0, x1);
+    // load + window + the first three stages: task = 8 consecutive slots of the bit-reversed order, i.e. points
+    // rev(task) + H/8 {0, 4, 2, 6, 1, 5, 3, 7} (H >= 8)
+    const int logT = logH - 3;
+    for (int idx = threadIdx.x; idx < mpb << logT; idx += blockDim.x) {
+        const int ml = idx & (mpb - 1), task = idx >> logP;
+        if (ml >= nm) continue;
+        const int j0 = logT ? (int)(__brev((unsigned)task) >> (32 - logT)) : 0;
+        double2 v[8];
+        TS x0[8], x1[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            const int j = j0 + ((((t & 1) << 2) | (t & 2) | (t >> 2)) << logT);
+            x0[t] = __ldg(src + (int64_t)(2 * j) * M + ml);
+            x1[t] = __ldg(src + (int64_t)(2 * j + 1) * M + ml);
+        }
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            const int j = j0 + ((((t & 1) << 2) | (t & 2) | (t >> 2)) << logT);
+            v[t] = make_double2((double)x0[t] * __ldg(window + 2 * j), (double)x1[t] * __ldg(window + 2 * j + 1));
+        }
+        first_stages(v);
+        double2 *z = zs + ml * stride + 9 * task;   // zp(8 task + t) = 9 task + t
+#pragma unroll
+        for (int t = 0; t < 8; ++t) z[t] = v[t];
     }
     __syncthreads();
-
-    // radix-2 DIT stages, up to three per pass
-    for (int st = 0; st < logH;) {
-        const int S = logH - st >= 3 ? 3 : logH - st;
-        const int logT = logH - S;   // H / 2^S tasks per mic
-        for (int idx = threadIdx.x; idx < nm << logT; idx += blockDim.x) {
-            const int ml = idx >> logT;
-            const int task = idx & ((1 << logT) - 1);
-            if (S == 3) fft_pass<3>(zs + ml * fft_stride(H), st, task, logH + 1, tw);
-            else if (S == 2) fft_pass<2>(zs + ml * fft_stride(H), st, task, logH + 1, tw);
-            else fft_pass<1>(zs + ml * fft_stride(H), st, task, logH + 1, tw);
-        }
-        __syncthreads();
-        st += S;
-    }
+    fft_passes(zs, nm, stride, 3, logH, logH + 1, tw);
 
     // real-input split: X[k] = E + W^k O,  E = (Z[k] + conj(Z[H-k]))/2,  O = -i (Z[k] - conj(Z[H-k]))/2
-    for (int idx = threadIdx.x; idx < nbins * nm; idx += blockDim.x) {
-        const int ml = idx % nm;
-        const int k = bin_lo + idx / nm;
-        const double2 *z = zs + ml * fft_stride(H);
-        const double2 zk = z[zp(k % H)];
-        const double2 zc = z[zp((H - k % H) % H)];
+    for (int idx = threadIdx.x; idx < nbins << logP; idx += blockDim.x) {
+        const int ml = idx & (mpb - 1);
+        if (ml >= nm) continue;
+        const int k = bin_lo + (idx >> logP), kh = k & (H - 1);
+        const double2 *z = zs + ml * stride;
+        const double2 zk = z[zp(kh)];
+        const double2 zc = z[zp((H - kh) & (H - 1))];
         const double er = 0.5 * (zk.x + zc.x), ei = 0.5 * (zk.y - zc.y);
         const double orr = 0.5 * (zk.y + zc.y), oi = -0.5 * (zk.x - zc.x);
-        double2 wk;
-        if (k < H) wk = tw[k];
-        else wk = make_double2(-1.0, 0.0);
-        const double xr = er + (wk.x * orr - wk.y * oi);
-        const double xi = ei + (wk.x * oi + wk.y * orr);
+        const double2 wk = k < H ? __ldg(tw + k) : make_double2(-1.0, 0.0);
+        const double xr = fma(wk.x, orr, fma(-wk.y, oi, er));
+        const double xi = fma(wk.x, oi, fma(wk.y, orr, ei));
         put_bin<OUT>(out, nw, (int)blockIdx.y, M, m0 + ml, k - bin_lo, xr, xi, R, KC, lo_elems);
     }
 }
@@ -464,19 +535,7 @@ __global__ void __launch_bounds__(256) fft_sub_kernel(const TS *__restrict__ sam
         zs[zp((int)(__brev((unsigned)i) >> (32 - logHs)))] = make_double2(x0, x1);
     }
     __syncthreads();
-    int logN = 0;
-    while ((1 << logN) < N) ++logN;
-    for (int st = 0; st < logHs;) {
-        const int S = logHs - st >= 3 ? 3 : logHs - st;
-        const int ntask = FFT_SUB_H >> S;
-        for (int task = threadIdx.x; task < ntask; task += blockDim.x) {
-            if (S == 3) fft_pass<3>(zs, st, task, logN, tw);
-            else if (S == 2) fft_pass<2>(zs, st, task, logN, tw);
-            else fft_pass<1>(zs, st, task, logN, tw);
-        }
-        __syncthreads();
-        st += S;
-    }
+    fft_passes(zs, 1, 0, 0, logHs, 31 - __clz(N), tw);
     double2 *dst = scratch + ((wi * M + m) * D + d) * (int64_t)FFT_SUB_H;
     for (int k = threadIdx.x; k < FFT_SUB_H; k += blockDim.x) dst[k] = zs[zp(k)];
 }
@@ -812,12 +871,20 @@ __global__ void __launch_bounds__(256) finalize_kernel(const void *__restrict__ 
     }
 }
 
-// Mics per CTA: at most 32 KB of complex doubles (N/2 per mic), so that several CTAs share an SM
-// and hide each other's barrier and FP64 latency; one mic for N > 4096.
+// Mics per CTA (a power of two) and threads: up to 74 KB of padded complex doubles and 256 threads, so that two or
+// three CTAs share an SM and hide each other's barriers and FP64 latency; for blocks of FFT_WIDE_N samples and more, of
+// which that would hold one or two mics and store 16 bytes of a row of complex64 spectra at a time, up to 150 KB and
+// 512 threads.
+// (Measured, CSM of 256 mics x 300,000 samples, block 8192, complex64: 6.29 -> 5.52 ms; 113 mics, block 2048: 0.93 ->
+// 0.91; block 512, 256 mics: 2.53 -> 2.65, so not below 2048.)
+constexpr int FFT_WIDE_N = 2048;
+static int fft_threads(int N) { return N >= FFT_WIDE_N ? 512 : 256; }
 static int fft_mics_per_block(int N)
 {
-    const int cap = 4096 / N;
-    return cap >= 16 ? 16 : (cap < 1 ? 1 : cap);
+    const size_t most = (N >= FFT_WIDE_N ? 150 : 74) * 1024;
+    int mpb = 16;
+    while (mpb > 1 && (size_t)mpb * fft_stride(N / 2) * sizeof(double2) > most) mpb >>= 1;
+    return mpb;
 }
 
 // Launch the windowed FFT of `num_windows` windows in output form `out_form`.
@@ -892,8 +959,8 @@ int fft_launch(const void *samples, int sample_dtype, int out_form, int num_mics
     do {                                                                                                          \
         auto kern = fft_window_kernel<TS, OF>;                                                                    \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                       \
-        kern<<<g1, 256, smem, s>>>(reinterpret_cast<const TS *>(samples), num_mics, block_size, hop, first_window, \
-                                   num_windows, mpb, window, tw, bin_lo, num_bins, out, R, KC, lo_elems);        \
+        kern<<<g1, fft_threads(block_size), smem, s>>>(reinterpret_cast<const TS *>(samples), num_mics, block_size, hop, \
+                                   first_window, num_windows, mpb, window, tw, bin_lo, num_bins, out, R, KC, lo_elems);        \
     } while (0)
 #define ACB_FFT_FORMS(TS)                                                \
     switch (out_form) {                                                  \
