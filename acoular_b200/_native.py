@@ -84,6 +84,7 @@ SIGNATURES = {
     'acb_csm_workspace_bytes': (_SZ, [_I, _I, _I64, _I]),
     'acb_csm_workspace_bytes_block': (_SZ, [_I, _I, _I64, _I, _I]),
     'acb_csm_accumulate': (_I, [_VP, _I, _I64, _I, _I, _I, _I64, _I64, _VP, _VP, _I, _I, _I, _VP, _VP, _SZ, _VP]),
+    'acb_csm_finished': (_I, [_VP, _I, _I64, _I, _I, _I, _I64, _I64, _VP, _VP, _I, _I, _I, _D, _VP, _VP, _SZ, _VP]),
     'acb_csm_finalize': (_I, [_VP, _I, _I, _I, _D, _VP, _VP]),
     'acb_map_f64': (_I, [ctypes.POINTER(MapParams), _VP, _VP, _VP, _VP, _VP, _VP, _VP, _VP]),
     'acb_beamformer_freq_f64': (_I, [ctypes.POINTER(MapParams), _VP, _D, _VP, _VP, _VP, _VP, _VP]),

@@ -4,8 +4,8 @@ An instance is one array recording with its own geometry, grid, FFT block size a
 the unit ``PowerSpectra`` + ``BeamformerBase`` process in the reference (acoular/spectra.py:366-416,
 acoular/fbeamform.py:475-510).  :class:`BatchPlan` keeps every instance's buffers resident and runs
 
-1. per instance: the windowed FFT + Welch accumulation for the instance's bins only
-   (``acb_csm_accumulate``) and the Hermitian finish (``acb_csm_finalize``);
+1. per instance: the windowed FFT + Welch sums for the instance's bins only, written as the finished
+   Hermitian matrix (``acb_csm_finished``);
 2. one persistent tensor-core launch for the maps of all instances (``acb_map_tc_batch``; up to 64
    instances per launch, one launch per steering type).
 
@@ -57,7 +57,7 @@ class BatchPlan:
         self.inst = list(instances)
         self.graph = None
         dev = self.dev
-        self.samples, self.upper, self.csm, self.k, self.mpos, self.gpos, self.out = [], [], [], [], [], [], []
+        self.samples, self.csm, self.k, self.mpos, self.gpos, self.out = [], [], [], [], [], []
         self.scale, self.windows, self.norm = [], [], []
         ws_bytes = 0
         for it in self.inst:
@@ -67,8 +67,6 @@ class BatchPlan:
             else:
                 dtype = torch.float32 if np.asarray(it.samples).dtype == np.float32 else torch.float64
             self.samples.append(torch.empty((S, M), dtype=dtype, device=dev))
-            cdt = torch.complex64 if it.precision == 'complex64' else torch.complex128
-            self.upper.append(torch.zeros((it.num_bins, M, M), dtype=cdt, device=dev))
             self.csm.append(torch.empty((it.num_bins, M, M), dtype=torch.complex128, device=dev))
             freqs = np.abs(np.fft.fftfreq(it.block_size, 1.0 / it.sample_freq)[: it.block_size // 2 + 1])
             bins = np.arange(it.bin_lo, it.bin_lo + it.num_bins)
@@ -106,11 +104,9 @@ class BatchPlan:
 
     def _launch(self):
         for i, it in enumerate(self.inst):
-            self.upper[i].zero_()
-            D.csm_upper_accumulate(self.samples[i], it.block_size, it.window, it.overlap, it.precision,
-                                   bin_lo=it.bin_lo, num_bins=it.num_bins, csm_upper=self.upper[i],
-                                   workspace=self.csm_ws, max_workspace_bytes=self.csm_ws.numel())
-            D.csm_finalize(self.upper[i], self.scale[i], out=self.csm[i])
+            D.csm_finished(self.samples[i], it.block_size, it.window, it.overlap, it.precision, self.scale[i],
+                           bin_lo=it.bin_lo, num_bins=it.num_bins, out=self.csm[i], workspace=self.csm_ws,
+                           max_workspace_bytes=self.csm_ws.numel())
         if self.form == 'tc':
             groups = {}
             for mi in self.map_instances:

@@ -3,8 +3,10 @@
 // Data flow per chunk of windows (all on the device, samples resident in HBM):
 //   fft_window_kernel : samples [S][M] (f32|f64) -> window (FP64) -> rFFT (FP64, radix-2 in shared
 //                       memory) -> spectra [bin][window][mic] rounded to the CSM precision
-//   gram_kernel       : csm_upper[bin][r][c] += sum_w conj(X[bin][w][c]) * X[bin][w][r], r <= c,
-//                       64x64 upper-triangular tiles, windows streamed through shared memory
+//   gram_f64_kernel   : csm_upper[bin][r][c] += sum_w conj(X[bin][w][c]) * X[bin][w][r], r <= c,
+//   gram_c64_kernel     32x32 (FP64 matrix instruction) or 64x64 (packed FP32 FMAs) upper-triangular tiles,
+//                       windows streamed through shared memory; or the finished matrix where the
+//                       windows are one chunk
 //   finalize_kernel   : Hermitian completion and the 2/(N*sum(w^2)*num_blocks) scale
 //
 // The per-element accumulation runs sequentially over windows with the same two chained FMAs per
@@ -588,32 +590,56 @@ __global__ void __launch_bounds__(256) fft_combine_kernel(const double2 *__restr
 }
 
 // ------------------------------------------------------------------------------------------------
-// Welch Gram accumulation, upper-triangular 64x64 tiles; thread (tx, ty) owns rows ty+16i and
-// columns tx+16j of the tile (conflict-free shared-memory reads, coalesced stores).
+// Welch Gram accumulation in complex64, upper-triangular 64x64 tiles; thread (tx, ty) of 16 x 8 owns rows ty + 8 i
+// and columns tx + 16 j of the tile.  An element's (re, im) is one packed pair of FP32 accumulators, so that the
+// reference's two chained FMAs per component are two packed FMAs, (x_c, -y_c) x_r and then (y_c, x_c) y_r.  In a
+// diagonal tile the 8 x 16 blocks below the diagonal are left out.
+// Bound: FP32 FMAs (0.31 ms here) and the issue slots of the operand pairs' moves.  8 x 4 elements per thread, as 4 x 4
+// made it shared-memory bound (89 % of its wavefronts).  Measured (B200): 2049 bins x 113 mics x 147 windows
+// 821 -> 500 us.
+// With `out` the sums are not added to csm but written, scaled, as the full Hermitian complex128 matrix.
 // ------------------------------------------------------------------------------------------------
-template <bool C64>
-struct GramT {
-    using V = typename std::conditional<C64, float2, double2>::type;
-    using S = typename std::conditional<C64, float, double>::type;
-};
-
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-
 constexpr int GT = 64;   // tile edge
 constexpr int GKC = 16;  // windows per shared-memory stage
+constexpr int GTHREADS = 128;
 
-template <bool C64>
-__global__ void __launch_bounds__(256) gram_kernel(const void *__restrict__ spec_, int M, int64_t nw,
-                                                   void *__restrict__ csm_)
+__device__ __forceinline__ void ffma2(float2 &acc, float ax, float ay, float b)
 {
-    using V = typename GramT<C64>::V;
-    using S = typename GramT<C64>::S;
-    __shared__ V xr_s[GKC][GT];
-    __shared__ V xc_s[GKC][GT];
-    const V *spec = reinterpret_cast<const V *>(spec_);
-    V *csm = reinterpret_cast<V *>(csm_);
+    asm("{\n\t.reg .b64 ra, rb, rc;\n\t"
+        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %4};\n\tmov.b64 rc, {%0, %1};\n\t"
+        "fma.rn.f32x2 rc, ra, rb, rc;\n\tmov.b64 {%0, %1}, rc;\n\t}"
+        : "+f"(acc.x), "+f"(acc.y)
+        : "f"(ax), "f"(ay), "f"(b));
+}
 
+// One stage of `kc` windows into the accumulators.
+template <bool DIAG>
+__device__ __forceinline__ void gram64_stage(const float2 *xr, const float2 *xc, int kc, float2 (&acc)[8][4])
+{
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll 4
+    for (int kk = 0; kk < kc; ++kk) {
+        float2 r[8], c[4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = xr[kk * GT + ty + 8 * i];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j] = xc[kk * GT + tx + 16 * j];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (DIAG && i > 2 * j + 1) continue;
+                ffma2(acc[i][j], c[j].x, -c[j].y, r[i].x);
+                ffma2(acc[i][j], c[j].y, c[j].x, r[i].y);
+            }
+    }
+}
+
+__global__ void __launch_bounds__(GTHREADS, 4) gram_c64_kernel(const float2 *__restrict__ spec, int M, int64_t nw,
+                                                               float2 *__restrict__ csm, double2 *__restrict__ out,
+                                                               double scale)
+{
+    __shared__ float2 g64_sm[2][2][GKC][GT];   // [stage][rows | columns]
     // upper-triangular tile index -> (ti, tj), ti <= tj
     const int T = (M + GT - 1) / GT;
     int t = blockIdx.x, ti = 0;
@@ -625,64 +651,69 @@ __global__ void __launch_bounds__(256) gram_kernel(const void *__restrict__ spec
     const int f = blockIdx.y;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int r0 = ti * GT, c0 = tj * GT;
+    const bool diag = ti == tj;
 
-    S acc_re[4][4], acc_im[4][4];
-    V *base = csm + (int64_t)f * M * M;
+    float2 acc[8][4];
+    float2 *base = csm + (int64_t)f * M * M;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
-            V v = {0, 0};
-            if (r < M && c < M && r <= c) v = base[(int64_t)r * M + c];
-            acc_re[i][j] = v.x;
-            acc_im[i][j] = v.y;
+            const int r = r0 + ty + 8 * i, c = c0 + tx + 16 * j;
+            acc[i][j] = make_float2(0.f, 0.f);
+            if (!out && r < M && c < M && r <= c) acc[i][j] = base[(int64_t)r * M + c];
         }
 
-    const V *sp = spec + (int64_t)f * nw * M;
-    for (int64_t k0 = 0; k0 < nw; k0 += GKC) {
+    const float2 *sp = spec + (int64_t)f * nw * M;
+    const int lm = threadIdx.x & (GT - 1), lk = threadIdx.x / GT;   // this thread's mic and first window of a stage
+    auto load = [&](int64_t k0, int buf) {
+#pragma unroll
+        for (int u = 0; u < GKC; u += GTHREADS / GT) {
+            const int64_t k = k0 + lk + u;
+            const bool in = k < nw;
+            const float2 *src = sp + (in ? k : 0) * M;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&g64_sm[buf][0][lk + u][lm]);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src + min(r0 + lm, M - 1)),
+                         "r"(in && r0 + lm < M ? 8 : 0)
+                         : "memory");
+            if (!diag)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + GKC * GT * 8),
+                             "l"(src + min(c0 + lm, M - 1)), "r"(in && c0 + lm < M ? 8 : 0)
+                             : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load(0, 0);
+    int buf = 0;
+    for (int64_t k0 = 0; k0 < nw; k0 += GKC, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();   // this stage has landed for every thread, and the other buffer is read by none any more
+        if (k0 + GKC < nw) load(k0 + GKC, buf ^ 1);
         const int kc = (int)((nw - k0) < GKC ? (nw - k0) : GKC);
-        for (int idx = threadIdx.x; idx < GKC * GT; idx += blockDim.x) {
-            const int kk = idx / GT, m = idx % GT;
-            V a = {0, 0}, b = {0, 0};
-            if (kk < kc) {
-                if (r0 + m < M) a = sp[(k0 + kk) * M + r0 + m];
-                if (c0 + m < M) b = sp[(k0 + kk) * M + c0 + m];
-            }
-            xr_s[kk][m] = a;
-            xc_s[kk][m] = b;
-        }
-        __syncthreads();
-        for (int kk = 0; kk < kc; ++kk) {
-            V xr[4], xc[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) xr[i] = xr_s[kk][ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) xc[j] = xc_s[kk][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    // temp = conj(X[c]) = (tr, ti); csm += temp * X[r]
-                    const S tr = xc[j].x, tim = -xc[j].y;
-                    acc_re[i][j] = fma_rn(-tim, xr[i].y, fma_rn(tr, xr[i].x, acc_re[i][j]));
-                    acc_im[i][j] = fma_rn(tr, xr[i].y, fma_rn(tim, xr[i].x, acc_im[i][j]));
-                }
-        }
-        __syncthreads();
+        const float2 *xr = &g64_sm[buf][0][0][0];
+        if (diag) gram64_stage<true>(xr, xr, kc, acc);
+        else gram64_stage<false>(xr, xr + GKC * GT, kc, acc);
     }
+    double2 *ob = out + (int64_t)f * M * M;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
-            if (r < M && c < M && r <= c) {
-                V v;
-                v.x = acc_re[i][j];
-                v.y = acc_im[i][j];
-                base[(int64_t)r * M + c] = v;
-            }
+            const int r = r0 + ty + 8 * i, c = c0 + tx + 16 * j;
+            if (r >= M || c >= M || r > c) continue;
+            if (out) put_hermitian(ob, M, r, c, (double)acc[i][j].x, (double)acc[i][j].y, scale);
+            else base[(int64_t)r * M + c] = acc[i][j];
         }
+}
+
+static int gram_c64_launch(const void *spec, int M, int64_t nw, int nbins, void *csm, void *out, double scale,
+                           cudaStream_t s)
+{
+    const int T = (M + GT - 1) / GT;
+    gram_c64_kernel<<<dim3(T * (T + 1) / 2, nbins), GTHREADS, 0, s>>>(
+        reinterpret_cast<const float2 *>(spec), M, nw, reinterpret_cast<float2 *>(csm),
+        reinterpret_cast<double2 *>(out), scale);
+    return check_launch();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -694,7 +725,8 @@ __global__ void __launch_bounds__(256) gram_kernel(const void *__restrict__ spec
 // elements), so this is the reference's order of two chained FMAs per window and component, bit for bit.
 // CTA = 32 x 32 tile of one bin's upper triangle, 4 warps of 16 x 16; 16 windows per stage, three stages of cp.async,
 // four CTAs per SM.  Rows are padded to 36 mics, so that the operand reads of 4 mics x 2 windows (A) and 8 mics x 2
-// windows (B) fall on different banks.  16 x 8 blocks entirely below the diagonal or past M are skipped.
+// windows (B) fall on different banks.  16 x 8 blocks entirely below the diagonal or past M are skipped.  With `out`
+// the sums are not added to csm but written, scaled, as the full Hermitian matrix.
 // Bound: the FP64 pipe (4 M^2 K flop per bin).  Measured (B200): 513 bins x 256 mics x 999 windows 7.84 -> 5.0 ms
 // (27 TFLOP/s; 64 x 64 tiles of 32 x 16 per warp 5.2 ms, half of the diagonal tiles idle); 65 bins x 64 mics x 799
 // windows 281 -> 115 us (195 CTAs where the 64 x 64 tiles of the FMA form were 65).
@@ -713,7 +745,8 @@ __device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], do
 }
 
 __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restrict__ spec, int M, int64_t nw,
-                                                          double2 *__restrict__ csm)
+                                                          double2 *__restrict__ csm, double2 *__restrict__ out,
+                                                          double scale)
 {
     constexpr int T = GF_T, LD = GF_LD, NB = 2;
     extern __shared__ double2 gf_sm[];   // [stage][row mics | column mics][window][LD]
@@ -767,7 +800,7 @@ __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restr
         for (int e = 0; e < 4; ++e) {
             const int r = rw + g + 8 * (e >> 1), c = cb + 2 * t + (e & 1);
             double2 v = make_double2(0.0, 0.0);
-            if (c < M && r <= c) v = base[(int64_t)r * M + c];
+            if (!out && c < M && r <= c) v = base[(int64_t)r * M + c];
             re[j][e] = v.x;
             im[j][e] = v.y;
         }
@@ -811,16 +844,20 @@ __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restr
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int r = rw + g + 8 * (e >> 1), c = cw + 8 * j + 2 * t + (e & 1);
-            if (c < M && r <= c) base[(int64_t)r * M + c] = make_double2(re[j][e], im[j][e]);
+            if (c >= M || r > c) continue;
+            if (out) put_hermitian(out + (int64_t)f * M * M, M, r, c, re[j][e], im[j][e], scale);
+            else base[(int64_t)r * M + c] = make_double2(re[j][e], im[j][e]);
         }
 }
 
-static int gram_f64_launch(const void *spec, int M, int64_t nw, int nbins, void *csm, cudaStream_t s)
+static int gram_f64_launch(const void *spec, int M, int64_t nw, int nbins, void *csm, void *out, double scale,
+                           cudaStream_t s)
 {
     const int T = (M + GF_T - 1) / GF_T;
     cudaFuncSetAttribute(gram_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GF_SMEM);
-    gram_f64_kernel<<<dim3(T * (T + 1) / 2, nbins), 128, GF_SMEM, s>>>(reinterpret_cast<const double2 *>(spec), M, nw,
-                                                                      reinterpret_cast<double2 *>(csm));
+    gram_f64_kernel<<<dim3(T * (T + 1) / 2, nbins), 128, GF_SMEM, s>>>(
+        reinterpret_cast<const double2 *>(spec), M, nw, reinterpret_cast<double2 *>(csm),
+        reinterpret_cast<double2 *>(out), scale);
     return check_launch();
 }
 
@@ -831,7 +868,7 @@ template <bool C64>
 __global__ void __launch_bounds__(256) finalize_kernel(const void *__restrict__ up_, int M, double scale,
                                                        double2 *__restrict__ out)
 {
-    using V = typename GramT<C64>::V;
+    using V = typename std::conditional<C64, float2, double2>::type;
     __shared__ double2 tile[32][33];
     const V *up = reinterpret_cast<const V *>(up_);
     const int f = blockIdx.z;
@@ -1004,16 +1041,14 @@ int acb_calc_csm_c128(void *csm, const void *spec, int num_freqs, int num_mics, 
 {
     if (!csm || !spec) return ACB_ERR_ARG;
     if (num_freqs <= 0 || num_mics <= 0) return ACB_ERR_SHAPE;
-    return gram_f64_launch(spec, num_mics, 1, num_freqs, csm, as_stream(stream));
+    return gram_f64_launch(spec, num_mics, 1, num_freqs, csm, nullptr, 1.0, as_stream(stream));
 }
 
 int acb_calc_csm_c64(void *csm, const void *spec, int num_freqs, int num_mics, void *stream)
 {
     if (!csm || !spec) return ACB_ERR_ARG;
     if (num_freqs <= 0 || num_mics <= 0) return ACB_ERR_SHAPE;
-    const int T = (num_mics + GT - 1) / GT;
-    gram_kernel<true><<<dim3(T * (T + 1) / 2, num_freqs), 256, 0, as_stream(stream)>>>(spec, num_mics, 1, csm);
-    return check_launch();
+    return gram_c64_launch(spec, num_mics, 1, num_freqs, csm, nullptr, 1.0, as_stream(stream));
 }
 
 size_t acb_csm_workspace_bytes(int num_mics, int num_bins, int64_t num_windows, int precision)
@@ -1033,12 +1068,13 @@ size_t acb_csm_workspace_bytes_block(int num_mics, int num_bins, int64_t num_win
     return sc ? (base + 255) / 256 * 256 + sc : base;
 }
 
-int acb_csm_accumulate(const void *samples, int sample_dtype, int64_t num_samples, int num_mics, int block_size,
-                       int hop, int64_t first_window, int64_t num_windows, const double *window,
-                       const void *twiddle, int bin_lo, int num_bins, int precision, void *csm_upper,
+// Windows into sums: added to csm_upper, or, with csm_out, written as the finished matrix (scale applied, Hermitian).
+static int csm_windows(const void *samples, int sample_dtype, int64_t num_samples, int num_mics, int block_size,
+                       int hop, int64_t first_window, int64_t num_windows, const double *window, const void *twiddle,
+                       int bin_lo, int num_bins, int precision, void *csm_upper, double scale, void *csm_out,
                        void *workspace, size_t workspace_bytes, void *stream)
 {
-    if (!samples || !window || !twiddle || !csm_upper) return ACB_ERR_ARG;
+    if (!samples || !window || !twiddle || (!csm_upper && !csm_out)) return ACB_ERR_ARG;
     if (sample_dtype != ACB_F32 && sample_dtype != ACB_F64) return ACB_ERR_ARG;
     const bool tc = precision == ACB_CSM_TC_TF32 || precision == ACB_CSM_TC_BF16X3;
     if (precision != ACB_C128 && precision != ACB_C64 && !tc) return ACB_ERR_ARG;
@@ -1047,7 +1083,7 @@ int acb_csm_accumulate(const void *samples, int sample_dtype, int64_t num_sample
     if (block_size < 16 || (block_size & (block_size - 1))) return ACB_ERR_SHAPE;
     if (block_size > 4 * FFT_MAX_N) return ACB_ERR_UNSUPPORTED;
     if (bin_lo < 0 || num_bins <= 0 || bin_lo + num_bins > block_size / 2 + 1) return ACB_ERR_SHAPE;
-    if (num_windows == 0) return ACB_OK;
+    if (num_windows == 0) return csm_out ? ACB_ERR_SHAPE : ACB_OK;
     if ((first_window + num_windows - 1) * (int64_t)hop + block_size > num_samples) return ACB_ERR_SHAPE;
     if (num_windows > 65535) return ACB_ERR_SHAPE;  // one grid row per window
     const size_t need = acb_csm_workspace_bytes_block(num_mics, num_bins, num_windows, precision, block_size);
@@ -1061,14 +1097,35 @@ int acb_csm_accumulate(const void *samples, int sample_dtype, int64_t num_sample
     const double2 *tw = reinterpret_cast<const double2 *>(twiddle);
     if (tc)
         return csm_tc_accumulate(samples, sample_dtype, num_mics, block_size, hop, first_window, num_windows, window,
-                                 tw, bin_lo, num_bins, precision == ACB_CSM_TC_TF32, csm_upper, workspace, scratch, s);
+                                 tw, bin_lo, num_bins, precision == ACB_CSM_TC_TF32, csm_upper, csm_out, scale,
+                                 workspace, scratch, s);
     int st = fft_launch(samples, sample_dtype, precision == ACB_C64 ? OUT_C64 : OUT_C128, num_mics, block_size, hop,
                         first_window, num_windows, window, tw, bin_lo, num_bins, workspace, 0, 0, 0, scratch, s);
     if (st) return st;
-    if (precision == ACB_C128) return gram_f64_launch(workspace, num_mics, num_windows, num_bins, csm_upper, s);
-    const int T = (num_mics + GT - 1) / GT;
-    gram_kernel<true><<<dim3(T * (T + 1) / 2, num_bins), 256, 0, s>>>(workspace, num_mics, num_windows, csm_upper);
-    return check_launch();
+    auto gram = precision == ACB_C64 ? gram_c64_launch : gram_f64_launch;
+    return gram(workspace, num_mics, num_windows, num_bins, csm_upper, csm_out, scale, s);
+}
+
+int acb_csm_accumulate(const void *samples, int sample_dtype, int64_t num_samples, int num_mics, int block_size,
+                       int hop, int64_t first_window, int64_t num_windows, const double *window,
+                       const void *twiddle, int bin_lo, int num_bins, int precision, void *csm_upper,
+                       void *workspace, size_t workspace_bytes, void *stream)
+{
+    if (!csm_upper) return ACB_ERR_ARG;
+    return csm_windows(samples, sample_dtype, num_samples, num_mics, block_size, hop, first_window, num_windows, window,
+                       twiddle, bin_lo, num_bins, precision, csm_upper, 1.0, nullptr, workspace, workspace_bytes,
+                       stream);
+}
+
+int acb_csm_finished(const void *samples, int sample_dtype, int64_t num_samples, int num_mics, int block_size,
+                     int hop, int64_t first_window, int64_t num_windows, const double *window, const void *twiddle,
+                     int bin_lo, int num_bins, int precision, double scale, void *csm_out, void *workspace,
+                     size_t workspace_bytes, void *stream)
+{
+    if (!csm_out) return ACB_ERR_ARG;
+    return csm_windows(samples, sample_dtype, num_samples, num_mics, block_size, hop, first_window, num_windows, window,
+                       twiddle, bin_lo, num_bins, precision, nullptr, scale, csm_out, workspace, workspace_bytes,
+                       stream);
 }
 
 int acb_csm_finalize(const void *csm_upper, int num_bins, int num_mics, int precision, double scale, void *csm_out,

@@ -19,12 +19,20 @@ size_t fft_scratch_bytes(int num_mics, int block_size, int64_t num_windows);
 // which it does for the tile forms up to blocks of 8192 samples (the FP32 four-window transform).
 bool fft_tiles_written_whole(int block_size);
 
-// Tensor-core Welch accumulation into the complex128 upper triangle (csm_tc.cu).
+// The finished matrix's entries (r, c), r <= c, and (c, r) from the sum (x, y): what finalize_kernel writes.
+__device__ __forceinline__ void put_hermitian(double2 *out, int M, int r, int c, double x, double y, double scale)
+{
+    out[(int64_t)r * M + c] = make_double2(x * scale, y * scale);
+    if (r != c) out[(int64_t)c * M + r] = make_double2(x * scale, -y * scale);
+}
+
+// Tensor-core Welch accumulation into the complex128 upper triangle, or, with csm_out, straight into the finished
+// matrix (csm_tc.cu).
 int csm_tc_row_tiles(int num_mics);
 size_t csm_tc_workspace_bytes(int num_mics, int num_bins, int64_t num_windows);
 int csm_tc_accumulate(const void *samples, int sample_dtype, int num_mics, int block_size, int hop,
                       int64_t first_window, int64_t num_windows, const double *window, const double2 *tw,
-                      int bin_lo, int num_bins, bool tf32, void *csm_upper, void *workspace, void *fft_scratch,
-                      cudaStream_t s);
+                      int bin_lo, int num_bins, bool tf32, void *csm_upper, void *csm_out, double scale,
+                      void *workspace, void *fft_scratch, cudaStream_t s);
 
 }  // namespace acb

@@ -52,7 +52,9 @@ struct GtcArgs {
     int64_t lo_bytes;          // BF16: byte offset of the lo tiles from the hi tiles
     int R, KC, M, nbins, nper;
     int64_t nitems;
-    double2 *csm;              // complex128 [nbins][M][M], upper triangle accumulated
+    double2 *csm;              // complex128 [nbins][M][M], upper triangle accumulated (out null)
+    double2 *out;              // or the finished matrix, scaled and Hermitian
+    double scale;
     uint64_t wait_limit_ns;
     GtcItem it[GTC_MAX_ITEMS];
 };
@@ -209,6 +211,7 @@ __global__ void __launch_bounds__(GTC_THREADS, 1) gram_tc_kernel(const __grid_co
             tc::tc_fence_after();
             const int r = (GTC_ROWT * 32 * g.rb + rho) >> 1;   // mic of this row
             double2 *crow = a.csm + ((int64_t)bin * a.M + r) * a.M;
+            double2 *obin = a.out + (int64_t)bin * a.M * a.M;
             for (int j = 0; j < g.nc; ++j) {
                 float v[32], w[32];
                 tc::tmem_ld_x32(taddr + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 256 + 32 * j), v);
@@ -224,12 +227,14 @@ __global__ void __launch_bounds__(GTC_THREADS, 1) gram_tc_kernel(const __grid_co
                     const float dim_im = p ? v[2 * (t2 + 8) + 1] : w[2 * t2 + 1];      // D[2r+1][2c+1]
                     const int c = cb + t2;
                     if (r < a.M && c < a.M && c >= r) {
-                        double2 cur = crow[c];
+                        double2 cur = make_double2(0.0, 0.0);
+                        if (!a.out) cur = crow[c];
                         cur.x += (double)dre_re + (double)dim_im;
                         // the diagonal sum_w |X_w[r]|^2 is real; its two mirrored accumulator
                         // entries differ by FP32 rounding only
                         if (c != r) cur.y += (double)dim_re - (double)dre_im;
-                        crow[c] = cur;
+                        if (a.out) put_hermitian(obin, a.M, r, c, cur.x, cur.y, a.scale);
+                        else crow[c] = cur;
                     }
                 }
             }
@@ -257,8 +262,8 @@ size_t csm_tc_workspace_bytes(int num_mics, int num_bins, int64_t num_windows)
 
 int csm_tc_accumulate(const void *samples, int sample_dtype, int num_mics, int block_size, int hop,
                       int64_t first_window, int64_t num_windows, const double *window, const double2 *tw,
-                      int bin_lo, int num_bins, bool tf32, void *csm_upper, void *workspace, void *fft_scratch,
-                      cudaStream_t s)
+                      int bin_lo, int num_bins, bool tf32, void *csm_upper, void *csm_out, double scale,
+                      void *workspace, void *fft_scratch, cudaStream_t s)
 {
     const int R = csm_tc_row_tiles(num_mics);
     const int KC = (int)((num_windows + 31) / 32);
@@ -296,6 +301,8 @@ int csm_tc_accumulate(const void *samples, int sample_dtype, int num_mics, int b
     a.nper = n;
     a.nitems = (int64_t)n * num_bins;
     a.csm = reinterpret_cast<double2 *>(csm_upper);
+    a.out = reinterpret_cast<double2 *>(csm_out);
+    a.scale = scale;
     a.wait_limit_ns = tc_wait_limit_ns();
     int dev = 0, nsm = kNumSMs;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

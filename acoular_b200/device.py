@@ -79,6 +79,37 @@ def window_vector(window: str, block_size: int, device) -> tuple[torch.Tensor, f
 CSM_PRECISIONS = {'complex128': N.C128, 'complex64': N.C64, 'tc_tf32': N.CSM_TC_TF32, 'tc_bf16x3': N.CSM_TC_BF16X3}
 
 
+def _samples_shape(samples: torch.Tensor):
+    if samples.dim() != 2 or not samples.is_contiguous():
+        msg = 'samples must be a contiguous (num_samples, num_mics) tensor'
+        raise ValueError(msg)
+    return samples.shape
+
+
+def _csm_inputs(samples: torch.Tensor, block_size: int, window: str, overlap: str, precision: str, num_bins: int,
+                windows: int, max_workspace_bytes: int):
+    """What the CSM entries take: (samples, their dtype code, hop, window, twiddles, precision code, windows per
+    chunk, workspace bytes of a chunk)."""
+    dev = samples.device
+    M = samples.shape[1]
+    prec = CSM_PRECISIONS[precision]
+    if samples.dtype not in (torch.float32, torch.float64):
+        samples = samples.to(torch.float64)
+    sd = N.F32 if samples.dtype == torch.float32 else N.F64
+    wv, _ = window_vector(window, block_size, dev)
+    tw = twiddles(block_size, dev)
+    size = N.lib().acb_csm_workspace_bytes_block
+    if prec in (N.CSM_TC_TF32, N.CSM_TC_BF16X3):
+        # the tensor-core operand pads every chunk to whole blocks of 32 windows
+        per32 = size(M, num_bins, 32, prec, block_size)
+        chunk = int(max(32, min(65504, max_workspace_bytes // max(per32, 1) * 32)))
+        chunk = min(chunk, -(-max(windows, 1) // 32) * 32)
+    else:
+        per_win = size(M, num_bins, 1, prec, block_size)
+        chunk = int(max(1, min(65535, max_workspace_bytes // max(per_win, 1), windows if windows > 0 else 1)))
+    return samples, sd, block_size // OVERLAPS[overlap], wv, tw, prec, chunk, size(M, num_bins, chunk, prec, block_size)
+
+
 def csm_upper_accumulate(samples: torch.Tensor, block_size: int, window: str, overlap: str,
                          precision: str = 'complex128', bin_lo: int = 0, num_bins: int | None = None,
                          csm_upper: torch.Tensor | None = None, workspace: torch.Tensor | None = None,
@@ -91,38 +122,16 @@ def csm_upper_accumulate(samples: torch.Tensor, block_size: int, window: str, ov
     Gram: TF32 or split-BF16 operands, FP32 accumulation per chunk of windows, complex128 sums).
     Returns ``(csm_upper, n_windows)``; ``csm_upper`` is (num_bins, M, M) complex128/complex64.
     """
-    dev = samples.device
-    if samples.dim() != 2 or not samples.is_contiguous():
-        msg = 'samples must be a contiguous (num_samples, num_mics) tensor'
-        raise ValueError(msg)
-    S, M = samples.shape
-    ov = OVERLAPS[overlap]
-    hop = block_size // ov
-    F = block_size // 2 + 1
-    nb = F - bin_lo if num_bins is None else num_bins
-    prec = CSM_PRECISIONS[precision]
-    cdt = torch.complex64 if prec == N.C64 else torch.complex128
+    S, M = _samples_shape(samples)
+    nb = block_size // 2 + 1 - bin_lo if num_bins is None else num_bins
+    K = num_windows(S, block_size, OVERLAPS[overlap]) if windows is None else windows
+    samples, sd, hop, wv, tw, prec, chunk, need = _csm_inputs(samples, block_size, window, overlap, precision, nb, K,
+                                                              max_workspace_bytes)
     if csm_upper is None:
-        csm_upper = torch.zeros((nb, M, M), dtype=cdt, device=dev)
-    K = num_windows(S, block_size, ov) if windows is None else windows
-    sd = N.F32 if samples.dtype == torch.float32 else N.F64
-    if samples.dtype not in (torch.float32, torch.float64):
-        samples = samples.to(torch.float64)
-        sd = N.F64
-    wv, _ = window_vector(window, block_size, dev)
-    tw = twiddles(block_size, dev)
-    if prec in (N.CSM_TC_TF32, N.CSM_TC_BF16X3):
-        # the tensor-core operand pads every chunk to whole blocks of 32 windows
-        per32 = N.lib().acb_csm_workspace_bytes_block(M, nb, 32, prec, block_size)
-        chunk = int(max(32, min(65504, max_workspace_bytes // max(per32, 1) * 32)))
-        chunk = min(chunk, -(-max(K, 1) // 32) * 32)
-        need = N.lib().acb_csm_workspace_bytes_block(M, nb, chunk, prec, block_size)
-    else:
-        per_win = N.lib().acb_csm_workspace_bytes_block(M, nb, 1, prec, block_size)
-        chunk = int(max(1, min(65535, max_workspace_bytes // max(per_win, 1), K if K > 0 else 1)))
-        need = N.lib().acb_csm_workspace_bytes_block(M, nb, chunk, prec, block_size)
+        cdt = torch.complex64 if prec == N.C64 else torch.complex128
+        csm_upper = torch.zeros((nb, M, M), dtype=cdt, device=samples.device)
     if workspace is None or workspace.numel() < need:
-        workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+        workspace = torch.empty(need, dtype=torch.uint8, device=samples.device)
     st = N.stream_handle()
     L = N.lib()
     w = first_window
@@ -134,6 +143,32 @@ def csm_upper_accumulate(samples: torch.Tensor, block_size: int, window: str, ov
                                      workspace.numel(), st), 'acb_csm_accumulate')
         w += nw
     return csm_upper, K
+
+
+def csm_finished(samples: torch.Tensor, block_size: int, window: str, overlap: str, precision: str, scale: float,
+                 bin_lo: int = 0, num_bins: int | None = None, out: torch.Tensor | None = None,
+                 workspace: torch.Tensor | None = None,
+                 max_workspace_bytes: int = DEFAULT_WORKSPACE_BYTES) -> torch.Tensor:
+    """The finished CSM (num_bins, M, M) complex128, ``scale`` applied: in one pass where the windows fit one
+    workspace, else (or without a complete window) the accumulated upper triangle and :func:`csm_finalize`; the same
+    bits either way."""
+    S, M = _samples_shape(samples)
+    nb = block_size // 2 + 1 - bin_lo if num_bins is None else num_bins
+    K = num_windows(S, block_size, OVERLAPS[overlap])
+    samples, sd, hop, wv, tw, prec, chunk, need = _csm_inputs(samples, block_size, window, overlap, precision, nb, K,
+                                                              max_workspace_bytes)
+    if out is None:
+        out = torch.empty((nb, M, M), dtype=torch.complex128, device=samples.device)
+    if not 0 < K <= chunk:
+        up, _ = csm_upper_accumulate(samples, block_size, window, overlap, precision, bin_lo, nb, workspace=workspace,
+                                     max_workspace_bytes=max_workspace_bytes)
+        return csm_finalize(up, scale, out=out)
+    if workspace is None or workspace.numel() < need:
+        workspace = torch.empty(need, dtype=torch.uint8, device=samples.device)
+    N.check(N.lib().acb_csm_finished(samples.data_ptr(), sd, S, M, block_size, hop, 0, K, wv.data_ptr(), tw.data_ptr(),
+                                     bin_lo, nb, prec, float(scale), out.data_ptr(), workspace.data_ptr(),
+                                     workspace.numel(), N.stream_handle()), 'acb_csm_finished')
+    return out
 
 
 _copy_streams: dict = {}
@@ -163,14 +198,12 @@ def calc_csm(samples: torch.Tensor, block_size: int = 1024, window: str = 'Recta
              precision: str = 'complex128', bin_lo: int = 0, num_bins: int | None = None,
              max_workspace_bytes: int = DEFAULT_WORKSPACE_BYTES) -> torch.Tensor:
     """Full CSM (num_bins, M, M) complex128 on the device, as ``PowerSpectra.calc_csm`` returns it."""
-    ov = OVERLAPS[overlap]
-    up, _ = csm_upper_accumulate(samples, block_size, window, overlap, precision, bin_lo, num_bins,
-                                 max_workspace_bytes=max_workspace_bytes)
     _, weight = window_vector(window, block_size, samples.device)
-    nblk = num_blocks(samples.shape[0], block_size, ov)
+    nblk = num_blocks(samples.shape[0], block_size, OVERLAPS[overlap])
     with np.errstate(divide='ignore', invalid='ignore'):
         scale = np.float64(2.0 / block_size) / np.float64(weight) / np.float64(nblk)
-    return csm_finalize(up, float(scale))
+    return csm_finished(samples, block_size, window, overlap, precision, float(scale), bin_lo, num_bins,
+                        max_workspace_bytes=max_workspace_bytes)
 
 
 # ------------------------------------------------------------------------------------------------

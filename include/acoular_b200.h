@@ -86,6 +86,14 @@ int acb_csm_accumulate(const void *samples, int sample_dtype, int64_t num_sample
                        int precision, void *csm_upper, void *workspace, size_t workspace_bytes,
                        void *stream);
 
+/* acb_csm_accumulate of one chunk into zeros and acb_csm_finalize in one: the same matrix, bit for bit, without the
+ * clearing, the accumulation buffer and the finalising pass.  For requests whose windows all fit one workspace;
+ * num_windows >= 1.  csm_out: complex128 [num_bins][num_mics][num_mics]. */
+int acb_csm_finished(const void *samples, int sample_dtype, int64_t num_samples, int num_mics, int block_size,
+                     int hop, int64_t first_window, int64_t num_windows, const double *window, const void *twiddle,
+                     int bin_lo, int num_bins, int precision, double scale, void *csm_out, void *workspace,
+                     size_t workspace_bytes, void *stream);
+
 /* Hermitian completion and scaling (acoular/spectra.py:411-416):
  *   csm_out[f, r, c] = scale * (r <= c ? upper[f, r, c] : conj(upper[f, c, r]))
  * upper in `precision`; csm_out always complex128 (as the reference returns). */
