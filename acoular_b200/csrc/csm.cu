@@ -151,6 +151,11 @@ __device__ __forceinline__ void first_stages(double2 (&v)[8])
     butterfly(v[3], v[7], make_double2(-h, -h));
 }
 
+// Blocks from this size on take wide CTAs (more mics, 512 threads; see fft_mics_per_block and fft4_mics_per_block).
+// (Measured, CSM of 256 mics x 300,000 samples, block 8192, complex64: 6.29 -> 5.52 ms; 113 mics, block 2048: 0.93 ->
+// 0.91; block 512, 256 mics: 2.53 -> 2.65, so not below 2048.)
+constexpr int FFT_WIDE_N = 2048;
+
 // Output forms of the spectra (OUT): complex128 or complex64 [bin][window][mic] for the FP64 /
 // FP32 Gram; or the tensor-core Gram's operand tiles, TF32 (OUT_TF32) or split BF16 hi + lo
 // (OUT_BF16), 32 x 32 tiles [bin][window/32][component/32] with component 2m = Re, 2m + 1 = Im of
@@ -253,6 +258,10 @@ __global__ void __launch_bounds__(512) fft_window_kernel(const TS *__restrict__ 
 // The tile layout is K-major: a 16-byte core-matrix row holds 4 consecutive windows (TF32) or 8
 // (BF16) of one spectrum component, so a CTA that transforms 4 consecutive windows of `mpb` mics
 // stores whole 16-byte rows (TF32) or half rows (BF16) instead of one 4-byte value per window.
+// Bound: shared-memory wavefronts (81 % of their rate): three passes' worth of 8-byte accesses and the split's.  The
+// first three stages run on the points as they are loaded, and a thread keeps its task's twiddles over the sequences.
+// Measured (B200): 999 windows x 256 mics x 1024 samples to TF32 tiles 1.06 -> 0.92 ms; CSM of 64 mics x 300,000
+// samples, block 4096: 0.56 -> 0.36 ms (wide CTAs).
 // The transform runs in FP32 (the operands are rounded to TF32 or split into BF16 hi + lo right
 // after it, so FP64 arithmetic buys nothing): complex points are 8 bytes, half the shared-memory
 // traffic of the FP64 transform.  Padded windows (>= the chunk's count, up to 32 KC) and padded
@@ -270,33 +279,33 @@ __host__ __device__ constexpr int fft_stride_f(int H, int mpb)
     return H + (H >> 4) + ((((32 / mpb) & 15) - (H + (H >> 4))) & 15);
 }
 
-// s (1..3) consecutive radix-2 DIT stages, the first of length 2^(sg + 1), on a bit-reversed FP32
-// sequence (see fft_pass).  The twiddles come from a shared-memory table in stage order: the stage of
-// length L = 2 hf reads W_L^i (i < hf) at tws[hf + i], so consecutive threads read consecutive
-// entries (the natural-order table read with the stride N / L put up to 16 threads on one bank).  The
-// entries are the FP32 roundings of the same W_N^e as the natural-order table.  All lengths are powers
-// of two, so the index arithmetic is shifts and masks.
+// s (1..3) consecutive radix-2 DIT stages, the first of length 2 half1, on the 2^s points of a task (see fft_pass).
+// The twiddles come from a shared-memory table in stage order: the stage of length L = 2 hf reads W_L^i (i < hf) at
+// tws[hf + i], so consecutive threads read consecutive entries (the natural-order table read with the stride N / L put
+// up to 16 threads on one bank).  The entries are the FP32 roundings of the same W_N^e as the natural-order table.
+// A task's twiddle at stage q is entry (task mod half1) + (t mod 2^q) half1 of the stage's table: 2^q distinct values.
 template <int S>
-__device__ __forceinline__ void fft_pass_f(float2 *__restrict__ z, int sg, int task, const float2 *__restrict__ tws)
+struct PassTwiddlesF {
+    float2 w[(1 << S) - 1];   // stage q at 2^q - 1 + u
+    __device__ __forceinline__ void load(int sg, int task, const float2 *__restrict__ tws)
+    {
+        const int half1 = 1 << sg, tb = task & (half1 - 1);
+#pragma unroll
+        for (int q = 0; q < S; ++q)
+#pragma unroll
+            for (int u = 0; u < (1 << q); ++u) w[(1 << q) - 1 + u] = tws[(half1 << q) + tb + u * half1];
+    }
+};
+
+template <int S>
+__device__ __forceinline__ void stages_f(float2 (&v)[1 << S], const PassTwiddlesF<S> &tw)
 {
-    const int half1 = 1 << sg;
-    const int base = ((task >> sg) << (sg + S)) + (task & (half1 - 1));
-    float2 v[1 << S];
 #pragma unroll
-    for (int t = 0; t < (1 << S); ++t) v[t] = z[zpf(base + t * half1)];
-    // the twiddle of point base + t half1 at stage q is entry (task mod half1) + (t mod 2^q) half1 of the
-    // stage's table: 2^q distinct values, each read once
-    const int tb = task & (half1 - 1);
-#pragma unroll
-    for (int q = 0; q < S; ++q) {
-        const int hf = half1 << q;                       // half the stage length L = 2^(sg + 1 + q)
-        float2 wq[1 << (S - 1)];
-#pragma unroll
-        for (int u = 0; u < (1 << q); ++u) wq[u] = tws[hf + tb + u * half1];
+    for (int q = 0; q < S; ++q)
 #pragma unroll
         for (int t = 0; t < (1 << S); ++t) {
             if (t & (1 << q)) continue;
-            const float2 w = wq[t & ((1 << q) - 1)];
+            const float2 w = tw.w[(1 << q) - 1 + (t & ((1 << q) - 1))];
             const float2 b = v[t + (1 << q)];
             const float br = b.x * w.x - b.y * w.y;
             const float bi = b.x * w.y + b.y * w.x;
@@ -304,9 +313,30 @@ __device__ __forceinline__ void fft_pass_f(float2 *__restrict__ z, int sg, int t
             v[t] = make_float2(a.x + br, a.y + bi);
             v[t + (1 << q)] = make_float2(a.x - br, a.y - bi);
         }
-    }
+}
+
+// One pass over `nseq` sequences: a thread keeps one task and its twiddles and walks the sequences.
+template <int S>
+__device__ __forceinline__ void fft_pass_f(float2 *__restrict__ zs, int nseq, int st, int sg, int logH,
+                                           const float2 *__restrict__ tws)
+{
+    const int logT = logH - S, T = 1 << logT, nt = blockDim.x, half1 = 1 << sg;
+    const int grp = T < nt ? threadIdx.x >> logT : 0, ngrp = T < nt ? nt >> logT : 1;
+    for (int task = T < nt ? threadIdx.x & (T - 1) : threadIdx.x; task < T; task += nt) {
+        const int base = ((task >> sg) << (sg + S)) + (task & (half1 - 1));
+        PassTwiddlesF<S> w;
+        w.load(sg, task, tws);
+        for (int q = grp; q < nseq; q += ngrp) {
+            float2 *z = zs + q * st;
+            float2 v[1 << S];
 #pragma unroll
-    for (int t = 0; t < (1 << S); ++t) z[zpf(base + t * half1)] = v[t];
+            for (int t = 0; t < (1 << S); ++t) v[t] = z[zpf(base + t * half1)];
+            stages_f<S>(v, w);
+#pragma unroll
+            for (int t = 0; t < (1 << S); ++t) z[zpf(base + t * half1)] = v[t];
+        }
+    }
+    __syncthreads();
 }
 
 constexpr int FFT4_WIN = 4;   // windows per CTA
@@ -344,45 +374,63 @@ __device__ __forceinline__ void ld_row(const double *__restrict__ p, float (&x)[
     }
 }
 
-// Load, window and bit-reversed placement of the CTA's 4 windows x mpb mics: one thread per (window,
-// group of V mics, point j), j fastest, so that a warp's stores into the bit-reversed slots of one
-// sequence spread over the banks, and each thread loads rows 2j and 2j + 1 as one vector of V mics.
-// Windows past the chunk and padding mics are zeros (M % V == 0: a group is all in or all out).
+// Load, window and the first three stages of the CTA's 4 windows x mpb mics: one thread per (window, group of V mics,
+// task), the task fastest.  A task is 8 consecutive slots of the bit-reversed order, i.e. points rev(task) + H/8
+// {0, 4, 2, 6, 1, 5, 3, 7}; the thread loads rows 2j and 2j + 1 of each as one vector of V mics.  Windows past the
+// chunk and padding mics are zeros (M % V == 0: a group is all in or all out).
 template <typename TS, int V>
 __device__ __forceinline__ void fft4_load(const TS *__restrict__ samples, int M, int hop, int64_t w0, int64_t nw,
                                           int wg, int m0, int mpb, int H, int logH, int st,
-                                          const float *__restrict__ wf, float2 *__restrict__ zs)
+                                          const float *__restrict__ wf, const float2 *__restrict__ tws,
+                                          float2 *__restrict__ zs)
 {
     constexpr int logV = V == 4 ? 2 : (V == 2 ? 1 : 0);
     int logG = 0;
     while ((V << logG) < mpb) ++logG;                          // mpb / V groups
-    const int total = FFT4_WIN * H << logG;
-#pragma unroll 4
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        const int j = idx & (H - 1);
-        const int mg = (idx >> logH) & ((1 << logG) - 1);
-        const int wi = idx >> (logH + logG);
+    const int logT = logH - 3;
+    PassTwiddlesF<3> w3;
+    w3.load(0, 0, tws);
+    for (int idx = threadIdx.x; idx < (FFT4_WIN << logG) << logT; idx += blockDim.x) {
+        const int task = idx & ((1 << logT) - 1);
+        const int mg = (idx >> logT) & ((1 << logG) - 1);
+        const int wi = idx >> (logT + logG);
         const int64_t w = (int64_t)wg * FFT4_WIN + wi;
         const int m = m0 + (mg << logV);
-        float x0[V], x1[V];
-        if (w < nw && m < M) {
-            const TS *src = samples + ((w0 + w) * (int64_t)hop + 2 * j) * M + m;
-            ld_row<V>(src, x0);
-            ld_row<V>(src + M, x1);
-        } else {
+        const int j0 = logT ? (int)(__brev((unsigned)task) >> (32 - logT)) : 0;
+        float x0[8][V], x1[8][V];
+        const bool in = w < nw && m < M;
+        const TS *src = samples + ((w0 + w) * (int64_t)hop) * M + m;
 #pragma unroll
-            for (int e = 0; e < V; ++e) x0[e] = x1[e] = 0.f;
+        for (int t = 0; t < 8; ++t) {
+            const int j = j0 + ((((t & 1) << 2) | (t & 2) | (t >> 2)) << logT);
+            if (in) {
+                ld_row<V>(src + (int64_t)(2 * j) * M, x0[t]);
+                ld_row<V>(src + (int64_t)(2 * j + 1) * M, x1[t]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < V; ++e) x0[t][e] = x1[t][e] = 0.f;
+            }
         }
-        const float a0 = wf[2 * j], a1 = wf[2 * j + 1];
-        const int jr = logH ? (int)(__brev((unsigned)j) >> (32 - logH)) : 0;
-        float2 *z = zs + (wi * mpb + (mg << logV)) * st + zpf(jr);
+        float2 a[8];
 #pragma unroll
-        for (int e = 0; e < V; ++e) z[e * st] = make_float2(x0[e] * a0, x1[e] * a1);
+        for (int t = 0; t < 8; ++t)
+            a[t] = *reinterpret_cast<const float2 *>(wf + 2 * (j0 + ((((t & 1) << 2) | (t & 2) | (t >> 2)) << logT)));
+        float2 *z = zs + (wi * mpb + (mg << logV)) * st;
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            float2 v[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) v[t] = make_float2(__fmul_rn(x0[t][e], a[t].x), __fmul_rn(x1[t][e], a[t].y));
+            stages_f<3>(v, w3);
+#pragma unroll
+            for (int t = 0; t < 8; ++t) z[e * st + zpf(8 * task + t)] = v[t];
+        }
     }
+    __syncthreads();
 }
 
 template <typename TS, int OUT>
-__global__ void __launch_bounds__(256) fft4_tc_kernel(const TS *__restrict__ samples, int M, int N, int hop, int64_t w0,
+__global__ void __launch_bounds__(512) fft4_tc_kernel(const TS *__restrict__ samples, int M, int N, int hop, int64_t w0,
                                                       int64_t nw, int mpb, int vw, const double *__restrict__ window,
                                                       const double2 *__restrict__ tw, int bin_lo, int nbins,
                                                       void *__restrict__ out, int R, int KC, int64_t lo_elems)
@@ -407,24 +455,16 @@ __global__ void __launch_bounds__(256) fft4_tc_kernel(const TS *__restrict__ sam
     for (int i = threadIdx.x; i < N; i += blockDim.x) wf[i] = (float)window[i];
     __syncthreads();
 
-    if (vw == 4) fft4_load<TS, 4>(samples, M, hop, w0, nw, wg, m0, mpb, H, logH, st, wf, zs);
-    else if (vw == 2) fft4_load<TS, 2>(samples, M, hop, w0, nw, wg, m0, mpb, H, logH, st, wf, zs);
-    else fft4_load<TS, 1>(samples, M, hop, w0, nw, wg, m0, mpb, H, logH, st, wf, zs);
-    __syncthreads();
+    if (vw == 4) fft4_load<TS, 4>(samples, M, hop, w0, nw, wg, m0, mpb, H, logH, st, wf, tws, zs);
+    else if (vw == 2) fft4_load<TS, 2>(samples, M, hop, w0, nw, wg, m0, mpb, H, logH, st, wf, tws, zs);
+    else fft4_load<TS, 1>(samples, M, hop, w0, nw, wg, m0, mpb, H, logH, st, wf, tws, zs);
 
-    // radix-2 DIT stages, up to three per pass, over all 4 mpb sequences
-    const int nseq = FFT4_WIN * mpb;
-    for (int sg = 0; sg < logH;) {
+    // the other stages, up to three per pass, over all 4 mpb sequences
+    for (int sg = 3; sg < logH;) {
         const int S = logH - sg >= 3 ? 3 : logH - sg;
-        const int logT = logH - S;                                 // H / 2^S tasks per sequence
-        for (int idx = threadIdx.x; idx < nseq << logT; idx += blockDim.x) {
-            const int q = idx >> logT;
-            const int task = idx & ((1 << logT) - 1);
-            if (S == 3) fft_pass_f<3>(zs + q * st, sg, task, tws);
-            else if (S == 2) fft_pass_f<2>(zs + q * st, sg, task, tws);
-            else fft_pass_f<1>(zs + q * st, sg, task, tws);
-        }
-        __syncthreads();
+        if (S == 3) fft_pass_f<3>(zs, FFT4_WIN * mpb, st, sg, logH, tws);
+        else if (S == 2) fft_pass_f<2>(zs, FFT4_WIN * mpb, st, sg, logH, tws);
+        else fft_pass_f<1>(zs, FFT4_WIN * mpb, st, sg, logH, tws);
         sg += S;
     }
 
@@ -483,14 +523,18 @@ __global__ void __launch_bounds__(256) fft4_tc_kernel(const TS *__restrict__ sam
     }
 }
 
-// Mics per CTA of fft4_tc_kernel: about 72 KB of FP32 sequences (2 to 3 CTAs per SM), power of two
-// <= 16 (so that the 16 R padded mics split evenly); 0 if even one mic's 4 windows do not fit.
+// Mics per CTA of fft4_tc_kernel (a power of two <= 16, so that the 16 R padded mics split evenly) and its threads: up
+// to 72 KB of FP32 sequences and 256 threads; for blocks of 2048 samples and more, of which that would hold one or two
+// mics and load 4 or 8 bytes of a row at a time, up to 148 KB and 512 threads.  0 mics if even one mic's 4 windows do
+// not fit.
+static int fft4_threads(int N) { return N >= FFT_WIDE_N ? 512 : 256; }
 static int fft4_mics_per_block(int N)
 {
     const size_t tables = (size_t)(N / 2) * sizeof(float2) + (size_t)N * sizeof(float);
     if ((size_t)FFT4_WIN * fft_stride_f(N / 2, 1) * sizeof(float2) + tables >= 200 * 1024) return 0;
+    const size_t most = (N >= FFT_WIDE_N ? 148 : 72) * 1024;
     int mpb = 16;
-    while (mpb > 1 && (size_t)mpb * FFT4_WIN * fft_stride_f(N / 2, mpb) * sizeof(float2) > 72 * 1024) mpb >>= 1;
+    while (mpb > 1 && (size_t)mpb * FFT4_WIN * fft_stride_f(N / 2, mpb) * sizeof(float2) > most) mpb >>= 1;
     return mpb;
 }
 
@@ -912,9 +956,6 @@ __global__ void __launch_bounds__(256) finalize_kernel(const void *__restrict__ 
 // three CTAs share an SM and hide each other's barriers and FP64 latency; for blocks of FFT_WIDE_N samples and more, of
 // which that would hold one or two mics and store 16 bytes of a row of complex64 spectra at a time, up to 150 KB and
 // 512 threads.
-// (Measured, CSM of 256 mics x 300,000 samples, block 8192, complex64: 6.29 -> 5.52 ms; 113 mics, block 2048: 0.93 ->
-// 0.91; block 512, 256 mics: 2.53 -> 2.65, so not below 2048.)
-constexpr int FFT_WIDE_N = 2048;
 static int fft_threads(int N) { return N >= FFT_WIDE_N ? 512 : 256; }
 static int fft_mics_per_block(int N)
 {
@@ -965,18 +1006,21 @@ int fft_launch(const void *samples, int sample_dtype, int out_form, int num_mics
             // every tile row (16 R padded mics) and column (32 KC padded windows) is written
             const dim3 g4((unsigned)(R * 16 / mpb4), (unsigned)(KC * 32 / FFT4_WIN));
             const size_t smem4 = fft4_smem_bytes(block_size, mpb4);
-            // vector width of the sample loads: V mics of a row at once where M and the base allow it
+            // vector width of the sample loads: V mics of a row at once where M and the base allow it; 16 bytes at
+            // most for blocks of 128, whose tasks at 4 doubles would leave half the threads idle (64 mics: 229 us
+            // for 300,000 samples, 210 at 2)
             const size_t es = sample_dtype == ACB_F32 ? 4 : 8;
             int vw = 1;
             for (int v = 4; v >= 2 && vw == 1; v >>= 1)
-                if (v <= mpb4 && num_mics % v == 0 && reinterpret_cast<uintptr_t>(samples) % (v * es < 16 ? v * es : 16) == 0)
+                if (v <= mpb4 && num_mics % v == 0 && (v * es <= 16 || block_size >= 256) &&
+                    reinterpret_cast<uintptr_t>(samples) % (v * es < 16 ? v * es : 16) == 0)
                     vw = v;
 #define ACB_FFT4_LAUNCH(TS, OF)                                                                                     \
     do {                                                                                                            \
         auto kern = fft4_tc_kernel<TS, OF>;                                                                         \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4);                        \
-        kern<<<g4, 256, smem4, s>>>(reinterpret_cast<const TS *>(samples), num_mics, block_size, hop, first_window,  \
-                                    num_windows, mpb4, vw, window, tw, bin_lo, num_bins, out, R, KC, lo_elems);    \
+        kern<<<g4, fft4_threads(block_size), smem4, s>>>(reinterpret_cast<const TS *>(samples), num_mics, block_size,   \
+                                    hop, first_window, num_windows, mpb4, vw, window, tw, bin_lo, num_bins, out, R, KC, lo_elems);    \
     } while (0)
             if (sample_dtype == ACB_F32) {
                 if (out_form == OUT_TF32) ACB_FFT4_LAUNCH(float, OUT_TF32);
