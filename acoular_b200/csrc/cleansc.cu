@@ -21,8 +21,12 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "map_internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace acb {
 
@@ -86,54 +90,68 @@ __device__ __forceinline__ double2 cdiv(double2 x, double2 y)
 // quadratic form equals the steering type's map: v_m = e^{-i fl32(k r_m)} (times r_m for 'inverse',
 // over r_m for 'true level' / 'true location'; the map kernel's synthesis), divided by M (classic),
 // M r0 (inverse), r0 S (true level) or sqrt(M S) (true location), S = sum r^2 or sum 1/r^2.
-// One warp per grid point, lanes over the mics; out (B, G, M).
+// One warp per grid point, lanes over the mics; out (B, G, M), or with MIC_MAJOR (B, M, G): a warp then takes four of
+// its CTA's 32 points, which go out through a shared-memory tile [M][33].
+template <bool MIC_MAJOR>
 __global__ void __launch_bounds__(256) cleansc_steer_kernel(CscArgs a, double2 *__restrict__ out)
 {
-    const int lane = threadIdx.x & 31;
-    const int64_t g = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    extern __shared__ double2 st_sm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int b = blockIdx.y;
-    if (g >= a.G) return;
     const int M = a.M;
     const double k = a.k[b];
-    double gx = 0, gy = 0, gz = 0, r0;
-    if (a.rm) {
-        r0 = a.r0[g];
-    } else {
-        gx = a.gpos[g];
-        gy = a.gpos[a.G + g];
-        gz = a.gpos[2 * a.G + g];
-        r0 = a.ref_mode == 1 ? a.ref_dist : dist3(gx, gy, gz, a.ref0, a.ref1, a.ref2);
-    }
-    double2 *o = out + ((int64_t)b * a.G + g) * M;
     const SincosTable sct = sincos_table(a.table, a.mask, a.faithful != 0);
-    double S = 0.0;
-    for (int m = lane; m < M; m += 32) {
-        const double r = a.rm ? a.rm[g * M + m] : dist3(gx, gy, gz, a.mpos[m], a.mpos[M + m], a.mpos[2 * M + m]);
-        const float arg = __double2float_rn(__dmul_rn(k, r));
-        float c, sn;
-        sincos_f32_arg(arg, sct, c, sn);
-        double2 v = make_double2((double)c, -(double)sn);
-        if (a.steer_type == 2) {
-            v.x = __dmul_rn(v.x, r);
-            v.y = __dmul_rn(v.y, r);
-            S += r * r;
-        } else if (a.steer_type >= 3) {
-            v.x = __ddiv_rn(v.x, r);
-            v.y = __ddiv_rn(v.y, r);
-            S += 1.0 / (r * r);
+    constexpr int kPer = MIC_MAJOR ? 4 : 1;   // points per warp
+    const int64_t gb = (int64_t)blockIdx.x * 8 * kPer;
+    for (int i = 0; i < kPer; ++i) {
+        const int pt = warp * kPer + i;
+        const int64_t g = gb + pt;
+        if (g >= a.G) break;
+        double gx = 0, gy = 0, gz = 0, r0;
+        if (a.rm) {
+            r0 = a.r0[g];
+        } else {
+            gx = a.gpos[g];
+            gy = a.gpos[a.G + g];
+            gz = a.gpos[2 * a.G + g];
+            r0 = a.ref_mode == 1 ? a.ref_dist : dist3(gx, gy, gz, a.ref0, a.ref1, a.ref2);
         }
-        o[m] = v;
-    }
+        double2 *o = MIC_MAJOR ? st_sm + pt : out + ((int64_t)b * a.G + g) * M;
+        const int64_t step = MIC_MAJOR ? 33 : 1;
+        double S = 0.0;
+        for (int m = lane; m < M; m += 32) {
+            const double r = a.rm ? a.rm[g * M + m] : dist3(gx, gy, gz, a.mpos[m], a.mpos[M + m], a.mpos[2 * M + m]);
+            const float arg = __double2float_rn(__dmul_rn(k, r));
+            float c, sn;
+            sincos_f32_arg(arg, sct, c, sn);
+            double2 v = make_double2((double)c, -(double)sn);
+            if (a.steer_type == 2) {
+                v.x = __dmul_rn(v.x, r);
+                v.y = __dmul_rn(v.y, r);
+                S += r * r;
+            } else if (a.steer_type >= 3) {
+                v.x = __ddiv_rn(v.x, r);
+                v.y = __ddiv_rn(v.y, r);
+                S += 1.0 / (r * r);
+            }
+            o[m * step] = v;
+        }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) S += __shfl_xor_sync(0xffffffffu, S, off);
-    const double Md = (double)M;
-    const double nf = a.steer_type == 1 ? Md : a.steer_type == 2 ? Md * r0 : a.steer_type == 3 ? r0 * S : sqrt(Md * S);
-    const double inv = 1.0 / nf;
-    __syncwarp();
-    for (int m = lane; m < M; m += 32) {
-        const double2 v = o[m];
-        o[m] = make_double2(v.x * inv, v.y * inv);
+        for (int off = 16; off > 0; off >>= 1) S += __shfl_xor_sync(0xffffffffu, S, off);
+        const double Md = (double)M;
+        const double nf =
+            a.steer_type == 1 ? Md : a.steer_type == 2 ? Md * r0 : a.steer_type == 3 ? r0 * S : sqrt(Md * S);
+        const double inv = 1.0 / nf;
+        __syncwarp();
+        for (int m = lane; m < M; m += 32) {
+            const double2 v = o[m * step];
+            o[m * step] = make_double2(v.x * inv, v.y * inv);
+        }
     }
+    if (!MIC_MAJOR) return;
+    __syncthreads();
+    for (int m = warp; m < M; m += 8)
+        if (gb + lane < a.G) out[((int64_t)b * M + m) * a.G + gb + lane] = st_sm[m * 33 + lane];
 }
 
 __global__ void cleansc_init_kernel(int *active, float *result, int64_t n_result, int B)
@@ -337,6 +355,266 @@ __global__ void __launch_bounds__(kCscThreads) cleansc_step_kernel(CscArgs a, in
     if (threadIdx.x == 0) a.lam[b] = hmax;
 }
 
+// ------------------------------------------------------------------------------------------------
+// All iterations of a bin in one cluster of eight CTAs, for arrays whose CSM fits each CTA's shared memory and grids
+// whose map fits the cluster's registers (csc_cluster_fits).  Every CTA keeps the whole CSM and does the step's small
+// work for itself, the same bits in each; the grid points are split over the CTAs (a thread keeps the map values of up
+// to four), and the argmax is the one exchange: each CTA stores its candidate into every CTA's slots (two sets, used
+// alternately, so that one cluster barrier per iteration suffices) and picks the best of the eight.  The component's
+// map reads the steering vectors mic-major, lanes along the grid.
+// Bound: the serial chain of an iteration (the fixed point's sums and reciprocal square roots at the latency of FP64
+// instructions).  Two launches per iteration cost more than that: 5 bins x 1681 points x 64 mics, 128 iterations
+// 3.1 -> 1.07 ms (B200);
+// 8 bins x 3600 points x 112 mics, 60 iterations 4.3 -> 2.1; 3 bins x 8099 points x 33 mics 2.3 -> 1.17.
+// The fixed point stops when a step leaves every value as it was: the remaining ones would change nothing.
+// ------------------------------------------------------------------------------------------------
+constexpr int kCscCtas = 8, kCscClThreads = 256, kCscPoints = 4, kCscHistory = 64;
+constexpr int kCscClMics = 112;
+
+struct CscPeak {
+    double v;
+    long long g;
+};
+
+static __host__ __device__ size_t csc_cluster_smem(int M)
+{
+    return ((size_t)M * M + 3 * M + kCscClThreads) * sizeof(double2) + (size_t)M * sizeof(double);
+}
+
+__device__ __forceinline__ void better(double &v, int64_t &g, double ov, int64_t og)
+{
+    if (ov > v || (ov == v && og < g)) {   // the first index of the maximum
+        v = ov;
+        g = og;
+    }
+}
+
+template <int NP, int AHEAD, int MINB>
+__global__ void __launch_bounds__(kCscClThreads, MINB) cleansc_cluster_kernel(CscArgs a, const double2 *__restrict__ steer,
+                                                                        int r_diag, double norm)
+{
+    extern __shared__ double2 cl_sm[];
+    __shared__ CscPeak peaks[2][kCscCtas], wpeak[kCscClThreads / 32];
+    __shared__ double powers[kCscHistory];   // the last peaks, by iteration modulo its length
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const int b = blockIdx.x / kCscCtas;
+    const int M = a.M, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t G = a.G;
+    double2 *C = cl_sm, *w = C + M * M, *d1 = w + M, *hh = d1 + M, *part = hh + M;
+    double *ww = reinterpret_cast<double *>(part + kCscClThreads);
+    double2 *Cg = a.csm + (int64_t)b * M * M;
+    for (int e = tid; e < M * M; e += kCscClThreads) C[e] = Cg[e];
+    // this thread's grid points and their map values
+    double h[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        const int64_t g = (int64_t)q * kCscCtas * kCscClThreads + rank * kCscClThreads + tid;
+        h[q] = g < G ? a.h[(int64_t)b * G + g] : -INFINITY;
+    }
+    const double k = a.k[b];
+    const SincosTable sct = sincos_table(a.table, a.mask, a.faithful != 0);
+    const double2 *sv = steer + (int64_t)b * M * G;
+    const int Mp = (M + 31) & ~31, ngrp = kCscClThreads / Mp;   // matvec: ngrp threads per row
+    cluster.sync();   // every CTA runs before the first remote store
+
+    for (int j = 0; j < a.J; ++j) {
+        // 1. the peak (and, after the first iteration, nothing else: h was updated at the end of the last one)
+        double best = -INFINITY;
+        int64_t bi = G;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const int64_t g = (int64_t)q * kCscCtas * kCscClThreads + rank * kCscClThreads + tid;
+            if (g < G) better(best, bi, h[q], g);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double ov = __shfl_xor_sync(0xffffffffu, best, o);
+            const int64_t og = __shfl_xor_sync(0xffffffffu, bi, o);
+            better(best, bi, ov, og);
+        }
+        if (lane == 0) wpeak[warp] = CscPeak{best, bi};
+        __syncthreads();
+        if (tid < kCscCtas) {
+            for (int u = 0; u < kCscClThreads / 32; ++u) better(best, bi, wpeak[u].v, wpeak[u].g);
+            *cluster.map_shared_rank(&peaks[j & 1][rank], tid) = CscPeak{best, bi};
+        }
+        cluster.sync();
+        best = -INFINITY;
+        bi = G;
+#pragma unroll
+        for (int u = 0; u < kCscCtas; ++u) better(best, bi, peaks[j & 1][u].v, peaks[j & 1][u].g);
+        if (bi >= G) break;   // no comparable value (NaN map)
+        const int64_t xi = bi;
+        const double hmax = best;
+        const bool stop = j > a.stopn && hmax > powers[(j - a.stopn) % kCscHistory];
+        if (rank == 0 && tid == kCscClThreads - 1) {
+            float *r = a.result + (int64_t)b * G + xi;
+            *r = __double2float_rn(__dadd_rn((double)*r, __dmul_rn(a.damp, hmax)));
+        }
+        if (stop) break;   // the same decision in every CTA
+
+        // 2. steering vector of the peak: transfer x_m = (cos p - i sin p) r0 / rm, p = fl32(k (rm - r0))
+        double2 x = make_double2(0.0, 0.0);
+        if (tid < M) {
+            double gx = 0, gy = 0, gz = 0, r0x;
+            if (a.rm) {
+                r0x = a.r0[xi];
+            } else {
+                gx = a.gpos[xi];
+                gy = a.gpos[G + xi];
+                gz = a.gpos[2 * G + xi];
+                r0x = a.ref_mode == 1 ? a.ref_dist : dist3(gx, gy, gz, a.ref0, a.ref1, a.ref2);
+            }
+            const double rmm =
+                a.rm ? a.rm[xi * M + tid] : dist3(gx, gy, gz, a.mpos[tid], a.mpos[M + tid], a.mpos[2 * M + tid]);
+            const float arg = __double2float_rn(__dmul_rn(k, __dsub_rn(rmm, r0x)));
+            float c, s;
+            sincos_f32_arg(arg, sct, c, s);
+            x = make_double2(__ddiv_rn(__dmul_rn((double)c, r0x), rmm), __ddiv_rn(__dmul_rn(-(double)s, r0x), rmm));
+            ww[tid] = __dadd_rn(__dmul_rn(x.x, x.x), __dmul_rn(x.y, x.y));   // Re x conj(x)
+        }
+        __syncthreads();
+        if (tid == 0) powers[j % kCscHistory] = hmax;   // read again after more barriers only
+        double nrm = 0.0;
+        if (a.steer_type >= 3) {   // einsum('ij,ij->i', x, x.conj())
+            for (int m = lane; m < M; m += 32) nrm += ww[m];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+            if (a.steer_type == 4) nrm = __dsqrt_rn(__dmul_rn(nrm, (double)M));
+        }
+        if (tid < M) {
+            if (a.steer_type == 1) {   // x / |x| / M
+                x = cdiv_real(cdiv_real(x, hypot(x.x, x.y)), (double)M);
+            } else if (a.steer_type == 2) {   // 1 / conj(x) / M
+                x = cdiv_real(cdiv(make_double2(1.0, 0.0), make_double2(x.x, -x.y)), (double)M);
+            } else {   // x / sum |x|^2  |  x / sqrt(sum |x|^2 M)
+                x = cdiv_real(x, nrm);
+            }
+            // * sqrt(normfactor), then the conjugate
+            w[tid] = make_double2(__dmul_rn(x.x, a.sqrt_norm), -__dmul_rn(x.y, a.sqrt_norm));
+        }
+        __syncthreads();
+
+        // 3. D1 = (C^T - diag C) w / hmax: D1_a = sum_{m != a} C[m][a] w_m, the mics m split over ngrp threads per a
+        {
+            const int r = tid % Mp, grp = tid / Mp;
+            double sr[2] = {0.0, 0.0}, si[2] = {0.0, 0.0};
+            if (r < M && grp < ngrp) {
+                const int per = (M + ngrp - 1) / ngrp, m1 = min(M, (grp + 1) * per);
+                for (int m = grp * per; m < m1; m += 2) {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        if (m + u >= m1 || m + u == r) continue;
+                        const double2 c = C[(m + u) * M + r], v = w[m + u];
+                        sr[u] = fma(c.x, v.x, fma(-c.y, v.y, sr[u]));
+                        si[u] = fma(c.x, v.y, fma(c.y, v.x, si[u]));
+                    }
+                }
+                part[grp * Mp + r] = make_double2(sr[0] + sr[1], si[0] + si[1]);
+            }
+        }
+        __syncthreads();
+
+        // the first steering values of step 6 go out now: they land while warp 0 iterates
+        double2 pre[AHEAD];
+        auto fetch = [&](int64_t g, int m0) {
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u)
+                pre[u] = __ldg(sv + (int64_t)min(m0 + u, M - 1) * G + min(g, G - 1));
+        };
+        fetch((int64_t)rank * kCscClThreads + tid, 0);
+
+        // 4. 20 fixed-point steps: hh = (D1 + |hh|^2 w) / sqrt(1 + sum_m |w_m|^2 |hh_m|^2), from hh = w, in warp 0
+        if (warp == 0) {
+            double2 q[kCscClMics / 32 + 1], v[kCscClMics / 32 + 1], d[kCscClMics / 32 + 1];
+            double wv[kCscClMics / 32 + 1];
+            const double inv = cdiv_real(make_double2(1.0, 0.0), hmax).x;
+#pragma unroll
+            for (int u = 0; u <= kCscClMics / 32; ++u) {
+                const int m = lane + 32 * u;
+                v[u] = d[u] = make_double2(0.0, 0.0);
+                if (m < M) {
+                    v[u] = w[m];
+                    double2 t = part[m];
+                    for (int e = 1; e < ngrp; ++e) t = make_double2(t.x + part[e * Mp + m].x, t.y + part[e * Mp + m].y);
+                    d[u] = make_double2(t.x * inv, t.y * inv);
+                }
+                q[u] = v[u];
+                wv[u] = v[u].x * v[u].x + v[u].y * v[u].y;
+            }
+            for (int it = 0; it < 20; ++it) {
+                double sum = 0.0, H[kCscClMics / 32 + 1];
+#pragma unroll
+                for (int u = 0; u <= kCscClMics / 32; ++u) {
+                    H[u] = fma(q[u].x, q[u].x, q[u].y * q[u].y);
+                    sum = fma(wv[u], H[u], sum);
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                const double scl = rsqrt(1.0 + sum);
+                bool same = true;
+#pragma unroll
+                for (int u = 0; u <= kCscClMics / 32; ++u) {
+                    const double2 n = make_double2(fma(H[u], v[u].x, d[u].x) * scl, fma(H[u], v[u].y, d[u].y) * scl);
+                    same = same && n.x == q[u].x && n.y == q[u].y;
+                    q[u] = n;
+                }
+                if (__all_sync(0xffffffffu, same)) break;
+            }
+#pragma unroll
+            for (int u = 0; u <= kCscClMics / 32; ++u)
+                if (lane + 32 * u < M) hh[lane + 32 * u] = q[u];
+        }
+        __syncthreads();
+
+        // 5. C[r][c] -= damp (hmax (hh_c conj(hh_r)))
+        for (int r = warp; r < M; r += kCscClThreads / 32) {
+            const double2 y = hh[r];
+            for (int c = lane; c < M; c += 32) {
+                const double2 u = hh[c];
+                const double pr = __dsub_rn(__dmul_rn(u.x, y.x), __dmul_rn(u.y, -y.y));
+                const double pi = __dadd_rn(__dmul_rn(u.x, -y.y), __dmul_rn(u.y, y.x));
+                double2 e = C[r * M + c];
+                e.x = __dsub_rn(e.x, __dmul_rn(a.damp, __dmul_rn(hmax, pr)));
+                e.y = __dsub_rn(e.y, __dmul_rn(a.damp, __dmul_rn(hmax, pi)));
+                C[r * M + c] = e;
+            }
+        }
+        // 6. h -= damp times the map of the component (hmax, conj(hh)): t_m = hh_m v_m
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            const int64_t g = (int64_t)p * kCscCtas * kCscClThreads + rank * kCscClThreads + tid;
+            if (g >= G) break;
+            double fr[4] = {0, 0, 0, 0}, fi[4] = {0, 0, 0, 0}, dg[4] = {0, 0, 0, 0};
+            for (int m = 0; m < M; m += AHEAD) {
+                if (p || m) fetch(g, m);
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    if (m + u >= M) break;
+                    const double2 s = pre[u], q = hh[m + u];
+                    const double tr = q.x * s.x - q.y * s.y, ti = q.x * s.y + q.y * s.x;
+                    fr[u & 3] += tr;
+                    fi[u & 3] += ti;
+                    if (r_diag) dg[u & 3] += tr * tr + ti * ti;
+                }
+            }
+            const double sr = (fr[0] + fr[1]) + (fr[2] + fr[3]), si = (fi[0] + fi[1]) + (fi[2] + fi[3]);
+            double full = sr * sr + si * si;
+            if (r_diag) full -= (dg[0] + dg[1]) + (dg[2] + dg[3]);
+            h[p] = __dsub_rn(h[p], __dmul_rn(a.damp, full * hmax * norm));
+        }
+    }
+    __syncthreads();
+    if (rank == 0)
+        for (int e = tid; e < M * M; e += kCscClThreads) Cg[e] = C[e];   // the cleaned matrix
+}
+
+static bool csc_cluster_fits(int M, int64_t G, int stopn)
+{
+    return M <= kCscClMics && G <= (int64_t)kCscPoints * kCscCtas * kCscClThreads && stopn >= 1 && stopn < kCscHistory;
+}
+
 struct CscWorkspace {
     size_t h, h1, powers, lam, vec, active, steer, total;
 };
@@ -437,7 +715,37 @@ int acb_cleansc_f64(const acb_map_params *p, void *csm, const double *wavenumber
     st = map_plain_launch(&q, B, csm, wavenumber, mpos, gpos, r0, rm, a.h, s);
     if (st) return st;
     double2 *steer = reinterpret_cast<double2 *>(ws + lay.steer);
-    cleansc_steer_kernel<<<dim3((unsigned)((G + 7) / 8), B), 256, 0, s>>>(a, steer);
+    if (csc_cluster_fits(M, G, stopn)) {
+        const size_t tile = (size_t)M * 33 * sizeof(double2), smem = csc_cluster_smem(M);
+        // few bins: 16 steering values in flight per thread and all the registers that takes; more bins than one CTA per
+        // SM holds (15 clusters): 8, and 128 registers for two (60 bins of 64 mics: 2.14 against 3.43 ms)
+        const bool few = B * kCscCtas <= 120, small = G <= kCscCtas * kCscClThreads;
+        auto kern = few ? (small ? cleansc_cluster_kernel<1, 16, 1> : cleansc_cluster_kernel<kCscPoints, 16, 1>)
+                        : (small ? cleansc_cluster_kernel<1, 8, 2> : cleansc_cluster_kernel<kCscPoints, 8, 2>);
+        if (cudaFuncSetAttribute(cleansc_steer_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+            return ACB_ERR_CUDA;
+        cleansc_steer_kernel<true><<<dim3((unsigned)((G + 31) / 32), B), 256, tile, s>>>(a, steer);
+        st = check_launch();
+        if (st) return st;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(B * kCscCtas));
+        cfg.blockDim = dim3(kCscClThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kCscCtas;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaLaunchKernelEx(&cfg, kern, a, static_cast<const double2 *>(steer), p->r_diag, p->norm) != cudaSuccess)
+            return ACB_ERR_CUDA;
+        return check_launch();
+    }
+    cleansc_steer_kernel<false><<<dim3((unsigned)((G + 7) / 8), B), 256, 0, s>>>(a, steer);
     st = check_launch();
     if (st) return st;
     const size_t smem = (size_t)M * (3 * sizeof(double2) + sizeof(double));
