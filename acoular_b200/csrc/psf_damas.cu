@@ -21,6 +21,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "tc_common.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -318,6 +319,260 @@ __global__ void __launch_bounds__(kDamasThreads) damas_kernel(const double *__re
         for (int64_t i = threadIdx.x; i < G; i += kDamasThreads) xg[i] = xs[i];
 }
 
+// ------------------------------------------------------------------------------------------------
+// The same sweeps with the solver fed two blocks ahead, for four or more blocks of rows and clusters of four or eight
+// CTAs.  CTA 0 solves: warp 0 takes the rows of one block after another (step t: block t mod nblk), lane i owning row i,
+// and three warps bring it, per step, three 32 x 32 tiles of the block's columns: of its own rows and of the next two
+// blocks' rows.  As each new value x_j is broadcast, every lane also adds its contribution to its rows of the next two
+// blocks, off the serial path, so that a step starts as soon as the sums over all other columns are there.  Those
+// come from the other CTAs: CTA r > 0 holds a slice of the columns, and for block t it needs the values of step t - 3
+// and before (the solver adds those of t - 1 and t - 2 itself; right of the block and, within it, right of each row
+// the previous sweep's values count), so it has two steps' time.  New values and sums travel as asynchronous stores
+// counted on mbarriers (rings of four; a ring's slot is used again only after an exchange in the other direction that
+// follows its last use): no cluster barrier in a step.
+// Bound: the solver's step, 2700 cycles: 60 per row (one FMA, a compare and a shuffle are 50 of them) and 800 to take in
+// the sums and publish the values.  Measured (B200): 5 bins x 1681 points x 100 sweeps 21.2 -> 7.6 ms; 2 bins x 4000
+// points 71 -> 35 (the form above spends 7600 cycles a step, of them 2000 in its cluster barrier).  Four rows at a time,
+// every lane solving their triangle for itself, was slower (80 a row: the extra FMAs' issue slots).
+// ------------------------------------------------------------------------------------------------
+constexpr int kGsTile = kDamasRows * kDamasPad, kGsStages = 3, kGsRing = 4;
+
+__host__ __device__ inline int64_t gs_smem_bytes(int64_t G)
+{
+    const int64_t nblk = (G + kDamasRows - 1) / kDamasRows;
+    return (nblk * kDamasRows + (int64_t)kGsStages * 3 * kGsTile + kGsRing * kDamasMaxCta * kDamasRows) * 8;
+}
+
+// 8 bytes to the same place of CTA `rank`'s shared memory, counted on that CTA's mbarrier.
+__device__ __forceinline__ void gs_send(int rank, const double *dst, double v, const uint64_t *bar)
+{
+    uint32_t ra, rb;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(tc::smem_u32(dst)), "r"(rank));
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(tc::smem_u32(bar)), "r"(rank));
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(ra), "d"(v),
+                 "r"(rb)
+                 : "memory");
+}
+
+// Bounded wait (half a second, or the flag raised by another thread): then it returns at once and the caller carries on.
+__device__ __forceinline__ void gs_wait(const uint64_t *bar, uint32_t parity, volatile int *gave_up)
+{
+    const uint32_t addr = tc::smem_u32(bar);
+    uint64_t t0 = 0;
+    while (true) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 100000;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(addr), "r"(parity)
+            : "memory");
+        if (ok || *gave_up) return;
+        const uint64_t t = tc::globaltimer_ns();
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > 500ull * 1000 * 1000) *gave_up = 1;
+    }
+}
+
+// max(0, u), and 0 for NaN as fmax gives it, on the integer pipe (sign bit or an exponent of ones with mantissa)
+__device__ __forceinline__ double gs_clamp(double u)
+{
+    return (uint32_t)__double2hiint(u) > 0x7ff00000u ? 0.0 : u;
+}
+
+__global__ void __launch_bounds__(kDamasThreads) damas_ahead_kernel(const double *__restrict__ A, int64_t G,
+                                                                   const double *__restrict__ y,
+                                                                   double *__restrict__ x, int n_iter, double relax)
+{
+    extern __shared__ double sm[];
+    __shared__ uint64_t xbar[kGsRing], pbar[kGsRing], tbar[kGsStages];
+    __shared__ int gave_up_s;
+    volatile int *gave_up = &gave_up_s;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int64_t bin = blockIdx.x / C;
+    const int nblk = (int)((G + kDamasRows - 1) / kDamasRows);
+    double *xs = sm;                                     // [nblk * 32], zeros past G
+    double *tiles = xs + (int64_t)nblk * kDamasRows;     // [stage][own rows | next | the one after][column][33]
+    double *part = tiles + kGsStages * 3 * kGsTile;      // [ring][CTA][32] (CTA 0's are used)
+    const double *Ab = A + bin * G * G;
+    const double *yg = y + bin * G;
+    double *xg = x + bin * G;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t steps = (int64_t)n_iter * nblk;
+
+    for (int64_t i = threadIdx.x; i < (int64_t)nblk * kDamasRows; i += kDamasThreads) xs[i] = i < G ? xg[i] : 0.0;
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < kGsRing; ++q) {
+            tc::mbar_init(&xbar[q], 1);
+            tc::mbar_init(&pbar[q], 1);
+        }
+        for (int q = 0; q < kGsStages; ++q) tc::mbar_init(&tbar[q], 96);
+        gave_up_s = 0;
+        tc::fence_mbar_init();
+        for (int q = 0; q < kGsRing; ++q)   // the first round of each ring
+            if (rank == 0) tc::mbar_arrive_expect_tx(&pbar[q], (uint32_t)((C - 1) * kDamasRows * 8));
+            else tc::mbar_arrive_expect_tx(&xbar[q], kDamasRows * 8);
+    }
+    cluster.sync();
+
+    if (rank == 0 && warp == 0) {
+        // ---------------- the solver
+        double acc1 = 0.0, acc2 = 0.0;   // -relax times the new values' part of row `lane` of the next two blocks
+        double yv = lane < G ? yg[lane] : 0.0;
+        int k = 0;
+        for (int64_t t = 0; t < steps; ++t) {
+            const int64_t g0 = (int64_t)k * kDamasRows;
+            const bool row = g0 + lane < G;
+            const int st = (int)(t % kGsStages), slot = (int)(t % kGsRing);
+            const double *D = tiles + st * 3 * kGsTile + lane, *N1 = D + kGsTile, *N2 = N1 + kGsTile;
+            const double xold = xs[g0 + lane];
+            const double c = fma(relax, yv, fma(1.0 - relax, xold, acc1));
+            gs_wait(&tbar[st], (uint32_t)(t / kGsStages) & 1, gave_up);
+            gs_wait(&pbar[slot], (uint32_t)(t / kGsRing) & 1, gave_up);
+            double sum[2] = {0.0, 0.0};
+#pragma unroll
+            for (int r = 1; r < kDamasMaxCta; ++r)
+                if (r < C) sum[r & 1] += part[(slot * kDamasMaxCta + r) * kDamasRows + lane];
+            if (lane == 0 && t + kGsRing < steps && !*gave_up)
+                tc::mbar_arrive_expect_tx(&pbar[slot], (uint32_t)((C - 1) * kDamasRows * 8));
+            double u = row ? fma(-relax, sum[0] + sum[1], c) : 0.0;
+            acc1 = acc2;
+            acc2 = 0.0;
+            k = k + 1 == nblk ? 0 : k + 1;
+            const int64_t gn = (int64_t)k * kDamasRows + lane;
+            yv = gn < G ? __ldg(yg + gn) : 0.0;
+            double xv = 0.0;
+#pragma unroll
+            for (int j = 0; j < kDamasRows; ++j) {
+                const double d = j < lane ? -relax * D[j * kDamasPad] : 0.0;
+                const double n1 = -relax * N1[j * kDamasPad], n2 = -relax * N2[j * kDamasPad];
+                const double xn = __shfl_sync(0xffffffffu, gs_clamp(u), j);
+                u = fma(d, xn, u);
+                acc1 = fma(n1, xn, acc1);
+                acc2 = fma(n2, xn, acc2);
+                xv = lane == j ? xn : xv;
+            }
+            xs[g0 + lane] = xv;
+            if (t + 3 < steps)   // the other CTAs wait for step t's values at step t + 3
+                for (int r = 1; r < C; ++r) gs_send(r, xs + g0 + lane, xv, &xbar[slot]);
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&xbar[slot]);
+        }
+    } else if (rank == 0 && warp <= 3) {
+        // ---------------- the solver's tiles: rows of block t (+ 1, + 2), columns of block t
+        const int which = warp - 1;
+        for (int64_t t = 0; t < steps; ++t) {
+            // the stage was read at step t - 3
+            if (t >= kGsStages) gs_wait(&xbar[(t - kGsStages) % kGsRing], (uint32_t)((t - kGsStages) / kGsRing) & 1,
+                                        gave_up);
+            const int64_t g0 = (t % nblk) * kDamasRows, gr = ((t + which) % nblk) * kDamasRows;
+            const int st = (int)(t % kGsStages);
+            double *dst = tiles + (st * 3 + which) * kGsTile + lane * kDamasPad;   // column `lane`
+            const bool col = g0 + lane < G;
+#pragma unroll 8
+            for (int i = 0; i < kDamasRows; ++i) {
+                const bool in = col && gr + i < G;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(tc::smem_u32(dst + i)),
+                             "l"(Ab + (in ? (gr + i) * G + g0 + lane : 0)), "r"(in ? 8 : 0)
+                             : "memory");
+            }
+            asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+            tc::mbar_arrive(&tbar[st]);
+        }
+    } else if (rank > 0) {
+        // ---------------- sums over this CTA's columns: rows warp and warp + 16 of every block
+        const int nch = (nblk + C - 2) / (C - 1);            // column blocks of a slice
+        const int b0 = (rank - 1) * nch, b1 = min(b0 + nch, nblk);
+        const int ngrp = b1 > b0 ? (b1 - b0 + 7) / 8 : 1;    // in groups of 8 column blocks
+        // column blocks of the slice in which this lane has a column, and the lane's place in row `warp` of block 0
+        const int mine = b1 > b0 ? b1 - b0 - ((int64_t)b1 * kDamasRows > G && (int64_t)(b1 - 1) * kDamasRows + lane >= G)
+                                 : 0;
+        const double *row0 = Ab + (int64_t)warp * G + (int64_t)b0 * kDamasRows + lane;
+        const double *xl = xs + b0 * kDamasRows + lane;
+        const int64_t half = 16 * G, block = kDamasRows * G;
+        double a0[8], a1[8];
+        // the group's elements of rows `warp` and `warp` + 16 of the block whose row `warp` is at `r`, if they exist
+        auto fetch = [&](const double *r, bool ok0, bool ok1, int grp) {
+            const double *r0 = r + grp * (8 * kDamasRows), *r1 = r0 + half;
+            const int n0 = ok0 ? mine - grp * 8 : 0, n1 = ok1 ? mine - grp * 8 : 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                a0[q] = a1[q] = 0.0;
+                if (q < n0) a0[q] = __ldg(r0 + q * kDamasRows);
+                if (q < n1) a1[q] = __ldg(r1 + q * kDamasRows);
+            }
+        };
+        const bool last0 = (int64_t)(nblk - 1) * kDamasRows + warp < G, last1 = (int64_t)(nblk - 1) * kDamasRows + warp + 16 < G;
+        int k = 0;
+        const double *rk = row0;   // row `warp` of block k
+        if (steps > 0) fetch(rk, true, true, 0);
+        for (int64_t t = 0; t < steps; ++t) {
+            const int kn = k + 1 == nblk ? 0 : k + 1;
+            const double *rn = kn ? rk + block : row0;
+            if (t >= 3) {
+                gs_wait(&xbar[(t - 3) % kGsRing], (uint32_t)((t - 3) / kGsRing) & 1, gave_up);
+                if (threadIdx.x == 0 && t + 1 < steps && !*gave_up)
+                    tc::mbar_arrive_expect_tx(&xbar[(t - 3) % kGsRing], kDamasRows * 8);   // for step t + 1
+            }
+            // places in the slice of block k and of the blocks solved at steps t - 1 and t - 2 (the solver's)
+            const int ek = k - b0, e1 = t >= 1 ? (k == 0 ? nblk - 1 : k - 1) - b0 : -1;
+            const int e2 = t >= 2 ? (k <= 1 ? nblk - 2 + k : k - 2) - b0 : -1;
+            double s0 = 0.0, s1 = 0.0;
+            for (int grp = 0; grp < ngrp; ++grp) {
+                double c0[8], c1[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    c0[q] = a0[q];
+                    c1[q] = a1[q];
+                }
+                // the next group, or the next block's first, lands while this one is summed and waited for
+                if (grp + 1 < ngrp) fetch(rk, k + 1 < nblk || last0, k + 1 < nblk || last1, grp + 1);
+                else if (t + 1 < steps) fetch(rn, kn + 1 < nblk || last0, kn + 1 < nblk || last1, 0);
+                double p0 = 0.0, p1 = 0.0;
+                const int left = b1 - b0 - grp * 8, gk = ek - grp * 8, g1 = e1 - grp * 8, g2 = e2 - grp * 8;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    if (q >= left || q == g1 || q == g2) continue;   // uniform
+                    const double xv = xl[(grp * 8 + q) * kDamasRows];
+                    double v0 = c0[q], v1 = c1[q];
+                    if (q == gk) {   // within the block only the columns right of the row
+                        v0 = lane <= warp ? 0.0 : v0;
+                        v1 = lane <= warp + 16 ? 0.0 : v1;
+                    }
+                    if (q & 1) {
+                        p0 = fma(v0, xv, p0);
+                        p1 = fma(v1, xv, p1);
+                    } else {
+                        s0 = fma(v0, xv, s0);
+                        s1 = fma(v1, xv, s1);
+                    }
+                }
+                s0 += p0;
+                s1 += p1;
+            }
+            // lanes 0..15 end up with row warp's sum, the others with row warp + 16's
+            const double give = lane < 16 ? s1 : s0;
+            double s = (lane < 16 ? s0 : s1) + __shfl_xor_sync(0xffffffffu, give, 16);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            const int slot = (int)(t % kGsRing);
+            if ((lane & 15) == 0)
+                gs_send(0, part + (slot * kDamasMaxCta + rank) * kDamasRows + warp + (lane ? 16 : 0), s, &pbar[slot]);
+            k = kn;
+            rk = rn;
+        }
+    }
+    if (*gave_up) __nanosleep(1000000);   // let what is still under way land before a CTA ends
+    cluster.sync();
+    if (rank == 0) {
+        const bool bad = *gave_up != 0;   // a wait ran out: no result
+        for (int64_t i = threadIdx.x; i < G; i += kDamasThreads)
+            xg[i] = bad ? __longlong_as_double(0x7ff8000000000000ll) : xs[i];
+    }
+}
+
 }  // namespace acb
 
 using namespace acb;
@@ -377,12 +632,17 @@ int acb_damas_gauss_seidel_f64(const double *psf, int64_t num_grid, int num_bins
     }
     if (C != 1 && C != 2 && C != 4 && C != 8) return ACB_ERR_ARG;
     if ((int64_t)num_bins * C > 0x7fffffff) return ACB_ERR_SHAPE;
-    if (cudaFuncSetAttribute(damas_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    // the form two blocks ahead: at least six blocks, four CTAs, and its tiles beside the solution
+    const int64_t smem_ahead = gs_smem_bytes(num_grid);
+    const bool ahead = num_grid > 5 * kDamasRows && C >= 4 && smem_ahead <= smem_max - 1024;
+    auto kern = ahead ? damas_ahead_kernel : damas_kernel;
+    const size_t smem_used = ahead ? (size_t)smem_ahead : smem;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_used) != cudaSuccess)
         return ACB_ERR_CUDA;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(num_bins * C));
     cfg.blockDim = dim3(kDamasThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = smem_used;
     cfg.stream = as_stream(stream);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -391,7 +651,7 @@ int acb_damas_gauss_seidel_f64(const double *psf, int64_t num_grid, int num_bins
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, damas_kernel, psf, num_grid, dirty_map, solution, n_iter, relax) != cudaSuccess)
+    if (cudaLaunchKernelEx(&cfg, kern, psf, num_grid, dirty_map, solution, n_iter, relax) != cudaSuccess)
         return ACB_ERR_CUDA;
     return check_launch();
 }
