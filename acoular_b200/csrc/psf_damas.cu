@@ -7,8 +7,7 @@
 //     P = |sum_m e^{-i fl32(k (rm[g,m] - rm[s,m]))} w_m|^2 * n^2,
 // the four steering types weighting w_m and n as the reference does; the phase is rounded to float32
 // and its cos/sin are the C library's float32 ones (the exception table of the plain map).
-// CTA = 32 grid points (lanes) x 8 sources (warps); the grid points' distance rows are staged in
-// shared memory, each source's row is read as a broadcast.
+// CTA = 32 grid points x 32 sources; their distance rows and reciprocals are staged in shared memory.
 //
 // DAMAS: per bin, n_iter sweeps over g = 0 .. G-1 in order, each x[g] = max(0, (1 - relax) x[g] +
 // relax (y[g] - sum_{h != g} A[g][h] x[h])) with the latest x.  The sweep is sequential by
@@ -27,93 +26,141 @@ namespace cg = cooperative_groups;
 
 namespace acb {
 
-constexpr int kPsfLanes = 32;
+constexpr int kPsfTile = 32;      // grid points and sources per CTA
 constexpr int kPsfWarps = 8;
-constexpr int kPsfMics = 4;     // mics whose phases a lane evaluates together
+constexpr int kPsfPer = kPsfTile / kPsfWarps;   // sources per warp (and phases a lane evaluates together)
+constexpr int kPsfMics = 32;      // mics per shared-memory chunk: 33 KB, four CTAs per SM (64: 0.67 ms below)
 
+// Distances and their reciprocals of a tile's 32 grid points, mic-major, and of its 32 sources, source-major.
+constexpr int kPsfG = kPsfMics * (kPsfTile + 1), kPsfS = kPsfTile * (kPsfMics + 1);
+constexpr int kPsfSmem = 2 * (kPsfG + kPsfS) * (int)sizeof(double);
+
+// CTA = 32 grid points (lanes) x 32 sources (four per warp).  The phase of (g, s) is minus that of (s, g), so that
+// where the sources are the grid itself (checked on the tile's own indices), a tile right of the diagonal also gives
+// its mirror image, whose CTA then has nothing to do.  The mirrored sums differ in their weights only: w for P(g; s),
+// wm for P(s; g), the same for 'true level' and 'true location'.
+// Bound: issue slots of the phase evaluation (about 100 instructions).  Measured (B200): 1681 x 1681 x 64 mics
+// 1.03 -> 0.51 ms.
 template <int ST>
-__global__ void __launch_bounds__(256) psf_kernel(int M, int64_t G, int S, const int64_t *__restrict__ src,
-                                                  const double *__restrict__ r0, const double *__restrict__ rm,
-                                                  double k, const uint64_t *__restrict__ table, uint64_t mask,
-                                                  int faithful, int mc, int round_f32, double *__restrict__ out)
+__global__ void __launch_bounds__(256, 4) psf_kernel(int M, int64_t G, int S, const int64_t *__restrict__ src,
+                                                     const double *__restrict__ r0, const double *__restrict__ rm,
+                                                     double k, const uint64_t *__restrict__ table, uint64_t mask,
+                                                     int faithful, int round_f32, double *__restrict__ out)
 {
-    extern __shared__ double rg_s[];   // [mc][32]: distance rows of this CTA's grid points, mic-major
+    extern __shared__ double psf_sm[];
+    double *rg_s = psf_sm, *ig_s = rg_s + kPsfG;        // [mic][point, 33]
+    double *rs_s = ig_s + kPsfG, *is_s = rs_s + kPsfS;   // [source][mic, 33]
+    __shared__ int64_t src_s[kPsfTile];
+    __shared__ double help_s[2 * kPsfTile];              // sums of 1 / r^2: points, sources
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t g = (int64_t)blockIdx.x * kPsfLanes + lane;
-    const int sidx = blockIdx.y * kPsfWarps + warp;
-    int64_t s = sidx < S ? src[sidx] : 0;
-    const bool src_ok = s >= 0 && s < G;   // an index outside the grid yields NaN, never a stray read
-    s = src_ok ? s : 0;
-    const bool valid = g < G && sidx < S;
-    const double *rs = rm + s * M;
+    const int64_t gb = (int64_t)blockIdx.x * kPsfTile;
+    const int sb = blockIdx.y * kPsfTile;
+    const int64_t g = gb + lane;
+    bool own = true;   // this tile's points and sources are the grid's in order
+    if (threadIdx.x < kPsfTile) {
+        const int i = sb + threadIdx.x;
+        const int64_t s = i < S ? src[i] : 0;
+        src_s[threadIdx.x] = s;
+        own = i >= S || s == i;
+    } else if (threadIdx.x < 2 * kPsfTile) {
+        const int64_t i = gb + threadIdx.x - kPsfTile;
+        own = i >= S || src[i] == i;
+    }
+    const bool sym = __syncthreads_and(own) && S == G && gb != sb;
+    if (sym && gb > sb) return;   // the tile on the other side of the diagonal writes this one
     const SincosTable sct = sincos_table(table, mask, faithful != 0);
-    double re = 0.0, im = 0.0, help = 0.0;
-    double rs_l = 1.0, irs_l = 1.0;
-    for (int m0 = 0; m0 < M; m0 += mc) {
-        const int n = min(mc, M - m0);
+    double re[kPsfPer], im[kPsfPer], rem[kPsfPer], imm[kPsfPer];
+#pragma unroll
+    for (int j = 0; j < kPsfPer; ++j) re[j] = im[j] = rem[j] = imm[j] = 0.0;
+    if (threadIdx.x < 2 * kPsfTile) help_s[threadIdx.x] = 0.0;
+    for (int m0 = 0; m0 < M; m0 += kPsfMics) {
+        const int n = min(kPsfMics, M - m0);
         __syncthreads();
-        for (int i = threadIdx.x; i < n * kPsfLanes; i += blockDim.x) {
-            const int mm = i / kPsfLanes, l = i % kPsfLanes;
-            const int64_t gg = (int64_t)blockIdx.x * kPsfLanes + l;
-            rg_s[i] = gg < G ? rm[gg * M + m0 + mm] : 1.0;
+        for (int i = threadIdx.x; i < kPsfTile * kPsfMics; i += blockDim.x) {
+            const int p = i / kPsfMics, m = i % kPsfMics;
+            if (m >= n) continue;
+            const double a = gb + p < G ? rm[(gb + p) * M + m0 + m] : 1.0;
+            int64_t s = src_s[p];
+            s = s >= 0 && s < G ? s : 0;   // an index outside the grid yields NaN, never a stray read
+            const double b = rm[s * M + m0 + m];
+            rg_s[m * (kPsfTile + 1) + p] = a;
+            ig_s[m * (kPsfTile + 1) + p] = 1.0 / a;
+            rs_s[p * (kPsfMics + 1) + m] = b;
+            is_s[p * (kPsfMics + 1) + m] = 1.0 / b;
         }
         __syncthreads();
-        // every lane runs the loop (the shuffles need the whole warp); invalid lanes write nothing.  Four mics at
-        // a time, so that their table lookups are in flight together (four divide the 32 of a shuffle block)
-        for (int mm = 0; mm < n; mm += kPsfMics) {
-            if ((mm & 31) == 0) {   // lane l holds the source distance of mic mm + l and its reciprocal
-                rs_l = mm + lane < n ? __ldg(rs + m0 + mm + lane) : 1.0;
-                irs_l = 1.0 / rs_l;
+        if (ST >= 3 && threadIdx.x < 2 * kPsfTile) {
+            double h = help_s[threadIdx.x];
+            for (int m = 0; m < n; ++m) {
+                const double q = threadIdx.x < kPsfTile ? ig_s[m * (kPsfTile + 1) + threadIdx.x]
+                                                        : is_s[(threadIdx.x - kPsfTile) * (kPsfMics + 1) + m];
+                h = fma(q, q, h);
             }
-            SincosPending pend[kPsfMics];
+            help_s[threadIdx.x] = h;
+        }
+        const double *rsw = rs_s + warp * kPsfPer * (kPsfMics + 1), *isw = is_s + warp * kPsfPer * (kPsfMics + 1);
+        for (int m = 0; m < n; ++m) {
+            const double rg = rg_s[m * (kPsfTile + 1) + lane], ig = ig_s[m * (kPsfTile + 1) + lane];
+            SincosPending pend[kPsfPer];
 #pragma unroll
-            for (int u = 0; u < kPsfMics; ++u) {
-                const double rsm = __shfl_sync(0xffffffffu, rs_l, (mm + u) & 31);
-                const double rg = rg_s[min(mm + u, n - 1) * kPsfLanes + lane];
-                pend[u] = sincos_begin(__double2float_rn(__dmul_rn(k, __dsub_rn(rg, rsm))), sct);
-            }
+            for (int j = 0; j < kPsfPer; ++j)
+                pend[j] = sincos_begin(__double2float_rn(__dmul_rn(k, __dsub_rn(rg, rsw[j * (kPsfMics + 1) + m]))), sct);
 #pragma unroll
-            for (int u = 0; u < kPsfMics; ++u) {
-                const double irs = __shfl_sync(0xffffffffu, irs_l, (mm + u) & 31);
-                if (mm + u >= n) break;   // uniform
-                const double rg = rg_s[(mm + u) * kPsfLanes + lane];
-                sincos_finish(pend[u], sct);
+            for (int j = 0; j < kPsfPer; ++j) {
+                sincos_finish(pend[j], sct);
+                const double c = (double)pend[j].c, sn = -(double)pend[j].s;
                 // (cos - i sin) / rs  [* rg (inverse) | / rg (true level, true location)]; the divisions as
-                // products with reciprocals (within an ulp of the quotients)
-                double tr = __dmul_rn((double)pend[u].c, irs), ti = __dmul_rn(-(double)pend[u].s, irs);
-                if (ST == 2) {
-                    tr = __dmul_rn(tr, rg);
-                    ti = __dmul_rn(ti, rg);
-                } else if (ST >= 3) {
-                    const double ig = 1.0 / rg;
-                    tr = __dmul_rn(tr, ig);
-                    ti = __dmul_rn(ti, ig);
-                    help += ig * ig;
+                // products with reciprocals (within an ulp of the quotients); the mirror image's sine is negated
+                const double is = isw[j * (kPsfMics + 1) + m];
+                const double w = ST == 1 ? is : ST == 2 ? is * rg : is * ig;
+                re[j] = fma(c, w, re[j]);
+                im[j] = fma(sn, w, im[j]);
+                if (ST < 3 && sym) {
+                    const double wm = ST == 1 ? ig : ig * rsw[j * (kPsfMics + 1) + m];
+                    rem[j] = fma(c, wm, rem[j]);
+                    imm[j] = fma(sn, wm, imm[j]);
                 }
-                re += tr;
-                im += ti;
             }
         }
     }
-    if (!valid) return;
+    __syncthreads();
+    double *tile = psf_sm;   // [point][source, 33]
     const double Md = (double)M;
-    const double a2 = re * re + im * im;
-    double res;
-    if (ST == 1) {
-        const double nf = r0[s] / Md;
-        res = a2 * (nf * nf);
-    } else if (ST == 2) {
-        const double nf = r0[s] / r0[g] / Md;
-        res = a2 * (nf * nf);
-    } else if (ST == 3) {
-        const double nf = r0[s] / r0[g] / help;
-        res = a2 * (nf * nf);
-    } else {
-        const double nf = r0[s];
-        res = a2 * (nf * nf) / Md / help;
+    // P(a; b) from the sum's squared magnitude, the reference distances and a's sum of 1 / r^2
+    auto value = [&](double a2, double ra, double rb, double help) {
+        double nf, res;
+        if (ST == 1) {
+            nf = rb / Md;
+            res = a2 * (nf * nf);
+        } else if (ST == 2) {
+            nf = rb / ra / Md;
+            res = a2 * (nf * nf);
+        } else if (ST == 3) {
+            nf = rb / ra / help;
+            res = a2 * (nf * nf);
+        } else {
+            res = a2 * (rb * rb) / Md / help;
+        }
+        return round_f32 ? (double)__double2float_rn(res) : res;
+    };
+    const double ra = g < G ? r0[g] : 1.0;
+#pragma unroll
+    for (int j = 0; j < kPsfPer; ++j) {
+        const int q = warp * kPsfPer + j;
+        const int64_t s = src_s[q];
+        const bool ok = s >= 0 && s < G;
+        const double rb = r0[ok ? s : 0];
+        const double a2 = re[j] * re[j] + im[j] * im[j];
+        tile[lane * (kPsfTile + 1) + q] =
+            ok ? value(a2, ra, rb, help_s[lane]) : __longlong_as_double(0x7ff8000000000000ll);
+        if (sym && sb + q < S && g < G) {
+            const double m2 = ST < 3 ? rem[j] * rem[j] + imm[j] * imm[j] : a2;
+            out[(int64_t)(sb + q) * S + g] = value(m2, rb, ra, help_s[kPsfTile + q]);
+        }
     }
-    if (!src_ok) res = __longlong_as_double(0x7ff8000000000000ll);
-    out[g * S + sidx] = round_f32 ? (double)__double2float_rn(res) : res;
+    __syncthreads();
+    for (int p = warp; p < kPsfTile; p += kPsfWarps)
+        if (gb + p < G && sb + lane < S) out[(gb + p) * S + sb + lane] = tile[p * (kPsfTile + 1) + lane];
 }
 
 constexpr int kDamasThreads = 512;
@@ -590,18 +637,16 @@ int acb_psf_f64(const acb_map_params *p, int num_sources, const int64_t *sources
         return ACB_ERR_ARG;
     const int M = p->num_mics;
     const int64_t G = p->num_grid;
-    const int mc = M < 256 ? M : 256;
-    const size_t smem = (size_t)mc * kPsfLanes * sizeof(double);
-    const dim3 grid((unsigned)((G + kPsfLanes - 1) / kPsfLanes), (unsigned)((num_sources + kPsfWarps - 1) / kPsfWarps));
-    if (grid.y > 65535) return ACB_ERR_SHAPE;
+    const dim3 grid((unsigned)((G + kPsfTile - 1) / kPsfTile), (unsigned)((num_sources + kPsfTile - 1) / kPsfTile));
+    if ((num_sources + 7) / 8 > 65535) return ACB_ERR_SHAPE;
     const uint64_t mask = p->glibc_faithful ? (uint64_t)p->sincos_table_slots - 1 : 0;
     cudaStream_t s = as_stream(stream);
-#define ACB_PSF(ST)                                                                                          \
-    do {                                                                                                     \
-        cudaFuncSetAttribute(psf_kernel<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
-        psf_kernel<ST><<<grid, kPsfLanes * kPsfWarps, smem, s>>>(M, G, num_sources, sources, r0, rm, wavenumber, \
-                                                                p->sincos_table, mask, p->glibc_faithful, mc, \
-                                                                round_f32, out_psf);                         \
+#define ACB_PSF(ST)                                                                                           \
+    do {                                                                                                      \
+        cudaFuncSetAttribute(psf_kernel<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPsfSmem);          \
+        psf_kernel<ST><<<grid, 32 * kPsfWarps, kPsfSmem, s>>>(M, G, num_sources, sources, r0, rm, wavenumber, \
+                                                             p->sincos_table, mask, p->glibc_faithful,        \
+                                                             round_f32, out_psf);                             \
     } while (0)
     switch (p->steer_type) {
     case 1: ACB_PSF(1); break;
