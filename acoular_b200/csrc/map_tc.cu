@@ -22,13 +22,15 @@
 // Pipeline step: one A stage (16 KB), i.e. one chunk (split BF16, TF32) or two (FP16, 8 KB each).
 // Every role works per step: one steering arrival, one R' tile barrier, one MMA commit, one
 // epilogue wait and release.
-//   warp 5      : bulk copies of the step's R' tiles (pre-laid in HBM in the shared-memory
+//   warp 20     : bulk copies of the step's R' tiles (pre-laid in HBM in the shared-memory
 //                 core-matrix order by tc_prep_kernel) into a 128 KB tile ring, running ahead
-//   warp 1      : TMEM allocation; one thread issues tcgen05.mma (A = steering chunk, B = R'
-//                 tiles) and commits to the step's mbarrier
-//   warps 0,9,2,3: epilogue (TMEM lane quarters 0..3): after the step's MMAs, read the final
+//   warp 1      : TMEM allocation; issues tcgen05.mma (A = steering chunk, B = R' tiles) and
+//                 commits to the step's mbarrier
+//   warps 0,21,2,3: epilogue (TMEM lane quarters 0..3): after the step's MMAs, read the final
 //                 accumulator columns from TMEM and dot them with the steering chunks read back
 //                 from the A stage
+//   warps 22,23 : finishing: an item's sums to its map values (scale, group sums, normalisation,
+//                 store), beside the next item's steps
 //   16 warps    : steering synthesis (four threads per grid point, 4 mics of each chunk), packed
 //                 FP32: distance by rsqrt, the phase (k as a float-float; reduced by a three-term
 //                 2*pi for split BF16), hardware sincos, the operand conversion into the A stage.
@@ -72,29 +74,31 @@ constexpr int TC_SYNTH_WARPS = 4 * TC_PARTS;  // TC_PARTS warps per TMEM lane qu
 constexpr int TC_SYNTH_THREADS = 32 * TC_SYNTH_WARPS;
 constexpr int TC_EPI_WARPS = 4;             // one per TMEM lane quarter
 constexpr int TC_EPI_THREADS = 32 * TC_EPI_WARPS;
-// Warp layout.  A warp's scheduler (SM sub-partition) is warp % 4.  The single-thread MMA issuer must
-// not share its scheduler with many compute-bound synthesis warps: a scheduler that always has a
-// ready FMA warp leaves the issuer's scalar instructions waiting for issue slots, and the tensor pipe
-// idles (measured on B200: a tcgen05.mma stream 50x slower next to FMA-bound warps on the same
-// scheduler, unchanged when they sit on the other three).  Scheduler 1 holds the MMA issuer (warp 1),
-// the bulk-copy producer (warp 5), the epilogue warp of TMEM lane quarter 1 (warp 9; a warp reads the
-// TMEM lanes of quarter warp % 4) and one synthesis warp (13); warps 17 and 21 idle.  Schedulers 0, 2
-// and 3 hold one epilogue warp and five synthesis warps each.  Six warps per scheduler leave 80
-// registers per thread (registers are allocated per scheduler, 16,384 each).
+// Warp layout.  A warp's scheduler (SM sub-partition) is warp % 4, and an epilogue warp reads the TMEM
+// lanes of quarter warp % 4.  Each scheduler holds four synthesis warps (4..19), one epilogue warp (0,
+// 21, 2, 3) and one of the MMA issuer (1), the bulk-copy producer (20) and the finishing warps (22, 23).
+// Six warps per scheduler leave 80 registers per thread (registers are allocated per scheduler, 16,384
+// each).
+// What bounds the FP16 form (256 mics, 160,801 points, 513 bins): no pipe is full (issue 55 %, MUFU
+// 46 %, tensor 25 %); the synthesis warps, four to a scheduler, wait on their own chains.  Measured there:
+// the MMAs issued by one divergent lane took 1330 of a step's 2300 clocks, by a converged warp's elected
+// lane 690, and the map values' divisions and loads held the epilogue, and with it the next item's first
+// step, for 400 clocks per step until they moved to warps of their own; together 40.5 -> 38.0 ms
+// (finishing warps alone 39.3, the issue alone 41.0).  64 mics, 10,201 points, 64 bins, FP16: 137 ->
+// 114 us; 560 mics, 32 bins, TF32: 1300 -> 1099 us; 600 mics, 3721 points, split BF16: 757 -> 627 us.
 constexpr int TC_WARPS = 24;
 constexpr int TC_THREADS = 32 * TC_WARPS;
 constexpr int TC_WARP_MMA = 1;
-constexpr int TC_WARP_PRODUCER = 5;
-__host__ __device__ constexpr bool tc_is_epi(int w) { return w == 0 || w == 2 || w == 3 || w == 9; }
+constexpr int TC_WARP_PRODUCER = 20;
+// finishing warps: lane quarters 0, 1 and 2, 3
+constexpr int TC_FIN_THREADS = 64;
+__host__ __device__ constexpr int tc_fin_index(int w) { return w == 22 ? 0 : w == 23 ? 1 : -1; }
+__host__ __device__ constexpr bool tc_is_epi(int w) { return w == 0 || w == 2 || w == 3 || w == 21; }
 // index 0..15 of a synthesis warp, -1 for other warps
 __host__ __device__ constexpr int tc_synth_index(int w)
 {
-    return (w < 4 || w >= TC_WARPS || w == 5 || w == 9 || w == 17 || w == 21)
-               ? -1
-               : (w - 4) - (w > 5) - (w > 9) - (w > 17) - (w > 21);
+    return w < 4 || w >= 4 + TC_SYNTH_WARPS ? -1 : w - 4;
 }
-static_assert(tc_synth_index(4) == 0 && tc_synth_index(13) == 7 && tc_synth_index(23) == TC_SYNTH_WARPS - 1,
-              "synthesis warp indices");
 
 // 2*pi = P2A + P2B + P2C (Cody-Waite split; P2A has 8 significant bits so n*P2A is exact)
 __device__ constexpr float TC_P2A = 0x1.92p+2f;
@@ -123,38 +127,9 @@ struct TcInst {
     uint8_t sp0[TC_MAX_SPLIT + 1];  // pass group s covers passes [sp0[s], sp0[s+1])
     double2 *part;             // [nbins * ntiles][splits][128] partial (B, S) when splits > 1
     int *cnt;                  // [nbins * ntiles][4] finished groups per epilogue warp (zeroed per launch)
-    int small;                 // every item number of the batch < 2^31: item decoding in 32-bit arithmetic
+    // a CTA's next item lies gridDim.x items on: that stride as (bins, tiles, groups), set at the launch
+    int d_bin, d_tile, d_split;
 };
-
-// Position of a work item inside its instance: items run (bin, tile, group) with the group fastest.
-struct TcItem {
-    int64_t base;              // bin * ntiles + tile
-    int bin, split, pa, pz;    // passes [pa, pz)
-    int64_t tile;
-};
-
-__device__ __forceinline__ TcItem decode_item(const TcInst &in, int64_t item)
-{
-    TcItem t;
-    if (in.small) {
-        // 32-bit division: the decode sits on the single-thread MMA issuer's path once per item
-        const uint32_t local = (uint32_t)(item - in.item_off), sp = (uint32_t)in.splits, nt = (uint32_t)in.ntiles;
-        const uint32_t base = local / sp;
-        t.split = (int)(local - base * sp);
-        t.base = base;
-        t.bin = (int)(base / nt);
-        t.tile = base - (uint32_t)t.bin * nt;
-    } else {
-        const int64_t local = item - in.item_off;
-        t.split = (int)(local % in.splits);
-        t.base = local / in.splits;
-        t.bin = (int)(t.base / in.ntiles);
-        t.tile = t.base % in.ntiles;
-    }
-    t.pa = in.sp0[t.split];
-    t.pz = in.sp0[t.split + 1];
-    return t;
-}
 
 constexpr int TC_MAX_INST = 64;
 
@@ -177,6 +152,52 @@ __device__ __forceinline__ int find_inst(const TcBatch &b, int64_t item)
     }
     return lo;
 }
+
+// A CTA's walk over its work items blockIdx.x, + gridDim.x, ...  Inside an instance items run
+// (bin, tile, group) with the group fastest; a step adds the stride's digits with carries, so the
+// divisions of a decode run once per instance only: every role's per-item work sits between two items'
+// steps, and short items feel it (40 mics, 40,401 points, 60 bins, FP16: 364 -> 325 us).
+struct TcWalk {
+    int64_t item;
+    int ii, bin, tile, split;
+
+    __device__ __forceinline__ void locate(const TcBatch &b)
+    {
+        ii = find_inst(b, item);
+        const TcInst &in = b.inst[ii];
+        const int64_t local = item - in.item_off, base = local / in.splits;
+        split = (int)(local - base * in.splits);
+        bin = (int)(base / in.ntiles);
+        tile = (int)(base - bin * in.ntiles);
+    }
+    __device__ __forceinline__ void start(const TcBatch &b)
+    {
+        item = blockIdx.x;
+        locate(b);
+    }
+    __device__ __forceinline__ void next(const TcBatch &b)
+    {
+        item += gridDim.x;
+        if (ii + 1 < b.n_inst && item >= b.inst[ii + 1].item_off) {
+            locate(b);
+            return;
+        }
+        const TcInst &in = b.inst[ii];
+        split += in.d_split;
+        tile += in.d_tile;
+        bin += in.d_bin;
+        if (split >= in.splits) {
+            split -= in.splits;
+            ++tile;
+        }
+        if (tile >= in.ntiles) {
+            tile -= (int)in.ntiles;
+            ++bin;
+        }
+    }
+    // the item's tile among the instance's (bin, tile) pairs
+    __device__ __forceinline__ int64_t base(const TcInst &in) const { return bin * in.ntiles + tile; }
+};
 
 constexpr int TC_NB = 8;       // chunk barrier ring (full_b / done); the producer runs <= 7 chunks ahead
 // The epilogue waits on every step's `done` barrier in turn; the MMAs of step T + TC_NB complete the
@@ -207,9 +228,8 @@ constexpr int TC_HALF = 2;    // FP16, R' scaled per bin by a power of two
 // FP16's full 11-bit precision down to 2^-14 of that scale; the map sums are scaled back by 2^-e.
 // The largest entry of each bin is found first (tc_binmax_kernel) and kept as FP64 bits in the
 // workspace half that the FP16 tiles leave unused.
-__device__ __forceinline__ int tc_half_shift(const unsigned long long *bmax, int bin)
+__device__ __forceinline__ int tc_half_shift(double mx)
 {
-    const double mx = __longlong_as_double((long long)bmax[bin]);
     int ex = 0;
     if (mx > 0.0) frexp(mx, &ex);   // mx < 2^ex
     return mx > 0.0 ? 15 - ex : 0;
@@ -272,7 +292,7 @@ __global__ void __launch_bounds__(256) tc_prep_kernel(const double2 *__restrict_
     const double2 *Cb = csm + (int64_t)bin * M * M;
     __nv_bfloat16 *th = rh + (int64_t)bin * bin_stride + (int64_t)tile_index(C, i, j) * TC_TILE_ELEMS;
     __nv_bfloat16 *tl = rl + (int64_t)bin * bin_stride + (int64_t)tile_index(C, i, j) * TC_TILE_ELEMS;
-    const int shift = PREC == TC_HALF ? tc_half_shift(reinterpret_cast<const unsigned long long *>(rl), bin) : 0;
+    const int shift = PREC == TC_HALF ? tc_half_shift(reinterpret_cast<const double *>(rl)[bin]) : 0;
     for (int e = threadIdx.x; e < TC_TILE_ELEMS; e += blockDim.x) {
         const int rr = e >> 5, kk = e & 31;
         const double val = tc_rprime(Cb, M, r_diag, i, j, rr, kk);
@@ -308,47 +328,42 @@ struct TcSmem {
     }
     __host__ __device__ static constexpr int mic_off(int ns) { return b_base(ns) + 2 * TC_RING * TC_TILE_BYTES; }
     __host__ __device__ static constexpr int red_off(int ns, int Mp) { return mic_off(ns) + Mp * 16; }
-    // per-item normalisation partial sums, double-buffered by item parity: [2][parts][128]
-    __host__ __device__ static constexpr int bar_off(int ns, int Mp) { return red_off(ns, Mp) + 2 * TC_PARTS * TC_ROWS * 8; }
-    __host__ __device__ static constexpr int nbars() { return 2 * TC_ASTAGES_MAX + 3 * TC_NB + 4 + 2; }
+    // per-item sums, double-buffered by item parity: normalisation [2][parts][128], epilogue [2][128]
+    __host__ __device__ static constexpr int bar_off(int ns, int Mp) { return red_off(ns, Mp) + 2 * (TC_PARTS + 1) * TC_ROWS * 8; }
+    __host__ __device__ static constexpr int nbars() { return 2 * TC_ASTAGES_MAX + 3 * TC_NB + 6 + 2; }
     __host__ __device__ static constexpr int total(int ns, int Mp) { return bar_off(ns, Mp) + nbars() * 8 + 16; }
 };
 
-// Reference distance of grid point g (loaded at an item's start, so the epilogue does not wait for
-// the grid positions after the item's last step).
-__device__ __forceinline__ double ref_distance(const TcInst &a, int64_t g)
-{
-    if (a.ref_mode == 1 || g >= a.G) return a.ref_dist;
-    return dist3(a.gpos[g], a.gpos[a.G + g], a.gpos[2 * a.G + g], a.ref0, a.ref1, a.ref2);
-}
-
 // Normalisation of the steering type (acoular/fastFuncs.py:293-310) and clipping.
+// Two points per thread (g0 and g0 + 32), their divisions side by side.
 template <int ST>
-__device__ __forceinline__ void finish_point(const TcInst &a, double scalar, double S, double r0, int bin, int64_t g,
-                                             double *out_map, double *out_norm)
+__device__ __forceinline__ void finish_points(const TcInst &a, const double (&scalar)[2], const double (&S)[2],
+                                              const double (&r0)[2], const bool (&live)[2], int bin, int64_t g0)
 {
     const double Md = (double)a.M;
-    double res, ns;
-    if (ST == 1) {
-        ns = 1.0 / Md;
-        res = scalar / (Md * Md) * a.norm;
-    } else if (ST == 2) {
-        const double nf = Md * r0;
-        const double nf2 = nf * nf;
-        ns = S / nf2;
-        res = scalar / nf2 * a.norm;
-    } else if (ST == 3) {
-        const double nf = r0 * S;
-        ns = 1.0 / (r0 * r0) / S;
-        res = scalar / (nf * nf) * a.norm;
-    } else {
-        const double nf = Md * S;
-        ns = 1.0 / Md;
-        res = scalar / nf * a.norm;
+    double nf[2], res[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (ST == 1) nf[h] = Md * Md;
+        else if (ST == 2) nf[h] = (Md * r0[h]) * (Md * r0[h]);
+        else if (ST == 3) nf[h] = (r0[h] * S[h]) * (r0[h] * S[h]);
+        else nf[h] = Md * S[h];
     }
-    if (a.clip && res < 0.0) res = 0.0;
-    out_map[(int64_t)bin * a.G + g] = res;
-    if (out_norm) out_norm[(int64_t)bin * a.G + g] = ns;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        res[h] = scalar[h] / nf[h] * a.norm;
+        if (a.clip && res[h] < 0.0) res[h] = 0.0;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int64_t g = g0 + 32 * h;
+        if (!live[h] || g >= a.G) continue;
+        a.out[(int64_t)bin * a.G + g] = res[h];
+        if (a.out_norm) {
+            const double ns = ST == 2 ? S[h] / nf[h] : ST == 3 ? 1.0 / (r0[h] * r0[h]) / S[h] : 1.0 / Md;
+            a.out_norm[(int64_t)bin * a.G + g] = ns;
+        }
+    }
 }
 
 // Persistent kernel: one CTA per SM walks the batch's work items (instance, bin, 128-point tile)
@@ -372,6 +387,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) map_tc_kernel(const __grid_cons
     const int NST = b.nstages;
     float4 *mp4 = reinterpret_cast<float4 *>(smem + TcSmem::mic_off(NST));        // [MPX] (x, y, z, w)
     double *red = reinterpret_cast<double *>(smem + TcSmem::red_off(NST, MPX));   // [2][parts][128] sums S
+    double *accs = red + 2 * TC_PARTS * TC_ROWS;                                  // [2][128] epilogue sums
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + TcSmem::bar_off(NST, MPX));
     uint64_t *full_a = bars;                          // [NST] step T written to A stage T % NST
     uint64_t *afree = bars + TC_ASTAGES_MAX;          // [NST] epilogue of step T has released A stage T % NST
@@ -379,11 +395,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) map_tc_kernel(const __grid_cons
     uint64_t *done = full_b + TC_NB;                  // [8]  MMAs of step T complete
     uint64_t *tfree = done + TC_NB;                   // [8]  epilogue has read all columns of window W
     uint64_t *s_ready = tfree + TC_NB;                // [2]  synthesis sums S of item parity written
-    // [2] epilogue has read the sums S of item parity: an item can have fewer steps than the A ring
-    // has stages, so the synthesis warps may finish item li + 2 before the epilogue reaches item li
+    // [2] the finishing warps have read the sums of item parity: an item can have fewer steps than the A
+    // ring has stages, so the synthesis warps may finish item li + 2 before the epilogue reaches item li
     uint64_t *s_free = s_ready + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(s_free + 2);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(s_free + 3);
+    uint64_t *acc_ready = s_free + 2;                 // [2]  epilogue sums of item parity written
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_ready + 2);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(acc_ready + 3);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t nmine = b.nitems > blockIdx.x ? (b.nitems - 1 - blockIdx.x) / gridDim.x + 1 : 0;
@@ -401,8 +418,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) map_tc_kernel(const __grid_cons
         for (int s = 0; s < TC_NB; ++s) tc::mbar_init(&tfree[s], TC_EPI_THREADS);
         tc::mbar_init(&s_ready[0], TC_SYNTH_THREADS);
         tc::mbar_init(&s_ready[1], TC_SYNTH_THREADS);
-        tc::mbar_init(&s_free[0], TC_EPI_THREADS);
-        tc::mbar_init(&s_free[1], TC_EPI_THREADS);
+        tc::mbar_init(&s_free[0], TC_FIN_THREADS);
+        tc::mbar_init(&s_free[1], TC_FIN_THREADS);
+        tc::mbar_init(&acc_ready[0], TC_EPI_THREADS);
+        tc::mbar_init(&acc_ready[1], TC_EPI_THREADS);
         *abort_flag = 0;
         tc::fence_mbar_init();
     }
@@ -426,15 +445,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) map_tc_kernel(const __grid_cons
             uint32_t U = 0;
             int T = 0, freed = -1, lastT = -1;
             bool ok = true;
-            for (int64_t li = 0; li < nmine && ok; ++li) {
-                const int64_t item = blockIdx.x + li * gridDim.x;
-                const TcInst &in = b.inst[find_inst(b, item)];
-                const TcItem it = decode_item(in, item);
+            TcWalk it;
+            it.start(b);
+            for (int64_t li = 0; li < nmine && ok; ++li, it.next(b)) {
+                const TcInst &in = b.inst[it.ii];
+                const int pa = in.sp0[it.split], pz = in.sp0[it.split + 1];
                 const int C = in.C, pw = in.pw;
                 const int64_t bin = it.bin;
                 const __nv_bfloat16 *bh = in.rh + (TF32 ? 2 : 1) * bin * in.bin_stride;   // FP16: halves
                 const __nv_bfloat16 *bl = in.rl + bin * in.bin_stride;
-                for (int pp = it.pa; pp < it.pz && ok; ++pp) {
+                for (int pp = pa; pp < pz && ok; ++pp) {
                     const int jb = pp * pw, je = min(C, jb + pw);
                     for (int i0 = 0; i0 < je && ok; i0 += CPS, ++T) {
                         const int i1 = min(je, i0 + CPS);
@@ -493,112 +513,101 @@ __global__ void __launch_bounds__(TC_THREADS, 1) map_tc_kernel(const __grid_cons
         }
     } else if (warp == TC_WARP_MMA) {
         // ---------------- MMA issuer ----------------
-        // Kept lean: it sits on every step's critical path.  Descriptors are built once and
-        // advanced by adding byte offsets >> 4 to their 14-bit start-address field; ring and
-        // stage indices are 32-bit counters advanced incrementally.
-        if (lane == 0) {
-            // BF16: 8-row x 8-element core matrices, 4 per 32-component row group (SBO 512);
-            // TF32: 8-row x 4-element core matrices, 8 per row group (SBO 1024)
-            constexpr uint32_t SBO = TF32 ? 1024 : 512;
-            const uint64_t a_base = tc::sdesc_noswizzle(tc::smem_u32(smem + TcSmem::a_off(0, 0)), 128, SBO);
-            const uint64_t b_base = tc::sdesc_noswizzle(tc::smem_u32(smem + TcSmem::b_off(NST, 0, 0)), 128, SBO);
-            constexpr uint32_t A_STEP = TC_A_BYTES >> 4;          // next (stage, hi|lo) block
-            constexpr uint32_t T_STEP = (TF32 ? 2 : 1) * (TC_TILE_BYTES >> 4);   // next ring tile
-            constexpr uint32_t LO_B = (TC_RING * TC_TILE_BYTES) >> 4;
-            // operand format: 0 = FP16, 1 = BF16 (kind::f16), 2 = TF32 (kind::tf32)
-            const uint32_t idesc0 = tc::idesc_m128(TF32 ? 2 : (HALF ? 0 : 1), 0);
-            int sa = 0, ua = 0;     // A stage and its phase parity
-            int sb = 0, ub = 0;     // step barrier slot and parity
-            uint32_t slot0 = 0;     // ring slot of the step's first tile
-            int lastb = -1, lastu = 0;
-            // accumulator windows (one per column pass) rotate through TMEM in slots of the
-            // instance's width; a slot is reused once the epilogue has released the window that
-            // last held it.  An instance change drains all windows and restarts the rotation.
-            int W = 0, w_start = 0, wpt = 1, width = 512, cur_inst = -1;
-            bool ok = true;
-            for (int64_t li = 0; li < nmine && ok; ++li) {
-                const int64_t item = blockIdx.x + li * gridDim.x;
-                const int ii = find_inst(b, item);
-                const TcItem it = decode_item(b.inst[ii], item);
-                const int C = b.inst[ii].C, pw = b.inst[ii].pw;
-                if (ii != cur_inst) {
-                    if (W > 0)
-                        ok = tc::mbar_wait(&tfree[(W - 1) & (TC_NB - 1)], (uint32_t)(((W - 1) / TC_NB) & 1), abort_flag,
-                                           b.wait_limit_ns);
-                    width = TC_CHUNK * min(C, pw);
-                    wpt = min(TC_NB, 512 / width);
-                    w_start = W;
-                    cur_inst = ii;
-                }
-                for (int pp = it.pa; pp < it.pz && ok; ++pp, ++W) {
-                    const int jb = pp * pw, je = min(C, jb + pw);
-                    if (W - w_start >= wpt)
-                        ok = tc::mbar_wait(&tfree[(W - wpt) & (TC_NB - 1)], (uint32_t)(((W - wpt) / TC_NB) & 1),
-                                           abort_flag, b.wait_limit_ns);
-                    const uint32_t wcol = taddr + (uint32_t)(((W - w_start) % wpt) * width);
-                    for (int i0 = 0; i0 < je && ok; i0 += CPS) {
-                        ok = tc::mbar_wait(&full_a[sa], (uint32_t)ua, abort_flag, b.wait_limit_ns) &&
-                             tc::mbar_wait(&full_b[sb], (uint32_t)ub, abort_flag, b.wait_limit_ns);
-                        if (!ok) break;
-                        tc::tc_fence_after();
-                        for (int i = i0; i < min(je, i0 + CPS); ++i) {
-                            const int j0 = max(i, jb), n = je - j0;
-                            const uint32_t dcol = wcol + (uint32_t)(TC_CHUNK * (j0 - jb));
-                            // split the step's n tiles into runs of <= 8 (N <= 256) that do not wrap
-                            const int run0 = min(min(n, 8), (int)(RING - slot0));
-                            const uint32_t slot1 = (slot0 + run0) & (RING - 1);
-                            const int rest = n - run0;
-                            const int run1 = min(min(rest, 8), (int)(RING - slot1));
-                            const uint32_t slot2 = (slot1 + run1) & (RING - 1);
-                            const int run2 = rest - run1;   // at most one more run (n <= 16)
-                            // BF16: K steps of 16 (2) x products hi*hi, hi*lo, lo*hi; TF32: K steps of 8 (4) x 1;
-                            // FP16: K steps of 16 (2) x 1
-                            constexpr int KS = TF32 ? 4 : 2, NPROD = SPLIT ? 3 : 1;
+        // It sits on every step's critical path.  The whole warp runs the loop and one elected lane
+        // issues, so every descriptor, column and instruction word is the same in all lanes.
+        const bool leader = tc::elect_one();
+        // BF16: 8-row x 8-element core matrices, 4 per 32-component row group (SBO 512);
+        // TF32: 8-row x 4-element core matrices, 8 per row group (SBO 1024)
+        constexpr uint32_t SBO = TF32 ? 1024 : 512;
+        const uint64_t a_base = tc::sdesc_noswizzle(tc::smem_u32(smem + TcSmem::a_off(0, 0)), 128, SBO);
+        const uint64_t b_base = tc::sdesc_noswizzle(tc::smem_u32(smem + TcSmem::b_off(NST, 0, 0)), 128, SBO);
+        constexpr uint32_t A_STEP = TC_A_BYTES >> 4;          // next (stage, hi|lo) block
+        constexpr uint32_t T_STEP = (TF32 ? 2 : 1) * (TC_TILE_BYTES >> 4);   // next ring tile
+        constexpr uint32_t LO_B = (TC_RING * TC_TILE_BYTES) >> 4;
+        // operand format: 0 = FP16, 1 = BF16 (kind::f16), 2 = TF32 (kind::tf32)
+        const uint32_t idesc0 = tc::idesc_m128(TF32 ? 2 : (HALF ? 0 : 1), 0);
+        const uint32_t tbase = __shfl_sync(0xffffffffu, taddr, 0);
+        int sa = 0, ua = 0;     // A stage and its phase parity
+        int sb = 0, ub = 0;     // step barrier slot and parity
+        uint32_t slot = 0;      // ring slot of the next tile
+        int lastb = -1, lastu = 0;
+        // accumulator windows (one per column pass) rotate through TMEM in slots of the
+        // instance's width; a slot is reused once the epilogue has released the window that
+        // last held it.  An instance change drains all windows and restarts the rotation.
+        int W = 0, w_start = 0, wslot = 0, wpt = 1, width = 512, cur_inst = -1;
+        bool ok = true;
+        TcWalk it;
+        it.start(b);
+        for (int64_t li = 0; li < nmine && ok; ++li, it.next(b)) {
+            const int ii = it.ii, pa = b.inst[ii].sp0[it.split], pz = b.inst[ii].sp0[it.split + 1];
+            const int C = b.inst[ii].C, pw = b.inst[ii].pw;
+            if (ii != cur_inst) {
+                if (W > 0)
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait(&tfree[(W - 1) & (TC_NB - 1)],
+                                                               (uint32_t)(((W - 1) / TC_NB) & 1), abort_flag,
+                                                               b.wait_limit_ns));
+                width = TC_CHUNK * min(C, pw);
+                wpt = min(TC_NB, 512 / width);
+                w_start = W;
+                wslot = 0;
+                cur_inst = ii;
+            }
+            for (int pp = pa; pp < pz && ok; ++pp, ++W) {
+                const int jb = pp * pw, je = min(C, jb + pw);
+                if (W - w_start >= wpt)
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait(&tfree[(W - wpt) & (TC_NB - 1)],
+                                                               (uint32_t)(((W - wpt) / TC_NB) & 1), abort_flag,
+                                                               b.wait_limit_ns));
+                const uint32_t wcol = tbase + (uint32_t)(wslot * width);
+                if (++wslot == wpt) wslot = 0;
+                for (int i0 = 0; i0 < je && ok; i0 += CPS) {
+                    ok = __all_sync(0xffffffffu,
+                                    tc::mbar_wait(&full_a[sa], (uint32_t)ua, abort_flag, b.wait_limit_ns) &&
+                                        tc::mbar_wait(&full_b[sb], (uint32_t)ub, abort_flag, b.wait_limit_ns));
+                    if (!ok) break;
+                    tc::tc_fence_after();
+                    for (int i = i0; i < min(je, i0 + CPS); ++i) {
+                        const int j0 = max(i, jb), n = je - j0;
+                        uint32_t dcol = wcol + (uint32_t)(TC_CHUNK * (j0 - jb));
+                        // A: split-BF16 hi (lo for the third product), FP32, or FP16 chunk i - i0 of the stage
+                        const uint64_t ad0 = a_base + (uint64_t)((sa * 2 + (HALF ? i - i0 : 0)) * A_STEP);
+                        // BF16: K steps of 16 (2) x products hi*hi, hi*lo, lo*hi; TF32: K steps of 8 (4) x 1;
+                        // FP16: K steps of 16 (2) x 1
+                        constexpr int KS = TF32 ? 4 : 2, NPROD = SPLIT ? 3 : 1;
+                        // the chunk's n tiles in runs of <= 8 (N <= 256) that do not wrap in the ring
+                        for (int left = n; left > 0;) {
+                            const int run = min(min(left, 8), (int)(RING - slot));
+                            const uint32_t idesc = idesc0 | ((uint32_t)(run * 4) << 17);
+                            const uint64_t bd0 = b_base + (uint64_t)(slot * T_STEP);
 #pragma unroll
                             for (int ks = 0; ks < KS; ++ks) {
 #pragma unroll
                                 for (int prod = 0; prod < NPROD; ++prod) {
-                                    // A: split-BF16 hi (lo for the third product), FP32, or FP16 chunk
-                                    // i - i0 of the stage
-                                    const int ablk = sa * 2 + (HALF ? (i - i0) : (prod == 2));
-                                    const uint64_t ad = a_base + (uint64_t)(ablk * A_STEP + ks * 16);
-                                    const uint64_t bd = b_base + (uint64_t)((prod == 1 ? LO_B : 0u) + ks * 16);
+                                    const uint64_t ad = ad0 + (uint64_t)((prod == 2 ? A_STEP : 0u) + ks * 16);
+                                    const uint64_t bd = bd0 + (uint64_t)((prod == 1 ? LO_B : 0u) + ks * 16);
                                     const uint32_t accum = (i == 0 && ks == 0 && prod == 0) ? 0u : 1u;
-                                    const uint32_t n0 = idesc0 | ((uint32_t)(run0 * 4) << 17);
-                                    const uint32_t n1 = idesc0 | ((uint32_t)(run1 * 4) << 17);
-                                    const uint32_t n2 = idesc0 | ((uint32_t)(run2 * 4) << 17);
-                                    if (TF32) {
-                                        tc::mma_tf32(dcol, ad, bd + slot0 * T_STEP, n0, accum);
-                                        if (run1 > 0)
-                                            tc::mma_tf32(dcol + (uint32_t)(run0 * TC_CHUNK), ad, bd + slot1 * T_STEP, n1,
-                                                        accum);
-                                        if (run2 > 0)
-                                            tc::mma_tf32(dcol + (uint32_t)((run0 + run1) * TC_CHUNK), ad,
-                                                        bd + slot2 * T_STEP, n2, accum);
-                                    } else {
-                                        tc::mma_bf16(dcol, ad, bd + slot0 * T_STEP, n0, accum);
-                                        if (run1 > 0)
-                                            tc::mma_bf16(dcol + (uint32_t)(run0 * TC_CHUNK), ad, bd + slot1 * T_STEP, n1,
-                                                        accum);
-                                        if (run2 > 0)
-                                            tc::mma_bf16(dcol + (uint32_t)((run0 + run1) * TC_CHUNK), ad,
-                                                        bd + slot2 * T_STEP, n2, accum);
+                                    if (leader) {
+                                        if (TF32) tc::mma_tf32(dcol, ad, bd, idesc, accum);
+                                        else tc::mma_bf16(dcol, ad, bd, idesc, accum);
                                     }
                                 }
                             }
-                            slot0 = (slot0 + (uint32_t)n) & (RING - 1);
+                            dcol += (uint32_t)(run * TC_CHUNK);
+                            slot = (slot + (uint32_t)run) & (RING - 1);
+                            left -= run;
                         }
-                        tc::mma_commit(&done[sb]);
-                        lastb = sb;
-                        lastu = ub;
-                        if (++sa == NST) { sa = 0; ua ^= 1; }
-                        if (++sb == TC_NB) { sb = 0; ub ^= 1; }
                     }
+                    if (leader) tc::mma_commit(&done[sb]);
+                    __syncwarp();
+                    lastb = sb;
+                    lastu = ub;
+                    if (++sa == NST) { sa = 0; ua ^= 1; }
+                    if (++sb == TC_NB) { sb = 0; ub ^= 1; }
                 }
             }
-            // MMAs complete in issue order: the last commit covers all of them
-            if (lastb >= 0) tc::mbar_drain(&done[lastb], (uint32_t)lastu, tc::drain_limit_ns(b.wait_limit_ns));
         }
+        // MMAs complete in issue order: the last commit covers all of them
+        if (lastb >= 0) tc::mbar_drain(&done[lastb], (uint32_t)lastu, tc::drain_limit_ns(b.wait_limit_ns));
     } else if (tc_is_epi(warp)) {
         // ---------------- epilogue (warps 0, 9, 2, 3 for lane quarters 0..3): one thread per grid point
         // After step (p, i) with i >= 16p the accumulator columns of chunk i are final; dot them
@@ -609,28 +618,25 @@ __global__ void __launch_bounds__(TC_THREADS, 1) map_tc_kernel(const __grid_cons
         const uint32_t lane_addr = taddr + ((uint32_t)(q * 32) << 16);
         const int a_row = ((row >> 3) << 9) + ((row & 7) << 4);   // byte offset of the row's first chunk
         int T = 0, sa = 0;
-        int W = 0, w_start = 0, wpt = 1, width = 512, cur_inst = -1;   // same window rotation as the MMAs
+        int W = 0, wslot = 0, wpt = 1, width = 512, cur_inst = -1;   // same window rotation as the MMAs
         bool ok = true;
-        for (int64_t li = 0; li < nmine && ok; ++li) {
-            const int64_t item = blockIdx.x + li * gridDim.x;
-            const int ii = find_inst(b, item);
+        TcWalk it;
+        it.start(b);
+        for (int64_t li = 0; li < nmine && ok; ++li, it.next(b)) {
+            const int ii = it.ii;
             const TcInst &in = b.inst[ii];
-            const TcItem it = decode_item(in, item);
-            const int C = in.C, pw = in.pw;
+            const int C = in.C, pw = in.pw, pa = in.sp0[it.split], pz = in.sp0[it.split + 1];
             if (ii != cur_inst) {
                 width = TC_CHUNK * min(C, pw);
                 wpt = min(TC_NB, 512 / width);
-                w_start = W;
+                wslot = 0;
                 cur_inst = ii;
             }
-            const int bin = it.bin;
-            const int64_t g = it.tile * TC_ROWS + row;
-            // (split BF16 has no registers to spare across the steps: it loads them after the last one)
-            const double r0 = SPLIT ? 0.0 : ref_distance(in, g);
             double acc = 0.0;
-            for (int pp = it.pa; pp < it.pz && ok; ++pp, ++W) {
+            for (int pp = pa; pp < pz && ok; ++pp, ++W) {
                 const int jb = pp * pw, je = min(C, jb + pw);
-                const uint32_t wcol = lane_addr + (uint32_t)(((W - w_start) % wpt) * width);
+                const uint32_t wcol = lane_addr + (uint32_t)(wslot * width);
+                if (++wslot == wpt) wslot = 0;
                 for (int i0 = 0; i0 < je; i0 += CPS, ++T) {
                     ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[T & (TC_NB - 1)], (uint32_t)((T / TC_NB) & 1),
                                                                abort_flag, b.wait_limit_ns));
@@ -702,46 +708,107 @@ __global__ void __launch_bounds__(TC_THREADS, 1) map_tc_kernel(const __grid_cons
                 tc::mbar_arrive(&tfree[W & (TC_NB - 1)]);
             }
             if (!ok) break;
+            // the slot of item li - 2 must have been read
+            if (li >= 2) {
+                ok = __all_sync(0xffffffffu, tc::mbar_wait(&s_free[li & 1], (uint32_t)(((li >> 1) - 1) & 1),
+                                                           abort_flag, b.wait_limit_ns));
+                if (!ok) break;
+            }
+            accs[(li & 1) * TC_ROWS + row] = acc;
+            tc::mbar_arrive(&acc_ready[li & 1]);
+        }
+    } else if (tc_fin_index(warp) >= 0) {
+        // ---------------- finishing (warps 22, 23): an item's sums to its map values ----------------
+        // Two points per thread, positions and scale loaded one item ahead: with items of one step (24
+        // mics, 14,641 points, 100 bins, FP16) this warp's chain of loads and divisions is what bounds
+        // the CTA (one point after the other, loads at the item's start: inverse steering 227 us, this
+        // form 205, by the epilogue warps 217).
+        const int q0 = 2 * tc_fin_index(warp);
+        bool ok = true;
+        TcWalk nx;   // the item whose positions and scale are being loaded: one ahead of the sums
+        double px[2], py[2], pz[2], bmax = 0.0;
+        auto fetch = [&]() {
+            const TcInst &in = b.inst[nx.ii];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int64_t g = (int64_t)nx.tile * TC_ROWS + (q0 + h) * 32 + lane;
+                px[h] = py[h] = pz[h] = 0.0;
+                if (g < in.G && in.ref_mode != 1) {
+                    px[h] = in.gpos[g];
+                    py[h] = in.gpos[in.G + g];
+                    pz[h] = in.gpos[2 * in.G + g];
+                }
+            }
+            if (HALF) bmax = reinterpret_cast<const double *>(in.rl)[nx.bin];
+        };
+        nx.start(b);
+        if (nmine > 0) fetch();
+        for (int64_t li = 0; li < nmine && ok; ++li) {
+            const TcWalk it = nx;
+            const TcInst &in = b.inst[it.ii];
+            const int bin = it.bin;
+            const int64_t g0 = (int64_t)it.tile * TC_ROWS + q0 * 32 + lane;   // and g0 + 32
+            double accv[2], Sv[2], r0v[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                r0v[h] = in.ref_mode == 1 ? in.ref_dist : dist3(px[h], py[h], pz[h], in.ref0, in.ref1, in.ref2);
+            const int shift = HALF ? tc_half_shift(bmax) : 0;
+            nx.next(b);
+            if (li + 1 < nmine) fetch();
+            ok = __all_sync(0xffffffffu, tc::mbar_wait(&s_ready[li & 1], (uint32_t)((li >> 1) & 1), abort_flag,
+                                                       b.wait_limit_ns) &&
+                                             tc::mbar_wait(&acc_ready[li & 1], (uint32_t)((li >> 1) & 1), abort_flag,
+                                                           b.wait_limit_ns));
+            if (!ok) break;
+            const double *rs = red + (li & 1) * TC_PARTS * TC_ROWS;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int row = (q0 + h) * 32 + lane;
+                accv[h] = accs[(li & 1) * TC_ROWS + row];
+                Sv[h] = 0.0;
+#pragma unroll
+                for (int pp = 0; pp < TC_PARTS; ++pp) Sv[h] += rs[pp * TC_ROWS + row];
+            }
+            tc::mbar_arrive(&s_free[li & 1]);
             if (HALF) {
                 // undo the bin's R' scale; an FP16 steering value out of range (|w| >= 65520) shows as a
                 // non-finite sum and raises bit 2 of the error word
-                acc = ldexp(acc, -tc_half_shift(reinterpret_cast<const unsigned long long *>(in.rl), bin));
-                if (g < in.G && !isfinite(acc) && err) atomicOr(err, 2);
-            }
-            // normalisation sums of this item from the synthesis warps
-            ok = __all_sync(0xffffffffu, tc::mbar_wait(&s_ready[li & 1], (uint32_t)((li >> 1) & 1), abort_flag,
-                                                       b.wait_limit_ns));
-            if (!ok) break;
-            const double *rs = red + (li & 1) * TC_PARTS * TC_ROWS;
-            double S = 0.0;
 #pragma unroll
-            for (int pp = 0; pp < TC_PARTS; ++pp) S += rs[pp * TC_ROWS + row];
-            tc::mbar_arrive(&s_free[li & 1]);
+                for (int h = 0; h < 2; ++h) {
+                    accv[h] = ldexp(accv[h], -shift);
+                    if (g0 + 32 * h < in.G && !isfinite(accv[h]) && err) atomicOr(err, 2);
+                }
+            }
+            bool last[2] = {true, true};
             if (in.splits > 1) {
                 // publish this group's partial sums; the last group of the (bin, tile) to finish
                 // adds all groups' partials in group order and writes the map
-                // (per warp: a warp's 32 rows are counted on their own, so no barrier spans warps)
-                double2 *pb = in.part + it.base * in.splits * TC_ROWS;
-                pb[it.split * TC_ROWS + row] = make_double2(acc, S);
+                // (per lane quarter: its 32 rows are counted on their own, so no barrier spans warps)
+                double2 *pb = in.part + it.base(in) * in.splits * TC_ROWS + q0 * 32 + lane;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) pb[it.split * TC_ROWS + 32 * h] = make_double2(accv[h], Sv[h]);
                 __threadfence();
                 __syncwarp();
-                int last = 0;
-                if (lane == 0) last = atomicAdd(&in.cnt[it.base * 4 + q], 1) == in.splits - 1;
-                last = __shfl_sync(0xffffffffu, last, 0);
-                if (!last) continue;
+                int n = 0;
+                if (lane < 2) n = atomicAdd(&in.cnt[it.base(in) * 4 + q0 + lane], 1) == in.splits - 1;
+                last[0] = __shfl_sync(0xffffffffu, n, 0);
+                last[1] = __shfl_sync(0xffffffffu, n, 1);
                 __threadfence();
-                acc = 0.0;
-                S = 0.0;
-                for (int s = 0; s < in.splits; ++s) {
-                    const double2 v = __ldcg(pb + s * TC_ROWS + row);
-                    acc += v.x;
-                    S += v.y;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (!last[h]) continue;
+                    accv[h] = Sv[h] = 0.0;
+                    for (int s = 0; s < in.splits; ++s) {
+                        const double2 v = __ldcg(pb + s * TC_ROWS + 32 * h);
+                        accv[h] += v.x;
+                        Sv[h] += v.y;
+                    }
                 }
             }
-            if (g < in.G) finish_point<ST>(in, acc, S, SPLIT ? ref_distance(in, g) : r0, bin, g, in.out, in.out_norm);
+            finish_points<ST>(in, accv, Sv, r0v, last, bin, g0);
         }
     } else if (tc_synth_index(warp) >= 0) {
-        // ---------------- steering synthesis (16 warps off scheduler 1) ----------------
+        // ---------------- steering synthesis (16 warps) ----------------
         // Synthesis warp s serves grid points 32q..32q+31 (q = s % 4) and part p = s / 4 of every
         // chunk: mics 4p..4p+3 of the chunk's 16, i.e. one 16-byte core-matrix column of the A tile.
         // The arithmetic runs on mic pairs in packed FP32 (.f32x2): one instruction per pair.
@@ -757,30 +824,31 @@ __global__ void __launch_bounds__(TC_THREADS, 1) map_tc_kernel(const __grid_cons
         // the grid point and wave number of an item are loaded one item ahead, so that their global-memory
         // latency overlaps the previous item's steps (at the item's start for split BF16, whose
         // synthesis has no registers to spare)
-        float nx = -TC_FAR, ny = -TC_FAR, nz = -TC_FAR;
+        double nx = -TC_FAR, ny = -TC_FAR, nz = -TC_FAR;
         double nk = 0.0;
-        auto fetch = [&](int64_t lj) {
-            const int64_t itm = blockIdx.x + lj * gridDim.x;
-            const TcInst &ij = b.inst[find_inst(b, itm)];
-            const TcItem tj = decode_item(ij, itm);
-            const int64_t gj = tj.tile * TC_ROWS + row;
+        TcWalk it;
+        auto fetch = [&]() {
+            const TcInst &ij = b.inst[it.ii];
+            const int64_t gj = (int64_t)it.tile * TC_ROWS + row;
             nx = ny = nz = -TC_FAR;
             if (gj < ij.G) {
-                nx = (float)ij.gpos[gj];
-                ny = (float)ij.gpos[ij.G + gj];
-                nz = (float)ij.gpos[2 * ij.G + gj];
+                nx = ij.gpos[gj];
+                ny = ij.gpos[ij.G + gj];
+                nz = ij.gpos[2 * ij.G + gj];
             }
-            nk = ij.k[tj.bin];
+            nk = ij.k[it.bin];
         };
-        if (!SPLIT && nmine > 0) fetch(0);
+        it.start(b);
+        if (!SPLIT && nmine > 0) fetch();
         for (int64_t li = 0; li < nmine && ok; ++li) {
-            const int64_t item = blockIdx.x + li * gridDim.x;
-            const int ii = find_inst(b, item);
+            const int ii = it.ii;
             const TcInst &in = b.inst[ii];
-            if (SPLIT) fetch(li);
-            const float gxf = nx, gyf = ny, gzf = nz;
+            const int pa = in.sp0[it.split], pz = in.sp0[it.split + 1];
+            if (SPLIT) fetch();
+            const float gxf = (float)nx, gyf = (float)ny, gzf = (float)nz;
             const double k = nk;
-            if (!SPLIT && li + 1 < nmine) fetch(li + 1);
+            it.next(b);
+            if (!SPLIT && li + 1 < nmine) fetch();
             if (ii != cur_inst) {
                 // new instance: every synthesis thread is past the previous item, reload the mics
                 asm volatile("bar.sync 2, %0;" ::"r"(TC_SYNTH_THREADS) : "memory");
@@ -801,14 +869,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) map_tc_kernel(const __grid_cons
                 asm volatile("bar.sync 2, %0;" ::"r"(TC_SYNTH_THREADS) : "memory");
                 cur_inst = ii;
             }
-            const TcItem it = decode_item(in, item);
             const int C = in.C, pw = in.pw;
             const uint64_t GX = tc::f2_splat(gxf), GY = tc::f2_splat(gyf), GZ = tc::f2_splat(gzf);
             const float khi = (float)k, klo = (float)(k - (double)khi);
             const uint64_t KH = tc::f2_splat(khi), KL = tc::f2_splat(klo);
             const uint64_t NKH = tc::f2_splat(-khi), NKL = tc::f2_splat(-klo);
             double S = 0.0;
-            for (int pp = it.pa; pp < it.pz && ok; ++pp) {
+            for (int pp = pa; pp < pz && ok; ++pp) {
                 const int jb = pp * pw, je = min(C, jb + pw);
                 // packed FP32 running sums of the normalisation terms of 4 consecutive chunks (8 per lane),
                 // added to the FP64 sum per group: passes start at multiples of 4 chunks, so the groups, and
@@ -997,7 +1064,6 @@ static int tc_fill_inst(const acb_map_params *p, const void *csm, const double *
     in.sp0[1] = (uint8_t)in.P;
     in.part = nullptr;
     in.cnt = nullptr;
-    in.small = 0;   // set once the batch's item count is known
     return ACB_OK;
 }
 
@@ -1115,6 +1181,13 @@ static int tc_launch(TcBatch &bt, const acb_map_params *const *params, const voi
     // that no second CTA fits (a second one would stall in tcgen05.alloc until the first exits)
     if (smem < 116 * 1024) smem = 116 * 1024;
     const dim3 grid((unsigned)(bt.nitems < nsm ? bt.nitems : nsm));
+    for (int i = 0; i < bt.n_inst; ++i) {
+        TcInst &in = bt.inst[i];
+        const int64_t q = grid.x / in.splits;
+        in.d_split = (int)(grid.x % in.splits);
+        in.d_tile = (int)(q % in.ntiles);
+        in.d_bin = (int)(q / in.ntiles);
+    }
     using KernT = void (*)(const TcBatch, int *);
     static const KernT kernels[4][3] = {
         {map_tc_kernel<1, TC_SPLIT>, map_tc_kernel<1, TC_TF>, map_tc_kernel<1, TC_HALF>},
@@ -1161,7 +1234,6 @@ int acb_map_tc(const acb_map_params *p, int precision, const void *csm, const do
     const size_t need = acb_map_tc_workspace_bytes(p->num_mics, p->num_bins, precision);
     if (!workspace || workspace_bytes < need) return ACB_ERR_WORKSPACE;
     bt.nitems = bt.inst[0].ntiles * bt.inst[0].nbins;
-    bt.inst[0].small = bt.nitems < (int64_t(1) << 31);
     const acb_map_params *pp[1] = {p};
     const void *cc[1] = {csm};
     return tc_launch(bt, pp, cc, p->steer_type, precision, error_word, as_stream(stream));
@@ -1214,7 +1286,6 @@ int acb_map_tc_batch(const acb_map_params *params, const acb_map_io *io, int num
         cc[i] = io[i].csm;
     }
     bt.nitems = items;
-    for (int i = 0; i < num_instances; ++i) bt.inst[i].small = items < (int64_t(1) << 31);
     return tc_launch(bt, pp, cc, steer, precision, error_word, as_stream(stream));
 }
 
