@@ -182,7 +182,7 @@ class PowerSpectra:
     def _samples_device(self) -> torch.Tensor:
         x = self._samples_host_or_device()
         if x.device.type == 'cpu':
-            x = x.to(self._device(), non_blocking=x.is_pinned())
+            x = D.upload_samples(x, self._device())
         return x.contiguous()
 
     def _csm_streamed(self, x: torch.Tensor, prec: str, nchunks: int = 8) -> torch.Tensor:
