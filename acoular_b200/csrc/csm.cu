@@ -41,7 +41,9 @@ void set_cuda_error(cudaError_t e) { g_last_cuda_error = cudaGetErrorString(e); 
 // thread keeps its task's twiddles for all of its mics, and it reads four of the seven: the others are those times -i.
 // Bound: shared memory (seven 16-byte accesses per point) and the FP64 pipe, about 0.5 ms each for 999 windows x 256
 // mics x 1024 samples.  Measured (B200): that transform 2.65 -> 1.24 ms (before: two more trips through shared
-// memory, a twiddle load per butterfly and runtime divisions by the mic count in the index arithmetic).
+// memory, a twiddle load per butterfly and runtime divisions by the mic count in the index arithmetic).  The lane order of the load
+// and the paired bins of the split give 4 to 8 % of a whole CSM where few mics fit a CTA (113 mics, block 4096, 75 %
+// overlap, complex64: 995 -> 958 us; 16 mics, block 16384: 371 -> 342) and 0.2 to 1 % elsewhere.
 // ------------------------------------------------------------------------------------------------
 // Shared-memory slot of point j of a mic's sequence: one padding slot after every 8 points, so that
 // 8 threads reading 16-byte points 8 apart (the first pass) or 64 apart hit different banks.
@@ -151,6 +153,20 @@ __device__ __forceinline__ void first_stages(double2 (&v)[8])
     butterfly(v[3], v[7], make_double2(-h, -h));
 }
 
+// The low n bits of x in reverse order.
+__device__ __forceinline__ int bit_reverse(int x, int n) { return n ? (int)(__brev((unsigned)x) >> (32 - n)) : 0; }
+
+// The pairs (u, H - u), u = u0 .. u0 + n - 1 <= H / 2, that hold the bins bin_lo .. bin_lo + nbins - 1 of 0 .. H.
+struct SplitPairs {
+    int u0, n;
+    __device__ __forceinline__ SplitPairs(int bin_lo, int nbins, int H)
+    {
+        const int last = bin_lo + nbins - 1, a = min(bin_lo, H - bin_lo), b = min(last, H - last);
+        u0 = min(a, b);
+        n = (2 * bin_lo <= H && 2 * last >= H ? H >> 1 : max(a, b)) - u0 + 1;
+    }
+};
+
 // Blocks from this size on take wide CTAs (more mics, 512 threads; see fft_mics_per_block and fft4_mics_per_block).
 // (Measured, CSM of 256 mics x 300,000 samples, block 8192, complex64: 6.29 -> 5.52 ms; 113 mics, block 2048: 0.93 ->
 // 0.91; block 512, 256 mics: 2.53 -> 2.65, so not below 2048.)
@@ -211,10 +227,14 @@ __global__ void __launch_bounds__(512) fft_window_kernel(const TS *__restrict__ 
     // load + window + the first three stages: task = 8 consecutive slots of the bit-reversed order, i.e. points
     // rev(task) + H/8 {0, 4, 2, 6, 1, 5, 3, 7} (H >= 8)
     const int logT = logH - 3;
+    // Lanes run along the mics, then (fewer than 8 mics) along the task, so that eight lanes store to eight banks, then
+    // along the rows: the window's values of a warp lie next to one another.
+    const int tl = min(max(3 - logP, 0), logT);
     for (int idx = threadIdx.x; idx < mpb << logT; idx += blockDim.x) {
-        const int ml = idx & (mpb - 1), task = idx >> logP;
+        const int ml = idx & (mpb - 1), a = idx >> logP, jl = a >> tl, low = a & ((1 << tl) - 1);
         if (ml >= nm) continue;
-        const int j0 = logT ? (int)(__brev((unsigned)task) >> (32 - logT)) : 0;
+        const int task = low | (bit_reverse(jl, logT - tl) << tl);
+        const int j0 = jl | (bit_reverse(low, tl) << (logT - tl));
         double2 v[8];
         TS x0[8], x1[8];
 #pragma unroll
@@ -237,19 +257,25 @@ __global__ void __launch_bounds__(512) fft_window_kernel(const TS *__restrict__ 
     fft_passes(zs, nm, stride, 3, logH, logH + 1, tw);
 
     // real-input split: X[k] = E + W^k O,  E = (Z[k] + conj(Z[H-k]))/2,  O = -i (Z[k] - conj(Z[H-k]))/2
-    for (int idx = threadIdx.x; idx < nbins << logP; idx += blockDim.x) {
+    // (bins k and H - k share their two points: read once for both)
+    const SplitPairs sp(bin_lo, nbins, H);
+    for (int idx = threadIdx.x; idx < sp.n << logP; idx += blockDim.x) {
         const int ml = idx & (mpb - 1);
         if (ml >= nm) continue;
-        const int k = bin_lo + (idx >> logP), kh = k & (H - 1);
+        const int u = sp.u0 + (idx >> logP);
         const double2 *z = zs + ml * stride;
-        const double2 zk = z[zp(kh)];
-        const double2 zc = z[zp((H - kh) & (H - 1))];
-        const double er = 0.5 * (zk.x + zc.x), ei = 0.5 * (zk.y - zc.y);
-        const double orr = 0.5 * (zk.y + zc.y), oi = -0.5 * (zk.x - zc.x);
-        const double2 wk = k < H ? __ldg(tw + k) : make_double2(-1.0, 0.0);
-        const double xr = fma(wk.x, orr, fma(-wk.y, oi, er));
-        const double xi = fma(wk.x, oi, fma(wk.y, orr, ei));
-        put_bin<OUT>(out, nw, (int)blockIdx.y, M, m0 + ml, k - bin_lo, xr, xi, R, KC, lo_elems);
+        const double2 za = z[zp(u)], zb = z[zp((H - u) & (H - 1))];
+        auto bin = [&](int k, double2 zk, double2 zc) {
+            if (k < bin_lo || k >= bin_lo + nbins) return;
+            const double er = 0.5 * (zk.x + zc.x), ei = 0.5 * (zk.y - zc.y);
+            const double orr = 0.5 * (zk.y + zc.y), oi = -0.5 * (zk.x - zc.x);
+            const double2 wk = k < H ? __ldg(tw + k) : make_double2(-1.0, 0.0);
+            const double xr = fma(wk.x, orr, fma(-wk.y, oi, er));
+            const double xi = fma(wk.x, oi, fma(wk.y, orr, ei));
+            put_bin<OUT>(out, nw, (int)blockIdx.y, M, m0 + ml, k - bin_lo, xr, xi, R, KC, lo_elems);
+        };
+        bin(u, za, zb);
+        if (2 * u != H) bin(H - u, zb, za);
     }
 }
 
