@@ -107,13 +107,9 @@ static __device__ __noinline__ void sincos_any(double x, double *s, double *c) {
 // exact for n < 2^15) and its remainder; cos/sin of n pi/32 from the table, those of r from their Taylor series
 // (next terms 2e-20 and 4e-18), combined as C + (C (cos r - 1) - S sin r).  About one FP64 ulp; results near zero
 // (C = 0 exactly) keep the relative accuracy of r.  17 FP64 operations, no branch but the range check.
-__device__ __forceinline__ void sincos_reduced(float x, double &c, double &s)
+__device__ __forceinline__ void sincos_small(float x, double &c, double &s)   // |x| < 3000
 {
     const double xd = static_cast<double>(x);
-    if (!(fabsf(x) < 3000.0f)) {   // NaN and infinities too
-        sincos_any(xd, &s, &c);
-        return;
-    }
     const double magic = 6755399441055744.0;   // 1.5 2^52: the addition rounds to an integer
     const double t = fma(xd, 0x1.45f306dc9c883p+3, magic);
     const double nd = t - magic;
@@ -127,51 +123,92 @@ __device__ __forceinline__ void sincos_reduced(float x, double &c, double &s)
     s = fma(p.y, cm, fma(p.x, sr, p.y));
 }
 
-// Float32 cos/sin of a float32 argument: correctly rounded value through FP64 evaluation,
+// Float32 cos/sin of float32 arguments: correctly rounded value through FP64 evaluation,
 // optionally corrected to the host C library's cosf/sinf by the exception table.  The table holds
 // non-negative arguments; a negative one is looked up by its magnitude (the C library's cosf is even
 // and its sinf odd, bit for bit, and a delta on the bits of a float changes its magnitude).
-// In two halves, so that the loads of several arguments are in flight together: begin evaluates and loads the home
-// slot's word, finish corrects (about one lane in 150 walks the table).
+// K arguments at a time, in two halves, so that their loads are in flight together: begin evaluates and loads the home
+// slots' words, finish corrects (about one lane in 150 walks the table).  Issue slots bound the callers: the range
+// test and the test for a walk are one branch for all K, and the lookups are predicated loads, no branches.
+// Measured (B200; before: a branch per argument for each): FP64 map of 256 mics x 160,801 points x 12 bins 20.9 -> 20.4
+// ms, DAMAS of 64 mics 9.74 -> 9.63 ms.
+template <int K>
 struct SincosPending {
-    float x, c, s;
-    uint64_t word;   // the home slot's word, all ones where no lookup is needed
+    float x[K], c[K], s[K];
+    uint64_t word[K];   // the home slot's word, all ones where no lookup is needed
 };
 
-__device__ __forceinline__ SincosPending sincos_begin(float x, const SincosTable &t)
+// Load of a word where `p` holds, all ones elsewhere.
+__device__ __forceinline__ uint64_t sincos_word(const uint64_t *at, bool p)
 {
-    SincosPending v;
-    double sd, cd;
-    sincos_reduced(x, cd, sd);
-    v.x = x;
-    v.c = __double2float_rn(cd);
-    v.s = __double2float_rn(sd);
-    // distance of the FP64 values from a float32 rounding midpoint, from their 29 low mantissa bits
-    const int mc = abs((__double2loint(cd) & 0x1fffffff) - 0x10000000);
-    const int ms = abs((__double2loint(sd) & 0x1fffffff) - 0x10000000);
-    v.word = ~0ull;
-    if (min(mc, ms) <= t.tol) v.word = __ldg(t.table + ((sincos_hash(__float_as_uint(fabsf(x))) >> 20) & t.mask));
-    return v;
+    uint64_t w;
+    asm("{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "mov.b64 %0, -1;\n\t"
+        "@q ld.global.nc.b64 %0, [%1];\n\t}"
+        : "=&l"(w)
+        : "l"(at), "r"((int)p));
+    return w;
 }
 
-__device__ __forceinline__ void sincos_finish(SincosPending &v, const SincosTable &t)
+template <int K>
+__device__ __forceinline__ void sincos_begin(SincosPending<K> &v, const SincosTable &t)
 {
-    const uint32_t key = __float_as_uint(fabsf(v.x));
-    const uint32_t tag = 16u + static_cast<uint32_t>(sincos_hash(key) >> 60);
-    if (v.word != ~0ull && (((static_cast<uint32_t>(v.word) | t.untagged) >> tag) & 1u)) {
+    double sd[K], cd[K];
+    uint32_t big = 0;
+#pragma unroll
+    for (int q = 0; q < K; ++q) big = max(big, __float_as_uint(fabsf(v.x[q])));
+    if (big < 0x453b8000u) {   // 3000.0f; infinities and NaN compare above
+#pragma unroll
+        for (int q = 0; q < K; ++q) sincos_small(v.x[q], cd[q], sd[q]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < K; ++q) {
+            if (fabsf(v.x[q]) < 3000.0f) sincos_small(v.x[q], cd[q], sd[q]);
+            else sincos_any(static_cast<double>(v.x[q]), &sd[q], &cd[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+        v.c[q] = __double2float_rn(cd[q]);
+        v.s[q] = __double2float_rn(sd[q]);
+        // distance of the FP64 values from a float32 rounding midpoint, from their 29 low mantissa bits
+        const int mc = abs((__double2loint(cd[q]) & 0x1fffffff) - 0x10000000);
+        const int ms = abs((__double2loint(sd[q]) & 0x1fffffff) - 0x10000000);
+        v.word[q] = sincos_word(t.table + ((sincos_hash(__float_as_uint(fabsf(v.x[q]))) >> 20) & t.mask),
+                                min(mc, ms) <= t.tol);
+    }
+}
+
+template <int K>
+__device__ __forceinline__ void sincos_finish(SincosPending<K> &v, const SincosTable &t)
+{
+    bool walk[K], any = false;
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+        const uint32_t tag = 16u + static_cast<uint32_t>(sincos_hash(__float_as_uint(fabsf(v.x[q]))) >> 60);
+        walk[q] = v.word[q] != ~0ull && (((static_cast<uint32_t>(v.word[q]) | t.untagged) >> tag) & 1u);
+        any |= walk[q];
+    }
+    if (!any) return;
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+        if (!walk[q]) continue;
         int dc, ds;
-        sincos_exception(t, fabsf(v.x), dc, ds);
-        if (dc) v.c = __int_as_float(__float_as_int(v.c) + dc);
-        if (ds) v.s = __int_as_float(__float_as_int(v.s) + ds);
+        sincos_exception(t, fabsf(v.x[q]), dc, ds);
+        if (dc) v.c[q] = __int_as_float(__float_as_int(v.c[q]) + dc);
+        if (ds) v.s[q] = __int_as_float(__float_as_int(v.s[q]) + ds);
     }
 }
 
 __device__ __forceinline__ void sincos_f32_arg(float x, const SincosTable &t, float &c, float &s)
 {
-    SincosPending v = sincos_begin(x, t);
+    SincosPending<1> v;
+    v.x[0] = x;
+    sincos_begin(v, t);
     sincos_finish(v, t);
-    c = v.c;
-    s = v.s;
+    c = v.c[0];
+    s = v.s[0];
 }
 
 }  // namespace acb

@@ -48,15 +48,11 @@ struct MapArgs {
 // rounded to float32, cos - i sin of it as the C library's float32 functions give them, then the
 // weight w: r (inverse) or 1/r (true level, true location; the product is within an ulp of the quotient).
 // In two halves, so that a caller with several values has their table lookups in flight together.
-__device__ __forceinline__ SincosPending steer_begin(const SincosTable &sct, double k, double r)
-{
-    return sincos_begin(__double2float_rn(__dmul_rn(k, r)), sct);
-}
+__device__ __forceinline__ float steer_phase(double k, double r) { return __double2float_rn(__dmul_rn(k, r)); }
 
-__device__ __forceinline__ double2 steer_finish(int steer_type, const SincosTable &sct, SincosPending &v, double w)
+__device__ __forceinline__ double2 steer_value(int steer_type, float c, float s, double w)
 {
-    sincos_finish(v, sct);
-    double2 h = make_double2((double)v.c, -(double)v.s);
+    double2 h = make_double2((double)c, -(double)s);
     if (steer_type >= 2) {
         h.x *= w;
         h.y *= w;
@@ -124,8 +120,9 @@ __device__ __forceinline__ void synth_tile(const MapArgs &a, const SincosTable &
                     } else {
                         const double r = __ldg(rm + g * a.M + m0 + m);
                         const double w = steer_weight(a.steer_type, r);
-                        SincosPending v = steer_begin(sct, k, r);
-                        h = steer_finish(a.steer_type, sct, v, w);
+                        float c, s;
+                        sincos_f32_arg(steer_phase(k, r), sct, c, s);
+                        h = steer_value(a.steer_type, c, s, w);
                         if (sum) S[i] += w * w;
                     }
                 }
@@ -139,18 +136,20 @@ __device__ __forceinline__ void synth_tile(const MapArgs &a, const SincosTable &
         const bool ok = gb + p < a.G;
         for (int mb = threadIdx.x / kPts; mb < np; mb += kSynth * kStep) {
             double w[kSynth];
-            SincosPending v[kSynth];
+            SincosPending<kSynth> v;
 #pragma unroll
             for (int u = 0; u < kSynth; ++u) {
                 const int m = m0 + min(mb + u * kStep, n - 1);
                 const double r = dist3_weight(a.steer_type, g0, g1, g2, __ldg(mpos + m), __ldg(mpos + a.M + m),
                                               __ldg(mpos + 2 * a.M + m), w[u]);
-                v[u] = steer_begin(sct, k, r);
+                v.x[u] = steer_phase(k, r);
             }
+            sincos_begin(v, sct);
+            sincos_finish(v, sct);
 #pragma unroll
             for (int u = 0; u < kSynth; ++u) {
                 const int m = mb + u * kStep;
-                double2 h = steer_finish(a.steer_type, sct, v[u], w[u]);
+                double2 h = steer_value(a.steer_type, v.c[u], v.s[u], w[u]);
                 if (!ok || m >= n) h = make_double2(0.0, 0.0);
                 else if (sum) S[0] += w[u] * w[u];
                 if (m < np) hs[m * kPtsPad + p] = h;
@@ -578,10 +577,15 @@ __global__ void __launch_bounds__(kEigSmallThreads)
             }
             S = fma(w, w, S);
         }
-        SincosPending pend[NB];
+        constexpr int KP = NB < 2 ? NB : 2;   // all four at once spill (5.36 -> 5.62 ms); pairs 5.30
+        SincosPending<KP> pend[NB / KP];
         if (!CUSTOM) {
 #pragma unroll
-            for (int q = 0; q < NB; ++q) pend[q] = steer_begin(sct, k[q], r);
+            for (int q = 0; q < NB; ++q) pend[q / KP].x[q % KP] = steer_phase(k[q], r);
+#pragma unroll
+            for (int q = 0; q < NB / KP; ++q) sincos_begin(pend[q], sct);
+#pragma unroll
+            for (int q = 0; q < NB / KP; ++q) sincos_finish(pend[q], sct);
         }
 #pragma unroll
         for (int q = 0; q < NB; ++q) {
@@ -590,7 +594,7 @@ __global__ void __launch_bounds__(kEigSmallThreads)
                 h = __ldg(hv + m);
                 S += fma(h.x, h.x, __dmul_rn(h.y, h.y));
             } else {
-                h = steer_finish(a.steer_type, sct, pend[q], w);
+                h = steer_value(a.steer_type, pend[q / KP].c[q % KP], pend[q / KP].s[q % KP], w);
             }
             const double2 *vrow = V[q] + (int64_t)m * E;
 #pragma unroll

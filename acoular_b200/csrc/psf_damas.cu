@@ -101,14 +101,15 @@ __global__ void __launch_bounds__(256, 4) psf_kernel(int M, int64_t G, int S, co
         const double *rsw = rs_s + warp * kPsfPer * (kPsfMics + 1), *isw = is_s + warp * kPsfPer * (kPsfMics + 1);
         for (int m = 0; m < n; ++m) {
             const double rg = rg_s[m * (kPsfTile + 1) + lane], ig = ig_s[m * (kPsfTile + 1) + lane];
-            SincosPending pend[kPsfPer];
+            SincosPending<kPsfPer> pend;
 #pragma unroll
             for (int j = 0; j < kPsfPer; ++j)
-                pend[j] = sincos_begin(__double2float_rn(__dmul_rn(k, __dsub_rn(rg, rsw[j * (kPsfMics + 1) + m]))), sct);
+                pend.x[j] = __double2float_rn(__dmul_rn(k, __dsub_rn(rg, rsw[j * (kPsfMics + 1) + m])));
+            sincos_begin(pend, sct);
+            sincos_finish(pend, sct);
 #pragma unroll
             for (int j = 0; j < kPsfPer; ++j) {
-                sincos_finish(pend[j], sct);
-                const double c = (double)pend[j].c, sn = -(double)pend[j].s;
+                const double c = (double)pend.c[j], sn = -(double)pend.s[j];
                 // (cos - i sin) / rs  [* rg (inverse) | / rg (true level, true location)]; the divisions as
                 // products with reciprocals (within an ulp of the quotients); the mirror image's sine is negated
                 const double is = isw[j * (kPsfMics + 1) + m];
