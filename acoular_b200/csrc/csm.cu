@@ -793,18 +793,23 @@ static int gram_c64_launch(const void *spec, int M, int64_t nw, int nbins, void 
 //     Im C[r][c] = sum_k A[r][k] B'[k][c],                         B'[.][c] = (-y_c, x_c, ..),
 // and the instruction adds its products to an element as a chain of FMAs in ascending k (checked on 10^5 random
 // elements), so this is the reference's order of two chained FMAs per window and component, bit for bit.
-// CTA = 32 x 32 tile of one bin's upper triangle, 4 warps of 16 x 16; 16 windows per stage, three stages of cp.async,
+// CTA = 32 x 32 (small launches: 32 x 16, GF_NARROW) tile of one bin's upper triangle, 4 warps of 16 x 16 (16 x 8); 16
+// windows per stage, three stages of cp.async,
 // four CTAs per SM.  Rows are padded to 36 mics, so that the operand reads of 4 mics x 2 windows (A) and 8 mics x 2
 // windows (B) fall on different banks.  16 x 8 blocks entirely below the diagonal or past M are skipped.  With `out`
 // the sums are not added to csm but written, scaled, as the full Hermitian matrix.
 // Bound: the FP64 pipe (4 M^2 K flop per bin).  Measured (B200): 513 bins x 256 mics x 999 windows 7.84 -> 5.0 ms
 // (27 TFLOP/s; 64 x 64 tiles of 32 x 16 per warp 5.2 ms, half of the diagonal tiles idle); 65 bins x 64 mics x 799
-// windows 281 -> 115 us (195 CTAs where the 64 x 64 tiles of the FMA form were 65).
+// windows 281 -> 75 us (195 CTAs where the 64 x 64 tiles of the FMA form were 65), in 32 x 16 tiles 65 us.
 // ------------------------------------------------------------------------------------------------
 constexpr int GF_T = 32;       // tile edge
 constexpr int GF_LD = GF_T + 4;
 constexpr int GF_KW = 16;      // windows per stage
 constexpr int GF_STAGES = 3;
+// Fewer 32 x 32 tiles than this (all bins): 32 x 16 tiles, twice as many CTAs, so that no SM holds two tiles while its
+// neighbour holds one.  Measured (B200), microseconds of the whole CSM, 32 x 32 / 32 x 16: 65 tiles 61 / 45, 99 151 / 145,
+// 170 227 / 209, 195 110 / 101 and 96 / 73, 198 207 / 182; 255 249 / 262, 257 139 / 145, 330 319 / 352, 387 175 / 205.
+constexpr int64_t GF_NARROW = kNumSMs * 3 / 2;
 constexpr int GF_SMEM = GF_STAGES * 2 * GF_KW * GF_LD * (int)sizeof(double2);
 
 __device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], double b0, double b1)
@@ -814,29 +819,30 @@ __device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], do
         : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
 }
 
+template <int NB>
 __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restrict__ spec, int M, int64_t nw,
                                                           double2 *__restrict__ csm, double2 *__restrict__ out,
                                                           double scale)
 {
-    constexpr int T = GF_T, LD = GF_LD, NB = 2;
+    constexpr int T = GF_T, TC = 16 * NB, LD = GF_LD;   // T rows x TC columns
     extern __shared__ double2 gf_sm[];   // [stage][row mics | column mics][window][LD]
-    // upper-triangular tile index -> (ti, tj), ti <= tj
-    const int NT = (M + T - 1) / T;
+    // tile index -> row tile ti and column tile tj >= ti T / TC
+    const int NT = (M + TC - 1) / TC;
     int tile = blockIdx.x, ti = 0;
-    while (tile >= NT - ti) {
-        tile -= NT - ti;
+    while (tile >= NT - ti * (T / TC)) {
+        tile -= NT - ti * (T / TC);
         ++ti;
     }
-    const int tj = ti + tile;
+    const int tj = ti * (T / TC) + tile;
     const int f = blockIdx.y;
     const int lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    // warp -> 16 x 16 quarter, rotated over the CTAs: in a diagonal tile the lower-left quarter has nothing to do
+    // warp -> 16 x 8 NB quarter, rotated over the CTAs: in a diagonal tile the lower-left quarter has nothing to do
     const int quarter = ((threadIdx.x >> 5) + blockIdx.x + blockIdx.y) & 3;
     const int wr = quarter >> 1, wc = quarter & 1;
-    const int r0 = ti * T, c0 = tj * T;
-    const int rw = r0 + wr * 16, cw = c0 + wc * 16;   // this warp's first row and column
-    const bool same = ti == tj;
+    const int r0 = ti * T, c0 = tj * TC;
+    const int rw = r0 + wr * 16, cw = c0 + wc * 8 * NB;   // this warp's first row and column
+    const bool same = c0 < r0 + T;                        // the columns are among the rows
     const double2 *sp = spec + (int64_t)f * nw * M;
     double2 *base = csm + (int64_t)f * M * M;
 
@@ -852,7 +858,7 @@ __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restr
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src + min(r0 + m, M - 1)),
                          "r"(in && r0 + m < M ? 16 : 0)
                          : "memory");
-            if (!same)
+            if (!same && m < TC)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + GF_KW * LD * 16),
                              "l"(src + min(c0 + m, M - 1)), "r"(in && c0 + m < M ? 16 : 0)
                              : "memory");
@@ -885,9 +891,9 @@ __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restr
         __syncthreads();   // stage st has landed for every thread; stage st - 1 is read by none any more
         if (st + 2 < nst) load(st + 2);
         const double2 *xr = gf_sm + (st % GF_STAGES) * (2 * GF_KW * LD);
-        const double2 *xc = same ? xr : xr + GF_KW * LD;
+        const double2 *xc = same ? xr + (c0 - r0) : xr + GF_KW * LD;
         const double *ar = reinterpret_cast<const double *>(xr + (t >> 1) * LD + wr * 16 + g) + (t & 1);
-        const double2 *bc = xc + (t >> 1) * LD + wc * 16 + g;
+        const double2 *bc = xc + (t >> 1) * LD + wc * 8 * NB + g;
 #pragma unroll
         for (int w = 0; w < GF_KW; w += 4) {
             double b0[NB], b1[NB], q0[NB], q1[NB];
@@ -924,10 +930,15 @@ static int gram_f64_launch(const void *spec, int M, int64_t nw, int nbins, void 
                            cudaStream_t s)
 {
     const int T = (M + GF_T - 1) / GF_T;
-    cudaFuncSetAttribute(gram_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GF_SMEM);
-    gram_f64_kernel<<<dim3(T * (T + 1) / 2, nbins), 128, GF_SMEM, s>>>(
-        reinterpret_cast<const double2 *>(spec), M, nw, reinterpret_cast<double2 *>(csm),
-        reinterpret_cast<double2 *>(out), scale);
+    const bool narrow = (int64_t)T * (T + 1) / 2 * nbins < GF_NARROW;
+    const auto kernel = narrow ? gram_f64_kernel<1> : gram_f64_kernel<2>;
+    const int TC = narrow ? (M + 15) / 16 : T, per = narrow ? 2 : 1;
+    int tiles = 0;
+    for (int ti = 0; ti < T; ++ti) tiles += TC - per * ti;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GF_SMEM);
+    kernel<<<dim3(tiles, nbins), 128, GF_SMEM, s>>>(reinterpret_cast<const double2 *>(spec), M, nw,
+                                                    reinterpret_cast<double2 *>(csm), reinterpret_cast<double2 *>(out),
+                                                    scale);
     return check_launch();
 }
 
