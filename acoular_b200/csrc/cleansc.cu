@@ -9,7 +9,8 @@
 //   D1 = (C^T - diag C) w / hmax; 20 fixed-point steps hh = (D1 + |hh|^2 w) / sqrt(1 + sum |w|^2 |hh|^2);
 //   h -= damp * map of the single component (hmax, conj(hh)); C -= damp hmax (hh hh^H)^T.
 //
-// Device schedule: the steering vectors of every grid point are synthesised once per bin (normalised for
+// Device schedule (arrays and grids that fit run all iterations of a bin in one cluster, cleansc_cluster_kernel; this is
+// the one for the others): the steering vectors of every grid point are synthesised once per bin (normalised for
 // the steering type, cleansc_steer_kernel); then per iteration cleansc_step_kernel (one CTA per bin: the
 // map update h -= damp h1 fused with the argmax, then the peak's steering vector, D1, the fixed point and
 // the CSM update) and the eigenvalue-form map of the new component on the cached steering vectors

@@ -7,6 +7,7 @@
 //                          (beta real, tau complex, v_0 = 1), then updates the trailing matrix
 //                          A22 <- H^H A22 H = A22 - v w^H - w v^H, p = tau A22 v, w = p - (tau/2)(p^H v) v,
 //                          on A22's lower triangle only (half the memory traffic of the full update).
+//                          heevd_tridiag_cluster_kernel does it in the shared memory of a cluster where it fits.
 //   heevd_tql_kernel     : eigenvalues and eigenvectors of T by implicit QL sweeps with Wilkinson shifts
 //                          (the EISPACK tql2 scheme), eigenvectors accumulated in Z.  One warp forms a
 //                          sweep's plane rotations from d and e; the others apply those of the sweep before

@@ -357,7 +357,7 @@ def batched_block(steps, warmup, precision):
                        'block_sizes': sorted({int(w.block_size) for w in wls}), 'bins_per_instance': 30,
                        'csm': 'complex64', 'form': f'tc {precision}', 'steer_type': 'true level', 'r_diag': True},
             'accuracy': {'vs': 'plain FP64 form on the same CSMs', **worst, 'instances': errs},
-            'gpu_launches_per_step': '1 graph (per instance: FFT, Welch Gram, finalize; 1 batched map)',
+            'gpu_launches_per_step': '1 graph (per instance: FFT, Welch Gram; 1 batched map)',
             'clocks': clk.summary(), 'dtype': f'{precision} / f32 accum'}
 
 
@@ -648,7 +648,7 @@ def config1_block(steps, warmup):
                              'cores': O.num_threads(), 'kind': 'port',
                              'sample': 'the whole step: CSM of 799 windows x 65 bins + the 5-bin band map'},
             'accuracy': {'vs': 'oracle', 'max_rel_err': err, 'e2e_max_rel_err': err_e2e},
-            'gpu_launches_per_step': 4, 'dtype': 'f64'}
+            'gpu_launches_per_step': 3, 'dtype': 'f64'}
 
 
 def run_eig(args):
@@ -844,7 +844,7 @@ def run_damas(args):
            'steer_type': st, 'r_diag': True, 'psf': 'full (G x G per bin), float64',
            'csm': 'complex128, computed once', 'l2': 'psf of the band (113 MB) read 100x per step'},
           stage_ms={k: float(np.mean(v)) for k, v in st_ms.items()},
-          roofline={'kernel': 'damas_kernel', 'bound': 'hbm (latency: one 32-row block per step)',
+          roofline={'kernel': 'damas_ahead_kernel', 'bound': 'hbm (latency: one 32-row block per step)',
                     'achieved': achieved, 'peak': pk['hbm_gbs'], 'unit': 'GB/s', 'frac': achieved / pk['hbm_gbs'],
                     'traffic': None, 'bytes_per_launch': gs_bytes,
                     'sequential_steps_per_launch': n_iter * nblk,
@@ -858,7 +858,7 @@ def run_damas(args):
                'd2h_bytes_per_step': int(B * G * 8)},
           cpu_baseline={'value': 1.0 / cpu_s, 'unit': 'bins/s', 'cores': O.num_threads(), 'kind': 'port',
                         'sample': f'1 bin (bin {b0}): map + full PSF + {n_iter} sweeps'},
-          gpu_launches=f'{1 + B + 1} per step (map_plain_kernel, {B} psf_kernel, damas_kernel) + 1 copy',
+          gpu_launches=f'{1 + B + 1} per step (map_f64_kernel, {B} psf_kernel, damas_ahead_kernel) + 1 copy',
           clocks=clk.summary(), dtype='f64')
 
 
@@ -926,7 +926,6 @@ def run_cleansc(args):
         if it:
             e2e_ms.append((time.perf_counter() - ta) * 1e3)
     e2e_err = float(np.abs(band[B // 2] - ref).max() / np.abs(ref).max())
-    J = 2 * M
     _line('CLEAN-SC bins/s (BeamformerCleansc, 64 mics, 41x41 grid, 8 kHz third-octave band)', B / (ms / 1e3),
           'bins/s', ms, args,
           {'workload': 'cleansc_' + wl.name, 'mics': M, 'grid_points': G, 'bins': B, 'n_iter': 'auto (<= 128)',
@@ -938,8 +937,7 @@ def run_cleansc(args):
                'd2h_bytes_per_step': int(B * G * 4)},
           cpu_baseline={'value': 1.0 / cpu_s, 'unit': 'bins/s', 'cores': O.num_threads(), 'kind': 'port',
                         'sample': f'1 bin (bin {b0}): map + CLEAN-SC iterations'},
-          gpu_launches=f'{2 + 2 * J - 1} per step (init, map_plain_kernel, {J} cleansc_step_kernel, '
-                       f'{J - 1} map_eig_small_kernel; stopped bins return at once)',
+          gpu_launches='4 per step (init, map_f64_kernel, cleansc_steer_kernel, cleansc_cluster_kernel)',
           clocks=clk.summary(), dtype='f64')
 
 
@@ -1087,7 +1085,6 @@ def main():
     csm_prec = 'complex128' if form == 'f64' else f'tc_{csm_tc}'
     ws_bytes = NAT.lib().acb_csm_workspace_bytes(M, F, K, D.CSM_PRECISIONS[csm_prec])
     workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-    csm_up = torch.zeros((F, M, M), dtype=torch.complex128, device=dev)
     csm_full = torch.empty((F, M, M), dtype=torch.complex128, device=dev)
     _, weight = D.window_vector('Hanning', N, dev)
     scale = 2.0 / N / weight / D.num_blocks(wl.num_samples, N, 2)
@@ -1098,10 +1095,8 @@ def main():
     def step(record=False):
         if record:
             ev_csm.record()
-        csm_up.zero_()
-        D.csm_upper_accumulate(samples, N, 'Hanning', '50%', precision=csm_prec, csm_upper=csm_up, workspace=workspace,
-                               max_workspace_bytes=ws_bytes)
-        D.csm_finalize(csm_up, scale, out=csm_full)
+        D.csm_finished(samples, N, 'Hanning', '50%', csm_prec, scale, out=csm_full, workspace=workspace,
+                       max_workspace_bytes=ws_bytes)
         c = csm_full if nbins == F else csm_full[:nbins]
         if record:
             ev_map[0].record()
@@ -1197,7 +1192,7 @@ def main():
     achieved_tf = flops / (map_avg / 1e3) / 1e12
     if form == 'f64':
         roof = {'bound': 'fp64', 'achieved': achieved_tf, 'peak': gp['fp64_tflops'], 'unit': 'TFLOP/s',
-                'frac': achieved_tf / gp['fp64_tflops'], 'traffic': None, 'kernel': 'map_plain_kernel',
+                'frac': achieved_tf / gp['fp64_tflops'], 'traffic': None, 'kernel': 'map_f64_kernel',
                 'peak_kind': 'DGEMM measured in this run'}
     else:
         # denominator: the measured sustained BF16 rate of the peak file (dense FP16 runs at the BF16 rate,
@@ -1246,7 +1241,7 @@ def main():
     # the other configurations, each timed on its own (rank 0 at N = 1): their rates, errors and latencies
     extra = {}
     if rank == 0 and ws == 1 and not args.no_extra:
-        del samples, csm_up, csm_full, out, csm64, cs, ks
+        del samples, csm_full, out, csm64, cs, ks
         torch.cuda.empty_cache()
         extra['config1'] = config1_block(20, 3)
         extra['batched64'] = batched_block(10, 3, prec)
@@ -1275,17 +1270,17 @@ def main():
         if pmatrix is not None:
             line['precision_matrix'] = pmatrix
         line.update(extra)
-        line['gpu_launches'] = launches_per_step(F, nbins, K, M) * args.steps
+        line['gpu_launches'] = launches_per_step(form, prec) * args.steps
         print(json.dumps(line), flush=True)
     if ws > 1:
         import torch.distributed as dist
         dist.destroy_process_group()
 
 
-def launches_per_step(F, nbins, K, M):
-    # csm_up.zero_ is a torch fill (not counted); ours: fft + gram per workspace chunk, finalize, map
-    chunks = -(-K // 65535)
-    return 2 * chunks + 1 + 1
+def launches_per_step(form, prec):
+    # fft + gram (all windows fit the workspace: the Gram writes the finished CSM); the map, and for the tensor-core
+    # form its operand tiles and (FP16) the bins' largest entries
+    return 2 + (1 if form == 'f64' else 3 if prec == 'fp16' else 2)
 
 
 if __name__ == '__main__':

@@ -371,6 +371,9 @@ int acb_map_tc_noalloc(const acb_map_params *p, int precision, const void *csm, 
  * x in [0, max_arg) where the host C library's cosf/sinf differ from that value, with the
  * difference in units of the last place.  It is built by CALLING the host cosf/sinf on every
  * float32 in the range (no knowledge of their implementation is used).
+ * An entry's key is the argument's bits (upper half); beside the differences it carries tag bits of the keys whose home
+ * slot it is, and one more entry records how close to a rounding midpoint the exceptions lie, so that the kernels look up
+ * only the arguments that can be among them.  A table without that entry gives the same results, more slowly.
  * table_host: uint64 [slots] (slots a power of two, >= 2^22 recommended), filled here.
  * Returns the number of exception entries, or a negative acb_status on error. */
 int64_t acb_sincos_table_build_host(uint64_t *table_host, int64_t slots, float max_arg, int num_threads);
