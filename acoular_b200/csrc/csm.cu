@@ -992,13 +992,16 @@ __global__ void __launch_bounds__(256) finalize_kernel(const void *__restrict__ 
 // Mics per CTA (a power of two) and threads: up to 74 KB of padded complex doubles and 256 threads, so that two or
 // three CTAs share an SM and hide each other's barriers and FP64 latency; for blocks of FFT_WIDE_N samples and more, of
 // which that would hold one or two mics and store 16 bytes of a row of complex64 spectra at a time, up to 150 KB and
-// 512 threads.
+// 512 threads.  At most 64 mics and no more than twice what the array has, and no more threads (64 at least) than the
+// first pass has tasks: with 16 mics and 256 threads whatever the block, half the threads and more idled.  Measured
+// (B200), whole complex128 CSM: 64 mics, block 128 100 -> 92 us, block 64 145 -> 122, block 32 120 -> 98, block 16 147 ->
+// 118; 256 mics, block 128 1306 -> 1226; 113 mics, block 256 420 -> 410; 8 mics, block 128 45 -> 41.
 static int fft_threads(int N) { return N >= FFT_WIDE_N ? 512 : 256; }
-static int fft_mics_per_block(int N)
+static int fft_mics_per_block(int N, int M)
 {
     const size_t most = (N >= FFT_WIDE_N ? 150 : 74) * 1024;
-    int mpb = 16;
-    while (mpb > 1 && (size_t)mpb * fft_stride(N / 2) * sizeof(double2) > most) mpb >>= 1;
+    int mpb = 64;
+    while (mpb > 1 && (mpb >= 2 * M || (size_t)mpb * fft_stride(N / 2) * sizeof(double2) > most)) mpb >>= 1;
     return mpb;
 }
 
@@ -1070,14 +1073,15 @@ int fft_launch(const void *samples, int sample_dtype, int out_form, int num_mics
             return check_launch();
         }
     }
-    const int mpb = fft_mics_per_block(block_size);
+    const int mpb = fft_mics_per_block(block_size, num_mics);
     const dim3 g1((num_mics + mpb - 1) / mpb, (unsigned)num_windows);
     const size_t smem = (size_t)mpb * fft_stride(block_size / 2) * sizeof(double2);
 #define ACB_FFT_LAUNCH(TS, OF)                                                                                    \
     do {                                                                                                          \
         auto kern = fft_window_kernel<TS, OF>;                                                                    \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                       \
-        kern<<<g1, fft_threads(block_size), smem, s>>>(reinterpret_cast<const TS *>(samples), num_mics, block_size, hop, \
+        const int nt = max(64, min(fft_threads(block_size), mpb * (block_size / 16)));                             \
+        kern<<<g1, nt, smem, s>>>(reinterpret_cast<const TS *>(samples), num_mics, block_size, hop, \
                                    first_window, num_windows, mpb, window, tw, bin_lo, num_bins, out, R, KC, lo_elems);        \
     } while (0)
 #define ACB_FFT_FORMS(TS)                                                \
