@@ -660,8 +660,8 @@ __global__ void __launch_bounds__(256) fft_combine_kernel(const double2 *__restr
 }
 
 // ------------------------------------------------------------------------------------------------
-// Welch Gram accumulation in complex64, upper-triangular 64x64 tiles; thread (tx, ty) of 16 x 8 owns rows ty + 8 i
-// and columns tx + 16 j of the tile.  An element's (re, im) is one packed pair of FP32 accumulators, so that the
+// Welch Gram accumulation in complex64, upper-triangular T x T tiles (64, or 32: gram_c64_narrow); thread (tx, ty) of 16
+// x 8 owns rows ty + 8 i and columns tx + 16 j of the tile.  An element's (re, im) is one packed pair of FP32 accumulators, so that the
 // reference's two chained FMAs per component are two packed FMAs, (x_c, -y_c) x_r and then (y_c, x_c) y_r.  In a
 // diagonal tile the 8 x 16 blocks below the diagonal are left out.
 // Bound: FP32 FMAs (0.31 ms here) and the issue slots of the operand pairs' moves.  8 x 4 elements per thread, as 4 x 4
@@ -669,7 +669,7 @@ __global__ void __launch_bounds__(256) fft_combine_kernel(const double2 *__restr
 // 821 -> 500 us.
 // With `out` the sums are not added to csm but written, scaled, as the full Hermitian complex128 matrix.
 // ------------------------------------------------------------------------------------------------
-constexpr int GT = 64;   // tile edge
+constexpr int GT = 64;   // the larger tile's edge
 constexpr int GKC = 16;  // windows per shared-memory stage
 constexpr int GTHREADS = 128;
 
@@ -683,21 +683,21 @@ __device__ __forceinline__ void ffma2(float2 &acc, float ax, float ay, float b)
 }
 
 // One stage of `kc` windows into the accumulators.
-template <bool DIAG>
-__device__ __forceinline__ void gram64_stage(const float2 *xr, const float2 *xc, int kc, float2 (&acc)[8][4])
+template <bool DIAG, int T, int RI, int CJ>
+__device__ __forceinline__ void gram64_stage(const float2 *xr, const float2 *xc, int kc, float2 (&acc)[RI][CJ])
 {
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll 4
     for (int kk = 0; kk < kc; ++kk) {
-        float2 r[8], c[4];
+        float2 r[RI], c[CJ];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) r[i] = xr[kk * GT + ty + 8 * i];
+        for (int i = 0; i < RI; ++i) r[i] = xr[kk * T + ty + 8 * i];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) c[j] = xc[kk * GT + tx + 16 * j];
+        for (int j = 0; j < CJ; ++j) c[j] = xc[kk * T + tx + 16 * j];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < RI; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < CJ; ++j) {
                 if (DIAG && i > 2 * j + 1) continue;
                 ffma2(acc[i][j], c[j].x, -c[j].y, r[i].x);
                 ffma2(acc[i][j], c[j].y, c[j].x, r[i].y);
@@ -705,40 +705,42 @@ __device__ __forceinline__ void gram64_stage(const float2 *xr, const float2 *xc,
     }
 }
 
+template <int T>
 __global__ void __launch_bounds__(GTHREADS, 4) gram_c64_kernel(const float2 *__restrict__ spec, int M, int64_t nw,
                                                                float2 *__restrict__ csm, double2 *__restrict__ out,
                                                                double scale)
 {
-    __shared__ float2 g64_sm[2][2][GKC][GT];   // [stage][rows | columns]
+    constexpr int RI = T / 8, CJ = T / 16;
+    __shared__ float2 g64_sm[2][2][GKC][T];   // [stage][rows | columns]
     // upper-triangular tile index -> (ti, tj), ti <= tj
-    const int T = (M + GT - 1) / GT;
+    const int NT = (M + T - 1) / T;
     int t = blockIdx.x, ti = 0;
-    while (t >= T - ti) {
-        t -= T - ti;
+    while (t >= NT - ti) {
+        t -= NT - ti;
         ++ti;
     }
     const int tj = ti + t;
     const int f = blockIdx.y;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int r0 = ti * GT, c0 = tj * GT;
+    const int r0 = ti * T, c0 = tj * T;
     const bool diag = ti == tj;
 
-    float2 acc[8][4];
+    float2 acc[RI][CJ];
     float2 *base = csm + (int64_t)f * M * M;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < CJ; ++j) {
             const int r = r0 + ty + 8 * i, c = c0 + tx + 16 * j;
             acc[i][j] = make_float2(0.f, 0.f);
             if (!out && r < M && c < M && r <= c) acc[i][j] = base[(int64_t)r * M + c];
         }
 
     const float2 *sp = spec + (int64_t)f * nw * M;
-    const int lm = threadIdx.x & (GT - 1), lk = threadIdx.x / GT;   // this thread's mic and first window of a stage
+    const int lm = threadIdx.x & (T - 1), lk = threadIdx.x / T;   // this thread's mic and first window of a stage
     auto load = [&](int64_t k0, int buf) {
 #pragma unroll
-        for (int u = 0; u < GKC; u += GTHREADS / GT) {
+        for (int u = 0; u < GKC; u += GTHREADS / T) {
             const int64_t k = k0 + lk + u;
             const bool in = k < nw;
             const float2 *src = sp + (in ? k : 0) * M;
@@ -747,7 +749,7 @@ __global__ void __launch_bounds__(GTHREADS, 4) gram_c64_kernel(const float2 *__r
                          "r"(in && r0 + lm < M ? 8 : 0)
                          : "memory");
             if (!diag)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + GKC * GT * 8),
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + GKC * T * 8),
                              "l"(src + min(c0 + lm, M - 1)), "r"(in && c0 + lm < M ? 8 : 0)
                              : "memory");
         }
@@ -761,14 +763,14 @@ __global__ void __launch_bounds__(GTHREADS, 4) gram_c64_kernel(const float2 *__r
         if (k0 + GKC < nw) load(k0 + GKC, buf ^ 1);
         const int kc = (int)((nw - k0) < GKC ? (nw - k0) : GKC);
         const float2 *xr = &g64_sm[buf][0][0][0];
-        if (diag) gram64_stage<true>(xr, xr, kc, acc);
-        else gram64_stage<false>(xr, xr + GKC * GT, kc, acc);
+        if (diag) gram64_stage<true, T>(xr, xr, kc, acc);
+        else gram64_stage<false, T>(xr, xr + GKC * T, kc, acc);
     }
     double2 *ob = out + (int64_t)f * M * M;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < CJ; ++j) {
             const int r = r0 + ty + 8 * i, c = c0 + tx + 16 * j;
             if (r >= M || c >= M || r > c) continue;
             if (out) put_hermitian(ob, M, r, c, (double)acc[i][j].x, (double)acc[i][j].y, scale);
@@ -776,13 +778,26 @@ __global__ void __launch_bounds__(GTHREADS, 4) gram_c64_kernel(const float2 *__r
         }
 }
 
+// 32 x 32 tiles for arrays of up to 32 mics, and where the 64 x 64 tiles' last round over the SMs would be so empty that
+// at least 3 of 10 places stay free (up to three rounds).  Measured (B200), microseconds of the whole CSM, 64 / 32: 33
+// tiles 164 / 104, 65 99 / 88, 195 219 / 173, 330 303 / 261; 129 129 / 141, 257 231 / 251, 650 470 / 476; 32 mics, 513
+// bins 175 / 112; 8 mics, 65 bins 77 / 42.
+static bool gram_c64_narrow(int M, int64_t tiles)
+{
+    const int64_t rounds = (tiles + kNumSMs - 1) / kNumSMs;
+    return M <= 32 || (rounds <= 3 && 10 * rounds * kNumSMs >= 13 * tiles);
+}
+
 static int gram_c64_launch(const void *spec, int M, int64_t nw, int nbins, void *csm, void *out, double scale,
                            cudaStream_t s)
 {
     const int T = (M + GT - 1) / GT;
-    gram_c64_kernel<<<dim3(T * (T + 1) / 2, nbins), GTHREADS, 0, s>>>(
-        reinterpret_cast<const float2 *>(spec), M, nw, reinterpret_cast<float2 *>(csm),
-        reinterpret_cast<double2 *>(out), scale);
+    const bool narrow = gram_c64_narrow(M, (int64_t)T * (T + 1) / 2 * nbins);
+    const auto kernel = narrow ? gram_c64_kernel<32> : gram_c64_kernel<GT>;
+    const int NT = narrow ? (M + 31) / 32 : T;
+    kernel<<<dim3(NT * (NT + 1) / 2, nbins), GTHREADS, 0, s>>>(reinterpret_cast<const float2 *>(spec), M, nw,
+                                                               reinterpret_cast<float2 *>(csm),
+                                                               reinterpret_cast<double2 *>(out), scale);
     return check_launch();
 }
 
