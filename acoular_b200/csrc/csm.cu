@@ -43,7 +43,7 @@ void set_cuda_error(cudaError_t e) { g_last_cuda_error = cudaGetErrorString(e); 
 // mics x 1024 samples.  Measured (B200): that transform 2.65 -> 1.24 ms (before: two more trips through shared
 // memory, a twiddle load per butterfly and runtime divisions by the mic count in the index arithmetic).  The lane order of the load
 // and the paired bins of the split give 4 to 8 % of a whole CSM where few mics fit a CTA (113 mics, block 4096, 75 %
-// overlap, complex64: 995 -> 958 us; 16 mics, block 16384: 371 -> 342) and 0.2 to 1 % elsewhere.
+// overlap, complex64, in the six-FMA form: 995 -> 958 us; 16 mics, block 16384: 371 -> 342) and 0.2 to 1 % elsewhere.
 // ------------------------------------------------------------------------------------------------
 // Shared-memory slot of point j of a mic's sequence: one padding slot after every 8 points, so that
 // 8 threads reading 16-byte points 8 apart (the first pass) or 64 apart hit different banks.
@@ -51,22 +51,42 @@ __device__ __forceinline__ int zp(int j) { return j + (j >> 3); }
 // padded length of one mic's sequence of H points (an odd number of 16-byte slots past the padding)
 __host__ __device__ constexpr int fft_stride(int H) { return H + (H >> 3) + 1; }
 
-// (a, b) -> (a + w b, a - w b), the difference as 2 a - (a + w b): six FMAs
+// (a, b) -> (a + w b, a - w b), the difference as 2 a - (a + w b): six FMAs; PLAIN: w b first, then the sum and the
+// difference.  Spectra that are rounded to complex64 take the plain form with every twiddle from the table: their
+// rounding then falls the same way as with one stage at a time, where the six-FMA form moves one value in 10^7 by an ulp
+// (113 mics, block 4096, complex64: 957 -> 1010 us, the price of it).  So do the sub-sequences of the largest blocks.
+template <bool PLAIN>
 __device__ __forceinline__ void butterfly(double2 &a, double2 &b, double2 w)
 {
+    if (PLAIN) {
+        const double br = b.x * w.x - b.y * w.y;
+        const double bi = b.x * w.y + b.y * w.x;
+        b = make_double2(a.x - br, a.y - bi);
+        a = make_double2(a.x + br, a.y + bi);
+        return;
+    }
     const double re = fma(b.x, w.x, fma(-b.y, w.y, a.x)), im = fma(b.x, w.y, fma(b.y, w.x, a.y));
     b = make_double2(fma(2.0, a.x, -re), fma(2.0, a.y, -im));
     a = make_double2(re, im);
 }
 
 // Twiddles of one task of a pass of S stages, the first of length 2 half1: with tb = task mod half1, stage q uses
-// W_{2 half1 2^q}^{tb + u half1}, u < 2^q; w[q] holds u = 0 and w3 u = 1 of the third stage; u + 2^{q-1} is -i times u.
-template <int S>
+// W_{2 half1 2^q}^{tb + u half1}, u < 2^q; w[q] holds u = 0 and w3 u = 1 of the third stage; u + 2^{q-1} is -i times u
+// (PLAIN: all from the table, u at 2^q - 1 + u).
+template <int S, bool PLAIN>
 struct PassTwiddles {
-    double2 w[S], w3;
+    double2 w[PLAIN ? (1 << S) - 1 : S], w3;
     __device__ __forceinline__ void load(int sg, int task, int logN, const double2 *__restrict__ tw)
     {
         const int half1 = 1 << sg, tb = task & (half1 - 1);
+        if (PLAIN) {
+#pragma unroll
+            for (int q = 0; q < S; ++q)
+#pragma unroll
+                for (int u = 0; u < (1 << q); ++u)
+                    w[(1 << q) - 1 + u] = __ldg(tw + ((tb + u * half1) << (logN - (sg + 1 + q))));
+            return;
+        }
 #pragma unroll
         for (int q = 0; q < S; ++q) w[q] = __ldg(tw + (tb << (logN - (sg + 1 + q))));
         if (S == 3) w3 = __ldg(tw + ((tb + half1) << (logN - (sg + 3))));
@@ -75,8 +95,8 @@ struct PassTwiddles {
 
 // s (1..3) consecutive radix-2 DIT stages of lengths L1 = 2^(sg + 1), 2 L1, .., on a bit-reversed
 // sequence z (one mic).  Task `task` in [0, H / 2^s) owns points base + t * L1/2, t = 0 .. 2^s - 1.
-template <int S>
-__device__ __forceinline__ void fft_pass(double2 *__restrict__ z, int sg, int task, const PassTwiddles<S> &tws)
+template <int S, bool PLAIN>
+__device__ __forceinline__ void fft_pass(double2 *__restrict__ z, int sg, int task, const PassTwiddles<S, PLAIN> &tws)
 {
     const int half1 = 1 << sg;
     const int base = ((task >> sg) << (sg + S)) + (task & (half1 - 1));   // the pass spans 2^(sg + S) points
@@ -89,9 +109,13 @@ __device__ __forceinline__ void fft_pass(double2 *__restrict__ z, int sg, int ta
         for (int t = 0; t < (1 << S); ++t) {
             if (t & (1 << q)) continue;
             const int u = t & ((1 << q) - 1);
+            if (PLAIN) {
+                butterfly<true>(v[t], v[t + (1 << q)], tws.w[(1 << q) - 1 + u]);
+                continue;
+            }
             const double2 w1 = S == 3 && q == 2 && (u & 1) ? tws.w3 : tws.w[q];
             const bool rot = q > 0 && (u >> (q - 1));   // the upper half of the u: times -i
-            butterfly(v[t], v[t + (1 << q)], rot ? make_double2(w1.y, -w1.x) : w1);
+            butterfly<false>(v[t], v[t + (1 << q)], rot ? make_double2(w1.y, -w1.x) : w1);
         }
 #pragma unroll
     for (int t = 0; t < (1 << S); ++t) z[zp(base + t * half1)] = v[t];
@@ -99,7 +123,7 @@ __device__ __forceinline__ void fft_pass(double2 *__restrict__ z, int sg, int ta
 
 // The remaining stages st .. logH - 1 of `nm` sequences in shared memory.  A thread keeps one task per pass and
 // its twiddles, and walks the mics (all of them, or every ngrp-th where the CTA holds ngrp threads per task).
-template <int S>
+template <int S, bool PLAIN>
 __device__ __forceinline__ void fft_pass_mics(double2 *zs, int nm, int stride, int st, int logH, int logN,
                                               const double2 *__restrict__ tw)
 {
@@ -107,13 +131,14 @@ __device__ __forceinline__ void fft_pass_mics(double2 *zs, int nm, int stride, i
     const int nt = blockDim.x;
     const int grp = T < nt ? threadIdx.x >> logT : 0, ngrp = T < nt ? nt >> logT : 1;
     for (int task = T < nt ? threadIdx.x & (T - 1) : threadIdx.x; task < T; task += nt) {
-        PassTwiddles<S> w;
+        PassTwiddles<S, PLAIN> w;
         w.load(st, task, logN, tw);
-        for (int ml = grp; ml < nm; ml += ngrp) fft_pass<S>(zs + ml * stride, st, task, w);
+        for (int ml = grp; ml < nm; ml += ngrp) fft_pass<S, PLAIN>(zs + ml * stride, st, task, w);
     }
     __syncthreads();
 }
 
+template <bool PLAIN>
 __device__ __forceinline__ void fft_passes(double2 *zs, int nm, int stride, int st, int logH, int logN,
                                            const double2 *__restrict__ tw)
 {
@@ -121,9 +146,9 @@ __device__ __forceinline__ void fft_passes(double2 *zs, int nm, int stride, int 
         const int left = logH - st;
         // four left: 2 + 2 rather than 3 + 1
         const int S = left == 4 ? 2 : (left >= 3 ? 3 : left);
-        if (S == 3) fft_pass_mics<3>(zs, nm, stride, st, logH, logN, tw);
-        else if (S == 2) fft_pass_mics<2>(zs, nm, stride, st, logH, logN, tw);
-        else fft_pass_mics<1>(zs, nm, stride, st, logH, logN, tw);
+        if (S == 3) fft_pass_mics<3, PLAIN>(zs, nm, stride, st, logH, logN, tw);
+        else if (S == 2) fft_pass_mics<2, PLAIN>(zs, nm, stride, st, logH, logN, tw);
+        else fft_pass_mics<1, PLAIN>(zs, nm, stride, st, logH, logN, tw);
         st += S;
     }
 }
@@ -147,10 +172,26 @@ __device__ __forceinline__ void first_stages(double2 (&v)[8])
     }
     const double h = 0.70710678118654752440;
     pair(v[0], v[4]);
-    butterfly(v[1], v[5], make_double2(h, -h));
+    butterfly<false>(v[1], v[5], make_double2(h, -h));
     turn(v[6]);
     pair(v[2], v[6]);
-    butterfly(v[3], v[7], make_double2(-h, -h));
+    butterfly<false>(v[3], v[7], make_double2(-h, -h));
+}
+// The same from the table's W_4^1, W_8^1 and W_8^3 (see butterfly).
+__device__ __forceinline__ void first_stages_plain(double2 (&v)[8], double2 w41, double2 w81, double2 w83)
+{
+    const double2 one = make_double2(1.0, 0.0);
+#pragma unroll
+    for (int t = 0; t < 8; t += 2) butterfly<true>(v[t], v[t + 1], one);
+#pragma unroll
+    for (int t = 0; t < 8; t += 4) {
+        butterfly<true>(v[t], v[t + 2], one);
+        butterfly<true>(v[t + 1], v[t + 3], w41);
+    }
+    butterfly<true>(v[0], v[4], one);
+    butterfly<true>(v[1], v[5], w81);
+    butterfly<true>(v[2], v[6], w41);
+    butterfly<true>(v[3], v[7], w83);
 }
 
 // The low n bits of x in reverse order.
@@ -223,6 +264,8 @@ __global__ void __launch_bounds__(512) fft_window_kernel(const TS *__restrict__ 
     const int m0 = blockIdx.x * mpb;
     const int nm = min(mpb, M - m0);
     const TS *src = samples + (w * (int64_t)hop) * M + m0;
+    constexpr bool PLAIN = OUT == OUT_C64;   // see butterfly
+    const double2 w41 = __ldg(tw + (N >> 2)), w81 = __ldg(tw + (N >> 3)), w83 = __ldg(tw + 3 * (N >> 3));
 
     // load + window + the first three stages: task = 8 consecutive slots of the bit-reversed order, i.e. points
     // rev(task) + H/8 {0, 4, 2, 6, 1, 5, 3, 7} (H >= 8)
@@ -246,15 +289,18 @@ __global__ void __launch_bounds__(512) fft_window_kernel(const TS *__restrict__ 
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
             const int j = j0 + ((((t & 1) << 2) | (t & 2) | (t >> 2)) << logT);
-            v[t] = make_double2((double)x0[t] * __ldg(window + 2 * j), (double)x1[t] * __ldg(window + 2 * j + 1));
+            const double a0 = __ldg(window + 2 * j), a1 = __ldg(window + 2 * j + 1);
+            v[t] = PLAIN ? make_double2(__dmul_rn((double)x0[t], a0), __dmul_rn((double)x1[t], a1))
+                         : make_double2((double)x0[t] * a0, (double)x1[t] * a1);
         }
-        first_stages(v);
+        if (PLAIN) first_stages_plain(v, w41, w81, w83);
+        else first_stages(v);
         double2 *z = zs + ml * stride + 9 * task;   // zp(8 task + t) = 9 task + t
 #pragma unroll
         for (int t = 0; t < 8; ++t) z[t] = v[t];
     }
     __syncthreads();
-    fft_passes(zs, nm, stride, 3, logH, logH + 1, tw);
+    fft_passes<PLAIN>(zs, nm, stride, 3, logH, logH + 1, tw);
 
     // real-input split: X[k] = E + W^k O,  E = (Z[k] + conj(Z[H-k]))/2,  O = -i (Z[k] - conj(Z[H-k]))/2
     // (bins k and H - k share their two points: read once for both)
@@ -270,8 +316,8 @@ __global__ void __launch_bounds__(512) fft_window_kernel(const TS *__restrict__ 
             const double er = 0.5 * (zk.x + zc.x), ei = 0.5 * (zk.y - zc.y);
             const double orr = 0.5 * (zk.y + zc.y), oi = -0.5 * (zk.x - zc.x);
             const double2 wk = k < H ? __ldg(tw + k) : make_double2(-1.0, 0.0);
-            const double xr = fma(wk.x, orr, fma(-wk.y, oi, er));
-            const double xi = fma(wk.x, oi, fma(wk.y, orr, ei));
+            const double xr = PLAIN ? er + (wk.x * orr - wk.y * oi) : fma(wk.x, orr, fma(-wk.y, oi, er));
+            const double xi = PLAIN ? ei + (wk.x * oi + wk.y * orr) : fma(wk.x, oi, fma(wk.y, orr, ei));
             put_bin<OUT>(out, nw, (int)blockIdx.y, M, m0 + ml, k - bin_lo, xr, xi, R, KC, lo_elems);
         };
         bin(u, za, zb);
@@ -607,7 +653,7 @@ __global__ void __launch_bounds__(256) fft_sub_kernel(const TS *__restrict__ sam
         zs[zp((int)(__brev((unsigned)i) >> (32 - logHs)))] = make_double2(x0, x1);
     }
     __syncthreads();
-    fft_passes(zs, 1, 0, 0, logHs, 31 - __clz(N), tw);
+    fft_passes<true>(zs, 1, 0, 0, logHs, 31 - __clz(N), tw);
     double2 *dst = scratch + ((wi * M + m) * D + d) * (int64_t)FFT_SUB_H;
     for (int k = threadIdx.x; k < FFT_SUB_H; k += blockDim.x) dst[k] = zs[zp(k)];
 }
