@@ -199,15 +199,15 @@ __global__ void __launch_bounds__(GTC_THREADS, 1) gram_tc_kernel(const __grid_co
         const int q = warp & 3;
         const int rho = q * 32 + lane;              // accumulator row = component in the row block
         const int p = lane & 1;                     // 0: Re row 2r, 1: Im row 2r+1
-        bool ok = true;
-        for (int64_t li = 0; li < nmine && ok; ++li) {
+        int64_t li = 0;
+        for (; li < nmine; ++li) {
             const int64_t item = blockIdx.x + li * gridDim.x;
             const int64_t bin = item / a.nper;
             const GtcItem g = a.it[item - bin * a.nper];
             const int buf = (int)(li & 1);
-            ok = __all_sync(0xffffffffu,
-                            tc::mbar_wait(&accf[buf], (uint32_t)((li >> 1) & 1), abort_flag, a.wait_limit_ns));
-            if (!ok) break;
+            if (!__all_sync(0xffffffffu,
+                            tc::mbar_wait(&accf[buf], (uint32_t)((li >> 1) & 1), abort_flag, a.wait_limit_ns)))
+                break;
             tc::tc_fence_after();
             const int r = (GTC_ROWT * 32 * g.rb + rho) >> 1;   // mic of this row
             double2 *crow = a.csm + ((int64_t)bin * a.M + r) * a.M;
@@ -240,6 +240,19 @@ __global__ void __launch_bounds__(GTC_THREADS, 1) gram_tc_kernel(const __grid_co
             }
             tc::tc_fence_before();
             tc::mbar_arrive(&acce[buf]);
+        }
+        // A wait ran out: the items from here on have no sums.  Their entries become NaN, not what the buffer held: the
+        // finished matrix is written into memory that nothing has cleared.
+        for (; li < nmine; ++li) {
+            const int64_t item = blockIdx.x + li * gridDim.x;
+            const int64_t bin = item / a.nper;
+            const GtcItem g = a.it[item - bin * a.nper];
+            const int r = (GTC_ROWT * 32 * g.rb + rho) >> 1;
+            const double nan = __longlong_as_double(0x7ff8000000000000ll);
+            // the row's two lanes take every other column
+            for (int c = max(r, 16 * g.c0) + p; r < a.M && c < min(a.M, 16 * (g.c0 + g.nc)); c += 2)
+                if (a.out) put_hermitian(a.out + (int64_t)bin * a.M * a.M, a.M, r, c, nan, nan, a.scale);
+                else a.csm[((int64_t)bin * a.M + r) * a.M + c] = make_double2(nan, nan);
         }
     }
     __syncthreads();

@@ -188,10 +188,10 @@ enum acb_tc_precision {
 size_t acb_map_tc_workspace_bytes(int num_mics, int num_bins, int precision);
 
 /* Limit of each bounded device-side wait in the tensor-core kernels (acb_map_tc, acb_map_tc_batch,
- * acb_map_tc_noalloc and the tensor-core CSM forms of acb_csm_accumulate); no counterpart in the
- * reference.  A wait that runs out sets the launch's error word to 1 (where one is given), the CTA
- * lets its own copies and MMAs finish, frees its tensor memory and exits, so the device context stays
- * usable.  Applies to launches enqueued after the call; 0 restores the default of 0.5 s.  Returns
+ * acb_map_tc_noalloc and the tensor-core CSM forms of acb_csm_accumulate and acb_csm_finished); no
+ * counterpart in the reference.  A wait that runs out sets the launch's error word to 1 (where one is
+ * given; the CSM forms write NaN to every entry whose sums are missing), the CTA lets its own copies
+ * and MMAs finish, frees its tensor memory and exits, so the device context stays usable.  Applies to launches enqueued after the call; 0 restores the default of 0.5 s.  Returns
  * the previous limit.  Process-wide (all devices and host threads). */
 uint64_t acb_tc_set_wait_limit_ns(uint64_t limit_ns);
 
