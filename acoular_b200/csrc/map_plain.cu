@@ -162,8 +162,9 @@ __device__ __forceinline__ void synth_tile(const MapArgs &a, const SincosTable &
 // sum Re(conj(h_a) C_ab h_b) for points g = lane / 4 and g + 8.  `diag`: the two ranges are the same mics, only
 // b > a counts, and half the (real) diagonal with `with_diag`.  Rows of C are read from global memory (L2) straight
 // into the B operand, two steps of 4 columns ahead: a lane's element C[a][b] serves the real and the imaginary
-// product, and every element is read once per CTA.  Rows and columns past the range repeat the last one: their
-// steering values are zeros.
+// product, and every element is read once per CTA.  What does not count takes no part, so that it may be infinite or NaN
+// (the diagonal of a CSM whose removal was asked for, say): entries left of the diagonal, a diagonal that is not wanted
+// and columns past the range enter as zeros, and rows past the range (their loads repeat the last one) are left out.
 template <int NW, int Q>
 __device__ __forceinline__ void quad_tile(const double2 *__restrict__ C, int M, const double2 *ha, int ra0, int na,
                                           const double2 *hb, int cb0, int nb, bool diag, bool with_diag, double &off0,
@@ -172,8 +173,7 @@ __device__ __forceinline__ void quad_tile(const double2 *__restrict__ C, int M, 
     constexpr int kRows = 8 * Q;   // rows per group
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int ngrp = (na + kRows - 1) / kRows;
-    const double dscale = with_diag ? 0.5 : 0.0;
+    const int ngrp = (na + kRows - 1) / kRows, whole = nb & ~3;
     for (int j = 0; j < ngrp; ++j) {
         // snake order over the warps (the groups' lengths fall with j), started at another warp in each CTA
         const int pos = j % NW;
@@ -210,7 +210,7 @@ __device__ __forceinline__ void quad_tile(const double2 *__restrict__ C, int M, 
                     c0[q] = c1[q];
                     c1[q] = __ldg(cp[q] + min(b + 8 + t, nb - 1));
                     const int d = b + t - a0 - 8 * q - g;   // column less row
-                    if (d <= 0) x = make_double2(d == 0 ? dscale * x.x : 0.0, 0.0);
+                    if (d <= 0 || b + t >= nb) x = make_double2(d == 0 && with_diag && b + t < nb ? 0.5 * x.x : 0.0, 0.0);
                     if (b >= a0 + 8 * q) {
                         mma_f64(re[q], h0.x, h1.x, h0.y, h1.y, x.x, -x.y);
                         mma_f64(im[q], h0.x, h1.x, h0.y, h1.y, x.y, x.x);
@@ -219,7 +219,7 @@ __device__ __forceinline__ void quad_tile(const double2 *__restrict__ C, int M, 
             }
         }
 #pragma unroll 2
-        for (; b < nb; b += 4) {
+        for (; b < whole; b += 4) {
             const double2 h0 = n0, h1 = n1;
             hp = hp < hend ? hp + 4 * kPtsPad : hp;
             n0 = hp[0];
@@ -234,11 +234,19 @@ __device__ __forceinline__ void quad_tile(const double2 *__restrict__ C, int M, 
                 mma_f64(im[q], h0.x, h1.x, h0.y, h1.y, x.y, x.x);
             }
         }
+        if (b < nb) {   // one to three columns left
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const double2 x = b + t < nb ? c0[q] : make_double2(0.0, 0.0);
+                mma_f64(re[q], n0.x, n1.x, n0.y, n1.y, x.x, -x.y);
+                mma_f64(im[q], n0.x, n1.x, n0.y, n1.y, x.y, x.x);
+            }
+        }
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
-            if (Q > 2 && a0 + 8 * q >= na) break;   // no such rows (their steering tile ends at a multiple of 16)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
+                if (a0 + 8 * q + 2 * t + e >= na) break;   // no such row
                 const double2 *r = ha + (a0 + 8 * q + 2 * t + e) * kPtsPad + g;
                 double2 h = r[0];
                 off0 = fma(h.x, re[q][e], fma(h.y, im[q][e], off0));
