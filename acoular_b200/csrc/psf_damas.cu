@@ -584,17 +584,15 @@ __global__ void __launch_bounds__(kDamasThreads) damas_ahead_kernel(const double
                 for (int q = 0; q < 8; ++q) {
                     if (q >= left || q == g1 || q == g2) continue;   // uniform
                     const double xv = xl[(grp * 8 + q) * kDamasRows];
-                    double v0 = c0[q], v1 = c1[q];
-                    if (q == gk) {   // within the block only the columns right of the row
-                        v0 = lane <= warp ? 0.0 : v0;
-                        v1 = lane <= warp + 16 ? 0.0 : v1;
-                    }
-                    if (q & 1) {
-                        p0 = fma(v0, xv, p0);
-                        p1 = fma(v1, xv, p1);
+                    double &t0 = q & 1 ? p0 : s0, &t1 = q & 1 ? p1 : s1;
+                    // within the block only the columns right of the row; the others are left out and not multiplied
+                    // by zero, as an old value (the dirty map's to begin with) may be infinite or NaN
+                    if (q == gk) {
+                        if (lane > warp) t0 = fma(c0[q], xv, t0);
+                        if (lane > warp + 16) t1 = fma(c1[q], xv, t1);
                     } else {
-                        s0 = fma(v0, xv, s0);
-                        s1 = fma(v1, xv, s1);
+                        t0 = fma(c0[q], xv, t0);
+                        t1 = fma(c1[q], xv, t1);
                     }
                 }
                 s0 += p0;
