@@ -583,11 +583,15 @@ __global__ void __launch_bounds__(kQlThreads) heevd_tql_kernel(const double *__r
         __syncthreads();
         if (s_m[buf] == 0) break;
     }
-    // ascending order, ties by index (as a stable sort)
+    // ascending order, ties by index (as a stable sort), NaN last: a permutation whatever the values, since the
+    // back-transformation reads columns by it
     for (int k = tid; k < M; k += kQlThreads) {
         const double dk = d[k];
         int rank = 0;
-        for (int j = 0; j < M; ++j) rank += (d[j] < dk) || (d[j] == dk && j < k);
+        for (int j = 0; j < M; ++j) {
+            const double dj = d[j];
+            rank += dk != dk ? dj == dj || j < k : dj < dk || (dj == dk && j < k);
+        }
         wall[(int64_t)b * M + rank] = dk;
         permall[(int64_t)b * M + rank] = k;
     }
