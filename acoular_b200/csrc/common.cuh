@@ -11,7 +11,8 @@ namespace acb {
 // Record the last CUDA error text for acb_last_cuda_error().
 void set_cuda_error(cudaError_t e);
 
-// Limit of one bounded device-side wait of the tensor-core kernels (acb_tc_set_wait_limit_ns).
+// Limit of one bounded device-side wait of the tensor-core kernels and of the exchanges inside a cluster
+// (acb_tc_set_wait_limit_ns).
 uint64_t tc_wait_limit_ns();
 
 inline int check_launch()

@@ -391,38 +391,6 @@ __host__ __device__ inline int64_t gs_smem_bytes(int64_t G)
     return (nblk * kDamasRows + (int64_t)kGsStages * 3 * kGsTile + kGsRing * kDamasMaxCta * kDamasRows) * 8;
 }
 
-// 8 bytes to the same place of CTA `rank`'s shared memory, counted on that CTA's mbarrier.
-__device__ __forceinline__ void gs_send(int rank, const double *dst, double v, const uint64_t *bar)
-{
-    uint32_t ra, rb;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(tc::smem_u32(dst)), "r"(rank));
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(tc::smem_u32(bar)), "r"(rank));
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(ra), "d"(v),
-                 "r"(rb)
-                 : "memory");
-}
-
-// Bounded wait (half a second, or the flag raised by another thread): then it returns at once and the caller carries on.
-__device__ __forceinline__ void gs_wait(const uint64_t *bar, uint32_t parity, volatile int *gave_up)
-{
-    const uint32_t addr = tc::smem_u32(bar);
-    uint64_t t0 = 0;
-    while (true) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 100000;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (ok || *gave_up) return;
-        const uint64_t t = tc::globaltimer_ns();
-        if (t0 == 0) t0 = t;
-        else if (t - t0 > 500ull * 1000 * 1000) *gave_up = 1;
-    }
-}
-
 // max(0, u), and 0 for NaN as fmax gives it, on the integer pipe (sign bit or an exponent of ones with mantissa)
 __device__ __forceinline__ double gs_clamp(double u)
 {
@@ -431,12 +399,13 @@ __device__ __forceinline__ double gs_clamp(double u)
 
 __global__ void __launch_bounds__(kDamasThreads) damas_ahead_kernel(const double *__restrict__ A, int64_t G,
                                                                    const double *__restrict__ y,
-                                                                   double *__restrict__ x, int n_iter, double relax)
+                                                                   double *__restrict__ x, int n_iter, double relax,
+                                                                   uint64_t limit_ns)
 {
     extern __shared__ double sm[];
     __shared__ uint64_t xbar[kGsRing], pbar[kGsRing], tbar[kGsStages];
-    __shared__ int gave_up_s;
-    volatile int *gave_up = &gave_up_s;
+    __shared__ int stop_s;
+    volatile int *stop = &stop_s;
     cg::cluster_group cluster = cg::this_cluster();
     const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     const int64_t bin = blockIdx.x / C;
@@ -457,7 +426,7 @@ __global__ void __launch_bounds__(kDamasThreads) damas_ahead_kernel(const double
             tc::mbar_init(&pbar[q], 1);
         }
         for (int q = 0; q < kGsStages; ++q) tc::mbar_init(&tbar[q], 96);
-        gave_up_s = 0;
+        stop_s = 0;
         tc::fence_mbar_init();
         for (int q = 0; q < kGsRing; ++q)   // the first round of each ring
             if (rank == 0) tc::mbar_arrive_expect_tx(&pbar[q], (uint32_t)((C - 1) * kDamasRows * 8));
@@ -477,13 +446,17 @@ __global__ void __launch_bounds__(kDamasThreads) damas_ahead_kernel(const double
             const double *D = tiles + st * 3 * kGsTile + lane, *N1 = D + kGsTile, *N2 = N1 + kGsTile;
             const double xold = xs[g0 + lane];
             const double c = fma(relax, yv, fma(1.0 - relax, xold, acc1));
-            gs_wait(&tbar[st], (uint32_t)(t / kGsStages) & 1, gave_up);
-            gs_wait(&pbar[slot], (uint32_t)(t / kGsRing) & 1, gave_up);
+            const bool here = tc::cluster_wait(&tbar[st], (uint32_t)(t / kGsStages) & 1, stop, limit_ns) &&
+                              tc::cluster_wait(&pbar[slot], (uint32_t)(t / kGsRing) & 1, stop, limit_ns);
+            if (!__all_sync(0xffffffffu, here)) {
+                tc::cluster_stop(stop, C);
+                break;
+            }
             double sum[2] = {0.0, 0.0};
 #pragma unroll
             for (int r = 1; r < kDamasMaxCta; ++r)
                 if (r < C) sum[r & 1] += part[(slot * kDamasMaxCta + r) * kDamasRows + lane];
-            if (lane == 0 && t + kGsRing < steps && !*gave_up)
+            if (lane == 0 && t + kGsRing < steps)
                 tc::mbar_arrive_expect_tx(&pbar[slot], (uint32_t)((C - 1) * kDamasRows * 8));
             double u = row ? fma(-relax, sum[0] + sum[1], c) : 0.0;
             acc1 = acc2;
@@ -504,7 +477,7 @@ __global__ void __launch_bounds__(kDamasThreads) damas_ahead_kernel(const double
             }
             xs[g0 + lane] = xv;
             if (t + 3 < steps)   // the other CTAs wait for step t's values at step t + 3
-                for (int r = 1; r < C; ++r) gs_send(r, xs + g0 + lane, xv, &xbar[slot]);
+                for (int r = 1; r < C; ++r) tc::cluster_send(r, xs + g0 + lane, xv, &xbar[slot]);
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&xbar[slot]);
         }
@@ -513,8 +486,13 @@ __global__ void __launch_bounds__(kDamasThreads) damas_ahead_kernel(const double
         const int which = warp - 1;
         for (int64_t t = 0; t < steps; ++t) {
             // the stage was read at step t - 3
-            if (t >= kGsStages) gs_wait(&xbar[(t - kGsStages) % kGsRing], (uint32_t)((t - kGsStages) / kGsRing) & 1,
-                                        gave_up);
+            const bool here = t < kGsStages || tc::cluster_wait(&xbar[(t - kGsStages) % kGsRing],
+                                                                (uint32_t)((t - kGsStages) / kGsRing) & 1, stop,
+                                                                limit_ns);
+            if (!__all_sync(0xffffffffu, here)) {
+                tc::cluster_stop(stop, C);
+                break;
+            }
             const int64_t g0 = (t % nblk) * kDamasRows, gr = ((t + which) % nblk) * kDamasRows;
             const int st = (int)(t % kGsStages);
             double *dst = tiles + (st * 3 + which) * kGsTile + lane * kDamasPad;   // column `lane`
@@ -560,8 +538,12 @@ __global__ void __launch_bounds__(kDamasThreads) damas_ahead_kernel(const double
             const int kn = k + 1 == nblk ? 0 : k + 1;
             const double *rn = kn ? rk + block : row0;
             if (t >= 3) {
-                gs_wait(&xbar[(t - 3) % kGsRing], (uint32_t)((t - 3) / kGsRing) & 1, gave_up);
-                if (threadIdx.x == 0 && t + 1 < steps && !*gave_up)
+                if (!__all_sync(0xffffffffu, tc::cluster_wait(&xbar[(t - 3) % kGsRing],
+                                                              (uint32_t)((t - 3) / kGsRing) & 1, stop, limit_ns))) {
+                    tc::cluster_stop(stop, C);
+                    break;
+                }
+                if (threadIdx.x == 0 && t + 1 < steps)
                     tc::mbar_arrive_expect_tx(&xbar[(t - 3) % kGsRing], kDamasRows * 8);   // for step t + 1
             }
             // places in the slice of block k and of the blocks solved at steps t - 1 and t - 2 (the solver's)
@@ -605,18 +587,15 @@ __global__ void __launch_bounds__(kDamasThreads) damas_ahead_kernel(const double
             for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             const int slot = (int)(t % kGsRing);
             if ((lane & 15) == 0)
-                gs_send(0, part + (slot * kDamasMaxCta + rank) * kDamasRows + warp + (lane ? 16 : 0), s, &pbar[slot]);
+                tc::cluster_send(0, part + (slot * kDamasMaxCta + rank) * kDamasRows + warp + (lane ? 16 : 0), s, &pbar[slot]);
             k = kn;
             rk = rn;
         }
     }
-    if (*gave_up) __nanosleep(1000000);   // let what is still under way land before a CTA ends
-    cluster.sync();
-    if (rank == 0) {
-        const bool bad = *gave_up != 0;   // a wait ran out: no result
+    const bool stopped = tc::cluster_end(cluster, stop);
+    if (rank == 0)   // a wait ran out, in whichever CTA: no result
         for (int64_t i = threadIdx.x; i < G; i += kDamasThreads)
-            xg[i] = bad ? __longlong_as_double(0x7ff8000000000000ll) : xs[i];
-    }
+            xg[i] = stopped ? __longlong_as_double(0x7ff8000000000000ll) : xs[i];
 }
 
 }  // namespace acb
@@ -679,8 +658,8 @@ int acb_damas_gauss_seidel_f64(const double *psf, int64_t num_grid, int num_bins
     // the form two blocks ahead: at least six blocks, four CTAs, and its tiles beside the solution
     const int64_t smem_ahead = gs_smem_bytes(num_grid);
     const bool ahead = num_grid > 5 * kDamasRows && C >= 4 && smem_ahead <= smem_max - 1024;
-    auto kern = ahead ? damas_ahead_kernel : damas_kernel;
     const size_t smem_used = ahead ? (size_t)smem_ahead : smem;
+    const void *kern = ahead ? reinterpret_cast<const void *>(damas_ahead_kernel) : reinterpret_cast<const void *>(damas_kernel);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_used) != cudaSuccess)
         return ACB_ERR_CUDA;
     cudaLaunchConfig_t cfg = {};
@@ -695,8 +674,11 @@ int acb_damas_gauss_seidel_f64(const double *psf, int64_t num_grid, int num_bins
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, kern, psf, num_grid, dirty_map, solution, n_iter, relax) != cudaSuccess)
-        return ACB_ERR_CUDA;
+    const cudaError_t err =
+        ahead ? cudaLaunchKernelEx(&cfg, damas_ahead_kernel, psf, num_grid, dirty_map, solution, n_iter, relax,
+                                   tc_wait_limit_ns())
+              : cudaLaunchKernelEx(&cfg, damas_kernel, psf, num_grid, dirty_map, solution, n_iter, relax);
+    if (err != cudaSuccess) return ACB_ERR_CUDA;
     return check_launch();
 }
 

@@ -88,6 +88,68 @@ __host__ __device__ constexpr uint64_t drain_limit_ns(uint64_t limit_ns)
     return 4 * limit_ns > 200000000ull ? 4 * limit_ns : 200000000ull;
 }
 
+// Data between the CTAs of a cluster: asynchronous stores to the same place of another CTA's shared memory, counted on
+// that CTA's mbarrier, and bounded waits for them.  One word per CTA, `stop`, ends a cluster early: whoever gives up
+// raises it in every CTA, no wait holds on beside it, and the roles leave their loops instead of going on with what they
+// have, so that nobody sends more than the step at hand.  cluster_end then tells every CTA alike.
+__device__ __forceinline__ uint32_t cluster_addr(const volatile void *p, int rank)
+{
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(const_cast<const void *>(p))), "r"(rank));
+    return a;
+}
+
+__device__ __forceinline__ void cluster_send(int rank, const double *dst, double v, const uint64_t *bar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(
+                     cluster_addr(dst, rank)),
+                 "d"(v), "r"(cluster_addr(bar, rank))
+                 : "memory");
+}
+
+// Wait for what the other CTAs send.  Gives up after `limit_ns` or where `stop` is raised; returns false then.
+__device__ __forceinline__ bool cluster_wait(const uint64_t *bar, uint32_t parity, const volatile int *stop,
+                                             uint64_t limit_ns)
+{
+    const uint32_t addr = smem_u32(bar), hint = limit_ns < 100000u ? (uint32_t)limit_ns : 100000u;
+    uint64_t t0 = 0;
+    while (true) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(addr), "r"(parity), "r"(hint)
+            : "memory");
+        if (ok) return true;
+        if (*stop) return false;
+        const uint64_t t = globaltimer_ns();
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > limit_ns) return false;
+    }
+}
+
+// Raise `stop` in all `nctas` CTAs of the cluster (each of them is between its first cluster barrier and cluster_end).
+__device__ __forceinline__ void cluster_stop(volatile int *stop, int nctas)
+{
+    for (int r = 0; r < nctas; ++r)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(stop, r)), "r"(1) : "memory");
+}
+
+// The end of a kernel's roles, by every thread of the cluster: whether it was stopped.  If so, what was still under way
+// has a millisecond to land before a CTA may exit.
+template <class Cluster>
+__device__ __forceinline__ bool cluster_end(Cluster &cluster, const volatile int *stop)
+{
+    cluster.sync();   // every send has been issued and every flag raised
+    if (!*stop) return false;
+    const uint64_t t0 = globaltimer_ns();
+    for (int i = 0; i < 100000 && globaltimer_ns() - t0 < 1000000; ++i) __nanosleep(1000);
+    cluster.sync();
+    return true;
+}
+
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Bulk global -> shared copy completing on an mbarrier (into the issuing CTA alone).

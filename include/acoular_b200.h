@@ -188,8 +188,9 @@ enum acb_tc_precision {
 size_t acb_map_tc_workspace_bytes(int num_mics, int num_bins, int precision);
 
 /* Limit of each bounded device-side wait in the tensor-core kernels (acb_map_tc, acb_map_tc_batch,
- * acb_map_tc_noalloc and the tensor-core CSM forms of acb_csm_accumulate and acb_csm_finished); no
- * counterpart in the reference.  A wait that runs out sets the launch's error word to 1 (where one is
+ * acb_map_tc_noalloc and the tensor-core CSM forms of acb_csm_accumulate and acb_csm_finished) and in
+ * the exchanges inside a cluster of acb_damas_gauss_seidel_f64, which says what one that runs out leaves;
+ * no counterpart in the reference.  A wait that runs out sets the launch's error word to 1 (where one is
  * given; the CSM forms write NaN to every entry whose sums are missing), the CTA lets its own copies
  * and MMAs finish, frees its tensor memory and exits, so the device context stays usable.  Applies to launches enqueued after the call; 0 restores the default of 0.5 s.  Returns
  * the previous limit.  Process-wide (all devices and host threads). */
@@ -257,7 +258,9 @@ int acb_psf_f64(const acb_map_params *p, int num_sources, const int64_t *sources
  *   result after n_iter Gauss-Seidel sweeps with relaxation `relax` (negative values set to 0).
  *   cta_per_bin: 1, 2, 4 or 8 CTAs (one cluster) per bin, 0 = choose from num_bins and the SM count.
  *   ACB_ERR_UNSUPPORTED when a bin's solution (8 G bytes + 38 KB) exceeds a CTA's shared memory
- *   (G above about 24,000). */
+ *   (G above about 24,000).
+ * The CTAs of a bin exchange values and sums with bounded waits (acb_tc_set_wait_limit_ns).  Where one runs out, that
+ * bin's solution is NaN throughout; the other bins' are not touched by it. */
 int acb_damas_gauss_seidel_f64(const double *psf, int64_t num_grid, int num_bins, const double *dirty_map,
                                double *solution, int n_iter, double relax, int cta_per_bin, void *stream);
 
