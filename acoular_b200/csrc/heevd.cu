@@ -184,39 +184,6 @@ __global__ void __launch_bounds__(kEvThreads) heevd_tridiag_kernel(double2 *__re
     }
 }
 
-// 16 bytes to the same place of CTA `rank`'s shared memory, counted on that CTA's mbarrier.
-__device__ __forceinline__ void send_to(int rank, const double2 *dst, double2 v, const uint64_t *bar)
-{
-    uint32_t ra, rb;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(tc::smem_u32(dst)), "r"(rank));
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(tc::smem_u32(bar)), "r"(rank));
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(ra),
-                 "d"(v.x), "d"(v.y), "r"(rb)
-                 : "memory");
-}
-
-// Bounded wait for data that other CTAs of the cluster sent; after the limit (half a second, or the flag raised by
-// another thread) it returns at once and the caller carries on, so that the kernel always ends.
-__device__ __forceinline__ void wait_sent(const uint64_t *bar, uint32_t parity, volatile int *gave_up)
-{
-    const uint32_t addr = tc::smem_u32(bar);
-    uint64_t t0 = 0;
-    while (true) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 100000;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (ok || *gave_up) return;
-        const uint64_t t = tc::globaltimer_ns();
-        if (t0 == 0) t0 = t;
-        else if (t - t0 > 500ull * 1000 * 1000) *gave_up = 1;
-    }
-}
-
 // The same reduction with the lower triangle in the shared memory of a cluster of C CTAs (rows r = rank + C l in CTA
 // `rank`, packed), for matrices that fit (up to about 150 rows in one CTA, 205 in two, 270 in four, 335 in eight).
 // The rank-2 update of step i - 1 and the product A22 v of step i are one pass over the stored elements: every CTA
@@ -237,13 +204,14 @@ __host__ __device__ constexpr int ev_packed(int rank, int C, int l) { return l *
 template <int MINB>
 __global__ void __launch_bounds__(kEvThreads, MINB)
     heevd_tridiag_cluster_kernel(const double2 *__restrict__ csm, int M, double *__restrict__ dall,
-                                 double *__restrict__ eall, double2 *__restrict__ tauall, double2 *__restrict__ vhall)
+                                 double *__restrict__ eall, double2 *__restrict__ tauall, double2 *__restrict__ vhall,
+                                 uint64_t limit_ns)
 {
     extern __shared__ double2 ev_sm[];
     __shared__ uint64_t bars[2];   // column; products
     __shared__ double red[2][kEvWarps];
-    __shared__ int gave_up_s;
-    volatile int *gave_up = &gave_up_s;
+    __shared__ int stop_s;
+    volatile int *stop = &stop_s;
     cg::cluster_group cluster = cg::this_cluster();
     const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     const int b = blockIdx.x / C;
@@ -263,7 +231,7 @@ __global__ void __launch_bounds__(kEvThreads, MINB)
     if (tid == 0) {
         tc::mbar_init(&bars[0], 1);
         tc::mbar_init(&bars[1], 1);
-        gave_up_s = 0;
+        stop_s = 0;
         tc::fence_mbar_init();
     }
     for (int l = warp; l < nl; l += kEvWarps) {
@@ -277,7 +245,7 @@ __global__ void __launch_bounds__(kEvThreads, MINB)
         double2 *x = x0 + (i & 1) * M;
         const int l0 = i < rank ? 0 : (i - rank) / C + 1;   // first own row below i
         // own part of column i of the updated matrix (row i itself included)
-        if (tid == 0 && !*gave_up) tc::mbar_arrive_expect_tx(&bars[0], (uint32_t)((M - i) * sizeof(double2)));
+        if (tid == 0) tc::mbar_arrive_expect_tx(&bars[0], (uint32_t)((M - i) * sizeof(double2)));
         const int lx = i % C == rank ? i / C : l0;
         const double2 vi = v[i], wi = w[i];
         for (int l = lx + tid; l < nl; l += kEvThreads) {
@@ -285,13 +253,15 @@ __global__ void __launch_bounds__(kEvThreads, MINB)
             const double2 t1 = cmulc(wi, v[r]), t2 = cmulc(vi, w[r]);   // v_r conj(w_i), w_r conj(v_i)
             const double2 a = rows[ev_packed(rank, C, l) + i];
             for (int k = 0; k < C; ++k)
-                send_to(k, x + r, make_double2(a.x - (t1.x + t2.x), a.y - (t1.y + t2.y)), &bars[0]);
+                tc::cluster_send(k, x + r, make_double2(a.x - (t1.x + t2.x), a.y - (t1.y + t2.y)), &bars[0]);
         }
-        wait_sent(&bars[0], i & 1, gave_up);
+        bool here = tc::cluster_wait(&bars[0], i & 1, stop, limit_ns);
         if (rank == 0 && tid == 0) d[i] = x[i].x;
-        if (i == M - 1) break;
-        if (tid == 0 && !*gave_up)
-            tc::mbar_arrive_expect_tx(&bars[1], (uint32_t)(C * (M - 1 - i) * sizeof(double2)));
+        if (i == M - 1) {
+            if (!here) tc::cluster_stop(stop, C);
+            break;
+        }
+        if (tid == 0) tc::mbar_arrive_expect_tx(&bars[1], (uint32_t)(C * (M - 1 - i) * sizeof(double2)));
         // the reflector, by every warp: beta = -sign(Re alpha) |(alpha, x)|, tau = (beta - alpha) / beta,
         // v = (1, x / (alpha - beta)); H = I where the column is real and reduced already
         double xn2 = 0.0;
@@ -384,9 +354,9 @@ __global__ void __launch_bounds__(kEvThreads, MINB)
                 s.y += q[u * M + c].y;
             }
             s = cmul(tu, s);
-            for (int k = 0; k < C; ++k) send_to(k, part + rank * M + c, s, &bars[1]);
+            for (int k = 0; k < C; ++k) tc::cluster_send(k, part + rank * M + c, s, &bars[1]);
         }
-        wait_sent(&bars[1], i & 1, gave_up);
+        here = tc::cluster_wait(&bars[1], i & 1, stop, limit_ns) && here;
         // w = p - (tau / 2) (p^H v) v
         double sr = 0.0, si = 0.0;
         for (int r = i + 1 + tid; r < M; r += kEvThreads) {
@@ -428,17 +398,24 @@ __global__ void __launch_bounds__(kEvThreads, MINB)
             e[i] = beta;
             tau[i] = tu;
         }
-        __syncthreads();
+        if (__syncthreads_or(!here)) {
+            tc::cluster_stop(stop, C);
+            break;
+        }
     }
-    if (*gave_up) {   // a wait ran out: no result; let what is still under way land before the CTA ends
-        if (tid == 0) d[0] = __longlong_as_double(0x7ff8000000000000ll);
-        __nanosleep(1000000);
+    const bool stopped = tc::cluster_end(cluster, stop);
+    if (rank == 0) {
+        if (tid == 0) {
+            e[M - 1] = 0.0;
+            tau[M - 1] = make_double2(0.0, 0.0);
+        }
+        if (stopped)   // a wait ran out, in whichever CTA: no result
+            for (int r = tid; r < M; r += kEvThreads) {
+                d[r] = __longlong_as_double(0x7ff8000000000000ll);
+                e[r] = 0.0;
+                tau[r] = make_double2(0.0, 0.0);
+            }
     }
-    if (rank == 0 && tid == 0) {
-        e[M - 1] = 0.0;
-        tau[M - 1] = make_double2(0.0, 0.0);
-    }
-    cluster.sync();
 }
 
 // d, e (B, M) -> eigenvalues w (B, M) ascending, Z (B, M, M) column-major (column j = eigenvector of the
@@ -464,15 +441,23 @@ __global__ void __launch_bounds__(kQlThreads) heevd_tql_kernel(const double *__r
     const int b = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31;
     double *Z = Zall + (int64_t)b * M * M;
+    int bad = 0;
     for (int k = tid; k < M; k += kQlThreads) {
         d[k] = dall[(int64_t)b * M + k];
         e[k] = eall[(int64_t)b * M + k];
+        bad |= d[k] != d[k] || e[k] != e[k];
     }
-    for (int64_t idx = tid; idx < (int64_t)M * M; idx += kQlThreads) Z[idx] = (idx / M == idx % M) ? 1.0 : 0.0;
-    if (tid == 0) s_fail = 0;
+    // a NaN in T (a NaN matrix, or a tridiagonalisation that gave up): no result, and no sweeps for one
+    bad = __syncthreads_or(bad);
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    if (bad)
+        for (int k = tid; k < M; k += kQlThreads) d[k] = nan;
+    for (int64_t idx = tid; idx < (int64_t)M * M; idx += kQlThreads)
+        Z[idx] = bad ? nan : (idx / M == idx % M) ? 1.0 : 0.0;
+    if (tid == 0) s_fail = bad;
     __syncthreads();
     const double eps = 2.220446049250313e-16;
-    int l = 0, iter = 0;   // warp 0: the eigenvalue being sought and its sweeps so far
+    int l = bad ? M : 0, iter = 0;   // warp 0: the eigenvalue being sought and its sweeps so far
     for (int sweep = 0;; ++sweep) {
         const int buf = sweep & 1;
         if (tid < 32) {
@@ -832,7 +817,9 @@ __global__ void __launch_bounds__(32 * kSelMax) heevd_select_kernel(const double
     const double eps = 2.220446049250313e-16;
     // Gershgorin interval, the norm of T and the pivot floor
     double lo = INFINITY, hi = -INFINITY, emax2 = 0.0;
+    bool bad = false;
     for (int i = lane; i < M; i += 32) {
+        bad |= d[i] != d[i] || e[i] != e[i];
         const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + fabs(e[i]);
         lo = fmin(lo, d[i] - r);
         hi = fmax(hi, d[i] + r);
@@ -843,6 +830,14 @@ __global__ void __launch_bounds__(32 * kSelMax) heevd_select_kernel(const double
         lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
         hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
         emax2 = fmax(emax2, __shfl_xor_sync(0xffffffffu, emax2, o));
+    }
+    double *zc = Zall + (int64_t)b * M * M + (int64_t)w * M;   // column w of Z
+    if (lane == 0) permall[(int64_t)b * M + w] = w;
+    if (__any_sync(0xffffffffu, bad)) {   // a NaN in T, which fmin, fmax and the counts would pass over: no result
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        if (lane == 0) wsel[(int64_t)b * sel.n + w] = nan;
+        for (int i = lane; i < M; i += 32) zc[i] = nan;
+        return;
     }
     const double pivmin = 2.2250738585072014e-308 * fmax(1.0, emax2);
     const double tnorm = fmax(fabs(lo), fabs(hi));
@@ -955,9 +950,7 @@ __global__ void __launch_bounds__(32 * kSelMax) heevd_select_kernel(const double
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const double inv = ss > 0.0 ? 1.0 / sqrt(ss) : 0.0;
-    double *zc = Zall + (int64_t)b * M * M + (int64_t)w * M;   // column w of Z
     for (int i = lane; i < M; i += 32) zc[i] = y[i] * inv;
-    if (lane == 0) permall[(int64_t)b * M + w] = w;
 }
 
 struct EvWorkspace {
@@ -1026,7 +1019,8 @@ static int tridiag_launch(const void *csm, int B, int M, double2 *A, double *d, 
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if (cudaLaunchKernelEx(&cfg, kern, static_cast<const double2 *>(csm), M, d, e, tau, vh) != cudaSuccess)
+        if (cudaLaunchKernelEx(&cfg, kern, static_cast<const double2 *>(csm), M, d, e, tau, vh, tc_wait_limit_ns()) !=
+            cudaSuccess)
             return ACB_ERR_CUDA;
         return check_launch();
     }

@@ -107,27 +107,48 @@ __device__ __forceinline__ void cluster_send(int rank, const double *dst, double
                  : "memory");
 }
 
-// Wait for what the other CTAs send.  Gives up after `limit_ns` or where `stop` is raised; returns false then.
+__device__ __forceinline__ void cluster_send(int rank, const double2 *dst, double2 v, const uint64_t *bar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(
+                     cluster_addr(dst, rank)),
+                 "d"(v.x), "d"(v.y), "r"(cluster_addr(bar, rank))
+                 : "memory");
+}
+
+__device__ __forceinline__ bool cluster_try(uint32_t bar, uint32_t parity, uint32_t hint_ns)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(hint_ns)
+        : "memory");
+    return ok != 0;
+}
+
+// A wait whose first try has failed, or with a limit so short that the first try counts.
+static __device__ __noinline__ bool cluster_wait_on(uint32_t bar, uint32_t parity, const volatile int *stop,
+                                                    uint64_t limit_ns)
+{
+    const uint64_t t0 = globaltimer_ns();
+    while (true) {
+        const bool ok = cluster_try(bar, parity, limit_ns < 100000u ? (uint32_t)limit_ns : 100000u);
+        const bool late = globaltimer_ns() - t0 > limit_ns;
+        if (ok) return !late;
+        if (late || *stop) return false;
+    }
+}
+
+// Wait for what the other CTAs send.  Gives up after `limit_ns` or where `stop` is raised; returns false then.  The
+// hardware suspends a try for some microseconds whatever its hint; what arrives after the limit is too late all the
+// same.  The loop is out of line: inline it made a step of the tridiagonalisation 5 % longer.
 __device__ __forceinline__ bool cluster_wait(const uint64_t *bar, uint32_t parity, const volatile int *stop,
                                              uint64_t limit_ns)
 {
-    const uint32_t addr = smem_u32(bar), hint = limit_ns < 100000u ? (uint32_t)limit_ns : 100000u;
-    uint64_t t0 = 0;
-    while (true) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(addr), "r"(parity), "r"(hint)
-            : "memory");
-        if (ok) return true;
-        if (*stop) return false;
-        const uint64_t t = globaltimer_ns();
-        if (t0 == 0) t0 = t;
-        else if (t - t0 > limit_ns) return false;
-    }
+    return (limit_ns >= 100000u && cluster_try(smem_u32(bar), parity, 100000u)) ||
+           cluster_wait_on(smem_u32(bar), parity, stop, limit_ns);
 }
 
 // Raise `stop` in all `nctas` CTAs of the cluster (each of them is between its first cluster barrier and cluster_end).

@@ -189,11 +189,13 @@ size_t acb_map_tc_workspace_bytes(int num_mics, int num_bins, int precision);
 
 /* Limit of each bounded device-side wait in the tensor-core kernels (acb_map_tc, acb_map_tc_batch,
  * acb_map_tc_noalloc and the tensor-core CSM forms of acb_csm_accumulate and acb_csm_finished) and in
- * the exchanges inside a cluster of acb_damas_gauss_seidel_f64, which says what one that runs out leaves;
- * no counterpart in the reference.  A wait that runs out sets the launch's error word to 1 (where one is
- * given; the CSM forms write NaN to every entry whose sums are missing), the CTA lets its own copies
- * and MMAs finish, frees its tensor memory and exits, so the device context stays usable.  Applies to launches enqueued after the call; 0 restores the default of 0.5 s.  Returns
- * the previous limit.  Process-wide (all devices and host threads). */
+ * the exchanges inside a cluster of acb_damas_gauss_seidel_f64, acb_heevd_f64 and acb_heevd_select_f64
+ * (which say what one that runs out leaves); no counterpart in the reference.  In the tensor-core
+ * kernels it sets the launch's error word to 1 (where one is given; the CSM forms write NaN to every
+ * entry whose sums are missing).  The CTA lets its own copies, stores and MMAs finish, frees its tensor
+ * memory and exits, so the device context stays usable.  Applies to launches enqueued after the call;
+ * 0 restores the default of 0.5 s.  Returns the previous limit.  Process-wide (all devices and host
+ * threads). */
 uint64_t acb_tc_set_wait_limit_ns(uint64_t limit_ns);
 
 /* Tensor-core form of the same map (acoular/fastFuncs.py:217-311 semantics, same arguments and
@@ -304,7 +306,8 @@ size_t acb_heevd_workspace_bytes(int num_mics, int num_bins);
  * ascending, eigvec complex128 [B][M][M] row-major with the eigenvectors in the columns (numpy's layout;
  * each column may differ from LAPACK's by a unit phase factor).  Householder tridiagonalisation, implicit QL
  * with Wilkinson shifts, back-transformation, all in FP64.  info int [B] (may be NULL): 1 where a QL iteration
- * did not converge in 60 steps.  M <= 4096. */
+ * did not converge in 60 steps, where the matrix holds a NaN, or where a bounded wait of the tridiagonalisation ran out
+ * (acb_tc_set_wait_limit_ns); in the last two cases the eigenvalues and eigenvectors of that bin are NaN.  M <= 4096. */
 int acb_heevd_f64(const void *csm, int num_bins, int num_mics, double *eigval, void *eigvec, int *info,
                   void *workspace, size_t workspace_bytes, void *stream);
 
@@ -316,6 +319,8 @@ int acb_heevd_f64(const void *csm, int num_bins, int num_mics, double *eigval, v
  * the selected eigenvalues by multisection on Sturm counts, their eigenvectors by inverse iteration, the
  * back-transformation; no QL sweeps.  Accurate for eigenvalues separated from the others; inside a cluster
  * of (nearly) equal eigenvalues the vector is some unit vector of the cluster's space, as any solver's is.
+ * Where the matrix holds a NaN, or a bounded wait of the tridiagonalisation ran out (acb_tc_set_wait_limit_ns), the
+ * eigenvalues and eigenvectors of that bin are NaN.
  * Workspace: acb_heevd_workspace_bytes(M, B).  M <= 4096 and (3 M + 5 M num_sel) 8 + M num_sel bytes of
  * shared memory <= 200 KB (ACB_ERR_UNSUPPORTED above). */
 int acb_heevd_select_f64(const void *csm, int num_bins, int num_mics, int num_sel, const int *sel, double *eigval,
