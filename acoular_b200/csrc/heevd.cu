@@ -424,9 +424,11 @@ __global__ void __launch_bounds__(kEvThreads, MINB)
 // Warp 0 forms the rotations of a sweep while the other warps apply those of the sweep before to Z, one barrier per
 // sweep.  Bound: the serial chain of a rotation (two products, the sum of squares, a reciprocal square root and five
 // more dependent operations); the library's hypot and a division made it twice as long, and the application
-// waited for it (64 matrices of 112 rows 4.2 -> 2.7 ms).  All lanes store the chain's values and the range test
-// runs beside the reciprocal square root: 2.7 -> 1.8 ms, 226 clocks per rotation (stores by lane 0 alone and the
-// test ahead of the root: about 350).  The application hides behind the chain (without it the time is the same).
+// waited for it (64 matrices of 112 rows 4.2 -> 2.7 ms).  Lane 0 runs the whole chain by itself, as a sweep reads
+// entries that it has stored to a little earlier, and the range test runs beside the reciprocal square root:
+// 2.7 -> 1.8 ms, 226 clocks per rotation (the loop in all lanes with only the stores in lane 0, and the test ahead of the
+// root: about 350; the loop in all lanes with a warp barrier per rotation: 240).  The application hides behind the chain
+// (without it the time is the same).
 __global__ void __launch_bounds__(kQlThreads) heevd_tql_kernel(const double *__restrict__ dall,
                                                                const double *__restrict__ eall, int M,
                                                                double *__restrict__ wall, double *__restrict__ Zall,
@@ -484,48 +486,47 @@ __global__ void __launch_bounds__(kQlThreads) heevd_tql_kernel(const double *__r
             } else {
                 ++iter;
                 double *cs = cs2 + buf * M, *sn = sn2 + buf * M;
-                // every lane follows the chain and stores the same values: no branch on the lane in it
-                double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-                const double h = fabs(g) < 1e150 ? sqrt(fma(g, g, 1.0)) : fabs(g);
-                double dn = d[m];   // d[i + 1] of the rotation at hand
-                g = dn - d[l] + e[l] / (g + copysign(h, g));
-                double s = 1.0, c = 1.0, p = 0.0;
-                double en = e[m - 1], dp = d[m - 1];   // read one rotation ahead of the stores
-                int i = m - 1;
-                bool restart = false;
-                __syncwarp();   // the first stores come after every lane's reads
-                for (; i >= l; --i) {
-                    const double ei = en, di = dp;
-                    const int j = max(i - 1, 0);
-                    en = e[j];
-                    dp = d[j];
-                    const double f = s * ei, bb = c * ei;
-                    const double x = fma(f, f, g * g);
-                    double rinv = rsqrt(x), r = x * rinv;
-                    if (!(x > 1e-280 && x < 1e280)) {
-                        r = hypot(f, g);
-                        if (r == 0.0) {   // split: deflate and restart from the same l
-                            e[i + 1] = 0.0;
-                            d[i + 1] = dn - p;
-                            e[m] = 0.0;
-                            restart = true;
-                            break;
-                        }
-                        rinv = 1.0 / r;
-                    }
-                    e[i + 1] = r;
-                    s = f * rinv;
-                    c = g * rinv;
-                    g = dn - p;
-                    r = (di - g) * s + 2.0 * c * bb;
-                    p = s * r;
-                    d[i + 1] = g + p;
-                    cs[i] = c;
-                    sn[i] = s;
-                    g = c * r - bb;
-                    dn = di;
-                }
+                __syncwarp();   // the search's reads come before the chain's stores
                 if (lane == 0) {
+                    double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
+                    const double h = fabs(g) < 1e150 ? sqrt(fma(g, g, 1.0)) : fabs(g);
+                    double dn = d[m];   // d[i + 1] of the rotation at hand
+                    g = dn - d[l] + e[l] / (g + copysign(h, g));
+                    double s = 1.0, c = 1.0, p = 0.0;
+                    double en = e[m - 1], dp = d[m - 1];   // read one rotation ahead of the stores
+                    int i = m - 1;
+                    bool restart = false;
+                    for (; i >= l; --i) {
+                        const double ei = en, di = dp;
+                        const int j = max(i - 1, 0);
+                        en = e[j];
+                        dp = d[j];
+                        const double f = s * ei, bb = c * ei;
+                        const double x = fma(f, f, g * g);
+                        double rinv = rsqrt(x), r = x * rinv;
+                        if (!(x > 1e-280 && x < 1e280)) {
+                            r = hypot(f, g);
+                            if (r == 0.0) {   // split: deflate and restart from the same l
+                                e[i + 1] = 0.0;
+                                d[i + 1] = dn - p;
+                                e[m] = 0.0;
+                                restart = true;
+                                break;
+                            }
+                            rinv = 1.0 / r;
+                        }
+                        e[i + 1] = r;
+                        s = f * rinv;
+                        c = g * rinv;
+                        g = dn - p;
+                        r = (di - g) * s + 2.0 * c * bb;
+                        p = s * r;
+                        d[i + 1] = g + p;
+                        cs[i] = c;
+                        sn[i] = s;
+                        g = c * r - bb;
+                        dn = di;
+                    }
                     if (!restart) {
                         d[l] = dn - p;
                         e[l] = g;
