@@ -723,10 +723,9 @@ int acb_cleansc_f64(const acb_map_params *p, void *csm, const double *wavenumber
         const bool few = B * kCscCtas <= 120, small = G <= kCscCtas * kCscClThreads;
         auto kern = few ? (small ? cleansc_cluster_kernel<1, 16, 1> : cleansc_cluster_kernel<kCscPoints, 16, 1>)
                         : (small ? cleansc_cluster_kernel<1, 8, 2> : cleansc_cluster_kernel<kCscPoints, 8, 2>);
-        if (cudaFuncSetAttribute(cleansc_steer_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return ACB_ERR_CUDA;
+        st = allow_smem(cleansc_steer_kernel<true>, tile);
+        if (!st) st = allow_smem(kern, smem);
+        if (st) return st;
         cleansc_steer_kernel<true><<<dim3((unsigned)((G + 31) / 32), B), 256, tile, s>>>(a, steer);
         st = check_launch();
         if (st) return st;
@@ -750,9 +749,8 @@ int acb_cleansc_f64(const acb_map_params *p, void *csm, const double *wavenumber
     st = check_launch();
     if (st) return st;
     const size_t smem = (size_t)M * (3 * sizeof(double2) + sizeof(double));
-    if (cudaFuncSetAttribute(cleansc_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return ACB_ERR_CUDA;
+    st = allow_smem(cleansc_step_kernel, smem);
+    if (st) return st;
     for (int j = 0; j < J; ++j) {
         cleansc_step_kernel<<<B, kCscThreads, smem, s>>>(a, j);
         st = check_launch();
@@ -807,9 +805,8 @@ int acb_cleansc_custom_f64(const acb_map_params *p, void *csm, const void *steer
     st = acb_map_custom_f64(&q, csm, steer, a.h, nullptr, stream);
     if (st) return st;
     const size_t smem = (size_t)M * (3 * sizeof(double2) + sizeof(double));
-    if (cudaFuncSetAttribute(cleansc_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return ACB_ERR_CUDA;
+    st = allow_smem(cleansc_step_kernel, smem);
+    if (st) return st;
     for (int j = 0; j < J; ++j) {
         cleansc_step_kernel<<<B, kCscThreads, smem, s>>>(a, j);
         st = check_launch();

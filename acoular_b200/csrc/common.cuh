@@ -25,6 +25,30 @@ inline int check_launch()
     return ACB_OK;
 }
 
+// Let `kern` be launched with `bytes` of dynamic shared memory.  The limit belongs to the function, not to the call, so it
+// only ever goes up, and at once to all that the device has left beside the kernel's static part: with each call's own size
+// another thread's call could lower it between this call's setting and its launch, which then fails.
+template <class... Args>
+inline int allow_smem(void (*kern)(Args...), size_t bytes)
+{
+    cudaFuncAttributes at;
+    cudaError_t e = cudaFuncGetAttributes(&at, kern);
+    if (e == cudaSuccess && bytes > (size_t)at.maxDynamicSharedSizeBytes) {
+        int dev = 0, most = 0;
+        e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        if (e == cudaSuccess) {
+            most -= (int)at.sharedSizeBytes;
+            e = (int64_t)bytes > most ? cudaErrorInvalidValue
+                                      : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        }
+    }
+    if (e == cudaSuccess) return ACB_OK;
+    cudaGetLastError();   // reported here, not by the next launch
+    set_cuda_error(e);
+    return ACB_ERR_CUDA;
+}
+
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 constexpr int kNumSMs = 148;

@@ -996,7 +996,7 @@ static int gram_f64_launch(const void *spec, int M, int64_t nw, int nbins, void 
     const int TC = narrow ? (M + 15) / 16 : T, per = narrow ? 2 : 1;
     int tiles = 0;
     for (int ti = 0; ti < T; ++ti) tiles += TC - per * ti;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GF_SMEM);
+    if (const int st = allow_smem(kernel, GF_SMEM)) return st;
     kernel<<<dim3(tiles, nbins), 128, GF_SMEM, s>>>(reinterpret_cast<const double2 *>(spec), M, nw,
                                                     reinterpret_cast<double2 *>(csm), reinterpret_cast<double2 *>(out),
                                                     scale);
@@ -1077,11 +1077,11 @@ int fft_launch(const void *samples, int sample_dtype, int out_form, int num_mics
         const dim3 gs((unsigned)num_mics, (unsigned)num_windows, (unsigned)(block_size / 2 / FFT_SUB_H));
         const size_t smem = (size_t)fft_stride(FFT_SUB_H) * sizeof(double2);
         if (sample_dtype == ACB_F32) {
-            cudaFuncSetAttribute(fft_sub_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (const int st = allow_smem(fft_sub_kernel<float>, smem)) return st;
             fft_sub_kernel<float><<<gs, 256, smem, s>>>(reinterpret_cast<const float *>(samples), num_mics, block_size,
                                                         hop, first_window, window, tw, sc);
         } else {
-            cudaFuncSetAttribute(fft_sub_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (const int st = allow_smem(fft_sub_kernel<double>, smem)) return st;
             fft_sub_kernel<double><<<gs, 256, smem, s>>>(reinterpret_cast<const double *>(samples), num_mics,
                                                          block_size, hop, first_window, window, tw, sc);
         }
@@ -1119,7 +1119,7 @@ int fft_launch(const void *samples, int sample_dtype, int out_form, int num_mics
 #define ACB_FFT4_LAUNCH(TS, OF)                                                                                     \
     do {                                                                                                            \
         auto kern = fft4_tc_kernel<TS, OF>;                                                                         \
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4);                        \
+        if (const int st_ = allow_smem(kern, smem4)) return st_;                                                    \
         kern<<<g4, fft4_threads(block_size), smem4, s>>>(reinterpret_cast<const TS *>(samples), num_mics, block_size,   \
                                     hop, first_window, num_windows, mpb4, vw, window, tw, bin_lo, num_bins, out, R, KC, lo_elems);    \
     } while (0)
@@ -1140,7 +1140,7 @@ int fft_launch(const void *samples, int sample_dtype, int out_form, int num_mics
 #define ACB_FFT_LAUNCH(TS, OF)                                                                                    \
     do {                                                                                                          \
         auto kern = fft_window_kernel<TS, OF>;                                                                    \
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                       \
+        if (const int st_ = allow_smem(kern, smem)) return st_;                                                   \
         const int nt = max(64, min(fft_threads(block_size), mpb * (block_size / 16)));                             \
         kern<<<g1, nt, smem, s>>>(reinterpret_cast<const TS *>(samples), num_mics, block_size, hop, \
                                    first_window, num_windows, mpb, window, tw, bin_lo, num_bins, out, R, KC, lo_elems);        \

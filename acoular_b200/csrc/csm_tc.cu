@@ -322,7 +322,7 @@ int csm_tc_accumulate(const void *samples, int sample_dtype, int num_mics, int b
     const unsigned grid = (unsigned)(a.nitems < nsm ? a.nitems : nsm);
     const int smem = gtc_smem_bytes();
     auto kern = tf32 ? gram_tc_kernel<true> : gram_tc_kernel<false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (const int st = allow_smem(kern, smem)) return st;
     kern<<<grid, GTC_THREADS, smem, s>>>(a, nullptr);
     return check_launch();
 }

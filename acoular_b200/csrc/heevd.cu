@@ -1006,8 +1006,7 @@ static int tridiag_launch(const void *csm, int B, int M, double2 *A, double *d, 
         const size_t smem = ev_cluster_smem(M, C);
         // two CTAs per SM where their memory fits: then with 128 registers (some spilled), else with all it needs
         auto kern = smem <= 110 * 1024 ? heevd_tridiag_cluster_kernel<2> : heevd_tridiag_cluster_kernel<1>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return ACB_ERR_CUDA;
+        if (const int st = allow_smem(kern, smem)) return st;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(B * C));
         cfg.blockDim = dim3(kEvThreads);
@@ -1031,9 +1030,7 @@ static int tridiag_launch(const void *csm, int B, int M, double2 *A, double *d, 
         return ACB_ERR_CUDA;
     }
     const size_t smem = 2 * (size_t)M * sizeof(double2);
-    if (cudaFuncSetAttribute(heevd_tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return ACB_ERR_CUDA;
+    if (const int st = allow_smem(heevd_tridiag_kernel, smem)) return st;
     heevd_tridiag_kernel<<<B, kEvThreads, smem, s>>>(A, M, d, e, tau, vh);
     return check_launch();
 }
@@ -1078,9 +1075,9 @@ int acb_heevd_f64(const void *csm, int num_bins, int num_mics, double *eigval, v
     double *Z = reinterpret_cast<double *>(ws + lay.Z);
     int *perm = reinterpret_cast<int *>(ws + lay.perm);
     const size_t sm2 = 6 * (size_t)M * sizeof(double);
-    if (cudaFuncSetAttribute(heevd_tql_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2) != cudaSuccess)
-        return ACB_ERR_CUDA;
-    int st = tridiag_launch(csm, B, M, A, d, e, tau, vh, s);
+    int st = allow_smem(heevd_tql_kernel, sm2);
+    if (st) return st;
+    st = tridiag_launch(csm, B, M, A, d, e, tau, vh, s);
     if (st) return st;
     heevd_tql_kernel<<<B, kQlThreads, sm2, s>>>(d, e, M, eigval, Z, perm, info);
     st = check_launch();
@@ -1088,8 +1085,8 @@ int acb_heevd_f64(const void *csm, int num_bins, int num_mics, double *eigval, v
     const size_t smem = (size_t)(M + 1) * W * sizeof(double2);
     // columns per warp: the slab's W columns over the 8 warps
     auto back = W >= 32 ? heevd_back_kernel<4> : (W >= 16 ? heevd_back_kernel<2> : heevd_back_kernel<1>);
-    if (cudaFuncSetAttribute(back, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return ACB_ERR_CUDA;
+    st = allow_smem(back, smem);
+    if (st) return st;
     back<<<dim3(B, (M + W - 1) / W), kEvThreads, smem, s>>>(vh, tau, Z, perm, M, W, M,
                                                            static_cast<double2 *>(eigvec));
     return check_launch();
@@ -1121,10 +1118,9 @@ int acb_heevd_select_f64(const void *csm, int num_bins, int num_mics, int num_se
     double2 *vh = reinterpret_cast<double2 *>(ws + lay.vh);
     double *Z = reinterpret_cast<double *>(ws + lay.Z);
     int *perm = reinterpret_cast<int *>(ws + lay.perm);
-    if (cudaFuncSetAttribute(heevd_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3) !=
-        cudaSuccess)
-        return ACB_ERR_CUDA;
-    int st = tridiag_launch(csm, B, M, A, d, e, tau, vh, s);
+    int st = allow_smem(heevd_select_kernel, sm3);
+    if (st) return st;
+    st = tridiag_launch(csm, B, M, A, d, e, tau, vh, s);
     if (st) return st;
     heevd_select_kernel<<<B, 32 * E, sm3, s>>>(d, e, M, es, eigval, Z, perm);
     st = check_launch();
@@ -1134,16 +1130,15 @@ int acb_heevd_select_f64(const void *csm, int num_bins, int num_mics, int num_se
         auto back = M <= 64 ? heevd_back_select_kernel<2>
                             : (M <= 128 ? heevd_back_select_kernel<4>
                                         : (M <= 256 ? heevd_back_select_kernel<8> : heevd_back_select_kernel<16>));
-        if (cudaFuncSetAttribute(back, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring) != cudaSuccess)
-            return ACB_ERR_CUDA;
+        st = allow_smem(back, ring);
+        if (st) return st;
         back<<<dim3(B, E), 32, ring, s>>>(vh, tau, Z, M, E, static_cast<double2 *>(eigvec));
         return check_launch();
     }
     // the E eigenvectors of T sit in columns 0 .. E-1 of each matrix's Z, perm[j] = j: one slab of E columns
     const size_t smem = (size_t)(M + 1) * E * sizeof(double2);
-    if (cudaFuncSetAttribute(heevd_back_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return ACB_ERR_CUDA;
+    st = allow_smem(heevd_back_kernel<1>, smem);
+    if (st) return st;
     heevd_back_kernel<1><<<dim3(B, 1), kEvThreads, smem, s>>>(vh, tau, Z, perm, M, E, E,
                                                               static_cast<double2 *>(eigvec));
     return check_launch();

@@ -673,7 +673,7 @@ static int launch_map_nw(const MapArgs &a, int nbins, const void *csm, const dou
     const int mc = a.M <= kMapOneTile ? a.M : kMapPairTile;
     const size_t smem = (size_t)(a.M <= mc ? 1 : 2) * ((mc + 15) & ~15) * kPtsPad * sizeof(double2);
     auto kern = map_f64_kernel<USE_RM, CUSTOM, NW>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (const int st = allow_smem(kern, smem)) return st;
     const dim3 grid((unsigned)((a.G + kPts - 1) / kPts), nbins);
     kern<<<grid, 32 * NW, smem, s>>>(a, reinterpret_cast<const double2 *>(csm), k, k_scalar, mpos, gpos, r0, rm, mc,
                                      out_map, out_norm, reinterpret_cast<const double2 *>(steer));
@@ -700,7 +700,7 @@ static int launch_eig_nw(const MapArgs &a, int nbins, int E, const double *eigva
     const int mc = a.M <= kMapOneTile ? a.M : kMapPairTile;
     const size_t smem = (size_t)((mc + 15) & ~15) * kPtsPad * sizeof(double2) + (a.r_diag ? mc * sizeof(double) : 0);
     auto kern = map_eig_kernel<USE_RM, CUSTOM, NW>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (const int st = allow_smem(kern, smem)) return st;
     const dim3 grid((unsigned)((a.G + kPts - 1) / kPts), nbins);
     kern<<<grid, 32 * NW, smem, s>>>(a, E, eigval, reinterpret_cast<const double2 *>(eigvec), k, k_scalar, mpos, gpos,
                                      r0, rm, mc, out_map, out_norm, reinterpret_cast<const double2 *>(steer), active);

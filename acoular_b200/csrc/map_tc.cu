@@ -1201,7 +1201,7 @@ static int tc_launch(TcBatch &bt, const acb_map_params *const *params, const voi
         {map_tc_kernel<3, TC_SPLIT>, map_tc_kernel<3, TC_TF>, map_tc_kernel<3, TC_HALF>},
         {map_tc_kernel<4, TC_SPLIT>, map_tc_kernel<4, TC_TF>, map_tc_kernel<4, TC_HALF>}};
     const KernT kern = kernels[steer_type - 1][precision];
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (const int st = allow_smem(kern, smem)) return st;
     kern<<<grid, TC_THREADS, smem, s>>>(bt, error_word);
     return check_launch();
 }

@@ -621,7 +621,7 @@ int acb_psf_f64(const acb_map_params *p, int num_sources, const int64_t *sources
     cudaStream_t s = as_stream(stream);
 #define ACB_PSF(ST)                                                                                           \
     do {                                                                                                      \
-        cudaFuncSetAttribute(psf_kernel<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPsfSmem);          \
+        if (const int st = allow_smem(psf_kernel<ST>, kPsfSmem)) return st;                                   \
         psf_kernel<ST><<<grid, 32 * kPsfWarps, kPsfSmem, s>>>(M, G, num_sources, sources, r0, rm, wavenumber, \
                                                              p->sincos_table, mask, p->glibc_faithful,        \
                                                              round_f32, out_psf);                             \
@@ -659,9 +659,7 @@ int acb_damas_gauss_seidel_f64(const double *psf, int64_t num_grid, int num_bins
     const int64_t smem_ahead = gs_smem_bytes(num_grid);
     const bool ahead = num_grid > 5 * kDamasRows && C >= 4 && smem_ahead <= smem_max - 1024;
     const size_t smem_used = ahead ? (size_t)smem_ahead : smem;
-    const void *kern = ahead ? reinterpret_cast<const void *>(damas_ahead_kernel) : reinterpret_cast<const void *>(damas_kernel);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_used) != cudaSuccess)
-        return ACB_ERR_CUDA;
+    if (const int st = ahead ? allow_smem(damas_ahead_kernel, smem_used) : allow_smem(damas_kernel, smem_used)) return st;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(num_bins * C));
     cfg.blockDim = dim3(kDamasThreads);
