@@ -63,6 +63,18 @@ __device__ __forceinline__ double dist3(double g0, double g1, double g2, double 
     return __dsqrt_rn(__fma_rn(d2, d2, __fma_rn(d1, d1, __dmul_rn(d0, d0))));
 }
 
+// D (16 x 8) += A (16 x 8) B (8 x 8), FP64.  Lane (g = lane / 4, t = lane % 4) holds A rows g, g + 8 at columns
+// t, t + 4 (a0: g,t  a1: g+8,t  a2: g,t+4  a3: g+8,t+4), B rows t, t + 4 of column g, and D rows g, g + 8 at
+// columns 2t, 2t + 1.  The products of one element are added as a chain of FMAs.
+__device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, double a2, double a3, double b0,
+                                        double b1)
+{
+    asm(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64.rn {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+        : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
+}
+
 // Exception table of the host C library's float32 cosf/sinf (built by acb_sincos_table_build_host): open
 // addressing, linear probing.  Entry layout: bits 63..32 = float bits of x, bits 31..16 = tags of the slot (below),
 // bits 15..8 = int8 ulp delta of cos, bits 7..0 = int8 ulp delta of sin; an all-ones word marks an empty slot.

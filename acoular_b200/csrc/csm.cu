@@ -873,13 +873,6 @@ constexpr int GF_STAGES = 3;
 constexpr int64_t GF_NARROW = kNumSMs * 3 / 2;
 constexpr int GF_SMEM = GF_STAGES * 2 * GF_KW * GF_LD * (int)sizeof(double2);
 
-__device__ __forceinline__ void mma_f64(double (&d)[4], const double (&a)[4], double b0, double b1)
-{
-    asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64.rn {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
-}
-
 template <int NB>
 __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restrict__ spec, int M, int64_t nw,
                                                           double2 *__restrict__ csm, double2 *__restrict__ out,
@@ -971,8 +964,8 @@ __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restr
 #pragma unroll
             for (int j = 0; j < NB; ++j)
                 if (use[j]) {
-                    mma_f64(re[j], a, b0[j], b1[j]);
-                    mma_f64(im[j], a, q0[j], q1[j]);
+                    mma_f64(re[j], a[0], a[1], a[2], a[3], b0[j], b1[j]);
+                    mma_f64(im[j], a[0], a[1], a[2], a[3], q0[j], q1[j]);
                 }
         }
     }

@@ -65,18 +65,6 @@ __device__ __forceinline__ double steer_weight(int steer_type, double r)
     return steer_type == 2 ? r : steer_type >= 3 ? 1.0 / r : 1.0;
 }
 
-// D (16 x 8) += A (16 x 8) B (8 x 8), FP64.  Lane (g = lane / 4, t = lane % 4) holds A rows g, g + 8 at columns
-// t, t + 4 (a0: g,t  a1: g+8,t  a2: g,t+4  a3: g+8,t+4), B rows t, t + 4 of column g, and D rows g, g + 8 at
-// columns 2t, 2t + 1.  The products of one element are added as a chain of FMAs.
-__device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, double a2, double a3, double b0,
-                                        double b1)
-{
-    asm(
-        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64.rn {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-        : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
-}
-
 // Distance of a grid point and a mic, and the steering weight: r (inverse) or 1/r (true level, true location; within
 // an ulp).  r is the correctly rounded square root that dist3 gives, formed from one reciprocal square root y, which
 // the weight needs anyway (P. Markstein's correction: s = d y, r = s + (d - s^2) y / 2).
