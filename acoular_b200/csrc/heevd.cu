@@ -814,7 +814,6 @@ __global__ void __launch_bounds__(32 * kSelMax) heevd_select_kernel(const double
         e[i] = ei;
     }
     __syncthreads();
-    if (w >= sel.n) return;
     const double eps = 2.220446049250313e-16;
     // Gershgorin interval, the norm of T and the pivot floor
     double lo = INFINITY, hi = -INFINITY, emax2 = 0.0;
@@ -846,10 +845,10 @@ __global__ void __launch_bounds__(32 * kSelMax) heevd_select_kernel(const double
     lo -= fudge;
     hi += fudge;
     const int k = sel.idx[w];
-    // the scaled squares; every rank's warp writes the same values
+    // the scaled squares, by all ranks' warps together (each has formed the same norm from T)
     const double tsc = tnorm > 0.0 ? scalbn(1.0, -ilogb(tnorm)) : 1.0;
-    for (int i = lane; i < M; i += 32) e2[i] = (e[i] * tsc) * (e[i] * tsc);
-    __syncwarp();
+    for (int i = tid; i < M; i += blockDim.x) e2[i] = (e[i] * tsc) * (e[i] * tsc);
+    __syncthreads();
     for (int it = 0; it < 64; ++it) {
         const double width = hi - lo;
         if (width <= fmax(2.0 * eps * fmax(fabs(lo), fabs(hi)), eps * tnorm) || width <= 4.0 * pivmin) break;
