@@ -372,6 +372,8 @@ __global__ void __launch_bounds__(kCscThreads) cleansc_step_kernel(CscArgs a, in
 constexpr int kCscCtas = 8, kCscClThreads = 256, kCscPoints = 4, kCscHistory = 64;
 constexpr int kCscClMics = 112;
 
+constexpr size_t kCscStepSmem = 2048 * (3 * sizeof(double2) + sizeof(double));   // cleansc_step_kernel's at the most mics
+
 struct CscPeak {
     double v;
     long long g;
@@ -723,8 +725,8 @@ int acb_cleansc_f64(const acb_map_params *p, void *csm, const double *wavenumber
         const bool few = B * kCscCtas <= 120, small = G <= kCscCtas * kCscClThreads;
         auto kern = few ? (small ? cleansc_cluster_kernel<1, 16, 1> : cleansc_cluster_kernel<kCscPoints, 16, 1>)
                         : (small ? cleansc_cluster_kernel<1, 8, 2> : cleansc_cluster_kernel<kCscPoints, 8, 2>);
-        st = allow_smem(cleansc_steer_kernel<true>, tile);
-        if (!st) st = allow_smem(kern, smem);
+        st = allow_smem(cleansc_steer_kernel<true>, tile, (size_t)kCscClMics * 33 * sizeof(double2));
+        if (!st) st = allow_smem(kern, smem, csc_cluster_smem(kCscClMics));
         if (st) return st;
         cleansc_steer_kernel<true><<<dim3((unsigned)((G + 31) / 32), B), 256, tile, s>>>(a, steer);
         st = check_launch();
@@ -749,7 +751,7 @@ int acb_cleansc_f64(const acb_map_params *p, void *csm, const double *wavenumber
     st = check_launch();
     if (st) return st;
     const size_t smem = (size_t)M * (3 * sizeof(double2) + sizeof(double));
-    st = allow_smem(cleansc_step_kernel, smem);
+    st = allow_smem(cleansc_step_kernel, smem, kCscStepSmem);
     if (st) return st;
     for (int j = 0; j < J; ++j) {
         cleansc_step_kernel<<<B, kCscThreads, smem, s>>>(a, j);
@@ -805,7 +807,7 @@ int acb_cleansc_custom_f64(const acb_map_params *p, void *csm, const void *steer
     st = acb_map_custom_f64(&q, csm, steer, a.h, nullptr, stream);
     if (st) return st;
     const size_t smem = (size_t)M * (3 * sizeof(double2) + sizeof(double));
-    st = allow_smem(cleansc_step_kernel, smem);
+    st = allow_smem(cleansc_step_kernel, smem, kCscStepSmem);
     if (st) return st;
     for (int j = 0; j < J; ++j) {
         cleansc_step_kernel<<<B, kCscThreads, smem, s>>>(a, j);

@@ -25,24 +25,16 @@ inline int check_launch()
     return ACB_OK;
 }
 
-// Let `kern` be launched with `bytes` of dynamic shared memory.  The limit belongs to the function, not to the call, so it
-// only ever goes up, and at once to all that the device has left beside the kernel's static part: with each call's own size
-// another thread's call could lower it between this call's setting and its launch, which then fails.
+constexpr int kSmemMost = 227 * 1024;   // of a CTA on sm_100a, static and dynamic
+
+// Let `kern` be launched with `bytes` of dynamic shared memory; `most` is the largest that any call asks for.  The limit
+// belongs to the function, not to the call, so every call sets the same one: with each call's own size another thread's
+// call could lower it between this call's setting and its launch, which then fails.
 template <class... Args>
-inline int allow_smem(void (*kern)(Args...), size_t bytes)
+inline int allow_smem(void (*kern)(Args...), size_t bytes, size_t most)
 {
-    cudaFuncAttributes at;
-    cudaError_t e = cudaFuncGetAttributes(&at, kern);
-    if (e == cudaSuccess && bytes > (size_t)at.maxDynamicSharedSizeBytes) {
-        int dev = 0, most = 0;
-        e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        if (e == cudaSuccess) {
-            most -= (int)at.sharedSizeBytes;
-            e = (int64_t)bytes > most ? cudaErrorInvalidValue
-                                      : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        }
-    }
+    cudaError_t e = bytes > most ? cudaErrorInvalidValue
+                                 : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e == cudaSuccess) return ACB_OK;
     cudaGetLastError();   // reported here, not by the next launch
     set_cuda_error(e);
@@ -85,9 +77,10 @@ __device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, do
 //   tags  Bit 16 + tag of a slot's word is set for every key with this home slot (whoever occupies it), tag = 4
 //         other bits of the key's hash: unless the bit is set, one load answers the lookup, with no walk.
 // A table without the meta entry has no tags: tol is then half an ulp and every occupied home slot is walked.
-// Bound: issue slots (about 100 instructions per value); with a lookup and its walk for every value and the library's
-// sincos it was 194 instructions.  Measured (B200): map of one eigen-component, 16 bins x 160,801 points x 256 mics,
-// 7.9 -> 5.1 ms; point-spread function 1681 x 1681 x 64 mics 1.72 -> 1.03 ms.
+// Bound: issue slots.  Instructions per value, the caller's own work included: 111 in psf_kernel, 152 in
+// map_eig_small_kernel (23 and 33 of them FP64).  Measured (B200; before: a lookup and its walk for every value and the
+// library's sincos, 194 instructions): map of one eigen-component, 16 bins x 160,801 points x 256 mics, 7.9 -> 5.1 ms;
+// point-spread function 1681 x 1681 x 64 mics 1.72 -> 1.03 ms (3.7 and 0.48 with what those kernels changed since).
 struct SincosTable {
     const uint64_t *table;
     uint64_t mask;

@@ -1000,7 +1000,7 @@ static int gram_f64_launch(const void *spec, int M, int64_t nw, int nbins, void 
     const int TC = narrow ? (M + 15) / 16 : T, per = narrow ? 2 : 1;
     int tiles = 0;
     for (int ti = 0; ti < T; ++ti) tiles += TC - per * ti;
-    if (const int st = allow_smem(kernel, GF_SMEM)) return st;
+    if (const int st = allow_smem(kernel, GF_SMEM, GF_SMEM)) return st;
     kernel<<<dim3(tiles, nbins), 128, GF_SMEM, s>>>(reinterpret_cast<const double2 *>(spec), M, nw,
                                                     reinterpret_cast<double2 *>(csm), reinterpret_cast<double2 *>(out),
                                                     scale);
@@ -1061,10 +1061,11 @@ __global__ void __launch_bounds__(256) finalize_kernel(const void *__restrict__ 
 // first pass has tasks: with 16 mics and 256 threads whatever the block, half the threads and more idled.  Measured
 // (B200), whole complex128 CSM: 64 mics, block 128 100 -> 92 us, block 64 145 -> 122, block 32 120 -> 98, block 16 147 ->
 // 118; 256 mics, block 128 1306 -> 1226; 113 mics, block 256 420 -> 410; 8 mics, block 128 45 -> 41.
+constexpr size_t FFT_SMEM = 150 * 1024;   // the most of any block: 148 KB of a block of 16384
 static int fft_threads(int N) { return N >= FFT_WIDE_N ? 512 : 256; }
 static int fft_mics_per_block(int N, int M)
 {
-    const size_t most = (N >= FFT_WIDE_N ? 150 : 74) * 1024;
+    const size_t most = N >= FFT_WIDE_N ? FFT_SMEM : 74 * 1024;
     int mpb = 64;
     while (mpb > 1 && (mpb >= 2 * M || (size_t)mpb * fft_stride(N / 2) * sizeof(double2) > most)) mpb >>= 1;
     return mpb;
@@ -1081,11 +1082,11 @@ int fft_launch(const void *samples, int sample_dtype, int out_form, int num_mics
         const dim3 gs((unsigned)num_mics, (unsigned)num_windows, (unsigned)(block_size / 2 / FFT_SUB_H));
         const size_t smem = (size_t)fft_stride(FFT_SUB_H) * sizeof(double2);
         if (sample_dtype == ACB_F32) {
-            if (const int st = allow_smem(fft_sub_kernel<float>, smem)) return st;
+            if (const int st = allow_smem(fft_sub_kernel<float>, smem, smem)) return st;
             fft_sub_kernel<float><<<gs, 256, smem, s>>>(reinterpret_cast<const float *>(samples), num_mics, block_size,
                                                         hop, first_window, window, tw, sc);
         } else {
-            if (const int st = allow_smem(fft_sub_kernel<double>, smem)) return st;
+            if (const int st = allow_smem(fft_sub_kernel<double>, smem, smem)) return st;
             fft_sub_kernel<double><<<gs, 256, smem, s>>>(reinterpret_cast<const double *>(samples), num_mics,
                                                          block_size, hop, first_window, window, tw, sc);
         }
@@ -1123,7 +1124,7 @@ int fft_launch(const void *samples, int sample_dtype, int out_form, int num_mics
 #define ACB_FFT4_LAUNCH(TS, OF)                                                                                     \
     do {                                                                                                            \
         auto kern = fft4_tc_kernel<TS, OF>;                                                                         \
-        if (const int st_ = allow_smem(kern, smem4)) return st_;                                                    \
+        if (const int st_ = allow_smem(kern, smem4, 200 * 1024)) return st_;                                        \
         kern<<<g4, fft4_threads(block_size), smem4, s>>>(reinterpret_cast<const TS *>(samples), num_mics, block_size,   \
                                     hop, first_window, num_windows, mpb4, vw, window, tw, bin_lo, num_bins, out, R, KC, lo_elems);    \
     } while (0)
@@ -1144,7 +1145,7 @@ int fft_launch(const void *samples, int sample_dtype, int out_form, int num_mics
 #define ACB_FFT_LAUNCH(TS, OF)                                                                                    \
     do {                                                                                                          \
         auto kern = fft_window_kernel<TS, OF>;                                                                    \
-        if (const int st_ = allow_smem(kern, smem)) return st_;                                                   \
+        if (const int st_ = allow_smem(kern, smem, FFT_SMEM)) return st_;                                         \
         const int nt = max(64, min(fft_threads(block_size), mpb * (block_size / 16)));                             \
         kern<<<g1, nt, smem, s>>>(reinterpret_cast<const TS *>(samples), num_mics, block_size, hop, \
                                    first_window, num_windows, mpb, window, tw, bin_lo, num_bins, out, R, KC, lo_elems);        \

@@ -343,7 +343,7 @@ int csm_tc_accumulate(const void *samples, int sample_dtype, int num_mics, int b
     const int smem = gtc_smem_bytes();
     auto kern = a.out ? (tf32 ? gram_tc_kernel<true, true> : gram_tc_kernel<false, true>)
                       : (tf32 ? gram_tc_kernel<true, false> : gram_tc_kernel<false, false>);
-    if (const int st = allow_smem(kern, smem)) return st;
+    if (const int st = allow_smem(kern, smem, smem)) return st;
     kern<<<grid, GTC_THREADS, smem, s>>>(a, nullptr);
     return check_launch();
 }

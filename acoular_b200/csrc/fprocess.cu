@@ -198,10 +198,10 @@ int acb_cross_spectra(const void *spectra, int64_t num_windows, int num_freqs, i
     cudaStream_t s = as_stream(stream);
     const size_t smem = (size_t)num_mics * (precision == ACB_C64 ? sizeof(float2) : sizeof(double2));
     if (precision == ACB_C64) {
-        if (const int st = allow_smem(cross_spectra_kernel<true>, smem)) return st;
+        if (const int st = allow_smem(cross_spectra_kernel<true>, smem, kSmemMost)) return st;
         cross_spectra_kernel<true><<<(unsigned)nwf, 256, smem, s>>>(spectra, num_mics, scale, out);
     } else {
-        if (const int st = allow_smem(cross_spectra_kernel<false>, smem)) return st;
+        if (const int st = allow_smem(cross_spectra_kernel<false>, smem, kSmemMost)) return st;
         cross_spectra_kernel<false><<<(unsigned)nwf, 256, smem, s>>>(spectra, num_mics, scale, out);
     }
     return check_launch();

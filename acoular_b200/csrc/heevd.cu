@@ -36,6 +36,7 @@ constexpr int kEvWarps = kEvThreads / 32;
 // the QL kernel's CTA: one warp forms the rotations, four apply them; small, so that every matrix of a 513-bin request
 // has its CTA resident at once (the sweeps are a serial recurrence, so a matrix takes the same time in any wave)
 constexpr int kQlThreads = 160;
+constexpr int kEvMaxRows = 4096;
 constexpr int kQlMaxIter = 60;   // QL iterations per eigenvalue before giving up (info = 1)
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b)
@@ -1002,7 +1003,7 @@ static int tridiag_launch(const void *csm, int B, int M, double2 *A, double *d, 
         const size_t smem = ev_cluster_smem(M, C);
         // two CTAs per SM where their memory fits: then with 128 registers (some spilled), else with all it needs
         auto kern = smem <= 110 * 1024 ? heevd_tridiag_cluster_kernel<2> : heevd_tridiag_cluster_kernel<1>;
-        if (const int st = allow_smem(kern, smem)) return st;
+        if (const int st = allow_smem(kern, smem, (smem <= 110 * 1024 ? 110 : 225) * 1024)) return st;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(B * C));
         cfg.blockDim = dim3(kEvThreads);
@@ -1026,7 +1027,7 @@ static int tridiag_launch(const void *csm, int B, int M, double2 *A, double *d, 
         return ACB_ERR_CUDA;
     }
     const size_t smem = 2 * (size_t)M * sizeof(double2);
-    if (const int st = allow_smem(heevd_tridiag_kernel, smem)) return st;
+    if (const int st = allow_smem(heevd_tridiag_kernel, smem, 2 * kEvMaxRows * sizeof(double2))) return st;
     heevd_tridiag_kernel<<<B, kEvThreads, smem, s>>>(A, M, d, e, tau, vh);
     return check_launch();
 }
@@ -1056,7 +1057,7 @@ int acb_heevd_f64(const void *csm, int num_bins, int num_mics, double *eigval, v
 {
     if (!csm || !eigval || !eigvec || !workspace) return ACB_ERR_ARG;
     const int M = num_mics, B = num_bins;
-    if (M < 1 || B < 1 || M > 4096 || B > 65535) return ACB_ERR_SHAPE;
+    if (M < 1 || B < 1 || M > kEvMaxRows || B > 65535) return ACB_ERR_SHAPE;
     const EvWorkspace lay = ev_layout(M, B);
     if (workspace_bytes < lay.total) return ACB_ERR_WORKSPACE;
     const int W = ev_slab(M);
@@ -1071,7 +1072,7 @@ int acb_heevd_f64(const void *csm, int num_bins, int num_mics, double *eigval, v
     double *Z = reinterpret_cast<double *>(ws + lay.Z);
     int *perm = reinterpret_cast<int *>(ws + lay.perm);
     const size_t sm2 = 6 * (size_t)M * sizeof(double);
-    int st = allow_smem(heevd_tql_kernel, sm2);
+    int st = allow_smem(heevd_tql_kernel, sm2, 6 * kEvMaxRows * sizeof(double));
     if (st) return st;
     st = tridiag_launch(csm, B, M, A, d, e, tau, vh, s);
     if (st) return st;
@@ -1081,7 +1082,7 @@ int acb_heevd_f64(const void *csm, int num_bins, int num_mics, double *eigval, v
     const size_t smem = (size_t)(M + 1) * W * sizeof(double2);
     // columns per warp: the slab's W columns over the 8 warps
     auto back = W >= 32 ? heevd_back_kernel<4> : (W >= 16 ? heevd_back_kernel<2> : heevd_back_kernel<1>);
-    st = allow_smem(back, smem);
+    st = allow_smem(back, smem, 200 * 1024);
     if (st) return st;
     back<<<dim3(B, (M + W - 1) / W), kEvThreads, smem, s>>>(vh, tau, Z, perm, M, W, M,
                                                            static_cast<double2 *>(eigvec));
@@ -1093,7 +1094,7 @@ int acb_heevd_select_f64(const void *csm, int num_bins, int num_mics, int num_se
 {
     if (!csm || !sel || !eigval || !eigvec || !workspace) return ACB_ERR_ARG;
     const int M = num_mics, B = num_bins, E = num_sel;
-    if (M < 1 || B < 1 || M > 4096 || B > 65535 || E < 1 || E > kSelMax || E > M) return ACB_ERR_SHAPE;
+    if (M < 1 || B < 1 || M > kEvMaxRows || B > 65535 || E < 1 || E > kSelMax || E > M) return ACB_ERR_SHAPE;
     EvSel es;
     es.n = E;
     for (int j = 0; j < kSelMax; ++j) es.idx[j] = 0;
@@ -1114,7 +1115,7 @@ int acb_heevd_select_f64(const void *csm, int num_bins, int num_mics, int num_se
     double2 *vh = reinterpret_cast<double2 *>(ws + lay.vh);
     double *Z = reinterpret_cast<double *>(ws + lay.Z);
     int *perm = reinterpret_cast<int *>(ws + lay.perm);
-    int st = allow_smem(heevd_select_kernel, sm3);
+    int st = allow_smem(heevd_select_kernel, sm3, 200 * 1024);
     if (st) return st;
     st = tridiag_launch(csm, B, M, A, d, e, tau, vh, s);
     if (st) return st;
@@ -1126,14 +1127,14 @@ int acb_heevd_select_f64(const void *csm, int num_bins, int num_mics, int num_se
         auto back = M <= 64 ? heevd_back_select_kernel<2>
                             : (M <= 128 ? heevd_back_select_kernel<4>
                                         : (M <= 256 ? heevd_back_select_kernel<8> : heevd_back_select_kernel<16>));
-        st = allow_smem(back, ring);
+        st = allow_smem(back, ring, kBackRing * 512 * sizeof(double2));
         if (st) return st;
         back<<<dim3(B, E), 32, ring, s>>>(vh, tau, Z, M, E, static_cast<double2 *>(eigvec));
         return check_launch();
     }
     // the E eigenvectors of T sit in columns 0 .. E-1 of each matrix's Z, perm[j] = j: one slab of E columns
     const size_t smem = (size_t)(M + 1) * E * sizeof(double2);
-    st = allow_smem(heevd_back_kernel<1>, smem);
+    st = allow_smem(heevd_back_kernel<1>, smem, 200 * 1024);
     if (st) return st;
     heevd_back_kernel<1><<<dim3(B, 1), kEvThreads, smem, s>>>(vh, tau, Z, perm, M, E, E,
                                                               static_cast<double2 *>(eigvec));

@@ -12,9 +12,9 @@
 //   3. cross-warp sum, normalisation of the steering type, optional clipping of negatives.
 // Bound: the FP64 pipe (4 M^2 flop per point and bin at 37 TFLOP/s, DFMA and the matrix instruction alike).  The
 // matrix instruction needs no masks, no broadcasts and 1/30 of the instructions of an FMA form, and 16-point tiles
-// leave room for three CTAs per SM at 256 mics.  Measured (B200): 12 bins x 160,801 points x 256 mics 41.0 -> 20.9 ms
+// leave room for three CTAs per SM at 256 mics.  Measured (B200): 12 bins x 160,801 points x 256 mics 41.0 -> 20.4 ms
 // (14.5 ms of it the matrix instruction alone, 24.4 TFLOP/s of its 4 M^2); 6 bins x 15,903 points x 300 mics
-// 8.1 -> 1.41 ms; 5 bins x 1681 points x 64 mics 45 -> 22 us.
+// 8.4 -> 1.39 ms; 5 bins x 1681 points x 64 mics 45 -> 22 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(32 * NW) map_eig_kernel(MapArgs a, int E, cons
 // CLEAN-SC iteration's single component): one thread per grid point and NB bins walks the mics in order,
 // computes a mic's distance and weight once, synthesises the steering value of each bin and accumulates the
 // projections and the normalisation sum in registers.  Each component's mic sum runs in the reference's order.
-// Bound: issue slots of the steering synthesis.  Measured (B200): 16 bins x 160,801 points x 256 mics 5.1 -> 3.8 ms
+// Bound: issue slots of the steering synthesis.  Measured (B200): 16 bins x 160,801 points x 256 mics 5.1 -> 3.7 ms
 // with four bins per thread and their table lookups in flight together (two bins: 3.8 too; one: 4.5).
 constexpr int kEigSmall = 4;
 constexpr int kEigSmallThreads = 128;
@@ -652,6 +652,8 @@ static int make_args(const acb_map_params *p, MapArgs &a)
 // above, pairs of 384-mic tiles.  Four warps per CTA up to 256 mics (three CTAs or more per SM, so that one's
 // synthesis runs under another's matrix products), eight where only one or two CTAs fit.
 constexpr int kMapOneTile = 768, kMapPairTile = 384, kMapFourWarps = 256;
+// the largest tile, with the eigenvalue form's diagonal
+constexpr size_t kMapSmem = kMapOneTile * (kPtsPad * sizeof(double2) + sizeof(double));
 
 template <bool USE_RM, bool CUSTOM, int NW>
 static int launch_map_nw(const MapArgs &a, int nbins, const void *csm, const double *k, double k_scalar,
@@ -661,7 +663,7 @@ static int launch_map_nw(const MapArgs &a, int nbins, const void *csm, const dou
     const int mc = a.M <= kMapOneTile ? a.M : kMapPairTile;
     const size_t smem = (size_t)(a.M <= mc ? 1 : 2) * ((mc + 15) & ~15) * kPtsPad * sizeof(double2);
     auto kern = map_f64_kernel<USE_RM, CUSTOM, NW>;
-    if (const int st = allow_smem(kern, smem)) return st;
+    if (const int st = allow_smem(kern, smem, kMapSmem)) return st;
     const dim3 grid((unsigned)((a.G + kPts - 1) / kPts), nbins);
     kern<<<grid, 32 * NW, smem, s>>>(a, reinterpret_cast<const double2 *>(csm), k, k_scalar, mpos, gpos, r0, rm, mc,
                                      out_map, out_norm, reinterpret_cast<const double2 *>(steer));
@@ -688,7 +690,7 @@ static int launch_eig_nw(const MapArgs &a, int nbins, int E, const double *eigva
     const int mc = a.M <= kMapOneTile ? a.M : kMapPairTile;
     const size_t smem = (size_t)((mc + 15) & ~15) * kPtsPad * sizeof(double2) + (a.r_diag ? mc * sizeof(double) : 0);
     auto kern = map_eig_kernel<USE_RM, CUSTOM, NW>;
-    if (const int st = allow_smem(kern, smem)) return st;
+    if (const int st = allow_smem(kern, smem, kMapSmem)) return st;
     const dim3 grid((unsigned)((a.G + kPts - 1) / kPts), nbins);
     kern<<<grid, 32 * NW, smem, s>>>(a, E, eigval, reinterpret_cast<const double2 *>(eigvec), k, k_scalar, mpos, gpos,
                                      r0, rm, mc, out_map, out_norm, reinterpret_cast<const double2 *>(steer), active);

@@ -79,8 +79,8 @@ constexpr int TC_EPI_THREADS = 32 * TC_EPI_WARPS;
 // 21, 2, 3) and one of the MMA issuer (1), the bulk-copy producer (20) and the finishing warps (22, 23).
 // Six warps per scheduler leave 80 registers per thread (registers are allocated per scheduler, 16,384
 // each).
-// What bounds the FP16 form (256 mics, 160,801 points, 513 bins): no pipe is full (issue 55 %, MUFU
-// 46 %, tensor 25 %); the synthesis warps, four to a scheduler, wait on their own chains.  Measured there:
+// What bounds the FP16 form (256 mics, 160,801 points, 513 bins): no pipe is full (issue 63 %, MUFU
+// 50 %, tensor 29 %); the synthesis warps, four to a scheduler, wait on their own chains.  Measured there:
 // the MMAs issued by one divergent lane took 1330 of a step's 2300 clocks, by a converged warp's elected
 // lane 690, and the map values' divisions and loads held the epilogue, and with it the next item's first
 // step, for 400 clocks per step until they moved to warps of their own; together 40.5 -> 38.0 ms
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) map_tc_kernel(const __grid_cons
         // MMAs complete in issue order: the last commit covers all of them
         if (lastb >= 0) tc::mbar_drain(&done[lastb], (uint32_t)lastu, tc::drain_limit_ns(b.wait_limit_ns));
     } else if (tc_is_epi(warp)) {
-        // ---------------- epilogue (warps 0, 9, 2, 3 for lane quarters 0..3): one thread per grid point
+        // ---------------- epilogue (warps 0, 21, 2, 3 for lane quarters 0..3): one thread per grid point
         // After step (p, i) with i >= 16p the accumulator columns of chunk i are final; dot them
         // with the steering chunk as the MMA saw it (hi + lo from the A stage).  Every step then
         // releases its A stage.
@@ -1201,7 +1201,7 @@ static int tc_launch(TcBatch &bt, const acb_map_params *const *params, const voi
         {map_tc_kernel<3, TC_SPLIT>, map_tc_kernel<3, TC_TF>, map_tc_kernel<3, TC_HALF>},
         {map_tc_kernel<4, TC_SPLIT>, map_tc_kernel<4, TC_TF>, map_tc_kernel<4, TC_HALF>}};
     const KernT kern = kernels[steer_type - 1][precision];
-    if (const int st = allow_smem(kern, smem)) return st;
+    if (const int st = allow_smem(kern, smem, smem_max)) return st;
     kern<<<grid, TC_THREADS, smem, s>>>(bt, error_word);
     return check_launch();
 }

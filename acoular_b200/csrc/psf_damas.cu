@@ -39,8 +39,8 @@ constexpr int kPsfSmem = 2 * (kPsfG + kPsfS) * (int)sizeof(double);
 // where the sources are the grid itself (checked on the tile's own indices), a tile right of the diagonal also gives
 // its mirror image, whose CTA then has nothing to do.  The mirrored sums differ in their weights only: w for P(g; s),
 // wm for P(s; g), the same for 'true level' and 'true location'.
-// Bound: issue slots of the phase evaluation (about 100 instructions).  Measured (B200): 1681 x 1681 x 64 mics
-// 1.03 -> 0.51 ms.
+// Bound: issue slots (64 %; 111 instructions per phase, its sums included).  Measured (B200): 1681 x 1681 x 64 mics
+// 1.03 -> 0.48 ms.
 template <int ST>
 __global__ void __launch_bounds__(256, 4) psf_kernel(int M, int64_t G, int S, const int64_t *__restrict__ src,
                                                      const double *__restrict__ r0, const double *__restrict__ rm,
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kDamasThreads) damas_kernel(const double *__re
 }
 
 // ------------------------------------------------------------------------------------------------
-// The same sweeps with the solver fed two blocks ahead, for four or more blocks of rows and clusters of four or eight
+// The same sweeps with the solver fed two blocks ahead, for six or more blocks of rows and clusters of four or eight
 // CTAs.  CTA 0 solves: warp 0 takes the rows of one block after another (step t: block t mod nblk), lane i owning row i,
 // and three warps bring it, per step, three 32 x 32 tiles of the block's columns: of its own rows and of the next two
 // blocks' rows.  As each new value x_j is broadcast, every lane also adds its contribution to its rows of the next two
@@ -378,9 +378,9 @@ __global__ void __launch_bounds__(kDamasThreads) damas_kernel(const double *__re
 // the previous sweep's values count), so it has two steps' time.  New values and sums travel as asynchronous stores
 // counted on mbarriers (rings of four; a ring's slot is used again only after an exchange in the other direction that
 // follows its last use): no cluster barrier in a step.
-// Bound: the solver's step, 2700 cycles: 60 per row (one FMA, a compare and a shuffle are 50 of them) and 800 to take in
-// the sums and publish the values.  Measured (B200): 5 bins x 1681 points x 100 sweeps 21.2 -> 7.6 ms; 2 bins x 4000
-// points 71 -> 35 (the form above spends 7600 cycles a step, of them 2000 in its cluster barrier).  Four rows at a time,
+// Bound: the solver's step, 2550 cycles: 60 per row (one FMA, a compare and a shuffle are 50 of them) and the rest to take
+// in the sums and publish the values.  Measured (B200): 5 bins x 1681 points x 100 sweeps 21.2 -> 7.0 ms; 2 bins x 4000
+// points 71 -> 29 (the form above spends 7600 cycles a step, of them 2000 in its cluster barrier).  Four rows at a time,
 // every lane solving their triangle for itself, was slower (80 a row: the extra FMAs' issue slots).
 // ------------------------------------------------------------------------------------------------
 constexpr int kGsTile = kDamasRows * kDamasPad, kGsStages = 3, kGsRing = 4;
@@ -621,7 +621,7 @@ int acb_psf_f64(const acb_map_params *p, int num_sources, const int64_t *sources
     cudaStream_t s = as_stream(stream);
 #define ACB_PSF(ST)                                                                                           \
     do {                                                                                                      \
-        if (const int st = allow_smem(psf_kernel<ST>, kPsfSmem)) return st;                                   \
+        if (const int st = allow_smem(psf_kernel<ST>, kPsfSmem, kPsfSmem)) return st;                                   \
         psf_kernel<ST><<<grid, 32 * kPsfWarps, kPsfSmem, s>>>(M, G, num_sources, sources, r0, rm, wavenumber, \
                                                              p->sincos_table, mask, p->glibc_faithful,        \
                                                              round_f32, out_psf);                             \
@@ -659,7 +659,9 @@ int acb_damas_gauss_seidel_f64(const double *psf, int64_t num_grid, int num_bins
     const int64_t smem_ahead = gs_smem_bytes(num_grid);
     const bool ahead = num_grid > 5 * kDamasRows && C >= 4 && smem_ahead <= smem_max - 1024;
     const size_t smem_used = ahead ? (size_t)smem_ahead : smem;
-    if (const int st = ahead ? allow_smem(damas_ahead_kernel, smem_used) : allow_smem(damas_kernel, smem_used)) return st;
+    if (const int st = ahead ? allow_smem(damas_ahead_kernel, smem_used, smem_max - 1024)
+                             : allow_smem(damas_kernel, smem_used, smem_max))
+        return st;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(num_bins * C));
     cfg.blockDim = dim3(kDamasThreads);
