@@ -26,22 +26,23 @@ namespace cg = cooperative_groups;
 
 namespace acb {
 
-constexpr int kPsfTile = 32;      // grid points and sources per CTA
+constexpr int kPsfTile = 32;      // grid points per CTA, and its most sources
 constexpr int kPsfWarps = 8;
-constexpr int kPsfPer = kPsfTile / kPsfWarps;   // sources per warp (and phases a lane evaluates together)
 constexpr int kPsfMics = 32;      // mics per shared-memory chunk: 33 KB, four CTAs per SM (64: 0.67 ms below)
 
 // Distances and their reciprocals of a tile's 32 grid points, mic-major, and of its 32 sources, source-major.
 constexpr int kPsfG = kPsfMics * (kPsfTile + 1), kPsfS = kPsfTile * (kPsfMics + 1);
 constexpr int kPsfSmem = 2 * (kPsfG + kPsfS) * (int)sizeof(double);
 
-// CTA = 32 grid points (lanes) x 32 sources (four per warp).  The phase of (g, s) is minus that of (s, g), so that
-// where the sources are the grid itself (checked on the tile's own indices), a tile right of the diagonal also gives
-// its mirror image, whose CTA then has nothing to do.  The mirrored sums differ in their weights only: w for P(g; s),
-// wm for P(s; g), the same for 'true level' and 'true location'.
+// CTA = 32 grid points (lanes) x 8 PER sources (PER per warp, whose phases a lane evaluates together): 32 where there are
+// CTAs enough, fewer for a few sources, whose chains of phases are what takes the time then (psf_per).
+// MIRROR (as many sources as points, PER = 4): the phase of (g, s) is minus that of (s, g), so that where the sources are
+// the grid itself (checked on the tile's own indices), a tile right of the diagonal also gives its mirror image, whose
+// CTA then has nothing to do.  The mirrored sums differ in their weights only: w for P(g; s), wm for P(s; g), the same
+// for 'true level' and 'true location'.
 // Bound: issue slots (64 %; 111 instructions per phase, its sums included).  Measured (B200): 1681 x 1681 x 64 mics
 // 1.03 -> 0.48 ms.
-template <int ST>
+template <int ST, int PER, bool MIRROR>
 __global__ void __launch_bounds__(256, 4) psf_kernel(int M, int64_t G, int S, const int64_t *__restrict__ src,
                                                      const double *__restrict__ r0, const double *__restrict__ rm,
                                                      double k, const uint64_t *__restrict__ table, uint64_t mask,
@@ -53,25 +54,27 @@ __global__ void __launch_bounds__(256, 4) psf_kernel(int M, int64_t G, int S, co
     __shared__ int64_t src_s[kPsfTile];
     __shared__ double help_s[2 * kPsfTile];              // sums of 1 / r^2: points, sources
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int NS = kPsfWarps * PER;                  // the tile's sources
+    static_assert(!MIRROR || NS == kPsfTile, "a mirrored tile is square");
     const int64_t gb = (int64_t)blockIdx.x * kPsfTile;
-    const int sb = blockIdx.y * kPsfTile;
+    const int sb = blockIdx.y * NS;
     const int64_t g = gb + lane;
-    bool own = true;   // this tile's points and sources are the grid's in order
-    if (threadIdx.x < kPsfTile) {
+    bool own = MIRROR;   // this tile's points and sources are the grid's in order
+    if (threadIdx.x < NS) {
         const int i = sb + threadIdx.x;
         const int64_t s = i < S ? src[i] : 0;
         src_s[threadIdx.x] = s;
-        own = i >= S || s == i;
-    } else if (threadIdx.x < 2 * kPsfTile) {
+        if (MIRROR) own = i >= S || s == i;
+    } else if (MIRROR && threadIdx.x < 2 * kPsfTile) {
         const int64_t i = gb + threadIdx.x - kPsfTile;
         own = i >= S || src[i] == i;
     }
-    const bool sym = __syncthreads_and(own) && S == G && gb != sb;
+    const bool sym = __syncthreads_and(own) && gb != sb;
     if (sym && gb > sb) return;   // the tile on the other side of the diagonal writes this one
     const SincosTable sct = sincos_table(table, mask, faithful != 0);
-    double re[kPsfPer], im[kPsfPer], rem[kPsfPer], imm[kPsfPer];
+    double re[PER], im[PER], rem[PER], imm[PER];
 #pragma unroll
-    for (int j = 0; j < kPsfPer; ++j) re[j] = im[j] = rem[j] = imm[j] = 0.0;
+    for (int j = 0; j < PER; ++j) re[j] = im[j] = rem[j] = imm[j] = 0.0;
     if (threadIdx.x < 2 * kPsfTile) help_s[threadIdx.x] = 0.0;
     for (int m0 = 0; m0 < M; m0 += kPsfMics) {
         const int n = min(kPsfMics, M - m0);
@@ -80,16 +83,17 @@ __global__ void __launch_bounds__(256, 4) psf_kernel(int M, int64_t G, int S, co
             const int p = i / kPsfMics, m = i % kPsfMics;
             if (m >= n) continue;
             const double a = gb + p < G ? rm[(gb + p) * M + m0 + m] : 1.0;
+            rg_s[m * (kPsfTile + 1) + p] = a;
+            if (ST >= 3 || MIRROR) ig_s[m * (kPsfTile + 1) + p] = 1.0 / a;
+            if (p >= NS) continue;
             int64_t s = src_s[p];
             s = s >= 0 && s < G ? s : 0;   // an index outside the grid yields NaN, never a stray read
             const double b = rm[s * M + m0 + m];
-            rg_s[m * (kPsfTile + 1) + p] = a;
-            ig_s[m * (kPsfTile + 1) + p] = 1.0 / a;
             rs_s[p * (kPsfMics + 1) + m] = b;
             is_s[p * (kPsfMics + 1) + m] = 1.0 / b;
         }
         __syncthreads();
-        if (ST >= 3 && threadIdx.x < 2 * kPsfTile) {
+        if (ST >= 3 && threadIdx.x < (MIRROR ? 2 * kPsfTile : kPsfTile)) {
             double h = help_s[threadIdx.x];
             for (int m = 0; m < n; ++m) {
                 const double q = threadIdx.x < kPsfTile ? ig_s[m * (kPsfTile + 1) + threadIdx.x]
@@ -98,17 +102,19 @@ __global__ void __launch_bounds__(256, 4) psf_kernel(int M, int64_t G, int S, co
             }
             help_s[threadIdx.x] = h;
         }
-        const double *rsw = rs_s + warp * kPsfPer * (kPsfMics + 1), *isw = is_s + warp * kPsfPer * (kPsfMics + 1);
+        if (sb + warp * PER >= S) continue;   // no such sources
+        const double *rsw = rs_s + warp * PER * (kPsfMics + 1), *isw = is_s + warp * PER * (kPsfMics + 1);
         for (int m = 0; m < n; ++m) {
-            const double rg = rg_s[m * (kPsfTile + 1) + lane], ig = ig_s[m * (kPsfTile + 1) + lane];
-            SincosPending<kPsfPer> pend;
+            const double rg = rg_s[m * (kPsfTile + 1) + lane];
+            const double ig = ST >= 3 || MIRROR ? ig_s[m * (kPsfTile + 1) + lane] : 0.0;
+            SincosPending<PER> pend;
 #pragma unroll
-            for (int j = 0; j < kPsfPer; ++j)
+            for (int j = 0; j < PER; ++j)
                 pend.x[j] = __double2float_rn(__dmul_rn(k, __dsub_rn(rg, rsw[j * (kPsfMics + 1) + m])));
             sincos_begin(pend, sct);
             sincos_finish(pend, sct);
 #pragma unroll
-            for (int j = 0; j < kPsfPer; ++j) {
+            for (int j = 0; j < PER; ++j) {
                 const double c = (double)pend.c[j], sn = -(double)pend.s[j];
                 // (cos - i sin) / rs  [* rg (inverse) | / rg (true level, true location)]; the divisions as
                 // products with reciprocals (within an ulp of the quotients); the mirror image's sine is negated
@@ -116,7 +122,7 @@ __global__ void __launch_bounds__(256, 4) psf_kernel(int M, int64_t G, int S, co
                 const double w = ST == 1 ? is : ST == 2 ? is * rg : is * ig;
                 re[j] = fma(c, w, re[j]);
                 im[j] = fma(sn, w, im[j]);
-                if (ST < 3 && sym) {
+                if (MIRROR && ST < 3 && sym) {
                     const double wm = ST == 1 ? ig : ig * rsw[j * (kPsfMics + 1) + m];
                     rem[j] = fma(c, wm, rem[j]);
                     imm[j] = fma(sn, wm, imm[j]);
@@ -146,22 +152,41 @@ __global__ void __launch_bounds__(256, 4) psf_kernel(int M, int64_t G, int S, co
     };
     const double ra = g < G ? r0[g] : 1.0;
 #pragma unroll
-    for (int j = 0; j < kPsfPer; ++j) {
-        const int q = warp * kPsfPer + j;
+    for (int j = 0; j < PER; ++j) {
+        const int q = warp * PER + j;
         const int64_t s = src_s[q];
         const bool ok = s >= 0 && s < G;
         const double rb = r0[ok ? s : 0];
         const double a2 = re[j] * re[j] + im[j] * im[j];
         tile[lane * (kPsfTile + 1) + q] =
             ok ? value(a2, ra, rb, help_s[lane]) : __longlong_as_double(0x7ff8000000000000ll);
-        if (sym && sb + q < S && g < G) {
+        if (MIRROR && sym && sb + q < S && g < G) {
             const double m2 = ST < 3 ? rem[j] * rem[j] + imm[j] * imm[j] : a2;
             out[(int64_t)(sb + q) * S + g] = value(m2, rb, ra, help_s[kPsfTile + q]);
         }
     }
     __syncthreads();
     for (int p = warp; p < kPsfTile; p += kPsfWarps)
-        if (gb + p < G && sb + lane < S) out[(gb + p) * S + sb + lane] = tile[p * (kPsfTile + 1) + lane];
+        if (gb + p < G && lane < NS && sb + lane < S) out[(gb + p) * S + sb + lane] = tile[p * (kPsfTile + 1) + lane];
+}
+
+// Sources per warp: the most whose tiles are filled (at most a quarter of padding) and are CTAs enough.  Measured (B200),
+// microseconds at 4 / 2 / 1 per warp, 'true level': 64 mics x 1681 points: 1 source 87 / 55 / 42, 33 103 / 63 / 51, 200 (371
+// CTAs / 689 / 1325) 162 / 159 / 135, 400 (689 / 1325 / 2650) 294 / 246 / 242, 1000 (1696 / 3339) 537 / 527; x 10,201 points:
+// 64 (638 / 1276 / 2552) 281 / 246 / 247, 200 (2233 / 4147) 662 / 659 / 699, 1000 2951 / 3067 / 3356; 32 mics x 40,000 points:
+// 24 (1250 / 2500 / 3750) 212 / 210 / 193, 64 (2500 / 5000) 405 / 415 / 468.  The mirrored form: 1681 points 472 where they take
+// 857 / 926; 441 points (105 CTAs with anything to do) 124 / 86 / 103.  Before (8 sources per CTA, one per warp, whatever
+// their number) 1681 points: 1 source 96, 33 124, 200 264, 1000 1032, all 1697.
+constexpr int64_t kPsfManyCtas4 = 15 * kNumSMs, kPsfManyCtas2 = 17 * kNumSMs / 2;
+
+static int psf_per(int64_t G, int S)
+{
+    const int64_t tiles = (G + kPsfTile - 1) / kPsfTile;
+    for (int per = 4; per > 1; per >>= 1) {
+        const int64_t ns = kPsfWarps * per, cols = (S + ns - 1) / ns;
+        if (4 * cols * ns <= 5 * (int64_t)S && tiles * cols >= (per == 4 ? kPsfManyCtas4 : kPsfManyCtas2)) return per;
+    }
+    return 1;
 }
 
 constexpr int kDamasThreads = 512;
@@ -615,25 +640,31 @@ int acb_psf_f64(const acb_map_params *p, int num_sources, const int64_t *sources
         return ACB_ERR_ARG;
     const int M = p->num_mics;
     const int64_t G = p->num_grid;
-    const dim3 grid((unsigned)((G + kPsfTile - 1) / kPsfTile), (unsigned)((num_sources + kPsfTile - 1) / kPsfTile));
     if ((num_sources + 7) / 8 > 65535) return ACB_ERR_SHAPE;
+    const int64_t tiles = (G + kPsfTile - 1) / kPsfTile;
+    const bool mirror = num_sources == G && tiles * (tiles + 1) / 2 >= kNumSMs;
+    const int per = mirror ? 4 : psf_per(G, num_sources), ns = kPsfWarps * per;
+    const dim3 grid((unsigned)tiles, (unsigned)((num_sources + ns - 1) / ns));
     const uint64_t mask = p->glibc_faithful ? (uint64_t)p->sincos_table_slots - 1 : 0;
     cudaStream_t s = as_stream(stream);
-#define ACB_PSF(ST)                                                                                           \
-    do {                                                                                                      \
-        if (const int st = allow_smem(psf_kernel<ST>, kPsfSmem, kPsfSmem)) return st;                                   \
-        psf_kernel<ST><<<grid, 32 * kPsfWarps, kPsfSmem, s>>>(M, G, num_sources, sources, r0, rm, wavenumber, \
-                                                             p->sincos_table, mask, p->glibc_faithful,        \
-                                                             round_f32, out_psf);                             \
-    } while (0)
+    auto launch = [&](auto kern) {
+        if (const int st = allow_smem(kern, kPsfSmem, kPsfSmem)) return st;
+        kern<<<grid, 32 * kPsfWarps, kPsfSmem, s>>>(M, G, num_sources, sources, r0, rm, wavenumber, p->sincos_table, mask,
+                                                    p->glibc_faithful, round_f32, out_psf);
+        return check_launch();
+    };
+#define ACB_PSF(ST)                                                                             \
+    return mirror     ? launch(psf_kernel<ST, 4, true>)                                         \
+           : per == 4 ? launch(psf_kernel<ST, 4, false>)                                        \
+           : per == 2 ? launch(psf_kernel<ST, 2, false>)                                        \
+                      : launch(psf_kernel<ST, 1, false>)
     switch (p->steer_type) {
-    case 1: ACB_PSF(1); break;
-    case 2: ACB_PSF(2); break;
-    case 3: ACB_PSF(3); break;
-    default: ACB_PSF(4); break;
+    case 1: ACB_PSF(1);
+    case 2: ACB_PSF(2);
+    case 3: ACB_PSF(3);
+    default: ACB_PSF(4);
     }
 #undef ACB_PSF
-    return check_launch();
 }
 
 int acb_damas_gauss_seidel_f64(const double *psf, int64_t num_grid, int num_bins, const double *dirty_map,
