@@ -357,19 +357,19 @@ __global__ void __launch_bounds__(kCscThreads) cleansc_step_kernel(CscArgs a, in
 }
 
 // ------------------------------------------------------------------------------------------------
-// All iterations of a bin in one cluster of eight CTAs, for arrays whose CSM fits each CTA's shared memory and grids
+// All iterations of a bin in one cluster of one to eight CTAs (csc_ctas), for arrays whose CSM fits each CTA's shared memory and grids
 // whose map fits the cluster's registers (csc_cluster_fits).  Every CTA keeps the whole CSM and does the step's small
 // work for itself, the same bits in each; the grid points are split over the CTAs (a thread keeps the map values of up
 // to four), and the argmax is the one exchange: each CTA stores its candidate into every CTA's slots (two sets, used
-// alternately, so that one cluster barrier per iteration suffices) and picks the best of the eight.  The component's
-// map reads the steering vectors mic-major, lanes along the grid.
+// alternately, so that one cluster barrier per iteration suffices) and picks the best of them.  The component's
+// map reads the steering vectors mic-major, lanes along the grid.  A bin's result has the same bits whatever the cluster.
 // Bound: the serial chain of an iteration (the fixed point's sums and reciprocal square roots at the latency of FP64
 // instructions).  Two launches per iteration cost more than that: 5 bins x 1681 points x 64 mics, 128 iterations
 // 3.1 -> 1.07 ms (B200);
 // 8 bins x 3600 points x 112 mics, 60 iterations 4.3 -> 2.1; 3 bins x 8099 points x 33 mics 2.3 -> 1.17.
 // The fixed point stops when a step leaves every value as it was: the remaining ones would change nothing.
 // ------------------------------------------------------------------------------------------------
-constexpr int kCscCtas = 8, kCscClThreads = 256, kCscPoints = 4, kCscHistory = 64;
+constexpr int kCscMaxCtas = 8, kCscClThreads = 256, kCscPoints = 4, kCscHistory = 64;
 constexpr int kCscClMics = 112;
 
 constexpr size_t kCscStepSmem = 2048 * (3 * sizeof(double2) + sizeof(double));   // cleansc_step_kernel's at the most mics
@@ -392,16 +392,17 @@ __device__ __forceinline__ void better(double &v, int64_t &g, double ov, int64_t
     }
 }
 
-template <int NP, int AHEAD, int MINB>
+// NC: the cluster's CTAs, 0 where they are known at run time only (eight of them 1 to 2 % slower).
+template <int NP, int AHEAD, int MINB, int NC>
 __global__ void __launch_bounds__(kCscClThreads, MINB) cleansc_cluster_kernel(CscArgs a, const double2 *__restrict__ steer,
                                                                         int r_diag, double norm)
 {
     extern __shared__ double2 cl_sm[];
-    __shared__ CscPeak peaks[2][kCscCtas], wpeak[kCscClThreads / 32];
+    __shared__ CscPeak peaks[2][kCscMaxCtas], wpeak[kCscClThreads / 32];
     __shared__ double powers[kCscHistory];   // the last peaks, by iteration modulo its length
     cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
-    const int b = blockIdx.x / kCscCtas;
+    const int nctas = NC ? NC : (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int b = blockIdx.x / nctas;
     const int M = a.M, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t G = a.G;
     double2 *C = cl_sm, *w = C + M * M, *d1 = w + M, *hh = d1 + M, *part = hh + M;
@@ -412,7 +413,7 @@ __global__ void __launch_bounds__(kCscClThreads, MINB) cleansc_cluster_kernel(Cs
     double h[NP];
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
-        const int64_t g = (int64_t)q * kCscCtas * kCscClThreads + rank * kCscClThreads + tid;
+        const int64_t g = (int64_t)q * nctas * kCscClThreads + rank * kCscClThreads + tid;
         h[q] = g < G ? a.h[(int64_t)b * G + g] : -INFINITY;
     }
     const double k = a.k[b];
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(kCscClThreads, MINB) cleansc_cluster_kernel(Cs
         int64_t bi = G;
 #pragma unroll
         for (int q = 0; q < NP; ++q) {
-            const int64_t g = (int64_t)q * kCscCtas * kCscClThreads + rank * kCscClThreads + tid;
+            const int64_t g = (int64_t)q * nctas * kCscClThreads + rank * kCscClThreads + tid;
             if (g < G) better(best, bi, h[q], g);
         }
 #pragma unroll
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(kCscClThreads, MINB) cleansc_cluster_kernel(Cs
         }
         if (lane == 0) wpeak[warp] = CscPeak{best, bi};
         __syncthreads();
-        if (tid < kCscCtas) {
+        if (tid < nctas) {
             for (int u = 0; u < kCscClThreads / 32; ++u) better(best, bi, wpeak[u].v, wpeak[u].g);
             *cluster.map_shared_rank(&peaks[j & 1][rank], tid) = CscPeak{best, bi};
         }
@@ -446,7 +447,8 @@ __global__ void __launch_bounds__(kCscClThreads, MINB) cleansc_cluster_kernel(Cs
         best = -INFINITY;
         bi = G;
 #pragma unroll
-        for (int u = 0; u < kCscCtas; ++u) better(best, bi, peaks[j & 1][u].v, peaks[j & 1][u].g);
+        for (int u = 0; u < kCscMaxCtas; ++u)
+            if (u < nctas) better(best, bi, peaks[j & 1][u].v, peaks[j & 1][u].g);
         if (bi >= G) break;   // no comparable value (NaN map)
         const int64_t xi = bi;
         const double hmax = best;
@@ -587,7 +589,7 @@ __global__ void __launch_bounds__(kCscClThreads, MINB) cleansc_cluster_kernel(Cs
         // 6. h -= damp times the map of the component (hmax, conj(hh)): t_m = hh_m v_m
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-            const int64_t g = (int64_t)p * kCscCtas * kCscClThreads + rank * kCscClThreads + tid;
+            const int64_t g = (int64_t)p * nctas * kCscClThreads + rank * kCscClThreads + tid;
             if (g >= G) break;
             double fr[4] = {0, 0, 0, 0}, fi[4] = {0, 0, 0, 0}, dg[4] = {0, 0, 0, 0};
             for (int m = 0; m < M; m += AHEAD) {
@@ -615,7 +617,30 @@ __global__ void __launch_bounds__(kCscClThreads, MINB) cleansc_cluster_kernel(Cs
 
 static bool csc_cluster_fits(int M, int64_t G, int stopn)
 {
-    return M <= kCscClMics && G <= (int64_t)kCscPoints * kCscCtas * kCscClThreads && stopn >= 1 && stopn < kCscHistory;
+    return M <= kCscClMics && G <= (int64_t)kCscPoints * kCscMaxCtas * kCscClThreads && stopn >= 1 && stopn < kCscHistory;
+}
+
+// CTAs of a bin's cluster, for B bins of G points whose CTAs fit `per_sm` to an SM.  Eight finish a bin soonest, but only 15
+// such clusters are resident per CTA of an SM, and the other bins wait for their turn: the size that makes the least of
+// rounds times a round's length, a round being about as long as the map of three points per thread and its own points.
+// Measured (B200), microseconds of 20 iterations, always eight CTAs / this rule / two launches per iteration: 64 mics x 100
+// points: 60 bins 784 / 423 / 844, 120 1495 / 443 / 861, 513 5894 / 917 / 1778; x 1681 points: 60 1093 / 939 / 1611, 513 8279 /
+// 6277 / 7896; 112 mics x 400 points: 60 2359 / 724 / 1569, 513 20,017 / 4680 / 6203; x 4000 points, 513: 43,201 / 34,568 /
+// 29,652 (the launches skip bins that stop early, which evens that out); 16 mics x 1681 points, 300: 2991 / 1537 / 2409.
+static int csc_ctas(int64_t G, int B, int per_sm)
+{
+    int best = kCscMaxCtas;
+    int64_t cost = INT64_MAX;
+    for (int c = kCscMaxCtas; c >= 1 && G <= (int64_t)kCscPoints * c * kCscClThreads; c >>= 1) {
+        const int64_t resident = per_sm * (c == 8 ? 15 : c == 4 ? 33 : kNumSMs / c);
+        const int64_t points = (G + c * kCscClThreads - 1) / (c * kCscClThreads);
+        const int64_t t = (B + resident - 1) / resident * (3 + points);
+        if (t < cost) {
+            cost = t;
+            best = c;
+        }
+    }
+    return best;
 }
 
 struct CscWorkspace {
@@ -720,11 +745,13 @@ int acb_cleansc_f64(const acb_map_params *p, void *csm, const double *wavenumber
     double2 *steer = reinterpret_cast<double2 *>(ws + lay.steer);
     if (csc_cluster_fits(M, G, stopn)) {
         const size_t tile = (size_t)M * 33 * sizeof(double2), smem = csc_cluster_smem(M);
+        const int per_sm = 2 * (smem + 2048) <= 228 * 1024 ? 2 : 1, C = csc_ctas(G, B, per_sm);
         // few bins: 16 steering values in flight per thread and all the registers that takes; more bins than one CTA per
-        // SM holds (15 clusters): 8, and 128 registers for two (60 bins of 64 mics: 2.14 against 3.43 ms)
-        const bool few = B * kCscCtas <= 120, small = G <= kCscCtas * kCscClThreads;
-        auto kern = few ? (small ? cleansc_cluster_kernel<1, 16, 1> : cleansc_cluster_kernel<kCscPoints, 16, 1>)
-                        : (small ? cleansc_cluster_kernel<1, 8, 2> : cleansc_cluster_kernel<kCscPoints, 8, 2>);
+        // SM holds: 8, and 128 registers for two (60 bins of 64 mics in clusters of eight: 2.14 against 3.43 ms)
+        const bool few = B * C <= 120, small = G <= C * kCscClThreads;
+        auto kern = few && C == 8 ? (small ? cleansc_cluster_kernel<1, 16, 1, 8> : cleansc_cluster_kernel<kCscPoints, 16, 1, 8>)
+                    : few         ? (small ? cleansc_cluster_kernel<1, 16, 1, 0> : cleansc_cluster_kernel<kCscPoints, 16, 1, 0>)
+                                  : (small ? cleansc_cluster_kernel<1, 8, 2, 0> : cleansc_cluster_kernel<kCscPoints, 8, 2, 0>);
         st = allow_smem(cleansc_steer_kernel<true>, tile, (size_t)kCscClMics * 33 * sizeof(double2));
         if (!st) st = allow_smem(kern, smem, csc_cluster_smem(kCscClMics));
         if (st) return st;
@@ -732,13 +759,13 @@ int acb_cleansc_f64(const acb_map_params *p, void *csm, const double *wavenumber
         st = check_launch();
         if (st) return st;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(B * kCscCtas));
+        cfg.gridDim = dim3((unsigned)(B * C));
         cfg.blockDim = dim3(kCscClThreads);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = kCscCtas;
+        attr[0].val.clusterDim.x = (unsigned)C;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
