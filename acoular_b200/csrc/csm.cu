@@ -859,8 +859,8 @@ static int gram_c64_launch(const void *spec, int M, int64_t nw, int nbins, void 
 // four CTAs per SM.  Rows are padded to 36 mics, so that the operand reads of 4 mics x 2 windows (A) and 8 mics x 2
 // windows (B) fall on different banks.  16 x 8 blocks entirely below the diagonal or past M are skipped.  With `out`
 // the sums are not added to csm but written, scaled, as the full Hermitian matrix.
-// A lane's two elements of a block are columns t and t + 4 (the instruction's column n stands for column n / 2 + 4 (n % 2)
-// of the block), so that four lanes read and write whole sectors of a row.  Measured (B200), 513 bins added to: 256 mics, 4
+// A lane's two elements of a block are two columns apart (gf_column), so that four lanes read and write whole sectors of a
+// row.  Measured (B200), 513 bins added to: 256 mics, 4
 // windows 164 -> 150 us, 33 windows 318 -> 271; 113 mics, 1 window 49 -> 41, 33 windows 108 -> 94 (lanes with columns 2 t and
 // 2 t + 1, and 16 windows' products whatever the stage holds; the FMA form before it 133, 455, 39 and 164).
 // Bound: the FP64 pipe (4 M^2 K flop per bin).  Measured (B200): 513 bins x 256 mics x 999 windows 7.84 -> 5.0 ms
@@ -876,6 +876,11 @@ constexpr int GF_STAGES = 3;
 // 170 227 / 209, 195 110 / 101 and 96 / 73, 198 207 / 182; 255 249 / 262, 257 139 / 145, 330 319 / 352, 387 175 / 205.
 constexpr int64_t GF_NARROW = kNumSMs * 3 / 2;
 constexpr int GF_SMEM = GF_STAGES * 2 * GF_KW * GF_LD * (int)sizeof(double2);
+
+// The column of an 8-column block that the instruction's column n stands for: 0 2 1 3 4 6 5 7.  Lane t's columns 2 t and
+// 2 t + 1 of the instruction are then 0, 1, 4, 5 and 2, 3, 6, 7 of the block over the four lanes (pairs fill sectors), and
+// neighbouring n two apart, so that their operand reads fall on different banks.
+__device__ __forceinline__ int gf_column(int n) { return ((n >> 1) & 1) + 4 * (n >> 2) + 2 * (n & 1); }
 
 template <int NB>
 __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restrict__ spec, int M, int64_t nw,
@@ -932,7 +937,7 @@ __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restr
         use[j] = rw <= cb + 7 && rw < M && cb < M;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int r = rw + g + 8 * (e >> 1), c = cb + t + 4 * (e & 1);
+            const int r = rw + g + 8 * (e >> 1), c = cb + gf_column(2 * t + (e & 1));
             double2 v = make_double2(0.0, 0.0);
             if (!out && c < M && r <= c) v = base[(int64_t)r * M + c];
             re[j][e] = v.x;
@@ -941,50 +946,55 @@ __global__ void __launch_bounds__(128, 4) gram_f64_kernel(const double2 *__restr
     }
 
     const int64_t nst = (nw + GF_KW - 1) / GF_KW;
-    load(0);
-    if (nst > 1) load(1);
-    for (int64_t st = 0; st < nst; ++st) {
-        if (st + 1 < nst) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    const double *ar = nullptr;
+    const double2 *bc = nullptr;
+    auto arrive = [&](int64_t st, bool more) {
+        if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
         else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();   // stage st has landed for every thread; stage st - 1 is read by none any more
         if (st + 2 < nst) load(st + 2);
         const double2 *xr = gf_sm + (st % GF_STAGES) * (2 * GF_KW * LD);
         const double2 *xc = same ? xr + (c0 - r0) : xr + GF_KW * LD;
-        const double *ar = reinterpret_cast<const double *>(xr + (t >> 1) * LD + wr * 16 + g) + (t & 1);
-        const double2 *bc = xc + (t >> 1) * LD + wc * 8 * NB + (g >> 1) + 4 * (g & 1);
-        auto four = [&](int w) {   // windows w .. w + 3 of the stage
-            double b0[NB], b1[NB], q0[NB], q1[NB];
+        ar = reinterpret_cast<const double *>(xr + (t >> 1) * LD + wr * 16 + g) + (t & 1);
+        bc = xc + (t >> 1) * LD + wc * 8 * NB + gf_column(g);
+    };
+    auto four = [&](int w) {   // windows w .. w + 3 of the stage
+        double b0[NB], b1[NB], q0[NB], q1[NB];
 #pragma unroll
-            for (int j = 0; j < NB; ++j) {
-                const double2 u = bc[w * LD + 8 * j], v = bc[(w + 2) * LD + 8 * j];
-                b0[j] = t & 1 ? u.y : u.x;
-                b1[j] = t & 1 ? v.y : v.x;
-                q0[j] = t & 1 ? u.x : -u.y;
-                q1[j] = t & 1 ? v.x : -v.y;
-            }
-            const double *p = ar + w * LD * 2;
-            const double a[4] = {p[0], p[16], p[4 * LD], p[4 * LD + 16]};
-#pragma unroll
-            for (int j = 0; j < NB; ++j)
-                if (use[j]) {
-                    mma_f64(re[j], a[0], a[1], a[2], a[3], b0[j], b1[j]);
-                    mma_f64(im[j], a[0], a[1], a[2], a[3], q0[j], q1[j]);
-                }
-        };
-        // of the last stage only the windows that are there: sums of a few windows are one stage
-        const int kw = (int)min((int64_t)GF_KW, nw - st * GF_KW);
-        if (kw == GF_KW) {
-#pragma unroll
-            for (int w = 0; w < GF_KW; w += 4) four(w);
-        } else {
-            for (int w = 0; w < kw; w += 4) four(w);
+        for (int j = 0; j < NB; ++j) {
+            const double2 u = bc[w * LD + 8 * j], v = bc[(w + 2) * LD + 8 * j];
+            b0[j] = t & 1 ? u.y : u.x;
+            b1[j] = t & 1 ? v.y : v.x;
+            q0[j] = t & 1 ? u.x : -u.y;
+            q1[j] = t & 1 ? v.x : -v.y;
         }
+        const double *p = ar + w * LD * 2;
+        const double a[4] = {p[0], p[16], p[4 * LD], p[4 * LD + 16]};
+#pragma unroll
+        for (int j = 0; j < NB; ++j)
+            if (use[j]) {
+                mma_f64(re[j], a[0], a[1], a[2], a[3], b0[j], b1[j]);
+                mma_f64(im[j], a[0], a[1], a[2], a[3], q0[j], q1[j]);
+            }
+    };
+    load(0);
+    if (nst > 1) load(1);
+    for (int64_t st = 0; st < nst - 1; ++st) {
+        arrive(st, true);
+#pragma unroll
+        for (int w = 0; w < GF_KW; w += 4) four(w);
     }
+    // of the last stage only the windows that are there: sums of a few windows are one stage
+    arrive(nst - 1, false);
+    const int kw = (int)(nw - (nst - 1) * GF_KW);
+#pragma unroll
+    for (int w = 0; w < GF_KW; w += 4)
+        if (w < kw) four(w);
 #pragma unroll
     for (int j = 0; j < NB; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int r = rw + g + 8 * (e >> 1), c = cw + 8 * j + t + 4 * (e & 1);
+            const int r = rw + g + 8 * (e >> 1), c = cw + 8 * j + gf_column(2 * t + (e & 1));
             if (c >= M || r > c) continue;
             if (out) put_hermitian(out + (int64_t)f * M * M, M, r, c, re[j][e], im[j][e], scale);
             else base[(int64_t)r * M + c] = make_double2(re[j][e], im[j][e]);
