@@ -861,8 +861,9 @@ static int gram_c64_launch(const void *spec, int M, int64_t nw, int nbins, void 
 // the sums are not added to csm but written, scaled, as the full Hermitian matrix.
 // A lane's two elements of a block are two columns apart (gf_column), so that four lanes read and write whole sectors of a
 // row.  Measured (B200), 513 bins added to: 256 mics, 4
-// windows 164 -> 150 us, 33 windows 318 -> 271; 113 mics, 1 window 49 -> 41, 33 windows 108 -> 94 (lanes with columns 2 t and
-// 2 t + 1, and 16 windows' products whatever the stage holds; the FMA form before it 133, 455, 39 and 164).
+// windows 164 -> 150 us, 33 windows 318 -> 270; 113 mics, 1 window 49 -> 41, 33 windows 108 -> 95 (lanes with columns 2 t and
+// 2 t + 1, and 16 windows' products whatever the stage holds; the FMA form before it 133, 455, 39 and 164).  999 windows of
+// 256 mics 6255 -> 6189 with the transform.
 // Bound: the FP64 pipe (4 M^2 K flop per bin).  Measured (B200): 513 bins x 256 mics x 999 windows 7.84 -> 5.0 ms
 // (27 TFLOP/s; 64 x 64 tiles of 32 x 16 per warp 5.2 ms, half of the diagonal tiles idle); 65 bins x 64 mics x 799
 // windows 281 -> 75 us (195 CTAs where the 64 x 64 tiles of the FMA form were 65), in 32 x 16 tiles 65 us.

@@ -818,9 +818,7 @@ __global__ void __launch_bounds__(32 * kSelMax) heevd_select_kernel(const double
     const double eps = 2.220446049250313e-16;
     // Gershgorin interval, the norm of T and the pivot floor
     double lo = INFINITY, hi = -INFINITY, emax2 = 0.0;
-    bool bad = false;
     for (int i = lane; i < M; i += 32) {
-        bad |= d[i] != d[i] || e[i] != e[i];
         const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + fabs(e[i]);
         lo = fmin(lo, d[i] - r);
         hi = fmax(hi, d[i] + r);
@@ -834,9 +832,6 @@ __global__ void __launch_bounds__(32 * kSelMax) heevd_select_kernel(const double
     }
     double *zc = Zall + (int64_t)b * M * M + (int64_t)w * M;   // column w of Z
     if (lane == 0) permall[(int64_t)b * M + w] = w;
-    // a NaN in T, which fmin, fmax and the counts would pass over: no result.  lam is NaN then, and through the solves its
-    // vector (an early return made the kernel 7 % slower)
-    const bool none = __any_sync(0xffffffffu, bad);
     const double pivmin = 2.2250738585072014e-308 * fmax(1.0, emax2);
     const double tnorm = fmax(fabs(lo), fabs(hi));
     const double fudge = 2.0 * eps * tnorm + 2.0 * pivmin;
@@ -847,7 +842,7 @@ __global__ void __launch_bounds__(32 * kSelMax) heevd_select_kernel(const double
     const double tsc = tnorm > 0.0 ? scalbn(1.0, -ilogb(tnorm)) : 1.0;
     for (int i = tid; i < M; i += blockDim.x) e2[i] = (e[i] * tsc) * (e[i] * tsc);
     __syncthreads();
-    for (int it = none ? 64 : 0; it < 64; ++it) {
+    for (int it = 0; it < 64; ++it) {
         const double width = hi - lo;
         if (width <= fmax(2.0 * eps * fmax(fabs(lo), fabs(hi)), eps * tnorm) || width <= 4.0 * pivmin) break;
         const double x = lo + width * (double)(lane + 1) / 33.0;
@@ -864,7 +859,11 @@ __global__ void __launch_bounds__(32 * kSelMax) heevd_select_kernel(const double
             hi = xh;
         }
     }
-    const double lam = none ? __longlong_as_double(0x7ff8000000000000ll) : 0.5 * (lo + hi);
+    // a NaN in T, which fmin, fmax and the counts pass over: no result.  lam is NaN then, and through the solves its
+    // vector (looked for ahead of the counts, with or without an early return, it made the kernel 7 % slower)
+    bool bad = false;
+    for (int i = lane; i < M; i += 32) bad |= d[i] != d[i] || e[i] != e[i];
+    const double lam = __any_sync(0xffffffffu, bad) ? __longlong_as_double(0x7ff8000000000000ll) : 0.5 * (lo + hi);
     if (lane == 0) {
         wsel[(int64_t)b * sel.n + w] = lam;
         const double tiny = tnorm > 0.0 ? eps * tnorm : 2.2250738585072014e-308;
