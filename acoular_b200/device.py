@@ -194,9 +194,10 @@ _STAGE_MIN, _STAGE_SLOT, _STAGE_THREADS = 8 << 20, 4 << 20, 4
 
 def upload_samples(x: torch.Tensor, device) -> torch.Tensor:
     """A host tensor as a tensor on ``device``.  Pageable memory may be changed once the call returns."""
-    if (not x.is_contiguous() or x.is_pinned() or x.numel() * x.element_size() < _STAGE_MIN
+    pinned = x.is_pinned()   # asks the driver
+    if (pinned or x.numel() * x.element_size() < _STAGE_MIN or not x.is_contiguous()
             or torch.get_num_threads() < _STAGE_THREADS or torch.cuda.is_current_stream_capturing()):
-        return x.to(device, non_blocking=x.is_pinned())
+        return x.to(device, non_blocking=pinned)
     out = torch.empty(x.shape, dtype=x.dtype, device=device)
     src, dst = x.view(-1), out.view(-1)
     n, step = src.numel(), _STAGE_SLOT // x.element_size()
