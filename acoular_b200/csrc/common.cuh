@@ -77,7 +77,7 @@ __device__ __forceinline__ void mma_f64(double (&d)[4], double a0, double a1, do
 //   tags  Bit 16 + tag of a slot's word is set for every key with this home slot (whoever occupies it), tag = 4
 //         other bits of the key's hash: unless the bit is set, one load answers the lookup, with no walk.
 // A table without the meta entry has no tags: tol is then half an ulp and every occupied home slot is walked.
-// Bound: issue slots.  Instructions per value, the caller's own work included: 111 in psf_kernel, 152 in
+// Bound: issue slots.  Instructions per value, the caller's own work included: 108 in psf_kernel, 152 in
 // map_eig_small_kernel (23 and 33 of them FP64).  Measured (B200; before: a lookup and its walk for every value and the
 // library's sincos, 194 instructions): map of one eigen-component, 16 bins x 160,801 points x 256 mics, 7.9 -> 5.1 ms;
 // point-spread function 1681 x 1681 x 64 mics 1.72 -> 1.03 ms (3.7 and 0.48 with what those kernels changed since).

@@ -7,7 +7,7 @@
 
 namespace acb {
 
-// Windowed rFFT of `num_windows` windows (FP64; FP32 for the operand tiles up to 8192 samples);
+// Windowed rFFT of `num_windows` windows (FP64; FP32 for the operand tiles up to 4096 samples);
 // out_form: 0 complex128 spectra, 1 complex64 spectra, 2 TF32 operand tiles, 3 split-BF16 operand tiles (R row tiles, KC window blocks, lo tiles
 // `lo_elems` after the hi tiles).  Blocks above 16384 samples need `scratch` of
 // fft_scratch_bytes(num_mics, block_size, num_windows) bytes (null otherwise).
@@ -16,7 +16,8 @@ int fft_launch(const void *samples, int sample_dtype, int out_form, int num_mics
                int num_bins, void *out, int R, int KC, int64_t lo_elems, void *scratch, cudaStream_t s);
 size_t fft_scratch_bytes(int num_mics, int block_size, int64_t num_windows);
 // True when fft_launch writes every element of the operand tiles (padding windows and mics as zeros),
-// which it does for the tile forms up to blocks of 8192 samples (the FP32 four-window transform).
+// which it does for the tile forms up to blocks of 4096 samples (the FP32 four-window transform; at 8192 one mic's
+// sequences and the tables take 200 KB, its limit).
 bool fft_tiles_written_whole(int block_size);
 
 // The finished matrix's entries (r, c), r <= c, and (c, r) from the sum (x, y): what finalize_kernel writes.

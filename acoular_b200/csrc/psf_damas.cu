@@ -40,7 +40,7 @@ constexpr int kPsfSmem = 2 * (kPsfG + kPsfS) * (int)sizeof(double);
 // the grid itself (checked on the tile's own indices), a tile right of the diagonal also gives its mirror image, whose
 // CTA then has nothing to do.  The mirrored sums differ in their weights only: w for P(g; s), wm for P(s; g), the same
 // for 'true level' and 'true location'.
-// Bound: issue slots (64 %; 111 instructions per phase, its sums included).  Measured (B200): 1681 x 1681 x 64 mics
+// Bound: issue slots (62 %; 108 instructions per phase, its sums included).  Measured (B200): 1681 x 1681 x 64 mics
 // 1.03 -> 0.48 ms.
 template <int ST, int PER, bool MIRROR>
 __global__ void __launch_bounds__(256, 4) psf_kernel(int M, int64_t G, int S, const int64_t *__restrict__ src,

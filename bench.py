@@ -737,7 +737,7 @@ def run_eig(args):
           map_rate=G * F / (float(np.mean(map_ms)) / 1e3), map_tflops_algorithmic=flops / (np.mean(map_ms) / 1e3) / 1e12,
           accuracy={'vs': 'oracle (numpy eigh + the reference eigen kernel restated)', 'bins': check_bins,
                     'max_rel_err': max(errs)},
-          gpu_launches_per_step='largest eigenpair (heevd_tridiag, heevd_select, heevd_back kernels) + 1 map_eig_small_kernel',
+          gpu_launches_per_step='largest eigenpair (heevd_tridiag_cluster, heevd_select, heevd_back_select kernels) + 1 map_eig_small_kernel',
           clocks=clk.summary(),
           dtype='f64')
 

@@ -132,7 +132,8 @@ typedef struct acb_map_params {
  *   mpos:      float64 [3][M];  gpos: float64 [3][G]
  *   out_map:   float64 [num_bins][G];  out_steer_norm: float64 [num_bins][G] or NULL
  * Distances and steering vectors are synthesised on the device from the positions.
- * error_word: int32 on the device or NULL (set nonzero on a device-detected fault). */
+ * error_word: not used (NULL or anything): this form has no device-side wait that could run out; the
+ * argument stands where the tensor-core form has it. */
 int acb_map_f64(const acb_map_params *p, const void *csm, const double *wavenumber, const double *mpos,
                 const double *gpos, double *out_map, double *out_steer_norm, int *error_word, void *stream);
 
